@@ -267,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   if (warp == 0) {
     // ========================= TMA producer: activations ========================
     // Stage sa = it % kActStages is free once the commit group of step it - kActStages retired.
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // activations belong to stream order
       uint32_t it = 0;
       ItemCursor cur = first_item(p);
@@ -294,7 +294,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     // post, one thread issuing all three copies of a step is good for a step per ~600 cycles, which is
     // the whole kernel's pace once two threads issue the MMAs.  Hence two producer threads, each
     // arriving on the stage's barrier with its own byte count.
-    if (lane == 0) {
+    if (elect_one()) {
       const bool meta = warp == kMetaProducerWarp;
       const uint32_t tx = meta ? (uint32_t)p.meta_rows * p.meta_row_bytes_s +
                                      (p.has_zp ? (uint32_t)p.meta_rows * p.meta_row_bytes_z : 0u)
@@ -331,7 +331,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     }
   } else if (DUAL && (warp == 1 || warp == kSecondIssuerWarp)) {
     // ========================= MMA issuers, DUAL: even steps / odd steps =========================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t q = warp == 1 ? 0u : 1u;
       const uint32_t idesc = make_idesc_f16(TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
@@ -371,7 +371,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     // dependent scalar code.  Hence: ring indices and parities are carried incrementally
     // (no division), the four MMAs of a step are one asm block, and the barrier polls take
     // the slow (bounded, instrumented) path only when the first poll fails.
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
       const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);  // LBO field

@@ -231,7 +231,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
 
   if (warp == 0) {
     // ========================= TMA producer: this CTA's 128 activation rows ========================
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // activations belong to stream order
       uint32_t it = 0;
       PairWalk walk(p, pair, num_pairs);
@@ -256,7 +256,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
   } else if (warp == kWeightProducerWarp) {
     // ==================== TMA producer: this CTA's packed weights and meta =================
     // (one thread: here the MMA thread sets the pace, and a second producer warp measured 3 % slower)
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t tx = kPackTileBytes + (uint32_t)p.meta_rows * p.meta_row_bytes_s +
                           (p.has_zp ? (uint32_t)p.meta_rows * p.meta_row_bytes_z : 0u);
       uint32_t it = 0;
@@ -288,7 +288,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     }
   } else if (warp == 1) {
     // =============================== MMA issuer: the leader's lane 0 =================================
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_f16(2 * TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
       const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);

@@ -91,6 +91,21 @@ inline cudaError_t ensure_dynamic_smem(Kernel kern, size_t bytes, std::atomic<in
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
+// True in exactly one lane of the (converged) warp.  Single-thread roles must be entered through this and
+// not through `lane == 0`: under elect.sync the compiler knows that one thread is active and moves the
+// operands of tcgen05.mma, tcgen05.commit and the bulk-tensor copies straight into uniform registers;
+// under an ordinary lane test it has to assume that they differ between lanes and wraps every such
+// instruction in a loop over their values.  Measured on B200: 54 against 9 cycles per tcgen05.mma
+// (N = 16, issue-bound), 370 cycles per iteration of a wait + expect_tx + copy loop under the lane test.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(pred));
+  return pred != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
