@@ -17,14 +17,15 @@
 // CTA; gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
 //
 // Persistent CTAs (one per SM) walk the tile list.  Warp roles:
-//   warp 0      TMA producer of the activation tiles (128-byte swizzle), kActStages stages
-//   warp 14     TMA producer of the packed int4 weight tiles (64 x 64 bytes per 64-k step),
-//               their scales and zero points, six stages
+//   warp 0      TMA producer of the activation tiles (128-byte swizzle)
 //   warp 1      MMA issuer (one elected lane); owns the TMEM allocation
 //   warps 2-5   epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
-//               through a second TMEM accumulator buffer
-//   warps 6-13  dequantizers, two groups of four warps on alternate steps: thread = one
-//               weight column n of the tile (TMEM lane n), 64 k per step = 32 TMEM columns
+//               through a second TMEM accumulator buffer where two fit
+//   warps 6-17  dequantizers, three groups of four warps on steps in turn: thread = one
+//               weight column n of the tile (TMEM lane n), 64 k = 32 TMEM columns
+//   warp 18     TMA producer of the packed int4 weight tiles
+//   warp 19     TMA producer of their scales and zero points
+// A step is 64 k, or 128 k for tiles of up to 128 rows (struct Shape).
 // Stages are handed over with mbarriers; every wait is bounded and, on expiry, sets
 // an error word and drains the CTA instead of hanging the GPU.
 //
@@ -51,27 +52,37 @@ namespace {
 
 using namespace tc;
 // Two rings.  The weight path (TMA -> shared memory -> dequantize -> tensor memory -> MMA) has a
-// loop latency of several step times, so it is eight stages deep; its stages are small (5.5 KB of
-// shared memory, 32 TMEM columns).  The activation path (TMA -> shared memory -> MMA) is short
-// but its stages are 32 KB, so it gets six.
-constexpr int kActStages = 6;
-// The weight ring in shared memory (packed tile + scales + zero points per stage) is a template
-// parameter of the kernels.
-constexpr int kDeqStages = 8;     // dequantized weights in tensor memory
-// tcgen05.commit costs about as much pipe time as one 128x256x16 MMA (measured: 128 cycles per MMA
-// back to back, 241 with a commit after each), so completion is signalled once per kCommitSteps
-// k steps and both rings are released at that granularity.
-constexpr int kCommitSteps = 1;
-constexpr int kDoneBars = kDeqStages / kCommitSteps;
-static_assert(kActStages % kCommitSteps == 0 && kDeqStages % kCommitSteps == 0, "rings are released per commit group");
-constexpr int kDeqGroups = 2;     // warp groups taking k steps in turn (three or four measured 3 % faster at most)
-constexpr int kNumDeqWarps = 4 * kDeqGroups;
-constexpr int kWarpsPerDeqGroup = kNumDeqWarps / kDeqGroups;
+// loop latency of several step times and small stages, so it is the deeper one; the activation path
+// (TMA -> shared memory -> MMA) is short but its stages are up to 32 KB.
+constexpr int kWarpsPerDeqGroup = 4;  // one warp per quarter of the TMEM lanes
 constexpr int kNumEpiWarps = 4;
-constexpr int kWeightProducerWarp = 2 + kNumEpiWarps + kNumDeqWarps;  // last warp
-constexpr int kSecondIssuerWarp = kWeightProducerWarp + 1;  // second MMA-issuing thread (DUAL kernels), else idle
-constexpr int kMetaProducerWarp = kWeightProducerWarp + 2;  // TMA producer of the scales and zero points
-constexpr int kThreads = 32 * (5 + kNumEpiWarps + kNumDeqWarps);
+constexpr int kFirstDeqWarp = 2 + kNumEpiWarps;
+
+// Shape of the one-CTA kernel, by activation rows per tile.
+//   KSUB    64-k sub-steps per pipeline step: what the roles hand to one another at a time
+//   ACT/WS  shared-memory stages of the activations / of the packed weights and meta
+//   DS      stages of dequantized weights in tensor memory (32 * KSUB columns each)
+//   NG      dequantizer groups of four warps, on steps in turn
+template <int KSUB_, int ACT_, int WS_, int DS_, int NG_>
+struct Shape {
+  static constexpr int KSUB = KSUB_, ACT = ACT_, WS = WS_, DS = DS_, NG = NG_;
+  static constexpr int kStepK = BLOCK_K * KSUB;
+  static constexpr int kWeightProducerWarp = kFirstDeqWarp + 4 * NG;
+  static constexpr int kMetaProducerWarp = kWeightProducerWarp + 1;
+  static constexpr int kThreads = 32 * (kMetaProducerWarp + 1);
+  static_assert(ACT <= DS, "an activation stage is released by the MMA_DONE barrier of its step");
+};
+// Up to 128 rows the math of a 64-k step is shorter than its hand-overs (three barriers, a commit, the polls
+// of five roles: ~400 cycles with loads, conversion and MMAs all left out), so a step carries 128 k.  Measured on
+// B200, 64-k against 128-k steps with three groups each: K = 8192, N = 28672, block 128: M = 64 54.6 vs 43.9 us,
+// M = 17 50.2 vs 40.3, M = 128 67.2 vs 58.0; M = 100, 4096 -> 11008 20.5 vs 16.3; M = 32, 4096 x 4096 10.1 vs 9.5.
+// Above 128 rows two 64-k steps of activations per stage leave three stages only (rowwise M = 333: 24.8 vs 27.4 us).
+// Groups: two / three / four at M = 64: 47.3 / 43.9 / 44.5 us; M = 32, 4096 x 4096: 9.7 / 9.5 / 10.3 us.
+using ShapeSmall = Shape<2, 6, 10, 6, 3>;  // BM <= 64:  two accumulators + six stages of 64 TMEM columns = 512
+using ShapeMid = Shape<2, 4, 8, 4, 3>;     // BM <= 128: two accumulators + four stages = 512
+using ShapeLarge = Shape<1, 6, 6, 8, 3>;   // BM <= 256
+// k per pipeline step of the kernel that takes tiles of BM rows
+inline int step_k(int BM) { return BM <= 64 ? ShapeSmall::kStepK : BM <= 128 ? ShapeMid::kStepK : ShapeLarge::kStepK; }
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s: far beyond any legitimate wait
 
 struct Params {
@@ -99,7 +110,8 @@ struct Params {
   int k_per_item;      // 64-k steps per work item
   int num_items;       // tiles << split_shift
   int balanced;
-  int k_steps;         // K / 64
+  int k_steps;         // steps of a tile: K / 64, or / 128 rounded up for tiles of up to 128 rows
+  int min_part;        // one-CTA kernel: range_bound's minimum in steps
   int total_steps;     // tiles * k_steps
   float* ws_partials;  // balanced: [cta][BM][128] fp32; otherwise [tile][split-1][BM][128]
   int gather_bulk;         // pair kernel, gather mode: peer copies as cp.async.bulk of whole rows
@@ -116,14 +128,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 // ---- work items -----------------------------------------------------------------------------
 
-constexpr int kMinPartSteps = 4;  // a range boundary closer than this to a tile boundary moves onto it
+constexpr int kMinPartSteps = 4;  // a range boundary closer than this (in 64-k steps) to a tile boundary moves onto it
+inline int min_part(int step_k) { return kMinPartSteps * BLOCK_K / step_k; }
 
 // First step of CTA b's range in balanced mode (b == grid: the end of the last range).
-__host__ __device__ inline int range_bound(int total_steps, int k_steps, int grid, int b) {
+__host__ __device__ inline int range_bound(int total_steps, int k_steps, int grid, int b, int min_part = kMinPartSteps) {
   int x = (int)((long long)b * total_steps / grid);
   const int r = x % k_steps;
-  if (r < kMinPartSteps) x -= r;
-  else if (r > k_steps - kMinPartSteps) x += k_steps - r;
+  if (r < min_part) x -= r;
+  else if (r > k_steps - min_part) x += k_steps - r;
   return x;
 }
 
@@ -138,8 +151,8 @@ struct ItemCursor {
 __device__ __forceinline__ ItemCursor first_item(const Params& p) {
   ItemCursor c;
   if (p.balanced) {
-    c.pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x);
-    c.end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1);
+    c.pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x, p.min_part);
+    c.end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1, p.min_part);
   } else {
     c.pos = (int)blockIdx.x;
     c.end = p.num_items;
@@ -179,50 +192,47 @@ struct SmemPlan {
   uint32_t act, pack, scale, zp, out, bars, total;
   uint32_t act_bytes;
 };
-__host__ __device__ inline SmemPlan make_plan(int BM, int kStages, int act_stages, uint32_t out_bytes = 0) {
+__host__ __device__ inline SmemPlan make_plan(int BM, int kStages, int act_stages, int ksub, uint32_t out_bytes = 0) {
   SmemPlan p;
-  p.act_bytes = (uint32_t)BM * 128u;
+  p.act_bytes = (uint32_t)(BM * 128 * ksub);  // BM is a multiple of 16: 1024-aligned sub-tiles of 64 k
   uint32_t o = 0;
-  p.act = o;   o += act_stages * ((p.act_bytes + 1023u) & ~1023u);  // 1024-aligned tiles
-  p.pack = o;  o += kStages * kPackTileBytes;
-  p.scale = o; o += kStages * kScaleTileBytes;
-  p.zp = o;    o += kStages * kZpTileBytes;
+  p.act = o;   o += act_stages * p.act_bytes;
+  p.pack = o;  o += kStages * kPackTileBytes * ksub;
+  p.scale = o; o += kStages * kScaleTileBytes * ksub;
+  p.zp = o;    o += kStages * kZpTileBytes * ksub;
   p.out = o;   o += out_bytes;  // output staging of the pair kernel's epilogue
   p.bars = o;  o += 512;
   p.total = o + 1024;  // slack to align the dynamic base to 1024
   return p;
 }
 
-// Barrier slots (8 bytes each) inside the barrier block.  Stage s of the TMA ring and stage s
-// of the dequantized ring belong to the same k step, so one "MMA done" barrier frees both.
-#define BLKQ4_TC_BARRIER_SLOTS(WS, ACT, DONE)                                                         \
+// Barrier slots (8 bytes each) inside the barrier block.  An "MMA done" barrier frees the activation stage and
+// the stage of dequantized weights of its step.
+#define BLKQ4_TC_BARRIER_SLOTS(WS, ACT, DS, DONE)                                                     \
   constexpr int kStages = (WS);                                                                                    \
   constexpr int BAR_ACT_FULL = 0;                        /* [kActStages] activation tile landed (-> MMA issuer) */  \
   constexpr int BAR_FULL = BAR_ACT_FULL + (ACT);         /* [kStages] packed weights + meta landed (-> dequantizers) */ \
   constexpr int BAR_PACK_FREE = BAR_FULL + kStages;      /* [kStages] packed weights / meta read (-> producer) */   \
   constexpr int BAR_DEQ_FULL = BAR_PACK_FREE + kStages;  /* [kDeqStages] dequantized stage in TMEM (-> MMA issuer) */ \
-  constexpr int BAR_MMA_DONE = BAR_DEQ_FULL + kDeqStages;  /* [kDoneBars] commit group g = it / kCommitSteps retired, index g % kDoneBars */ \
+  constexpr int BAR_MMA_DONE = BAR_DEQ_FULL + (DS);  /* MMAs of step it retired, index it % count */ \
   constexpr int BAR_ACC_FULL = BAR_MMA_DONE + (DONE);    /* [2] accumulator complete */                             \
   constexpr int BAR_ACC_EMPTY = BAR_ACC_FULL + 2;        /* [2] accumulator drained by the epilogue */              \
   constexpr int BAR_COUNT = BAR_ACC_EMPTY + 2;                                                                      \
   static_assert(BAR_COUNT * 8 + 16 <= 512, "barrier block too small");
 
-// DUAL (BM <= 128): two threads issue the MMAs, the even k steps into one accumulator and the odd
-// ones into a second, and the epilogue adds the two.  A thread gets one tcgen05.mma accepted per
-// ~130 cycles whatever its N (measured: N = 32 .. 256, TMEM or shared-memory first operand), while
-// the tensor pipe needs only N/2 cycles for it - two threads with accumulators of their own reach
-// 65 cycles per MMA at N <= 64 and 71 at N = 128.  The sum order is fixed, so results stay reproducible.
-template <bool COLWISE, int WS, bool DUAL>
-__global__ void __launch_bounds__(kThreads, 1)
+template <bool COLWISE, class S>
+__global__ void __launch_bounds__(S::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_pack,
                const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
                const Params p) {
-  BLKQ4_TC_BARRIER_SLOTS(WS, kActStages, kDoneBars)
+  constexpr int KSUB = S::KSUB, kActStages = S::ACT, kDeqStages = S::DS, kStepK = S::kStepK;
+  constexpr int kStepCols = kDeqCols * KSUB, kStepPackBytes = kPackTileBytes * KSUB;
+  constexpr int kStepScaleBytes = kScaleTileBytes * KSUB, kStepZpBytes = kZpTileBytes * KSUB;
+  BLKQ4_TC_BARRIER_SLOTS(S::WS, kActStages, kDeqStages, kDeqStages)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const SmemPlan plan = make_plan(p.BM, kStages, kActStages);
-  const uint32_t act_stride = (plan.act_bytes + 1023u) & ~1023u;
+  const SmemPlan plan = make_plan(p.BM, kStages, kActStages, KSUB);
   const uint32_t bars = base + plan.bars;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + plan.bars + BAR_COUNT * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + plan.bars + BAR_COUNT * 8 + 8);
@@ -244,9 +254,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       mbar_init(bar(BAR_PACK_FREE + i), kWarpsPerDeqGroup);
     }
     for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_DEQ_FULL + i), kWarpsPerDeqGroup);
-    for (int i = 0; i < kDoneBars; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
+    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(BAR_ACC_FULL + i), DUAL ? 2 : 1);
+      mbar_init(bar(BAR_ACC_FULL + i), 1);
       mbar_init(bar(BAR_ACC_EMPTY + i), kNumEpiWarps);
     }
     *abort_flag = 0;
@@ -277,28 +287,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         for (int ks = item.ks0; ks < item.ks0 + item.count; ++ks, ++it) {
           const int sa = it % kActStages;
           if (it >= (uint32_t)kActStages) {
-            const uint32_t g = (it - kActStages) / kCommitSteps;  // commit group of the stage's last user
-            if (!mbar_wait(bar(BAR_MMA_DONE + g % kDoneBars), (g / kDoneBars) & 1, abort_flag, 0x100 | sa))
+            const uint32_t g = it - kActStages;  // the stage's last user
+            if (!mbar_wait(bar(BAR_MMA_DONE + g % kDeqStages), (g / kDeqStages) & 1, abort_flag, 0x100 | sa))
               goto act_producer_done;
           }
           const uint32_t fb = bar(BAR_ACT_FULL + sa);
           mbar_arrive_expect_tx(fb, plan.act_bytes);
-          tma_load_2d(base + plan.act + sa * act_stride, &tm_act, ks * BLOCK_K, m_tile * p.BM, fb);
+#pragma unroll
+          for (int u = 0; u < KSUB; ++u)  // past the end of K the copy fills zeros
+            tma_load_2d(base + plan.act + sa * plan.act_bytes + u * (p.BM * 128), &tm_act, ks * kStepK + u * BLOCK_K,
+                        m_tile * p.BM, fb);
         }
       }
     act_producer_done:;
     }
-  } else if (warp == kWeightProducerWarp || warp == kMetaProducerWarp) {
+  } else if (warp == S::kWeightProducerWarp || warp == S::kMetaProducerWarp) {
     // ============ TMA producers: packed weights (one warp), scales and zero points (another) ============
-    // A thread gets one bulk-tensor copy accepted per ~110 cycles; with the stage wait and the byte-count
-    // post, one thread issuing all three copies of a step is good for a step per ~600 cycles, which is
-    // the whole kernel's pace once two threads issue the MMAs.  Hence two producer threads, each
-    // arriving on the stage's barrier with its own byte count.
+    // Two producer threads, each arriving on the stage's barrier with its own byte count: the stage wait,
+    // the byte-count post and up to three copies of a step are a serial chain for one thread.
     if (elect_one()) {
-      const bool meta = warp == kMetaProducerWarp;
+      const bool meta = warp == S::kMetaProducerWarp;
       const uint32_t tx = meta ? (uint32_t)p.meta_rows * p.meta_row_bytes_s +
                                      (p.has_zp ? (uint32_t)p.meta_rows * p.meta_row_bytes_z : 0u)
-                               : (uint32_t)kPackTileBytes;
+                               : (uint32_t)kStepPackBytes;
       uint32_t it = 0;
       ItemCursor cur = first_item(p);
       Item item;
@@ -311,74 +322,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
             goto w_producer_done;
           const uint32_t fb = bar(BAR_FULL + s);
           mbar_arrive_expect_tx(fb, tx);
-          const int k0 = ks * BLOCK_K;
+          const int k0 = ks * kStepK;
           if (!meta) {
-            tma_load_2d(base + plan.pack + s * kPackTileBytes, &tm_pack, k0, n_tile * (TILE_N / 2), fb);
+            tma_load_2d(base + plan.pack + s * kStepPackBytes, &tm_pack, k0, n_tile * (TILE_N / 2), fb);
           } else if (COLWISE) {
             // meta row-major [K/block, N]: box = meta_rows x 128 columns
             const int mrow = k0 >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &tm_scale, n_tile * TILE_N, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &tm_zp, n_tile * TILE_N, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &tm_scale, n_tile * TILE_N, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &tm_zp, n_tile * TILE_N, mrow, fb);
           } else {
             // meta column-major [K, N/block]: box = meta_rows (n blocks) x 64 k
             const int mrow = (n_tile * TILE_N) >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &tm_scale, k0, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &tm_zp, k0, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &tm_scale, k0, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &tm_zp, k0, mrow, fb);
           }
         }
       }
     w_producer_done:;
     }
-  } else if (DUAL && (warp == 1 || warp == kSecondIssuerWarp)) {
-    // ========================= MMA issuers, DUAL: even steps / odd steps =========================
-    if (elect_one()) {
-      const uint32_t q = warp == 1 ? 0u : 1u;
-      const uint32_t idesc = make_idesc_f16(TILE_N, p.BM);
-      const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
-      const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);
-      const uint32_t act_lo0 = desc_lo_flags | (((base + plan.act) >> 4) & 0x3FFFu);
-      const uint32_t act_lo_step = act_stride >> 4;
-      const uint32_t a_tmem0 = tmem_base + (uint32_t)p.a_col0;
-      const uint32_t d_tmem = tmem_base + q * (uint32_t)p.BM;  // one accumulator per issuer, no double buffering
-      uint32_t it = 0, tcount = 0;
-      ItemCursor cur = first_item(p);
-      Item item;
-      for (; next_item(p, cur, item); ++tcount) {
-        if (tcount >= 1u && !mbar_wait(bar(BAR_ACC_EMPTY), (tcount - 1u) & 1u, abort_flag, 0x200 | q)) goto mma2_done;
-        tc_fence_after();
-        uint32_t accumulate = 0u;
-        for (uint32_t st = it + ((it ^ q) & 1u); st < it + (uint32_t)item.count; st += 2) {
-          const uint32_t s = st % kDeqStages, sa = st % kActStages;
-          const uint32_t bar_a = bar(BAR_ACT_FULL) + 8u * sa, bar_d = bar(BAR_DEQ_FULL) + 8u * s;
-          const uint32_t par_sa = (st / kActStages) & 1u, par_s = (st / kDeqStages) & 1u;
-          if (!mbar_try_wait(bar_a, par_sa) && !mbar_wait(bar_a, par_sa, abort_flag, 0x210 | sa)) goto mma2_done;
-          if (!mbar_try_wait(bar_d, par_s) && !mbar_wait(bar_d, par_s, abort_flag, 0x220 | s)) goto mma2_done;
-          tc_fence_after();
-          umma_f16_ts_x4(d_tmem, a_tmem0 + s * kDeqCols, act_lo0 + sa * act_lo_step, desc_hi, idesc, accumulate);
-          accumulate = 1u;
-          umma_commit(bar(BAR_MMA_DONE) + 8u * (st % kDoneBars));
-        }
-        it += (uint32_t)item.count;
-        umma_commit(bar(BAR_ACC_FULL));  // arrives at once for an issuer without a step in this item
-      }
-    mma2_done:;
-    }
   } else if (warp == 1) {
     // =============================== MMA issuer =================================
-    // One thread drives the tensor pipe, and its own instruction stream is the critical
-    // path of the kernel: a 128x256x16 MMA takes 128 cycles, so the waits, address
+    // One thread drives the tensor pipe; a 128x256x16 MMA takes 128 cycles, so the waits, address
     // arithmetic, four issues and the commit of a 64-k step must fit in 512 cycles of
     // dependent scalar code.  Hence: ring indices and parities are carried incrementally
-    // (no division), the four MMAs of a step are one asm block, and the barrier polls take
+    // (no division), the four MMAs of 64 k are one asm block, and the barrier polls take
     // the slow (bounded, instrumented) path only when the first poll fails.
     if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
       const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);  // LBO field
       const uint32_t act_lo0 = desc_lo_flags | (((base + plan.act) >> 4) & 0x3FFFu);
-      const uint32_t act_lo_step = act_stride >> 4;
+      const uint32_t act_lo_step = plan.act_bytes >> 4, act_lo_sub = (uint32_t)p.BM * 128u >> 4;
       const uint32_t a_tmem0 = tmem_base + (uint32_t)p.a_col0;
-      uint32_t s = 0, sa = 0, par_s = 0, par_sa = 0, gdone = 0, it = 0, tcount = 0;
+      uint32_t s = 0, sa = 0, par_s = 0, par_sa = 0, tcount = 0;
       uint32_t ab = 0, par_acc = 0;
       // The barriers of step i + 1 are polled (without blocking) BEFORE the MMAs of step i are
       // issued, so that the poll's round trip to shared memory overlaps the issue instead of
@@ -391,7 +367,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       goto mma_done;                                                                                                \
     tc_fence_after();                                                                                               \
     const uint32_t d_tmem = tmem_base + ab * (uint32_t)p.BM;                                                        \
-    for (int ks = 0; ks < (COUNT); ++ks, ++it) {                                                                    \
+    for (int ks = 0; ks < (COUNT); ++ks) {                                                                          \
       const uint32_t bar_a = bar(BAR_ACT_FULL) + 8u * sa, bar_d = bar(BAR_DEQ_FULL) + 8u * s;                       \
       if (!ready_a && !mbar_try_wait(bar_a, par_sa) && !mbar_wait(bar_a, par_sa, abort_flag, 0x210 | sa))           \
         goto mma_done;                                                                                              \
@@ -399,16 +375,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         goto mma_done;                                                                                              \
       tc_fence_after();                                                                                             \
       /* 16 k = 8 TMEM columns of the weights, 32 bytes (2 descriptor units) of the activation row */              \
-      const uint32_t a_tmem = a_tmem0 + s * kDeqCols, b_lo = act_lo0 + sa * act_lo_step;                            \
+      const uint32_t a_tmem = a_tmem0 + s * kStepCols, b_lo = act_lo0 + sa * act_lo_step;                           \
+      const uint32_t done_bar = bar(BAR_MMA_DONE) + 8u * s;                                                         \
       if (++s == kDeqStages) { s = 0; par_s ^= 1u; }                                                                \
       if (++sa == kActStages) { sa = 0; par_sa ^= 1u; }                                                             \
       ready_a = mbar_test_wait(bar(BAR_ACT_FULL) + 8u * sa, par_sa);                                                \
       ready_d = mbar_test_wait(bar(BAR_DEQ_FULL) + 8u * s, par_s);                                                  \
       umma_f16_ts_x4(d_tmem, a_tmem, b_lo, desc_hi, idesc, ks > 0 ? 1u : 0u);                                       \
-      if (it % kCommitSteps == kCommitSteps - 1) {                                                                  \
-        umma_commit(bar(BAR_MMA_DONE) + 8u * gdone);                                                                \
-        if (++gdone == kDoneBars) gdone = 0;                                                                        \
-      }                                                                                                             \
+      _Pragma("unroll") for (int u = 1; u < KSUB; ++u)                                                              \
+        umma_f16_ts_x4(d_tmem, a_tmem + u * kDeqCols, b_lo + u * act_lo_sub, desc_hi, idesc, 1u);                   \
+      umma_commit(done_bar);                                                                                        \
     }                                                                                                               \
     umma_commit(bar(BAR_ACC_FULL + ab));                                                                            \
     if (++ab == (uint32_t)p.acc_bufs) { ab = 0; par_acc ^= 1u; }                                                    \
@@ -416,8 +392,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       if (!p.balanced) {
         for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++tcount) BLKQ4_TC_MMA_ITEM(p.k_per_item)
       } else {
-        int pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x);
-        const int end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1);
+        int pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x, p.min_part);
+        const int end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1, p.min_part);
         int to_tile_end = p.k_steps - pos % p.k_steps;
         for (; pos < end; ++tcount) {
           const int count = min(to_tile_end, end - pos);
@@ -438,7 +414,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     uint32_t tcount = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // output and workspace belong to stream order
     const size_t tile_floats = (size_t)p.BM * TILE_N;
-    uint32_t it_base = 0;  // global index of the item's first k step
     ItemCursor cur = first_item(p);
     Item item;
     for (; next_item(p, cur, item); ++tcount) {
@@ -446,27 +421,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       const int ab = tcount % p.acc_bufs;
       if (!mbar_wait(bar(BAR_ACC_FULL + ab), (tcount / p.acc_bufs) & 1, abort_flag, 0x300 | ab)) break;
       tc_fence_after();
-      // DUAL: the item's even steps were summed in accumulator 0 and its odd steps in accumulator 1 (an
-      // item of a single step wrote only one of them); the result is accumulator 0 + accumulator 1.
-      const bool have0 = !DUAL || item.count > 1 || (it_base & 1u) == 0u;
-      const bool have1 = DUAL && (item.count > 1 || (it_base & 1u) == 1u);
-      it_base += (uint32_t)item.count;
       auto load_acc = [&](int c0, uint32_t (&r)[32]) {
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        if (!DUAL) {
-          tmem_ld_32x32b_x32(lane_base + (uint32_t)(ab * p.BM + c0), r);
-          tmem_ld_wait();
-        } else if (have0 && have1) {
-          uint32_t r1[32];
-          tmem_ld_32x32b_x32(lane_base + (uint32_t)c0, r);
-          tmem_ld_32x32b_x32(lane_base + (uint32_t)(p.BM + c0), r1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
-        } else {
-          tmem_ld_32x32b_x32(lane_base + (uint32_t)((have1 ? p.BM : 0) + c0), r);
-          tmem_ld_wait();
-        }
+        tmem_ld_32x32b_x32(lane_base + (uint32_t)(ab * p.BM + c0), r);
+        tmem_ld_wait();
       };
       const int n_l = quarter * 32 + lane;
       if (item.role == 1) {
@@ -559,21 +517,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           p.ws_flags[item.flag] = 0u;
       }
     }
-  } else if (warp < kWeightProducerWarp) {
+  } else if (warp < S::kWeightProducerWarp) {
     // =============================== dequantizers ===============================
-    // Two groups of four warps take alternate 64-k steps, so that a group has two step times
-    // for the dependent chain wait -> load -> convert -> tcgen05.st -> arrive of one step.
+    // The groups of four warps take steps in turn, so that a group has as many step times as there are
+    // groups for the dependent chain wait -> load -> convert -> tcgen05.st -> arrive of one step.
     // A warp may only touch the TMEM lanes of its quarter (warp id % 4), and lane = row of the
     // MMA's first operand = weight column n of the tile: thread <-> n = 32 (warp % 4) + lane.
     // Column n lives in packed column np_l = 8 (n / 16) + n % 8 of the tile, in the "low"
     // nibble positions when n % 16 < 8 and 8 bits further up otherwise (the thread of n +- 8
-    // reads the same bytes).  Per step it reads the column's 64 bytes and writes 32 TMEM
+    // reads the same bytes).  Per 64 k it reads the column's 64 bytes and writes 32 TMEM
     // columns: column j = fp16 pair k = (2j, 2j + 1).
-    const int dw = warp - (2 + kNumEpiWarps);
-    const int group = dw / kWarpsPerDeqGroup;
+    const int group = (warp - kFirstDeqWarp) / kWarpsPerDeqGroup;
     const int n_l = 32 * (warp & 3) + lane;
     const int np_l = 8 * (n_l >> 4) + (n_l & 7);
-    const uint32_t nib_shift = (n_l & 8) ? 8u : 0u;
+    const uint32_t rot_lo = (n_l & 8) ? 30u : 6u, rot_hi = (n_l & 8) ? 26u : 2u;
     const uint32_t tmem_row = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)p.a_col0;
     uint32_t total_its = 0;
     {
@@ -581,20 +538,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       Item item;
       while (next_item(p, cur, item)) total_its += (uint32_t)item.count;
     }
-    for (uint32_t it = group; it < total_its; it += kDeqGroups) {
+    with_block_shift(p.block_shift, p.has_zp, [&](auto bsh, auto zp) {
+    for (uint32_t it = group; it < total_its; it += S::NG) {
       const int s = it % kStages, d = it % kDeqStages;
       if (it >= (uint32_t)kDeqStages) {
-        const uint32_t g = (it - kDeqStages) / kCommitSteps;  // commit group of the TMEM stage's last user
-        if (!mbar_wait(bar(BAR_MMA_DONE + g % kDoneBars), (g / kDoneBars) & 1, abort_flag, 0x410 | d)) break;
+        const uint32_t g = it - kDeqStages;  // the TMEM stage's last user
+        if (!mbar_wait(bar(BAR_MMA_DONE + d), (g / kDeqStages) & 1, abort_flag, 0x410 | d)) break;
       }
       if (!mbar_wait(bar(BAR_FULL + s), (it / kStages) & 1, abort_flag, 0x400 | s)) break;
       tc_fence_after();
-      const uint8_t* pk = base_ptr + plan.pack + s * kPackTileBytes + np_l * 64;
-      const uint8_t* sc_tile = base_ptr + plan.scale + s * kScaleTileBytes;
-      const uint8_t* zp_tile = base_ptr + plan.zp + s * kZpTileBytes;
-      uint32_t out[32];
-      dequant_step<COLWISE>(pk, sc_tile, zp_tile, n_l, nib_shift, p.block, p.block_shift, p.has_zp, out);
-      tmem_st_32x32b_x32(tmem_row + (uint32_t)(d * kDeqCols), out);
+      const uint8_t* pk = base_ptr + plan.pack + s * kStepPackBytes + np_l * kStepK;
+      const uint8_t* sc_tile = base_ptr + plan.scale + s * kStepScaleBytes;
+      const uint8_t* zp_tile = base_ptr + plan.zp + s * kStepZpBytes;
+      DequantSub<COLWISE, decltype(bsh)::value, decltype(zp)::value != 0, KSUB> sub[KSUB];
+#pragma unroll
+      for (int u = 0; u < KSUB; ++u) sub[u].load(pk, u, sc_tile, zp_tile, n_l);
+#pragma unroll
+      for (int u = 0; u < KSUB; ++u) {
+        uint32_t out[32];
+        sub[u].emit(sc_tile, zp_tile, u, n_l, rot_lo, rot_hi, out);
+        tmem_st_32x32b_x32(tmem_row + (uint32_t)(d * kStepCols + u * kDeqCols), out);
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -603,6 +567,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         mbar_arrive(bar(BAR_PACK_FREE + s));
       }
     }
+    });
   }
 
   // ---- teardown ----
@@ -639,7 +604,7 @@ struct SplitPlan {
 SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   const int BM = M >= 256 ? 256 : ((M + 15) / 16) * 16;
   const int tiles = ((M + BM - 1) / BM) * ((N + TILE_N - 1) / TILE_N);
-  const int k_steps = K / BLOCK_K;
+  const int k_steps = (K + step_k(BM) - 1) / step_k(BM);
   const int sms = sm_count() > 0 ? sm_count() : 148;
   SplitPlan best{0, 0, 0, 0};
   if (tiles > sms) {
@@ -651,7 +616,7 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
     const int rounds = (tiles + sms - 1) / sms;
     const long long total_steps = (long long)tiles * k_steps;
     static const bool off = getenv("BLKQ4_TC_NO_BALANCE") != nullptr;
-    if (!off && total_steps < (1ll << 30) / sms && total_steps / sms >= k_steps + 2 * kMinPartSteps &&
+    if (!off && total_steps < (1ll << 30) / sms && total_steps / sms >= k_steps + 2 * min_part(step_k(BM)) &&
         (double)tiles < 0.80 * rounds * sms) {
       const size_t flags = ((size_t)sms * sizeof(unsigned) + 255) & ~(size_t)255;
       const size_t total = flags + (size_t)sms * BM * TILE_N * sizeof(float);
@@ -663,7 +628,7 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   // second round of half-size items loses more to the fp32 exchange than it gains in balance.
   for (int shift = 1; shift <= 2; ++shift) {
     const int split = 1 << shift;
-    if (k_steps % split != 0 || k_steps / split < 8 || tiles * split > sms) continue;
+    if (k_steps % split != 0 || (k_steps / split) * step_k(BM) < 512 || tiles * split > sms) continue;
     const size_t flags = ((size_t)tiles * sizeof(unsigned) + 255) & ~(size_t)255;
     const size_t total = flags + (size_t)tiles * (split - 1) * BM * TILE_N * sizeof(float);
     if (total > ws_bytes_available) continue;
@@ -767,13 +732,13 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   p.out = out;
   p.bias = bias;
   // tensor memory: accumulators first, then the dequantized stages
-  // BM <= 128: two accumulators, one per MMA-issuing thread (DUAL kernels); above, a single accumulator
-  static const bool dual_off = getenv("BLKQ4_TC_NO_DUAL") != nullptr;
-  const bool dual = p.BM <= 128 && !dual_off;
-  p.acc_bufs = dual ? 1 : ((2 * p.BM + kDeqStages * kDeqCols <= 512) ? 2 : 1);
-  p.a_col0 = dual ? 2 * p.BM : p.acc_bufs * p.BM;
+  const int deq_cols = p.BM <= 64 ? ShapeSmall::DS * ShapeSmall::KSUB * kDeqCols
+                       : p.BM <= 128 ? ShapeMid::DS * ShapeMid::KSUB * kDeqCols
+                                     : ShapeLarge::DS * ShapeLarge::KSUB * kDeqCols;
+  p.acc_bufs = (2 * p.BM + deq_cols <= 512) ? 2 : 1;
+  p.a_col0 = p.acc_bufs * p.BM;
   {
-    const uint32_t need = (uint32_t)(p.a_col0 + kDeqStages * kDeqCols);
+    const uint32_t need = (uint32_t)(p.a_col0 + deq_cols);
     p.tmem_cols = 32;
     while (p.tmem_cols < need) p.tmem_cols <<= 1;
   }
@@ -788,17 +753,21 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     p.m_tiles = pp.m_tiles;
   }
 
+  // k per pipeline step: the box of the weights and of the meta spans it, the activations come in 64-k tiles
+  const int sk = pair ? BLOCK_K : step_k(p.BM);
   CUtensorMap tm_act, tm_pack, tm_scale, tm_zp;
   bool ok = encode_tensor_map_2d(&tm_act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)K, (uint64_t)M, BLOCK_K,
                       pair ? (uint32_t)(p.BM / 2) : (uint32_t)p.BM, CU_TENSOR_MAP_SWIZZLE_128B);
-  // No swizzle on the packed tile: the dequantizers' 16-byte loads of eight neighbouring packed
+  // Packed tiles of 128-byte rows carry the 128-byte swizzle: the dequantizers' 16-byte loads of eight
+  // neighbouring packed columns would otherwise all fall on the same banks.
+  // No swizzle on 64-byte rows: the dequantizers' 16-byte loads of eight neighbouring packed
   // columns (64 bytes apart) do conflict four ways, but a 64-byte TMA swizzle that removes the
   // conflicts measured 1-2 % SLOWER on the same GPU (c3 59.2 vs 58.2 us): those loads are not on
   // the critical path, the extra XOR per load is.
   ok = ok && encode_tensor_map_2d(&tm_pack, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)K, (uint64_t)(N / 2),
-                       BLOCK_K, TILE_N / 2, CU_TENSOR_MAP_SWIZZLE_NONE);
+                       (uint32_t)sk, TILE_N / 2, sk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
   if (colwise) {
-    p.meta_rows = block >= BLOCK_K ? 1 : BLOCK_K / block;
+    p.meta_rows = block >= sk ? 1 : sk / block;
     p.meta_row_bytes_s = TILE_N * 2;
     p.meta_row_bytes_z = TILE_N;
     ok = ok && encode_tensor_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, (uint64_t)N,
@@ -807,12 +776,12 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
                          (uint64_t)(K / block), TILE_N, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
   } else {
     p.meta_rows = block >= TILE_N ? 1 : TILE_N / block;
-    p.meta_row_bytes_s = BLOCK_K * 2;
-    p.meta_row_bytes_z = BLOCK_K;
+    p.meta_row_bytes_s = (uint32_t)sk * 2;
+    p.meta_row_bytes_z = (uint32_t)sk;
     ok = ok && encode_tensor_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, (uint64_t)K,
-                         (uint64_t)(N / block), BLOCK_K, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+                         (uint64_t)(N / block), (uint32_t)sk, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
     ok = ok && encode_tensor_map_2d(&tm_zp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, zp ? zp : packed, (uint64_t)K,
-                         (uint64_t)(N / block), BLOCK_K, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+                         (uint64_t)(N / block), (uint32_t)sk, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
   }
   if (!ok) return "cuTensorMapEncodeTiled failed";
 
@@ -832,7 +801,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     p.ws_flags = reinterpret_cast<unsigned*>(workspace);
     p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + pp.flags_bytes);
     auto kern = colwise ? gemm_tc_pair_kernel<true, kPairWeightStages> : gemm_tc_pair_kernel<false, kPairWeightStages>;
-    const SmemPlan plan = make_plan(kPairRows, kPairWeightStages, kPairActStages, kPairOutBytes);
+    const SmemPlan plan = make_plan(kPairRows, kPairWeightStages, kPairActStages, 1, kPairOutBytes);
     static std::atomic<int> granted[2][64];
     cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[colwise ? 1 : 0]);
     if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
@@ -869,24 +838,35 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   const int num_tiles = p.m_tiles * p.n_tiles;
   const SplitPlan sp = ws_ok ? plan_split(M, N, K, workspace_bytes) : SplitPlan{0, 0, 0, 0};
   p.split_shift = sp.split_shift;
-  p.k_per_item = (K / BLOCK_K) >> sp.split_shift;
+  p.k_steps = (K + sk - 1) / sk;
+  p.k_per_item = p.k_steps >> sp.split_shift;
+  p.min_part = min_part(sk);
   p.num_items = num_tiles << sp.split_shift;
   p.balanced = sp.balanced;
-  p.k_steps = K / BLOCK_K;
   p.total_steps = sp.balanced ? num_tiles * p.k_steps : 0;
   p.ws_flags = reinterpret_cast<unsigned*>(workspace);
   p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + sp.flags_bytes);
   const int grid = p.num_items < sms ? p.num_items : sms;
-  // (a 16-stage weight ring measured no faster than 6 with either kernel)
-  const SmemPlan plan = make_plan(p.BM, 6, kActStages);
-  auto kern = dual ? (colwise ? gemm_tc_kernel<true, 6, true> : gemm_tc_kernel<false, 6, true>)
-                   : (colwise ? gemm_tc_kernel<true, 6, false> : gemm_tc_kernel<false, 6, false>);
-  static std::atomic<int> granted[4][64];
-  cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[(colwise ? 1 : 0) + (dual ? 2 : 0)]);
+  using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params);
+  static std::atomic<int> granted[6][64];
+  Kern kern;
+  int threads, which;
+  SmemPlan plan;
+  auto pick = [&](auto shape, int idx) {
+    using S = decltype(shape);
+    kern = colwise ? (Kern)gemm_tc_kernel<true, S> : (Kern)gemm_tc_kernel<false, S>;
+    threads = S::kThreads;
+    which = 2 * idx + (colwise ? 1 : 0);
+    plan = make_plan(p.BM, S::WS, S::ACT, S::KSUB);
+  };
+  if (p.BM <= 64) pick(ShapeSmall{}, 0);
+  else if (p.BM <= 128) pick(ShapeMid{}, 1);
+  else pick(ShapeLarge{}, 2);
+  cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[which]);
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = plan.total;
   cfg.stream = stream;
   // BLKQ4_GEMM_EARLY_WEIGHT_FETCH: programmatic stream serialization, see the kernel's entry

@@ -36,6 +36,10 @@ constexpr int kPairRows = 128;  // most activation rows staged per CTA: half of 
 // both CTAs' activation copies and the arrivals of both CTAs' dequantizer warps - and the MMA thread
 // polls one barrier per step instead of two: every instruction of that thread is on the critical path.
 constexpr int kPairActStages = 8;     // 16 KB each
+constexpr int kDeqStages = 8;         // dequantized weights in tensor memory, 32 columns each
+constexpr int kDeqGroups = 2;         // warp groups taking k steps in turn (three or four measured slower)
+constexpr int kNumDeqWarps = 4 * kDeqGroups;
+constexpr int kWeightProducerWarp = kFirstDeqWarp + kNumDeqWarps;  // last warp
 constexpr int kPairWeightStages = 6;  // 5.5 KB each; deeper rings measured no faster
 constexpr int kPairCommitSteps = 1;   // a commit per two steps measured no faster
 // fp16 staging of a CTA's 128 x 256 output tile: the epilogue empties the accumulator into it, hands
@@ -127,7 +131,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
       : "memory");
 }
 
-// warps 0 .. kWeightProducerWarp only: the one-CTA kernel's second issuer and meta producer have no part here
+// warps 0 .. kWeightProducerWarp only: no meta producer here
 constexpr int kPairThreads = 32 * (kWeightProducerWarp + 1);
 
 // Work items of one pair.  Whole rounds: pair tiles `pair`, `pair + num_pairs`, ... in full.  Balanced
@@ -176,11 +180,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                     const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
                     const Params p) {
   constexpr int kActStages = kPairActStages, kDoneBars = kPairDoneBars, kCommitSteps = kPairCommitSteps;
-  BLKQ4_TC_BARRIER_SLOTS(WS, kPairActStages, kPairDoneBars)
+  BLKQ4_TC_BARRIER_SLOTS(WS, kPairActStages, kDeqStages, kPairDoneBars)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const SmemPlan plan = make_plan(kPairRows, kStages, kActStages, kPairOutBytes);
+  const SmemPlan plan = make_plan(kPairRows, kStages, kActStages, 1, kPairOutBytes);
   const uint32_t act_stride = (plan.act_bytes + 1023u) & ~1023u;
   const uint32_t bars = base + plan.bars;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + plan.bars + BAR_COUNT * 8);
@@ -588,7 +592,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int group = dw / kWarpsPerDeqGroup;
     const int n_l = 32 * (warp & 3) + lane;
     const int np_l = 8 * (n_l >> 4) + (n_l & 7);
-    const uint32_t nib_shift = (n_l & 8) ? 8u : 0u;
+    const uint32_t rot_lo = (n_l & 8) ? 30u : 6u, rot_hi = (n_l & 8) ? 26u : 2u;
     const uint32_t tmem_row = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + kAcol0;
     const uint32_t deq_full_leader = map_to_cta(bar(BAR_DEQ_FULL), 0);
     uint32_t total_its = 0;
@@ -597,6 +601,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       int item, ks0, count, role;
       while (walk.next(item, ks0, count, role)) total_its += (uint32_t)count;
     }
+    with_block_shift(p.block_shift, p.has_zp, [&](auto bsh, auto zp) {
     for (uint32_t it = group; it < total_its; it += kDeqGroups) {
       const int s = it % kStages, d = it % kDeqStages;
       if (it >= (uint32_t)kDeqStages) {
@@ -608,8 +613,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       const uint8_t* pk = base_ptr + plan.pack + s * kPackTileBytes + np_l * 64;
       const uint8_t* sc_tile = base_ptr + plan.scale + s * kScaleTileBytes;
       const uint8_t* zp_tile = base_ptr + plan.zp + s * kZpTileBytes;
+      DequantSub<COLWISE, decltype(bsh)::value, decltype(zp)::value != 0, 1> sub;
+      sub.load(pk, 0, sc_tile, zp_tile, n_l);
       uint32_t out[32];
-      dequant_step<COLWISE>(pk, sc_tile, zp_tile, n_l, nib_shift, p.block, p.block_shift, p.has_zp, out);
+      sub.emit(sc_tile, zp_tile, 0, n_l, rot_lo, rot_hi, out);
       tmem_st_32x32b_x32(tmem_row + (uint32_t)(d * kDeqCols), out);
       tmem_st_wait();
       tc_fence_before();
@@ -620,6 +627,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         mbar_arrive(bar(BAR_PACK_FREE + s));
       }
     }
+    });
   }
 
   // ---- teardown: neither CTA frees tensor memory or leaves while the other may still signal it ----

@@ -103,71 +103,121 @@ __host__ __device__ inline uint32_t make_idesc_f16(int umma_m, int umma_n) {
 }
 
 
-// One 64-k step of weight column n_l of a tile: reads the column's 64 packed bytes (`pk`, already
-// pointing at the packed column; `nib_shift` 0 or 8 selects which of the two columns sharing the bytes
-// this thread owns), the step's scale / zero-point tile, and produces the 32 fp16 pairs of the
-// dequantized stage: out[j] = k pair (2j, 2j + 1).  Numerics are the reference kernel's: fp16(16 + q)
+// One 64-k sub-step of weight column n_l of a tile (a step holds KSUB of them): `load` reads the column's 64
+// packed bytes and its scales / zero points from the stage in shared memory, `emit` produces the 32 fp16
+// pairs of the dequantized stage, out[j] = k pair (2j, 2j + 1).  Numerics are the reference kernel's: fp16(16 + q)
 // by bit placement, then fma.rn.f16 with rn(scale * (-16 - zp)).
-template <bool COLWISE>
-__device__ __forceinline__ void dequant_step(const uint8_t* pk, const uint8_t* sc_tile, const uint8_t* zp_tile,
-                                             int n_l, uint32_t nib_shift, int block, int block_shift, int has_zp,
-                                             uint32_t (&out)[32]) {
-  const uint32_t rot_lo = nib_shift ? 30u : 6u, rot_hi = nib_shift ? 26u : 2u;
+// Block size and zero points are template parameters and loading is separate from converting so that all
+// loads of a step are issued back to back: with a runtime block size every 16-k chunk had its own
+// dependent scale load and a branch on the zero points, and a step cost a dequantizer group ~2300 cycles of
+// mostly latency (M = 17, K = 8192, N = 28672, block 128: 46.1 us against 26.3 us without the conversion).
+template <int KSUB>
+struct PackedColumn {
+  uint4 w[4];
+  // `pk` points at the packed column; 128-byte rows are stored with the 128-byte swizzle (chunk c of packed
+  // column r lies at c ^ (r % 8)), so that the eight columns a quarter-warp reads fall on different banks
+  __device__ __forceinline__ void load(const uint8_t* pk, int sub, int n_l) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {  // 16-byte chunk: k in [16 c, 16 c + 16)
-    const uint4 wv = *reinterpret_cast<const uint4*>(pk + c * 16);
-    const uint32_t w4[4] = {wv.x, wv.y, wv.z, wv.w};
-    // scale / offset half2 for the k pairs (2r, 2r+1) [lo] and (2r+8, 2r+9) [hi] of word r
-    uint32_t s_lo[4], s_hi[4], o_lo[4], o_hi[4];
-    if (COLWISE) {
-      // scale tile: meta_rows x 128 fp16; the 16 k of a chunk share one block
-      const int mr = (block >= BLOCK_K) ? 0 : ((c * 16) >> block_shift);
-      const uint32_t sc = reinterpret_cast<const unsigned short*>(sc_tile)[mr * TILE_N + n_l];
-      const uint32_t z = has_zp ? (uint32_t)zp_tile[mr * TILE_N + n_l] : 8u;
-      const uint32_t sc2 = sc | (sc << 16);
+    for (int c = 0; c < 4; ++c) {
+      const int cc = sub * 4 + c;
+      w[c] = *reinterpret_cast<const uint4*>(pk + (KSUB == 2 ? ((cc ^ (n_l & 7)) * 16) : cc * 16));
+    }
+  }
+  // Column n0's nibbles sit at bits 0-3 / 16-19 (k = 2r, 2r+1) and 4-7 / 20-23 (k = 2r+8, 2r+9) of word r, column
+  // n0 + 8's eight bits further up; fp16(16 + q) by bit placement needs them at bits 6-9 / 22-25.  One
+  // rotation per operand does it (instead of a shift to this thread's nibbles and a second one into
+  // place): left by 6 / 2 for n0, by 30 / 26 (= right by 2 / 6) for n0 + 8; what wraps around falls
+  // outside the mask.
+  __device__ __forceinline__ static uint32_t half16plus(uint32_t w, uint32_t rot) {
+    return (__funnelshift_l(w, w, rot) & 0x03c003c0u) | 0x4c004c00u;
+  }
+};
+
+template <bool COLWISE, int BLOCK_SHIFT, bool HAS_ZP, int KSUB>
+struct DequantSub;
+
+// Column-wise blocks: meta tile = rows of 128 columns, one row per block of k.
+template <int BLOCK_SHIFT, bool HAS_ZP, int KSUB>
+struct DequantSub<true, BLOCK_SHIFT, HAS_ZP, KSUB> : PackedColumn<KSUB> {
+  static constexpr int kBlocks = BLOCK_SHIFT >= 6 ? 1 : (BLOCK_K >> BLOCK_SHIFT);  // of a sub-step
+  uint32_t s[kBlocks], z[kBlocks];
+  __device__ __forceinline__ void load(const uint8_t* pk, int sub, const uint8_t* sc_tile, const uint8_t* zp_tile, int n_l) {
+    PackedColumn<KSUB>::load(pk, sub, n_l);
+    const int row0 = BLOCK_SHIFT > 6 ? 0 : sub * kBlocks;
+#pragma unroll
+    for (int b = 0; b < kBlocks; ++b) {
+      s[b] = reinterpret_cast<const unsigned short*>(sc_tile)[(row0 + b) * TILE_N + n_l];
+      z[b] = HAS_ZP ? (uint32_t)zp_tile[(row0 + b) * TILE_N + n_l] : 8u;
+    }
+  }
+  __device__ __forceinline__ void emit(const uint8_t*, const uint8_t*, int, int, uint32_t rot_lo, uint32_t rot_hi,
+                                       uint32_t (&out)[32]) const {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {  // 16-byte chunk: k in [16 c, 16 c + 16) of the sub-step
+      const int b = BLOCK_SHIFT >= 6 ? 0 : ((c * 16) >> BLOCK_SHIFT);
+      const uint32_t sc2 = s[b] | (s[b] << 16);
       // fp16(-16 - z) by bit placement (0xcc00 is -16.0, mantissa step 1/64), times the scale
-      const uint32_t nz = 0xcc00u | (z << 6);
+      const uint32_t nz = 0xcc00u | (z[b] << 6);
       const uint32_t of2 = hmul2_u32(sc2, nz | (nz << 16));
+      const uint32_t w4[4] = {this->w[c].x, this->w[c].y, this->w[c].z, this->w[c].w};
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        s_lo[r] = s_hi[r] = sc2;
-        o_lo[r] = o_hi[r] = of2;
+        // chunk c, word r: k = 16 c + 2 r (+1) -> column 8 c + r; k + 8 -> column 8 c + 4 + r
+        out[8 * c + r] = hfma2_u32(sc2, this->half16plus(w4[r], rot_lo), of2);
+        out[8 * c + 4 + r] = hfma2_u32(sc2, this->half16plus(w4[r], rot_hi), of2);
       }
-    } else {
-      // scale tile: (128 / block) rows x 64 k fp16, k permuted per 16 as
-      // 0 1 8 9 2 3 10 11 ...; zero points 0 8 1 9 2 10 3 11 ...
-      const int mr = n_l / block;
-      const uint4* sp = reinterpret_cast<const uint4*>(sc_tile + mr * 128 + c * 32);
+    }
+  }
+};
+
+// Row-wise blocks: meta tile = (128 / block) rows of the step's k, permuted per 16 as 0 1 8 9 2 3 10 11 ...
+// (scales) and 0 8 1 9 2 10 3 11 ... (zero points).
+template <int BLOCK_SHIFT, bool HAS_ZP, int KSUB>
+struct DequantSub<false, BLOCK_SHIFT, HAS_ZP, KSUB> : PackedColumn<KSUB> {
+  __device__ __forceinline__ void load(const uint8_t* pk, int sub, const uint8_t*, const uint8_t*, int n_l) {
+    PackedColumn<KSUB>::load(pk, sub, n_l);
+  }
+  __device__ __forceinline__ void emit(const uint8_t* sc_tile, const uint8_t* zp_tile, int sub, int n_l, uint32_t rot_lo,
+                                       uint32_t rot_hi, uint32_t (&out)[32]) const {
+    const int mr = n_l >> BLOCK_SHIFT;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int cc = sub * 4 + c;
+      const uint4* sp = reinterpret_cast<const uint4*>(sc_tile + mr * (128 * KSUB) + cc * 32);
       const uint4 s0 = sp[0], s1 = sp[1];
       const uint32_t sw[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
       uint4 zv = make_uint4(0x08080808u, 0x08080808u, 0x08080808u, 0x08080808u);
-      if (has_zp) zv = *reinterpret_cast<const uint4*>(zp_tile + mr * 64 + c * 16);
+      if (HAS_ZP) zv = *reinterpret_cast<const uint4*>(zp_tile + mr * (64 * KSUB) + cc * 16);
       const uint32_t zw[4] = {zv.x, zv.y, zv.z, zv.w};
+      const uint32_t w4[4] = {this->w[c].x, this->w[c].y, this->w[c].z, this->w[c].w};
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        s_lo[r] = sw[2 * r];
-        s_hi[r] = sw[2 * r + 1];
         const uint32_t nz_lo = ((zw[r] << 6) & 0x03c003c0u) | 0xcc00cc00u;  // fp16(-16 - z)
         const uint32_t nz_hi = ((zw[r] >> 2) & 0x03c003c0u) | 0xcc00cc00u;
-        o_lo[r] = hmul2_u32(sw[2 * r], nz_lo);
-        o_hi[r] = hmul2_u32(sw[2 * r + 1], nz_hi);
+        out[8 * c + r] = hfma2_u32(sw[2 * r], this->half16plus(w4[r], rot_lo), hmul2_u32(sw[2 * r], nz_lo));
+        out[8 * c + 4 + r] = hfma2_u32(sw[2 * r + 1], this->half16plus(w4[r], rot_hi), hmul2_u32(sw[2 * r + 1], nz_hi));
       }
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      // Column n0's nibbles sit at bits 0-3 / 16-19 (k = 2r, 2r+1) and 4-7 / 20-23 (k = 2r+8, 2r+9), column
-      // n0 + 8's eight bits further up; fp16(16 + q) by bit placement needs them at bits 6-9 / 22-25.  One
-      // rotation per operand does it (instead of a shift to this thread's nibbles and a second one into
-      // place): left by 6 / 2 for n0, by 30 / 26 (= right by 2 / 6) for n0 + 8; what wraps around falls
-      // outside the mask.
-      const uint32_t h_lo = (__funnelshift_l(w4[r], w4[r], rot_lo) & 0x03c003c0u) | 0x4c004c00u;
-      const uint32_t h_hi = (__funnelshift_l(w4[r], w4[r], rot_hi) & 0x03c003c0u) | 0x4c004c00u;
-      const uint32_t d_lo = hfma2_u32(s_lo[r], h_lo, o_lo[r]);
-      const uint32_t d_hi = hfma2_u32(s_hi[r], h_hi, o_hi[r]);
-      // chunk c, word r: k = 16 c + 2 r (+1) -> column 8 c + r; k + 8 -> column 8 c + 4 + r
-      out[8 * c + r] = d_lo;
-      out[8 * c + 4 + r] = d_hi;
-    }
+  }
+};
+
+// Calls fn(block shift, zero points) with both as compile-time constants.
+template <int V>
+struct IntC {
+  static constexpr int value = V;
+};
+template <typename Fn>
+__device__ __forceinline__ void with_block_shift(int block_shift, int has_zp, Fn&& fn) {
+  if (has_zp) {
+    if (block_shift == 7) fn(IntC<7>{}, IntC<1>{});
+    else if (block_shift == 6) fn(IntC<6>{}, IntC<1>{});
+    else if (block_shift == 5) fn(IntC<5>{}, IntC<1>{});
+    else fn(IntC<4>{}, IntC<1>{});
+  } else {
+    if (block_shift == 7) fn(IntC<7>{}, IntC<0>{});
+    else if (block_shift == 6) fn(IntC<6>{}, IntC<0>{});
+    else if (block_shift == 5) fn(IntC<5>{}, IntC<0>{});
+    else fn(IntC<4>{}, IntC<0>{});
   }
 }
 

@@ -161,8 +161,9 @@ size_t blkq4_gemm_workspace_size(int m, int n, int k);
  *   out6[1]  activation rows per tile        out6[2]  output tiles
  *   out6[3]  K split (1, 2 or 4)             out6[4]  1 when the tiles are cut in balanced k-step ranges
  *   out6[5]  units the balanced ranges are cut for (SMs or pairs of SMs), else 0
- * blkq4_gemm_plan_range_bound returns the first k step of unit b's range in the balanced plan's
- * (tile, k step) sequence of total_steps = tiles * (k / 64) steps (b == units: the end). */
+ * blkq4_gemm_plan_range_bound returns the first k step of unit b's range in the (tile, k step) sequence of
+ * total_steps = tiles * k_steps steps of 64 k (b == units: the end).  Tiles of up to 128 rows run in steps of
+ * 128 k: there the kernel cuts by the same rule, with a shortest part of two such steps instead of four. */
 int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* out6);
 int blkq4_gemm_plan_range_bound(int total_steps, int k_steps, int units, int b);
 int blkq4_fp16_gemm_ws_sm100(

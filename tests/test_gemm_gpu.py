@@ -296,3 +296,23 @@ def test_output_canaries_untouched():
         assert (h[:256] == 7).all() and (h[256 + M * N :] == 7).all()
         want = O.dequant_gemm(block, colwise, a, N, pw, ps, pz)
         assert (bits(h[256 : 256 + M * N].reshape(M, N)) == bits(want)).all()
+
+
+@pytest.mark.parametrize("block,colwise,has_zp", [(64, True, True), (16, True, False), (32, False, True), (128, False, False)])
+@pytest.mark.parametrize("M", [17, 64, 65, 128, 129])
+def test_half_filled_last_step(M, block, colwise, has_zp):
+    """Tiles of up to 128 rows run in steps of 128 k: K an odd multiple of 64 leaves the last step half empty
+    (zero-filled), in whole rounds, split over K (17 steps of 128 k do not split, 20 do), and a single step."""
+    import torch
+
+    from gemmlib_b200 import capi
+
+    for N, K in [(384, 2112), (256, 2496), (128, 64)]:
+        a, pw, ps, pz = kat_problem(block, colwise, has_zp, M, N, K)
+        want = O.dequant_gemm(block, colwise, a, N, pw, ps, pz)
+        nbytes = capi.gemm_workspace_size(M, N, K)
+        ws = torch.zeros(max(nbytes, 256), dtype=torch.uint8, device="cuda")
+        for workspace in (None, ws):
+            got = gpu_gemm(block, colwise, a, N, pw, ps, pz, workspace=workspace)
+            assert (bits(got) == bits(want)).all(), (M, N, K, workspace is not None)
+        assert not ws[:256].any()
