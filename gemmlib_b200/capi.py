@@ -19,6 +19,7 @@ SYMBOLS = (
     "blkq4_fp16_gemm_sm100",
     "blkq4_fp16_gemm_ws_sm100",
     "blkq4_gemm_workspace_size",
+    "blkq4_gemm_workspace_size_sm100",
     "blkq4_fp16_gemm_static_ws_sm100",
     "blkq4_static_scratch_size",
     "blkq4_fp16_quant_sm80",
@@ -64,6 +65,8 @@ def _load() -> ctypes.CDLL:
     lib.blkq4_fp16_gemm_ws_sm100.restype = i
     lib.blkq4_gemm_workspace_size.argtypes = [i, i, i]
     lib.blkq4_gemm_workspace_size.restype = sz
+    lib.blkq4_gemm_workspace_size_sm100.argtypes = [i, b, i, i, i]
+    lib.blkq4_gemm_workspace_size_sm100.restype = sz
     lib.blkq4_fp16_gemm_static_ws_sm100.argtypes = [i, b, i, i, i, vp, vp, sz, vp, sz, vp, sz, vp, sz, vp, sz, vp, sz,
                                                     ctypes.c_uint, vp]
     lib.blkq4_fp16_gemm_static_ws_sm100.restype = i

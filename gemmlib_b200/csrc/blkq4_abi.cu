@@ -162,10 +162,12 @@ extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blockin
 
   // m > 16 is the reference's own threshold between its two tile configurations
   // (src/blkq4_f16_gemm_sm80.cu:343); here it separates the HBM-bound skinny
-  // kernel from the tcgen05 tensor-core kernel.
+  // kernels from the tcgen05 tensor-core kernel, which also takes the larger skinny problems
+  // whose blocking only the generic skinny kernel covers.
   const std::string e =
-      (m <= 16) ? blkq4::launch_gemv(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, flags)
-                : blkq4::launch_gemm_tc(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, workspace,
+      (m <= 16 && !blkq4::gemm_tc_takes_skinny(block_size, column_wise_blocking, m, n, k, s, z))
+          ? blkq4::launch_gemv(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, flags)
+          : blkq4::launch_gemm_tc(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, workspace,
                                           workspace_size, flags);
   if (!e.empty()) return fail(err, "Kernel execution failed: " + e);
   return 0;
@@ -187,6 +189,11 @@ extern "C" int blkq4_fp16_gemm_sm100(int block_size, bool column_wise_blocking, 
 extern "C" size_t blkq4_gemm_workspace_size(int m, int n, int k) {
   if (m <= 0 || n <= 0 || k <= 0 || (k % 64) != 0) return 0;
   return blkq4::gemm_tc_workspace_bytes(m, n, k);
+}
+
+extern "C" size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int n, int k) {
+  if (m <= 0 || n <= 0 || k <= 0 || (k % 64) != 0 || !blkq4::supported_block(block_size)) return 0;
+  return blkq4::gemm_tc_workspace_bytes_any(block_size, column_wise_blocking, m, n, k);
 }
 
 extern "C" int blkq4_fp16_gemm_sm80(int block_size, bool column_wise_blocking, int m, int n, int k,

@@ -86,6 +86,9 @@ bool gemm_tc_gather_supported(int M, int N, int K);
 // Bytes of zero-initialised workspace with which launch_gemm_tc would split K for this problem
 // (0: it would not).
 size_t gemm_tc_workspace_bytes(int M, int N, int K);
+// True when launch_gemm_tc runs this problem of up to 16 rows instead of launch_gemv, and the workspace for any M.
+bool gemm_tc_takes_skinny(int block, bool colwise, int M, int N, int K, const void* scales, const void* zp);
+size_t gemm_tc_workspace_bytes_any(int block, bool colwise, int M, int N, int K);
 // True when the preferred plan of the problem is the balanced one (more tiles than SMs): its workspace
 // only buys balance; without it the same kernel runs in whole rounds.
 bool gemm_tc_plan_balanced(int M, int N, int K);

@@ -98,26 +98,26 @@ struct Params {
   uint32_t meta_row_bytes_s, meta_row_bytes_z;  // bytes per box row
   __half* out;
   const __half* bias;  // fp16 [N] added to the fp16 result, or null
-  // Work items.  A tile's K range may be cut in parts that different CTAs compute: every part but
-  // one leaves an fp32 partial tile in the workspace, the remaining one adds them to its own.
-  //   balanced == 0: item = (tile, part), part < split covering k_per_item steps; CTA b takes items
-  //     b, b + grid, ...; the last part of a tile adds the others.
+  // Work items.  A tile's K range may be cut in parts that different CTAs compute.
+  //   balanced == 0: item = (tile, part), part < split covering k_per_item steps (the last one what is
+  //     left).  split == 1: CTA b takes items b, b + grid, ...  split > 1: one item per CTA, the parts of a
+  //     tile form a cluster and exchange their fp32 partial tiles through distributed shared memory.
   //   balanced == 1: the (tile, k step) sequence of the whole problem is cut in one contiguous range
   //     per CTA (range_bound), so that every SM gets the same number of steps whatever the tile
   //     count; a tile that straddles two ranges has its tail computed FIRST by the later CTA
   //     (partial tile, slot = that CTA) and its head LAST by the earlier CTA, which adds the partial.
-  int split_shift;     // log2(split), split in {1, 2, 4}
+  int split;
   int k_per_item;      // 64-k steps per work item
-  int num_items;       // tiles << split_shift
+  int num_items;       // tiles * split
   int balanced;
   int k_steps;         // steps of a tile: K / 64, or / 128 rounded up for tiles of up to 128 rows
   int min_part;        // one-CTA kernel: range_bound's minimum in steps
   int total_steps;     // tiles * k_steps
-  float* ws_partials;  // balanced: [cta][BM][128] fp32; otherwise [tile][split-1][BM][128]
+  float* ws_partials;  // balanced: [cta][BM][128] fp32
   int gather_bulk;         // pair kernel, gather mode: peer copies as cp.async.bulk of whole rows
   int n_fastest, n_pairs;  // pair kernel: tile order (0: the m tiles of a pair of weight columns run together; 1: the column pairs of an m tile)
   GatherTable gt;      // pair kernel, gt.world > 0: the result goes to every rank's gathered buffer instead of `out`
-  unsigned* ws_flags;  // balanced: [cta]; otherwise [tile]: arrivals (self-resetting)
+  unsigned* ws_flags;  // balanced: [cta]: arrivals (self-resetting)
 };
 
 // ---- PTX wrappers ---------------------------------------------------------------------------
@@ -142,8 +142,8 @@ __host__ __device__ inline int range_bound(int total_steps, int k_steps, int gri
 
 struct Item {
   int tile, ks0, count;
-  int role;    // 0: whole tile; 1: writes its partial tile to `slot`; 2: adds `nparts` partial tiles from `slot` on
-  int slot, flag, nparts;
+  int role;    // 0: whole tile; 1: writes its partial tile to `slot`; 2: adds the partial tile in `slot`; 3: part of a cluster's tile
+  int slot;
 };
 struct ItemCursor {
   int pos, end;  // balanced: steps of the range still to do; otherwise: next item index, item count
@@ -168,19 +168,16 @@ __device__ __forceinline__ bool next_item(const Params& p, ItemCursor& c, Item& 
     // a range is longer than a tile, so a cut tile has exactly two parts: its tail opens the later
     // CTA's range, its head closes the earlier one's
     it.role = it.ks0 > 0 ? 1 : (it.count < p.k_steps ? 2 : 0);
-    it.slot = it.flag = (int)blockIdx.x + (it.role == 2 ? 1 : 0);
-    it.nparts = 1;
+    it.slot = (int)blockIdx.x + (it.role == 2 ? 1 : 0);
     c.pos += it.count;
   } else {
-    const int split = 1 << p.split_shift;
-    it.tile = c.pos >> p.split_shift;
-    const int part = c.pos - (it.tile << p.split_shift);
+    const int split = p.split;
+    it.tile = c.pos / split;
+    const int part = c.pos - it.tile * split;
     it.ks0 = part * p.k_per_item;
-    it.count = p.k_per_item;
-    it.role = split == 1 ? 0 : (part < split - 1 ? 1 : 2);
-    it.slot = it.tile * (split - 1) + (it.role == 1 ? part : 0);
-    it.flag = it.tile;
-    it.nparts = split - 1;
+    it.count = min(p.k_per_item, p.k_steps - it.ks0);
+    it.role = split == 1 ? 0 : 3;
+    it.slot = 0;
     c.pos += (int)gridDim.x;
   }
   return true;
@@ -390,7 +387,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     if (++ab == (uint32_t)p.acc_bufs) { ab = 0; par_acc ^= 1u; }                                                    \
   }
       if (!p.balanced) {
-        for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++tcount) BLKQ4_TC_MMA_ITEM(p.k_per_item)
+        for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++tcount) {
+          const int count = min(p.k_per_item, p.k_steps - item % p.split * p.k_per_item);
+          BLKQ4_TC_MMA_ITEM(count)
+        }
       } else {
         int pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x, p.min_part);
         const int end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1, p.min_part);
@@ -427,6 +427,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         tmem_ld_wait();
       };
       const int n_l = quarter * 32 + lane;
+      if (item.role == 3) break;  // this CTA's only item: the cluster adds its parts up after the role branches
       if (item.role == 1) {
         // ---- a part that hands over: fp32 partial tile [m][n] to the workspace: for a row m
         //      the 32 lanes of a warp write 128 contiguous bytes.  (One line per lane, [n][m] with
@@ -445,16 +446,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(bar(BAR_ACC_EMPTY + ab));
-          atomicAdd(p.ws_flags + item.flag, 1u);
+          atomicAdd(p.ws_flags + item.slot, 1u);
         }
         continue;
       }
       if (item.role == 2) {
-        // ---- the part that finishes the tile: wait (bounded) for the other parts' partial tiles ----
+        // ---- the part that finishes the tile: wait (bounded) for the other part's partial tile ----
         if (lane == 0) {
-          const unsigned want = (unsigned)(item.nparts * kNumEpiWarps);
+          const unsigned want = (unsigned)kNumEpiWarps;
           const long long t0 = clock64();
-          while (*reinterpret_cast<volatile unsigned*>(p.ws_flags + item.flag) < want) {
+          while (*reinterpret_cast<volatile unsigned*>(p.ws_flags + item.slot) < want) {
             if (*abort_flag || clock64() - t0 > kWaitCycles) {
               *abort_flag = 1;
               atomicCAS(&g_gemm_tc_error, 0, 0x320 | quarter);
@@ -479,15 +480,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         uint32_t r[32];
         load_acc(c0, r);
         if (item.role == 2) {
-          // add the other parts in part order (a fixed order: the result is reproducible)
-          for (int q = 0; q < item.nparts; ++q) {
-            const float* sq = src_ws + (size_t)q * tile_floats + (size_t)c0 * TILE_N;
-            float f[32];
+          const float* sq = src_ws + (size_t)c0 * TILE_N;
+          float f[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) f[j] = (m0 + c0 + j < p.M) ? __ldcg(sq + (size_t)j * TILE_N) : 0.0f;
+          for (int j = 0; j < 32; ++j) f[j] = (m0 + c0 + j < p.M) ? __ldcg(sq + (size_t)j * TILE_N) : 0.0f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + f[j]);
-          }
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + f[j]);
         }
         int m = m0 + c0 + odd;
         __half* dst = p.out + (size_t)m * p.N + (n & ~1);
@@ -513,8 +511,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       if (lane == 0) {
         mbar_arrive(bar(BAR_ACC_EMPTY + ab));
         // the warp that completes the tile's count puts the flag back to zero for the next launch
-        if (item.role == 2 && atomicAdd(p.ws_flags + item.flag, 1u) == (unsigned)((item.nparts + 1) * kNumEpiWarps - 1))
-          p.ws_flags[item.flag] = 0u;
+        if (item.role == 2 && atomicAdd(p.ws_flags + item.slot, 1u) == (unsigned)(2 * kNumEpiWarps - 1))
+          p.ws_flags[item.slot] = 0u;
       }
     }
   } else if (warp < S::kWeightProducerWarp) {
@@ -570,6 +568,66 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     });
   }
 
+  if (p.split > 1) {
+    // ---- split K: the cluster's CTAs hold one fp32 partial tile each.  Part q owns rows [q slice, (q + 1) slice): every
+    //      CTA stores the other parts' rows of its partial tile into THEIR shared memory (over the activation
+    //      ring, idle once the MMAs of all parts have retired) and then adds up its own rows, in part order, with
+    //      all its threads.  With the partial tiles in global memory and one finishing CTA, which read them chunk by
+    //      chunk from L2 (one round trip per 32 rows and part), more parts cost more than they gave; 4096 x 4096,
+    //      us: M = 128, four parts 16.7 -> 11.0; M = 256, four parts 28.0 -> 15.7; M = 512, two parts 24.9 -> 20.9;
+    //      K = 4096, N = 1024, M = 128: four parts through memory 15.4, eight 21.7, eight in a cluster 8.2.
+    //      A cluster's CTAs are co-resident by construction, so nobody waits for a CTA that is not running.
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // all warps store to the output
+    __syncwarp();
+    cluster_sync_all();  // every part's epilogue warps have seen their accumulator complete
+    tc_fence_after();
+    const int split = p.split, part = (int)blockIdx.x % split, tile = (int)blockIdx.x / split;
+    const int n_tile = tile / p.m_tiles, m0 = (tile % p.m_tiles) * p.BM;
+    const int rows = min(p.BM, p.M - m0);
+    const int slice = 2 * ((p.BM + 2 * split - 1) / (2 * split));
+    const uint32_t region = base + plan.act;  // [part][slice][128] fp32
+    if (warp >= 2 && warp < S::kWeightProducerWarp) {
+      // a warp may read the TMEM lanes of its quarter: the epilogue and dequantizer warps share the columns
+      const int n_l = 32 * (warp & 3) + lane;
+      const uint32_t lane_base = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
+      for (int c0 = 32 * ((warp - 2) >> 2); c0 < rows; c0 += 32 * (S::NG + 1)) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(lane_base + (uint32_t)c0, v);
+        tmem_ld_wait();
+        int owner = c0 / slice, rr = c0 - owner * slice;
+        uint32_t dst = map_to_cta(region + (uint32_t)(((part * slice + rr) * TILE_N + n_l) * 4), (uint32_t)owner);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (c0 + j < rows) {
+            st_shared_cluster_f32(dst, v[j]);
+            dst += TILE_N * 4;
+            if (++rr == slice) {
+              rr = 0;
+              if (++owner < split) dst = map_to_cta(region + (uint32_t)((part * slice * TILE_N + n_l) * 4), (uint32_t)owner);
+            }
+          }
+        }
+      }
+    }
+    cluster_sync_all();
+    const int r0 = part * slice, mine = min(slice, rows - r0);
+    const float* src = reinterpret_cast<const float*>(base_ptr + plan.act);
+    for (int idx = threadIdx.x; idx < mine * (TILE_N / 2); idx += S::kThreads) {
+      const int rr = idx / (TILE_N / 2), n2 = 2 * (idx % (TILE_N / 2)), n = n_tile * TILE_N + n2;
+      if (n >= p.N) continue;
+      float2 sum = make_float2(0.0f, 0.0f);
+      for (int q = 0; q < split; ++q) {
+        const float2 f = *reinterpret_cast<const float2*>(src + (size_t)(q * slice + rr) * TILE_N + n2);
+        sum.x += f.x;
+        sum.y += f.y;
+      }
+      __half2 v = __floats2half2_rn(sum.x, sum.y);
+      // the bias is added to the rounded result in fp16, as above
+      if (p.bias) v = __hadd2(v, *reinterpret_cast<const __half2*>(p.bias + n));
+      *reinterpret_cast<__half2*>(p.out + (size_t)(m0 + r0 + rr) * p.N + n) = v;
+    }
+  }
+
   // ---- teardown ----
   tc_fence_before();
   __syncthreads();
@@ -590,13 +648,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
 
 namespace {
 
+constexpr int kMaxSplit = 8;  // parts of a tile: the portable cluster size
+
 // Work plan.  The kernel is persistent with one CTA per SM.  A problem with few output tiles
 // (prefill of a 4096-wide layer at M = 512: 64 tiles on 148 SMs) leaves SMs idle: cutting every
 // tile's K range in `split` work items fills them.  A problem with more tiles than SMs but not a
 // whole number of rounds (256 tiles: the second round keeps 108 of 148 SMs busy) is cut in one
 // contiguous range of k steps per CTA instead ("balanced", see Params).
 struct SplitPlan {
-  int split_shift;
+  int split, k_per_item;  // k_per_item steps per part, the last part what is left
   int balanced;
   size_t flags_bytes, total_bytes;  // workspace: [flags, 256-byte aligned][partials]
 };
@@ -606,7 +666,7 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   const int tiles = ((M + BM - 1) / BM) * ((N + TILE_N - 1) / TILE_N);
   const int k_steps = (K + step_k(BM) - 1) / step_k(BM);
   const int sms = sm_count() > 0 ? sm_count() : 148;
-  SplitPlan best{0, 0, 0, 0};
+  SplitPlan best{1, k_steps, 0, 0, 0};
   if (tiles > sms) {
     // balanced ranges: every range longer than a tile (a cut tile then has exactly two parts), and
     // only when whole rounds would leave more than a fifth of the SM time idle.  Measured on B200:
@@ -620,19 +680,38 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
         (double)tiles < 0.80 * rounds * sms) {
       const size_t flags = ((size_t)sms * sizeof(unsigned) + 255) & ~(size_t)255;
       const size_t total = flags + (size_t)sms * BM * TILE_N * sizeof(float);
-      if (total <= ws_bytes_available) best = SplitPlan{0, 1, flags, total};
+      if (total <= ws_bytes_available) best = SplitPlan{1, k_steps, 1, flags, total};
     }
     return best;
   }
-  // Split only when every work item still gets an SM of its own (one round): measured on B200 a
-  // second round of half-size items loses more to the fp32 exchange than it gains in balance.
-  for (int shift = 1; shift <= 2; ++shift) {
-    const int split = 1 << shift;
-    if (k_steps % split != 0 || (k_steps / split) * step_k(BM) < 512 || tiles * split > sms) continue;
-    const size_t flags = ((size_t)tiles * sizeof(unsigned) + 255) & ~(size_t)255;
-    const size_t total = flags + (size_t)tiles * (split - 1) * BM * TILE_N * sizeof(float);
-    if (total > ws_bytes_available) continue;
-    best = SplitPlan{shift, 0, flags, total};
+  // Split only when every work item still gets an SM of its own (one round).  The parts exchange their partial tiles
+  // through distributed shared memory, so they may be uneven and as many (of at least 512 k) as there are SMs for.
+  // The workspace stays the caller's opt-in (a split changes the order of the fp32 sums), of the size it has always
+  // been: that of the fp32 partial tiles of an even two- or four-way split, or one page of flags where K does not
+  // divide evenly.  A smaller one gets the split it would hold.  Up to 16 rows no opt-in is asked for: those
+  // calls never needed one.
+  auto even_split = [&](size_t avail, size_t* bytes) {
+    int split = 1;
+    *bytes = 0;
+    for (int parts = 2; parts <= 4; parts *= 2) {
+      const size_t flags = ((size_t)tiles * sizeof(unsigned) + 255) & ~(size_t)255;
+      const size_t total = flags + (size_t)tiles * (parts - 1) * BM * TILE_N * sizeof(float);
+      if (k_steps % parts != 0 || (k_steps / parts) * step_k(BM) < 512 || tiles * parts > sms || total > avail) continue;
+      split = parts;
+      *bytes = total;
+    }
+    return split;
+  };
+  size_t bytes = 0, all_bytes = 0;
+  const int fits = even_split(ws_bytes_available, &bytes), wanted = even_split(~(size_t)0, &all_bytes);
+  const bool free_split = M <= 16;
+  if (!free_split && fits < wanted) return SplitPlan{fits, k_steps / fits, 0, 0, bytes};
+  if (!free_split && ws_bytes_available < 256) return best;
+  for (int parts = 2; parts <= kMaxSplit; ++parts) {
+    const int per = (k_steps + parts - 1) / parts;
+    const int split = (k_steps + per - 1) / per;  // no empty part
+    if (split == 1 || per * step_k(BM) < 512 || tiles * split > sms) continue;
+    best = SplitPlan{split, per, 0, 0, free_split ? 0 : bytes ? bytes : 256};
   }
   return best;
 }
@@ -698,6 +777,31 @@ size_t gemm_tc_workspace_bytes(int M, int N, int K) {
   const PairPlan pp = plan_pair(M, N, K, ~(size_t)0);
   if (pp.use) return pp.total_bytes;
   return plan_split(M, N, K, ~(size_t)0).total_bytes;
+}
+
+// Which problems of up to 16 rows run here rather than on the generic skinny kernel (blkq4_gemv.cu): both convert
+// the weights to fp16 by the same formula and sum in fp32.  Only those whose blocking no other skinny kernel takes
+// (row-wise, or blocks of 16 and 32): the others scale fp32 sums instead, which is more accurate.
+// The generic kernel splits K over the eight warps of a CTA and streams its weights through registers; it is good for
+// about 1.6 TB/s and a short launch.  Measured on B200, generic against this one, us, block 32 column-wise with
+// zero points (row-wise):
+//   M = 8:  1024 x 4096 3.8 / 5.3 (4.4 / 5.4);  2048 x 8192 8.1 / 8.3 (9.6 / 9.8);  4096 x 4096 7.3 / 8.5 (8.8 / 10.1);
+//           4096 x 8192 13.1 / 11.3 (15.6 / 14.1);  4096 x 11008 18.4 / 13.7 (20.9 / 18.8);  11008 x 512 13.3 / 7.1
+//           (16.7 / 8.5);  8192 x 28672 75.3 / 42.0 (86.0 / 57.9)
+//   M = 16: 512 x 2048 5.5 / 3.4 (5.4 / 3.5);  1024 x 4096 5.6 / 5.4 (5.3 / 5.5);  2048 x 8192 7.8 / 8.5 (8.2 / 9.9);
+//           4096 x 4096 10.5 / 8.7 (11.0 / 10.4);  4096 x 8192 12.8 / 11.5 (13.3 / 14.2);  4096 x 11008 21.6 / 13.8
+//           (23.7 / 18.8);  11008 x 2048 24.9 / 10.8 (25.8 / 13.4);  8192 x 28672 79.2 / 42.3 (84.3 / 58.4)
+bool gemm_tc_takes_skinny(int block, bool colwise, int M, int N, int K, const void* scales, const void* zp) {
+  if (M > 16 || (colwise && block >= 64)) return false;
+  if (reinterpret_cast<uintptr_t>(scales) % 16 != 0 || reinterpret_cast<uintptr_t>(zp) % 16 != 0) return false;
+  const long long kn = (long long)K * N;
+  if (M <= 8) return K >= 8192 || kn >= (1ll << 25);
+  return !(N >= 8192 && K >= 2048 && kn <= (colwise ? 1ll << 24 : 1ll << 25));
+}
+
+size_t gemm_tc_workspace_bytes_any(int block, bool colwise, int M, int N, int K) {
+  if (M > 16) return gemm_tc_workspace_bytes(M, N, K);
+  return gemm_tc_takes_skinny(block, colwise, M, N, K, nullptr, nullptr) ? plan_split(M, N, K, ~(size_t)0).total_bytes : 0;
 }
 
 bool gemm_tc_split_plan_refusable(int M, int N, int K, size_t capacity) {
@@ -836,21 +940,20 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     return std::string();
   }
   const int num_tiles = p.m_tiles * p.n_tiles;
-  const SplitPlan sp = ws_ok ? plan_split(M, N, K, workspace_bytes) : SplitPlan{0, 0, 0, 0};
-  p.split_shift = sp.split_shift;
+  const SplitPlan sp = plan_split(M, N, K, ws_ok ? workspace_bytes : 0);
+  p.split = sp.split;  // split > 1: at most one item per SM
   p.k_steps = (K + sk - 1) / sk;
-  p.k_per_item = p.k_steps >> sp.split_shift;
+  p.k_per_item = sp.k_per_item;
   p.min_part = min_part(sk);
-  p.num_items = num_tiles << sp.split_shift;
   p.balanced = sp.balanced;
   p.total_steps = sp.balanced ? num_tiles * p.k_steps : 0;
   p.ws_flags = reinterpret_cast<unsigned*>(workspace);
   p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + sp.flags_bytes);
-  const int grid = p.num_items < sms ? p.num_items : sms;
   using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params);
   static std::atomic<int> granted[6][64];
   Kern kern;
   int threads, which;
+  size_t max_smem;
   SmemPlan plan;
   auto pick = [&](auto shape, int idx) {
     using S = decltype(shape);
@@ -858,6 +961,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     threads = S::kThreads;
     which = 2 * idx + (colwise ? 1 : 0);
     plan = make_plan(p.BM, S::WS, S::ACT, S::KSUB);
+    max_smem = make_plan(idx == 0 ? 64 : idx == 1 ? 128 : 256, S::WS, S::ACT, S::KSUB).total;
   };
   if (p.BM <= 64) pick(ShapeSmall{}, 0);
   else if (p.BM <= 128) pick(ShapeMid{}, 1);
@@ -865,16 +969,45 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[which]);
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = plan.total;
   cfg.stream = stream;
   // BLKQ4_GEMM_EARLY_WEIGHT_FETCH: programmatic stream serialization, see the kernel's entry
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  while (p.split > 1) {
+    // all clusters in one round, or fewer parts: an SM group holds whole clusters only
+    attr[0].val.clusterDim.x = (unsigned)p.split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(num_tiles * p.split);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    static std::atomic<int> fit[6][kMaxSplit + 1][64];  // clusters of this size that are resident at once
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool cached = dev >= 0 && dev < 64;
+    int n = cached ? fit[which][p.split][dev].load(std::memory_order_relaxed) : 0;
+    if (n <= 0) {
+      // asked with the largest shared-memory plan of the kernel, so that the answer holds for every BM
+      cfg.dynamicSmemBytes = max_smem;
+      e = ensure_dynamic_smem(kern, max_smem, granted[which]);
+      if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 0) {
+        cudaGetLastError();
+        n = 0;
+      }
+      cfg.dynamicSmemBytes = plan.total;
+      if (cached && n > 0) fit[which][p.split][dev].store(n, std::memory_order_relaxed);
+    }
+    if (n >= num_tiles) break;
+    p.k_per_item = (p.k_steps + p.split - 2) / (p.split - 1);
+    p.split = (p.k_steps + p.k_per_item - 1) / p.k_per_item;
+  }
+  p.num_items = num_tiles * p.split;
+  cfg.gridDim = dim3(p.num_items < sms ? p.num_items : sms);
+  cfg.attrs = p.split > 1 ? attr : attr + 1;
+  cfg.numAttrs = (p.split > 1 ? 1 : 0) + ((flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) ? 1 : 0);
   e = cudaLaunchKernelEx(&cfg, kern, tm_act, tm_pack, tm_scale, tm_zp, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
@@ -910,7 +1043,7 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
   const blkq4::SplitPlan sp = blkq4::plan_split(m, n, k, workspace_size);
   const int bm = m >= 256 ? 256 : ((m + 15) / 16) * 16;
   out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
-  out6[3] = 1 << sp.split_shift; out6[4] = sp.balanced; out6[5] = sp.balanced ? sms : 0;
+  out6[3] = sp.split; out6[4] = sp.balanced; out6[5] = sp.balanced ? sms : 0;
   return 0;
 }
 

@@ -50,21 +50,6 @@ constexpr int kPairDoneBars = (kPairActStages > kDeqStages ? kPairActStages : kD
 static_assert(kPairActStages == kDeqStages, "one barrier per step serves both rings");
 static_assert(kDeqStages % kPairCommitSteps == 0, "rings are released per commit group");
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of `local_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
 // Arrival on a barrier of the peer CTA.  What it publishes lives in tensor memory and is ordered by
 // tcgen05.wait::st / tcgen05.fence::before_thread_sync, so the arrive carries no cluster-scope release
 // (measured: with .release.cluster the peer's dequantizer warps took 2.7x as long per step).

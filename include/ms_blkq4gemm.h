@@ -142,24 +142,30 @@ int blkq4_fp16_gemm_sm100(
  * blkq4_gemm_workspace_size(m, n, k) bytes, 256-byte aligned, ZERO-INITIALISED once (the kernel
  * leaves it zeroed), used by one call at a time (calls on one stream may share it).  With it the
  * tensor-core kernel splits K when the output has too few 128 x 256 tiles to fill the GPU's SMs
- * (e.g. M = 512, N = 4096: 64 tiles on 148 SMs): parts of a tile's K range run on different SMs,
- * leave fp32 partial tiles in the workspace and the last part adds them in a fixed order.  With
+ * (e.g. M = 512, N = 4096: 64 tiles on 148 SMs): parts of a tile's K range run on different SMs
+ * of a cluster, which exchange fp32 partial tiles through distributed shared memory and add them in a fixed order
+ * (the workspace is the caller's opt-in to that order of sums; up to 16 rows none is needed).  With
  * more tiles than SMs (or than pairs of SMs, for m >= 256) but far from a whole number of rounds
  * (e.g. 224 tiles on 148 SMs) it cuts the tiles' k steps in one balanced range per SM (or pair)
- * instead, and a tile that straddles two ranges is finished through an fp32 partial tile in the same
- * way.  Results are reproducible run to run with the same workspace size.  A null or too small
+ * instead, and a tile that straddles two ranges is finished through an fp32 partial tile in the
+ * workspace.  Results are reproducible run to run with the same workspace size.  A null or too small
  * workspace, or a size query of 0, means the call runs exactly as blkq4_fp16_gemm_sm100.  No counterpart in the reference (its split-K template parameters
  * are unused, src/mickey/blk_q4/f16_gemm_sm80.h:86-90).
  */
 size_t blkq4_gemm_workspace_size(int m, int n, int k);
 
+/* No counterpart in the reference.  The same with the blocking, which decides for m <= 16 whether the tensor-core
+ * kernel takes the problem (row-wise blocks, or blocks of 16 and 32, at the larger sizes) and would cut it in
+ * balanced ranges; for m > 16 equal to blkq4_gemm_workspace_size. */
+size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int n, int k);
+
 /* No counterpart in the reference.  Host-only description of the work plan blkq4_fp16_gemm_ws_sm100 would
  * choose for the problem with a workspace of `workspace_size` bytes: nothing is launched and no device is
  * needed (the plan depends on the current device's SM count; 148 is assumed without a device).
- *   out6[0]  kernel: 0 = skinny kernels (m <= 16), 1 = tensor-core kernel with one CTA per tile,
+ *   out6[0]  kernel: 0 = m <= 16 (skinny kernels; some blockings and sizes run on kernel 1), 1 = tensor-core kernel with one CTA per tile,
  *            2 = tensor-core kernel with CTA pairs
  *   out6[1]  activation rows per tile        out6[2]  output tiles
- *   out6[3]  K split (1, 2 or 4)             out6[4]  1 when the tiles are cut in balanced k-step ranges
+ *   out6[3]  K split (1 .. 8)                out6[4]  1 when the tiles are cut in balanced k-step ranges
  *   out6[5]  units the balanced ranges are cut for (SMs or pairs of SMs), else 0
  * blkq4_gemm_plan_range_bound returns the first k step of unit b's range in the (tile, k step) sequence of
  * total_steps = tiles * k_steps steps of 64 k (b == units: the end).  Tiles of up to 128 rows run in steps of

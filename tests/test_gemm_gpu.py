@@ -316,3 +316,50 @@ def test_half_filled_last_step(M, block, colwise, has_zp):
             got = gpu_gemm(block, colwise, a, N, pw, ps, pz, workspace=workspace)
             assert (bits(got) == bits(want)).all(), (M, N, K, workspace is not None)
         assert not ws[:256].any()
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("block,colwise,has_zp,N,K", [
+    (32, True, True, 544, 192), (16, True, False, 96, 2112),       # one part; uneven parts of a cluster
+    (32, False, True, 2080, 1088), (128, False, False, 256, 4096),  # two parts; eight
+    (16, True, True, 4192, 8256), (64, False, True, 320, 8256),    # K from where up to 8 rows move
+    (32, True, False, 19200, 1792)])                               # more tiles than SMs
+def test_skinny_problems_on_the_tensor_core_kernel(M, block, colwise, has_zp, N, K):
+    """Up to 16 rows, blockings of the generic skinny kernel: the larger problems run on the tensor-core kernel.
+    Both sides of the rule, with and without a workspace, and with scales that are not 16-byte aligned (those
+    stay on the generic kernel), against the same bars."""
+    from gemmlib_b200 import capi
+
+    for ws in (None, torch.zeros(16 << 20, dtype=torch.uint8, device="cuda")):
+        check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
+        assert ws is None or not ws[:512].any()
+    if not colwise:
+        return  # the generic kernel reads row-wise meta 16 bytes at a time
+    w = gaussian_weight(N, K, seed=1)
+    a = gaussian_act(M, K, seed=2).cuda()
+    pw, ps, pz = (to_cuda(t) for t in O.quant_prepack(block, colwise, w.numpy(), has_zp))
+    off = torch.empty(ps.numel() + 8, dtype=torch.float16, device="cuda")
+    off[4:4 + ps.numel()] = ps
+    outs = []
+    for s in (ps, off[4:4 + ps.numel()]):
+        out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        capi.gemm(block, colwise, M, N, K, a, pw, s, pz, out)
+        outs.append(out.float())
+    # the two kernels convert alike and differ by the order of fp32 sums: an fp16 rounding apart
+    assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -10 * outs[0].abs().max()
+
+
+@pytest.mark.parametrize("case", [(32, False, True, 333, 2080, 4032), (64, True, True, 200, 640, 4160),
+                                  (16, True, False, 256, 512, 8256), (128, True, False, 100, 288, 8064)],
+                         ids=lambda c: "-".join(map(str, c)))
+def test_uneven_split(case):
+    """K ranges that do not divide evenly among the CTAs of a cluster."""
+    from gemmlib_b200 import capi
+
+    block, colwise, has_zp, M, N, K = case
+    need = capi.gemm_workspace_size(M, N, K)
+    assert need > 0 and capi.gemm_plan(M, N, K, need)["split"] > 1
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
+    assert not ws.any()
+    assert capi.gemm_plan(M, N, K, 0)["split"] == 1
