@@ -59,10 +59,10 @@ std::vector<torch::Tensor> blkq4linear_quant(int block_size, bool col_wise, bool
 }
 
 torch::Tensor blkq4linear_forward_out(int block_size, bool col_wise, int in_features, int out_features,
-                                      torch::Tensor input, torch::Tensor q_weights, torch::Tensor q_scales,
-                                      torch::Tensor q_zp, torch::Tensor output,
-                                      c10::optional<torch::Tensor> bias, int64_t flags,
-                                      c10::optional<torch::Tensor> workspace) {
+                                      const torch::Tensor& input, const torch::Tensor& q_weights,
+                                      const torch::Tensor& q_scales, const torch::Tensor& q_zp,
+                                      const torch::Tensor& output, const c10::optional<torch::Tensor>& bias,
+                                      int64_t flags, const c10::optional<torch::Tensor>& workspace) {
   TORCH_CHECK(input.scalar_type() == torch::kFloat16, "blkq4linear_forward only supports float16 inputs");
   TORCH_CHECK(input.dim() == 2 && input.size(1) == in_features,
               "Activation shape is not compatible with the weights");
@@ -113,6 +113,29 @@ torch::Tensor blkq4linear_forward(int block_size, bool col_wise, int in_features
                                  q_zp, output, c10::nullopt, 0, c10::nullopt);
 }
 
+// The whole of BlkQ4Linear.forward but a bias that cannot be fused: leading dimensions flattened, the output
+// allocated unless the caller brought one, the launch, the leading dimensions restored.  In one call because at
+// decode sizes the Python calls around the launch took longer than the kernel.
+torch::Tensor blkq4linear_linear(int block_size, bool col_wise, int in_features, int out_features,
+                                 const torch::Tensor& input, const torch::Tensor& q_weights,
+                                 const torch::Tensor& q_scales, const torch::Tensor& q_zp,
+                                 const c10::optional<torch::Tensor>& bias, int64_t flags,
+                                 const c10::optional<torch::Tensor>& workspace,
+                                 const c10::optional<torch::Tensor>& out) {
+  const bool flat = input.dim() == 2 && input.size(1) == in_features && input.is_contiguous();
+  const torch::Tensor x = flat ? input : input.reshape({-1, in_features});
+  torch::Tensor output =
+      out.has_value() ? out->view({-1, out_features})
+                      : torch::empty({x.size(0), out_features},
+                                     torch::TensorOptions().dtype(torch::kFloat16).device(x.device()));
+  blkq4linear_forward_out(block_size, col_wise, in_features, out_features, x, q_weights, q_scales, q_zp, output, bias,
+                          flags, workspace);
+  if (flat && !out.has_value()) return output;
+  auto shape = input.sizes().vec();
+  shape.back() = out_features;
+  return output.view(shape);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -122,6 +145,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("block_size"), py::arg("col_wise"), py::arg("in_features"), py::arg("out_features"),
         py::arg("input"), py::arg("q_weights"), py::arg("q_scales"), py::arg("q_zp"), py::arg("output"),
         py::arg("bias") = py::none(), py::arg("flags") = 0, py::arg("workspace") = py::none());
+  m.def("linear", &blkq4linear_linear, "BlkQ4Linear.forward: any leading dimensions, the output allocated unless given",
+        py::arg("block_size"), py::arg("col_wise"), py::arg("in_features"), py::arg("out_features"),
+        py::arg("input"), py::arg("q_weights"), py::arg("q_scales"), py::arg("q_zp"), py::arg("bias"), py::arg("flags"),
+        py::arg("workspace"), py::arg("out"));
+  m.def("gemm_workspace_size_blocked",
+        [](int block, bool col_wise, int m_, int n_, int k_) {
+          return int64_t(blkq4_gemm_workspace_size_sm100(block, col_wise, m_, n_, k_));
+        },
+        "gemm_workspace_size with the blocking, for any row count");
   m.def("gemm_workspace_size", [](int m_, int n_, int k_) { return int64_t(blkq4_gemm_workspace_size(m_, n_, k_)); },
         "Bytes of zeroed workspace with which the tensor-core kernel splits K (0: it does not)");
   m.attr("EARLY_WEIGHT_FETCH") = int(BLKQ4_GEMM_EARLY_WEIGHT_FETCH);

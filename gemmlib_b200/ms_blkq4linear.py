@@ -25,6 +25,9 @@ from torch import nn
 
 from . import ms_blkq4linear_ext
 
+_EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
+_linear = ms_blkq4linear_ext.linear
+_workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
 # Split-K workspaces: one zero-initialised buffer per (device, stream), shared by all layers (calls
 # on one stream run one at a time; the kernel leaves the buffer's flags zeroed).  Grown on demand.
@@ -94,25 +97,30 @@ class BlkQ4Linear(nn.Module):
         return None
 
     def forward(self, input, out=None):
-        lead = input.shape[:-1]
-        x = input.reshape(-1, self.in_features)
-        if out is None:
-            output = torch.empty(x.size(0), self.out_features, dtype=torch.float16, device=x.device)
-        else:
-            output = out.view(-1, self.out_features)
-        fused = self._fusable_bias(x)
-        flags = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH if (self.early_weight_fetch and self._settled) else 0
+        # Few and plain lookups: at decode sizes the host's time per call is what a caller sees.
+        block, col_wise, K, N = self.block_size, self.col_wise, self.in_features, self.out_features
+        bias = self.bias
+        fused = None if bias is None else self._fusable_bias(input)
+        settled = self._settled
+        flags = _EARLY if (settled and self.early_weight_fetch) else 0
         ws = None
-        if x.size(0) > 16 and self.split_k:
-            ws = split_k_workspace(x.device, ms_blkq4linear_ext.gemm_workspace_size(
-                x.size(0), self.out_features, self.in_features))
-        ms_blkq4linear_ext.forward_out(
-            self.block_size, self.col_wise, self.in_features, self.out_features,
-            x, self.q_weights, self.q_scales, self.q_zp, output, fused, flags, ws)
-        self._settled = True
-        if self.bias is not None and fused is None:
-            output += self.bias
-        return output.view(*lead, self.out_features)
+        if self.split_k:
+            rows = input.numel() // K
+            if rows > 16 or block < 64 or not col_wise:  # the others never use one
+                need = _workspace_size(block, col_wise, rows, N, K)
+                if need > 0:
+                    ws = split_k_workspace(input.device, need)
+        buf = self._buffers
+        if "q_weights" in buf and "q_scales" in buf and "q_zp" in buf:
+            packed = buf["q_weights"], buf["q_scales"], buf["q_zp"]
+        else:  # replaced on the module by something other than a buffer
+            packed = self.q_weights, self.q_scales, self.q_zp
+        output = _linear(block, col_wise, K, N, input, *packed, fused, flags, ws, out)
+        if not settled:
+            self._settled = True
+        if bias is not None and fused is None:
+            output += bias
+        return output
 
     def extra_repr(self):
         return (f"in_features={self.in_features}, out_features={self.out_features}, block_size={self.block_size}, "

@@ -138,3 +138,39 @@ def test_linear_stack_graph_replay_matches_eager():
         assert torch.equal(got.view(torch.int16), got2.view(torch.int16))
         want = bufs["h0"]
         assert torch.allclose(got.float(), want.float(), rtol=0, atol=2.0 ** -7 * max(1.0, float(want.abs().max())))
+
+
+@pytest.mark.parametrize("M", [1, 16, 24])
+def test_forward_takes_every_input_form(M):
+    """One native call does the flattening, the allocation and the view: strided and batched inputs,
+    a caller's output, a bias that cannot be fused, and a packed tensor that is no longer a buffer."""
+    from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
+
+    K, N = 256, 160
+    w = gaussian_weight(N, K, seed=4).cuda()
+    m = BlkQ4Linear(32, True, False, w)
+    x = gaussian_act(M, K, seed=5).cuda()
+    want = m(x)
+    assert want.shape == (M, N) and not want.requires_grad
+    strided = torch.empty(M, 2 * K, dtype=torch.float16, device="cuda")[:, ::2].copy_(x)
+    with pytest.raises(RuntimeError, match="contiguous"):  # two dimensions: taken as they are
+        m(strided)
+    turned = torch.stack([x, x]).transpose(0, 1)  # [M, 2, K], strided: flattening copies
+    assert torch.equal(m(turned), torch.stack([want, want]).transpose(0, 1))
+    assert torch.equal(m(x.view(1, M, 1, K)), want.view(1, M, 1, N))
+    if M == 1:
+        assert torch.equal(m(x.view(K)), want.view(N))
+    out = torch.zeros(M, 1, N, dtype=torch.float16, device="cuda")
+    got = m(x.view(M, 1, K), out=out)
+    assert got.data_ptr() == out.data_ptr() and torch.equal(out.view(M, N), want)
+    wide = torch.linspace(-1, 1, N).cuda()  # float32: added outside the kernel
+    m.bias = wide
+    assert torch.equal(m(x), want.clone().add_(wide))
+    m.bias = None
+    q = m.q_weights
+    del m.q_weights
+    m.q_weights = torch.nn.Parameter(q, requires_grad=False)
+    assert torch.equal(m(x), want)
+    for bad in (x.float(), x[:, :-64], x[:0]):
+        with pytest.raises(RuntimeError):
+            m(bad)
