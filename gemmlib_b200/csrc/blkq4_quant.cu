@@ -72,23 +72,25 @@ __device__ __forceinline__ unsigned long long pack_f32x2(float x, float y) {
   return r;
 }
 
-// Two weights v at once: q = clamp(round_half_away(v * r + zp), 0, 15), each in a 16-bit field with q at bits
-// POS .. POS + 3, fraction bits below and zeros above.
+// Two weights v at once: 15 - q with q = clamp(round_half_away(v * r + zp), 0, 15), each in a 16-bit field with
+// 15 - q at bits POS .. POS + 3, fraction bits below and zeros above.  nr2 and nz2 are -r and -zp.
 //
 // The reference's expression (f16_quant_sm80.cuh:295-296) is compiled by nvcc with its default fused multiply-add
-// contraction; the fma is explicit here.  For x >= 0 rounding halves away from zero is floor(x + 0.5), and negative x
-// end at 0 either way.  Adding 1.5 * 2^(23 - POS) + 0.5 with rounding toward zero leaves floor((x + 0.5) * 2^POS)
-// in the low mantissa bits (the sum is positive and its last place is 2^-POS), so one packed fp32 addition
-// does the rounding and the conversion; the low 16 bits are that integer in two's complement (|x| < 38: a
-// subnormal scale may be off by half of itself), which a packed 16-bit minimum with the negative values
-// flushed to zero clamps to [0, 16 * 2^POS - 1].
+// contraction; the fma is explicit here and gives -x for x = v * r + zp.  For x >= 0 rounding halves away from zero
+// is floor(x + 0.5), and negative x end at 0 either way.  With n = floor((x + 0.5) * 2^POS), adding
+// 1.5 * 2^(23 - POS) + 15.5 - 2^-POS with rounding toward +infinity leaves 16 * 2^POS - 1 - n in the low mantissa
+// bits (the sum is positive and its last place is 2^-POS), so one packed fp32 addition does the rounding and the
+// conversion; the low 16 bits are that integer in two's complement (|x| < 38: a subnormal scale may be off by
+// half of itself), which a packed 16-bit minimum with the negative values flushed to zero clamps to
+// [0, 16 * 2^POS - 1].  Why 15 - q: a NaN (a NaN weight, or an infinite one, whose block has r = 0) has all low
+// bits set, which is flushed to zero, and the reference's min(15, NaN) makes it q = 15.
 template <int POS>
-__device__ __forceinline__ uint32_t quantize_pair(uint32_t v, unsigned long long r2, unsigned long long zp2) {
+__device__ __forceinline__ uint32_t quantize_pair(uint32_t v, unsigned long long nr2, unsigned long long nz2) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
-  constexpr float kMagic = 1.5f * (float)(1 << (23 - POS)) + 0.5f;
+  constexpr float kMagic = (float)(1.5 * (1 << (23 - POS)) + 15.5 - 1.0 / (1 << POS));
   unsigned long long x;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack_f32x2(f.x, f.y)), "l"(r2), "l"(zp2));
-  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(x) : "l"(x), "l"(pack_f32x2(kMagic, kMagic)));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack_f32x2(f.x, f.y)), "l"(nr2), "l"(nz2));
+  asm("add.rp.f32x2 %0, %1, %2;" : "=l"(x) : "l"(x), "l"(pack_f32x2(kMagic, kMagic)));
   uint32_t lo, hi, q;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(x));
   constexpr uint32_t kMax = (16u << POS) - 1u;
@@ -105,10 +107,13 @@ __device__ __forceinline__ uint32_t select_bits(uint32_t a, uint32_t b, uint32_t
 
 // One packed word (reference dev_prepack_weights, f16_quant_sm80.cuh:362-417) of k = 2r, 2r + 1, 2r + 8, 2r + 9:
 // nibbles, from bit 0, of (2r, n0) (2r + 8, n0) (2r, n0 + 8) (2r + 8, n0 + 8), the same for 2r + 1 from bit 16.
-// a0, a1 / b0, b1: quantize_pair<4> of k pair 2r and quantize_pair<8> of k pair 2r + 8, columns n0 / n0 + 8.
+// a0, b0: quantize_pair<4> of k pair 2r, columns n0 and n0 + 8; a1, b1: quantize_pair<8> of k pair 2r + 8.  All
+// 32 bits come out complemented (~0xe4 = 0x1b), which turns every 15 - q into q.
 __device__ __forceinline__ uint32_t assemble_word(uint32_t a0, uint32_t a1, uint32_t b0, uint32_t b1) {
   const uint32_t a = select_bits(a0, a1, 0x00ff00ffu), b = select_bits(b0, b1, 0x00ff00ffu);
-  return select_bits(a >> 4, b << 4, 0x00ff00ffu);
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x1b;" : "=r"(d) : "r"(a >> 4), "r"(b << 4), "r"(0x00ff00ffu));
+  return d;
 }
 
 // 16 halves of a weight row.  ALIGNED: 16-byte loads.
@@ -187,7 +192,10 @@ quant_colwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   auto params = [&](uint32_t range, uint32_t f, uint32_t& m, float& rc) {
     __half sc;
     uint8_t z;
-    block_params(half_bits_to_float(range & 0xffffu), half_bits_to_float(range >> 16), half_bits_to_float(f), has_zp, sc, z, rc);
+    // the reference's scan starts from +-FLT_MAX, which an all-NaN block and one of infinities alone keep
+    const float mn = fminf(half_bits_to_float(range & 0xffffu), __FLT_MAX__);
+    const float mx = fmaxf(half_bits_to_float(range >> 16), -__FLT_MAX__);
+    block_params(mn, mx, half_bits_to_float(f), has_zp, sc, z, rc);
     m = (uint32_t)__half_as_ushort(sc) | ((uint32_t)z << 16);
   };
   if constexpr (G == 1) {
@@ -206,9 +214,9 @@ quant_colwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
     rcb = odd ? rc : orc;
   }
 
-  const float za = (float)(ma >> 16), zb = (float)(mb >> 16);
-  const unsigned long long ra2 = pack_f32x2(rca, rca), za2 = pack_f32x2(za, za);
-  const unsigned long long rb2 = pack_f32x2(rcb, rcb), zb2 = pack_f32x2(zb, zb);
+  const float za = -(float)(ma >> 16), zb = -(float)(mb >> 16);
+  const unsigned long long ra2 = pack_f32x2(-rca, -rca), za2 = pack_f32x2(za, za);
+  const unsigned long long rb2 = pack_f32x2(-rcb, -rcb), zb2 = pack_f32x2(zb, zb);
   uint32_t out[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -242,8 +250,8 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   constexpr int NB = 128 / BLOCK;             // blocks per k in the tile
   __shared__ uint2 s_range[kWarps][32];       // [16-column group][k pair] min2, max2
   __shared__ __align__(16) unsigned short s_first[kWarps][64];  // [group][k] the group's first column
-  __shared__ __align__(16) float s_recip[NB][64];
-  __shared__ __align__(16) float s_zp[NB][64];
+  __shared__ __align__(16) float s_recip[NB][64];  // -1 / scale
+  __shared__ __align__(16) float s_zp[NB][64];     // -zero point
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kl = lane & 3, npl = lane >> 2;   // chunk along k, packed column of the group
@@ -300,8 +308,8 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
     uint8_t z;
     float rc;
     block_params(mn, mx, half_bits_to_float(s_first[nb * GROUPS][k]), has_zp, sc, z, rc);
-    s_recip[nb][k] = rc;
-    s_zp[nb][k] = (float)z;
+    s_recip[nb][k] = -rc;
+    s_zp[nb][k] = -(float)z;
     // meta column-major [K, N / BLOCK], every 16 rows permuted (reference dev_prepack_scales, :457-547): source row
     // 2t + u + 8h goes to 4t + u + 2h (scales) and 4t + 2u + h (zero points)
     const int g16 = k & ~15, u = k & 1, t = (k >> 1) & 3, h = (k >> 3) & 1;

@@ -102,6 +102,36 @@ def test_edge_values_bit_exact_vs_oracle():
                 assert_same(got, want, f"block={block} colwise={colwise} zp={has_zp}")
 
 
+@pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
+@pytest.mark.parametrize("has_zp", [True, False])
+@pytest.mark.parametrize("colwise", [True, False])
+@pytest.mark.parametrize("block", [16, 32, 64, 128])
+def test_nan_and_infinite_weights_bit_exact_vs_oracle(block, colwise, has_zp, offset):
+    """A weight that is not finite becomes nibble 15 (min(15, NaN) of the reference; an infinity has a reciprocal
+    scale of 0), does not move the range its block's scan finds, and leaves the neighbours' bytes alone."""
+    K, N = 256, 128
+    nan, inf = np.float16("nan"), np.float16("inf")
+    w = (np.random.default_rng(block).standard_normal((N, K)) * 0.05).astype(np.float16)
+    w[0, ::5] = nan
+    w[1, 3] = -nan                           # sign bit set
+    w.view(np.uint16)[2, 7::16] = 0x7C01     # a signalling pattern
+    w[3, 1::9] = inf
+    w[4, 2::9] = -inf
+    w[5, 4::16], w[5, 11::16] = inf, -inf
+    w[6], w[7], w[8] = nan, inf, -inf
+    w[9] = 0.0
+    w[9, 3::16] = nan                        # zeros and a NaN
+    w[10], w[10, 1::2] = -0.0, nan
+    w[32:, ::7] = nan                        # row-wise: whole blocks of one k
+    w[64:, 64::8] = inf
+    w[:, 128::32] = -inf
+    want = O.quant_prepack(block, colwise, w, has_zp)
+    base = torch.empty(N * K + 8, dtype=torch.float16, device="cuda")
+    src = base[offset : offset + N * K].view(N, K).copy_(torch.from_numpy(w))
+    got = gpu_quant(block, colwise, src, has_zp)
+    assert_same(got, want, f"block={block} colwise={colwise} zp={has_zp}")
+
+
 def test_leading_dimension_and_unaligned_source():
     """ld > K, and a source whose rows are not 16-byte aligned (scalar-load path)."""
     K, N = 128, 64
