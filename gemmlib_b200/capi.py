@@ -171,11 +171,17 @@ def quant(block_size, column_wise, rows, columns, ld, weights, q_weights, q_scal
 
 
 EARLY_WEIGHT_FETCH = 1  # BLKQ4_GEMM_EARLY_WEIGHT_FETCH
+SKINNY_WORKSPACE = 2    # BLKQ4_GEMM_SKINNY_WORKSPACE
 
 
 def gemm_workspace_size(m: int, n: int, k: int) -> int:
     """Bytes of zeroed workspace with which the tensor-core kernel would split K (0: it would not)."""
     return int(lib.blkq4_gemm_workspace_size(m, n, k))
+
+
+def gemm_workspace_size_blocked(block_size: int, col_wise: bool, m: int, n: int, k: int) -> int:
+    """Bytes of zeroed workspace of a call with SKINNY_WORKSPACE (0: it would not use one)."""
+    return int(lib.blkq4_gemm_workspace_size_sm100(block_size, col_wise, m, n, k))
 
 
 def gather_supported(block_size: int, col_wise: bool, m: int, n_shard: int, k: int) -> bool:

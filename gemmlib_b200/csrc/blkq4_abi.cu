@@ -152,6 +152,10 @@ extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blockin
                  (has_offsets && reinterpret_cast<uintptr_t>(offsets_ptr) % 16 != 0)))
     return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets must be 16-byte aligned for m > 16)");
 
+  // Up to 16 rows blkq4_gemm_workspace_size is 0, so a caller may pass its prefill workspace along with decode calls
+  // that run on another stream; only BLKQ4_GEMM_SKINNY_WORKSPACE says that the workspace is this call's.
+  if (m <= 16 && !(flags & BLKQ4_GEMM_SKINNY_WORKSPACE)) workspace = nullptr, workspace_size = 0;
+
   auto stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   auto a = reinterpret_cast<const __half*>(act_ptr);
   auto w = reinterpret_cast<const uint8_t*>(weights_ptr);

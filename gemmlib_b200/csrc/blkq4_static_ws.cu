@@ -83,7 +83,7 @@ extern "C" int blkq4_fp16_gemm_static_ws_sm100(int block_size, bool column_wise_
   std::string why;
   void* scratch = static_scratch(why);
   if (!scratch) return fail(err, "Static scratch unavailable: " + why);
-  // up to 16 rows the scratch stays out of it: such calls may run on several streams at a time
+  // up to 16 rows the scratch stays out of it, whatever the flags: such calls may run on several streams at a time
   if (m <= 16) scratch = nullptr;
   return blkq4_fp16_gemm_ws_sm100(block_size, column_wise_blocking, m, n, k, stream, act_ptr, a_size, weights_ptr,
                                   weights_size, scales_ptr, scales_size, offsets_ptr, offsets_size, output_ptr,

@@ -153,9 +153,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         [](int block, bool col_wise, int m_, int n_, int k_) {
           return int64_t(blkq4_gemm_workspace_size_sm100(block, col_wise, m_, n_, k_));
         },
-        "gemm_workspace_size with the blocking, for any row count");
+        "Bytes of workspace of a call with SKINNY_WORKSPACE, for any row count");
   m.def("gemm_workspace_size", [](int m_, int n_, int k_) { return int64_t(blkq4_gemm_workspace_size(m_, n_, k_)); },
         "Bytes of zeroed workspace with which the tensor-core kernel splits K (0: it does not)");
   m.attr("EARLY_WEIGHT_FETCH") = int(BLKQ4_GEMM_EARLY_WEIGHT_FETCH);
+  m.attr("SKINNY_WORKSPACE") = int(BLKQ4_GEMM_SKINNY_WORKSPACE);
   m.def("library_version", []() { return std::string(blkq4_version()); });
 }

@@ -26,6 +26,7 @@ from torch import nn
 from . import ms_blkq4linear_ext
 
 _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
+_SKINNY_WS = ms_blkq4linear_ext.SKINNY_WORKSPACE
 _linear = ms_blkq4linear_ext.linear
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
@@ -110,6 +111,7 @@ class BlkQ4Linear(nn.Module):
                 need = _workspace_size(block, col_wise, rows, N, K)
                 if need > 0:
                     ws = split_k_workspace(input.device, need)
+                    flags |= _SKINNY_WS
         buf = self._buffers
         if "q_weights" in buf and "q_scales" in buf and "q_zp" in buf:
             packed = buf["q_weights"], buf["q_scales"], buf["q_zp"]

@@ -30,6 +30,7 @@ forward = _mod.forward
 forward_out = _mod.forward_out
 library_version = _mod.library_version
 EARLY_WEIGHT_FETCH = _mod.EARLY_WEIGHT_FETCH
+SKINNY_WORKSPACE = _mod.SKINNY_WORKSPACE
 gemm_workspace_size = _mod.gemm_workspace_size
 gemm_workspace_size_blocked = _mod.gemm_workspace_size_blocked
 linear = _mod.linear

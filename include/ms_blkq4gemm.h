@@ -149,14 +149,20 @@ int blkq4_fp16_gemm_sm100(
  * (e.g. 224 tiles on 148 SMs) it cuts the tiles' k steps in one balanced range per SM (or pair)
  * instead, and a tile that straddles two ranges is finished through an fp32 partial tile in the
  * workspace.  Results are reproducible run to run with the same workspace size.  A null or too small
- * workspace, or a size query of 0, means the call runs exactly as blkq4_fp16_gemm_sm100.  No counterpart in the reference (its split-K template parameters
- * are unused, src/mickey/blk_q4/f16_gemm_sm80.h:86-90).
+ * workspace, or a size query of 0, means the call runs exactly as blkq4_fp16_gemm_sm100: up to 16 rows, where
+ * the query is always 0, the workspace is neither read nor written, so that such calls may run on several streams
+ * at a time.  No counterpart in the reference (its split-K template parameters are unused,
+ * src/mickey/blk_q4/f16_gemm_sm80.h:86-90).
  */
 size_t blkq4_gemm_workspace_size(int m, int n, int k);
 
-/* No counterpart in the reference.  The same with the blocking, which decides for m <= 16 whether the tensor-core
- * kernel takes the problem (row-wise blocks, or blocks of 16 and 32, at the larger sizes) and would cut it in
- * balanced ranges; for m > 16 equal to blkq4_gemm_workspace_size. */
+/* Flag of blkq4_fp16_gemm_ws_sm100: use the workspace up to 16 rows too.  The call is then one of those that use it
+ * one at a time.  For more than 16 rows it changes nothing. */
+#define BLKQ4_GEMM_SKINNY_WORKSPACE 2u
+
+/* No counterpart in the reference.  The workspace of a call with BLKQ4_GEMM_SKINNY_WORKSPACE: the blocking decides
+ * for m <= 16 whether the tensor-core kernel takes the problem (row-wise blocks, or blocks of 16 and 32, at the
+ * larger sizes) and would cut it in balanced ranges; for m > 16 equal to blkq4_gemm_workspace_size. */
 size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int n, int k);
 
 /* No counterpart in the reference.  Host-only description of the work plan blkq4_fp16_gemm_ws_sm100 would

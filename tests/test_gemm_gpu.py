@@ -363,3 +363,37 @@ def test_uneven_split(case):
     check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
     assert not ws.any()
     assert capi.gemm_plan(M, N, K, 0)["split"] == 1
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("block,colwise,has_zp", [(32, True, True), (128, False, False)])
+def test_workspace_up_to_16_rows(M, block, colwise, has_zp):
+    """Up to 16 rows the workspace is the call's only with SKINNY_WORKSPACE: without the flag it is neither read nor
+    written (another stream may be using it), with it the tiles are cut in balanced ranges whose flag words come
+    back to zero and whose partial tiles replace what lay there (NaN)."""
+    from gemmlib_b200 import capi
+
+    N, K = 28672, 1216  # 224 tiles of ten steps, the last one half empty
+    assert capi.gemm_workspace_size(M, N, K) == 0
+    need = capi.gemm_workspace_size_blocked(block, colwise, M, N, K)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    flag_bytes = -(-4 * sms // 256) * 256
+    assert need == flag_bytes + sms * 16 * 128 * 4
+    w = gaussian_weight(N, K, seed=3)
+    a = gaussian_act(M, K, seed=M).numpy()
+    pw, ps, pz = O.quant_prepack(block, colwise, w.numpy(), has_zp)
+    rows = a.astype(np.float32) @ O.dequant(block, colwise, K, N, pw, ps, pz, kernel_formula=True).astype(np.float32).T
+    plain = gpu_gemm(block, colwise, a, N, pw, ps, pz)
+    # one fp16 rounding and fp32 sums of K terms in any order
+    tol = (2.0 ** -11 + K * 2.0 ** -24) * np.abs(rows).max() + 2.0 ** -11
+    assert np.abs(plain - rows).max() <= tol
+    foreign = torch.full((need,), 0xFF, dtype=torch.uint8, device="cuda")
+    assert (bits(gpu_gemm(block, colwise, a, N, pw, ps, pz, workspace=foreign)) == bits(plain)).all()
+    assert (foreign == 0xFF).all()
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    ws[flag_bytes:] = 0xFF
+    got = gpu_gemm(block, colwise, a, N, pw, ps, pz, flags=capi.SKINNY_WORKSPACE, workspace=ws)
+    assert np.abs(got - rows).max() <= tol
+    assert not ws[:flag_bytes].any()
+    written = (ws[flag_bytes:].view(sms, 16, 512) != 0xFF).any(-1)  # [cta][row]
+    assert written[:, :M].all(-1).sum() >= sms // 2 and not written[:, M:].any()
