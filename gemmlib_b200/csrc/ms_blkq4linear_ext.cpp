@@ -15,8 +15,16 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+#include <cuda_runtime.h>
 
 #include "ms_blkq4gemm.h"
 
@@ -136,6 +144,73 @@ torch::Tensor blkq4linear_linear(int block_size, bool col_wise, int in_features,
   return output.view(shape);
 }
 
+// ---- workspaces of calls that are being captured into a CUDA graph ----
+// The graph keeps the buffer's address, so the graph keeps the buffer: a user object of the graph holds the tensor
+// until the graph and everything instantiated from it are gone.  One buffer per capture and stream, its flag words
+// zeroed by a node of the same graph, so that graphs share nothing and may replay side by side.
+std::mutex g_dropped_mutex;
+std::vector<torch::Tensor>& g_dropped = *new std::vector<torch::Tensor>;  // outlives static destruction
+std::atomic<bool> g_any_dropped{false};
+std::atomic<int> g_graph_workspaces{0};
+
+// A user object's destructor may not call CUDA, so it leaves the buffer to the next call of graph_workspace.
+void drop_graph_workspace(void* held) {
+  auto* buffer = static_cast<torch::Tensor*>(held);
+  {
+    std::lock_guard<std::mutex> lock(g_dropped_mutex);
+    g_dropped.push_back(std::move(*buffer));
+    g_any_dropped.store(true);
+  }
+  delete buffer;
+  --g_graph_workspaces;
+}
+
+// The workspace of at least `nbytes` for the capture that is under way on the device's current stream (`stream`);
+// nothing when none is, an empty tensor when the graph cannot take one.  Called with the GIL held.
+c10::optional<torch::Tensor> graph_workspace(int device, uintptr_t stream_handle, int64_t nbytes) {
+  if (g_any_dropped.load()) {
+    std::vector<torch::Tensor> dropped;
+    std::lock_guard<std::mutex> lock(g_dropped_mutex);
+    dropped.swap(g_dropped);
+    g_any_dropped.store(false);
+  }
+  const auto stream = reinterpret_cast<cudaStream_t>(stream_handle);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &status, &id, &graph) != cudaSuccess) {
+    cudaGetLastError();
+    return c10::nullopt;
+  }
+  if (status == cudaStreamCaptureStatusNone) return c10::nullopt;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  const auto u8 = torch::TensorOptions().dtype(torch::kUInt8).device(torch::kCUDA, static_cast<c10::DeviceIndex>(device));
+  if (status != cudaStreamCaptureStatusActive) return torch::empty({0}, u8);
+
+  // the last capture of each stream; its tensor is there as long as that capture is under way (ids are never reused)
+  static auto& last = *new std::map<std::pair<int, cudaStream_t>, std::pair<unsigned long long, torch::Tensor*>>;
+  auto& slot = last[{device, stream}];
+  if (slot.first == id && slot.second && slot.second->numel() >= nbytes) return *slot.second;
+  auto* held = new torch::Tensor(torch::empty({nbytes}, u8));
+  ++g_graph_workspaces;
+  torch::Tensor buffer = *held;
+  cudaUserObject_t object = nullptr;
+  if (cudaUserObjectCreate(&object, held, drop_graph_workspace, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    cudaGetLastError();
+    drop_graph_workspace(held);
+    return torch::empty({0}, u8);
+  }
+  // flag words: at most one per SM, far below 64 KB; the partial tiles behind them need no clearing
+  if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaGetLastError();
+    cudaUserObjectRelease(object, 1);
+    return torch::empty({0}, u8);
+  }
+  slot = {id, held};
+  C10_CUDA_CHECK(cudaMemsetAsync(buffer.data_ptr(), 0, size_t(std::min<int64_t>(nbytes, 64 << 10)), stream));
+  return buffer;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -156,6 +231,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "Bytes of workspace of a call with SKINNY_WORKSPACE, for any row count");
   m.def("gemm_workspace_size", [](int m_, int n_, int k_) { return int64_t(blkq4_gemm_workspace_size(m_, n_, k_)); },
         "Bytes of zeroed workspace with which the tensor-core kernel splits K (0: it does not)");
+  m.def("graph_workspace", &graph_workspace,
+        "Workspace owned by the CUDA graph that the device's current stream is being captured into, else None",
+        py::arg("device"), py::arg("stream"), py::arg("nbytes"));
+  m.def("graph_workspaces", [] { return g_graph_workspaces.load(); }, "Workspaces that CUDA graphs hold at present");
   m.attr("EARLY_WEIGHT_FETCH") = int(BLKQ4_GEMM_EARLY_WEIGHT_FETCH);
   m.attr("SKINNY_WORKSPACE") = int(BLKQ4_GEMM_SKINNY_WORKSPACE);
   m.def("library_version", []() { return std::string(blkq4_version()); });

@@ -15,10 +15,13 @@ epilogue (bit-identical to the reference's separate ``output += bias``, one pass
 output less); and, from the second call on, the skinny kernel is launched with
 ``BLKQ4_GEMM_EARLY_WEIGHT_FETCH`` (set ``early_weight_fetch = False`` on a layer whose
 packed tensors are rewritten by work queued on the same stream as ``forward``); prefill
-shapes with too few output tiles to fill the GPU split K through a workspace shared per
-(device, stream) (``split_k = False`` turns that off).
+shapes with too few output tiles to fill the GPU split K through a workspace that eager calls share
+per (device, stream) and that a CUDA graph owns (``split_k = False`` turns that off).
 """
 from __future__ import annotations
+
+import contextlib
+import threading
 
 import torch
 from torch import nn
@@ -28,18 +31,45 @@ from . import ms_blkq4linear_ext
 _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
 _SKINNY_WS = ms_blkq4linear_ext.SKINNY_WORKSPACE
 _linear = ms_blkq4linear_ext.linear
+_graph_workspace = ms_blkq4linear_ext.graph_workspace
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
-# Split-K workspaces: one zero-initialised buffer per (device, stream), shared by all layers (calls
-# on one stream run one at a time; the kernel leaves the buffer's flags zeroed).  Grown on demand.
+# Split-K workspaces.  Eager calls: one zero-initialised buffer per (device, stream), shared by all layers (calls
+# on one stream run one at a time; the kernel leaves the buffer's flags zeroed).  Grown on demand, the smaller
+# buffer going back to the allocator, which orders its reuse behind the stream's work.
+# A CUDA graph keeps the address it was captured with and replays on any stream, so it never sees these: its
+# buffers belong to the graph (``graph_workspace``) or to whoever captures it (``workspaces_owned_by``).
 _WORKSPACES = {}
+_owner = threading.local()
+
+
+@contextlib.contextmanager
+def workspaces_owned_by(workspaces: dict):
+    """Within the block this thread's calls take their split-K workspaces from ``workspaces``
+    ((device, stream) -> buffers, the last one in use).  The caller keeps the dict as long as a graph captured
+    in the block may replay; unlike a graph's own workspace these need no zeroing node."""
+    before = getattr(_owner, "workspaces", None)
+    _owner.workspaces = workspaces
+    try:
+        yield workspaces
+    finally:
+        _owner.workspaces = before
 
 
 def split_k_workspace(device, nbytes: int):
     if nbytes <= 0:
         return None
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (index, torch.cuda.current_stream(device).cuda_stream)
+    owned = getattr(_owner, "workspaces", None)
+    if owned is not None:
+        buffers = owned.setdefault(key, [])  # a captured call keeps the buffer it got: none is dropped here
+        if not buffers or buffers[-1].numel() < nbytes:
+            buffers.append(torch.zeros(nbytes, dtype=torch.uint8, device=device))
+        return buffers[-1]
+    ws = _graph_workspace(*key, nbytes)
+    if ws is not None:
+        return ws
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 16 << 20), dtype=torch.uint8, device=device)
@@ -96,6 +126,12 @@ class BlkQ4Linear(nn.Module):
                 and b.numel() == self.out_features and b.is_contiguous()):
             return b
         return None
+
+    def workspace_bytes(self, rows):
+        """Split-K workspace that ``forward`` uses for ``rows`` activation rows (0: none)."""
+        if not self.split_k:
+            return 0
+        return _workspace_size(self.block_size, self.col_wise, rows, self.out_features, self.in_features)
 
     def forward(self, input, out=None):
         # Few and plain lookups: at decode sizes the host's time per call is what a caller sees.

@@ -34,3 +34,5 @@ SKINNY_WORKSPACE = _mod.SKINNY_WORKSPACE
 gemm_workspace_size = _mod.gemm_workspace_size
 gemm_workspace_size_blocked = _mod.gemm_workspace_size_blocked
 linear = _mod.linear
+graph_workspace = _mod.graph_workspace
+graph_workspaces = _mod.graph_workspaces

@@ -20,7 +20,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import BlkQ4Linear
+from .ms_blkq4linear import BlkQ4Linear, split_k_workspace, workspaces_owned_by
 
 
 class LinearStack:
@@ -35,6 +35,7 @@ class LinearStack:
         self.steps = list(steps)
         self.between = dict(between or {})
         self._graphs: Dict[int, Tuple[torch.cuda.CUDAGraph, Dict[str, torch.Tensor]]] = {}
+        self._split_k: Dict[int, dict] = {}  # row count -> split-K workspaces of its graph
         self.device = self.steps[0][0].q_weights.device
         self.stream = torch.cuda.Stream(self.device)
         written = {"x"}
@@ -67,13 +68,20 @@ class LinearStack:
     def _capture(self, M: int):
         bufs = self._workspace(M)
         self.stream.wait_stream(torch.cuda.current_stream(self.device))
-        with torch.cuda.stream(self.stream):
-            for _ in range(2):  # the first pass settles every layer (plain launches), the second warms up
+        with workspaces_owned_by({}) as split_k:
+            with torch.cuda.stream(self.stream):
+                # the largest at once: the layers do not outgrow one buffer after another
+                split_k_workspace(self.device, max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps
+                                                    if isinstance(lyr, BlkQ4Linear)), default=0))
+                for _ in range(2):  # the first pass settles every layer (plain launches), the second warms up
+                    self._run_eager(bufs)
+            self.stream.synchronize()
+            for buffers in split_k.values():
+                del buffers[:-1]  # outgrown in the first pass
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=self.stream):
                 self._run_eager(bufs)
-        self.stream.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=self.stream):
-            self._run_eager(bufs)
+        self._split_k[M] = split_k
         self._graphs[M] = (graph, bufs)
         return self._graphs[M]
 

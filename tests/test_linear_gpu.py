@@ -174,3 +174,79 @@ def test_forward_takes_every_input_form(M):
     for bad in (x.float(), x[:, :-64], x[:0]):
         with pytest.raises(RuntimeError):
             m(bad)
+
+
+def _balanced_layer():
+    """224 output tiles on 148 SMs: every row count cuts balanced ranges through a workspace."""
+    from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = (torch.randn(28672, 1216, generator=g, device="cuda") * 0.02).half()
+    return BlkQ4Linear(32, True, False, w)
+
+
+def test_stack_graphs_own_their_workspaces():
+    """A graph's workspace outlives the capture of a row count that needs a larger one, is no other graph's and not
+    the eager calls', so a replay reads and writes only its own memory."""
+    from gemmlib_b200 import ms_blkq4linear as L
+    from gemmlib_b200.stack import LinearStack
+
+    layer = _balanced_layer()
+    st = LinearStack([(layer, "x", "y")])
+    x = gaussian_act(16, 1216, seed=8).cuda()
+    want = layer(x)  # the eager workspace
+    first = st.forward(x, "y").clone()
+    held = {M: [b for buffers in st._split_k[M].values() for b in buffers] for M in (16,)}
+    ptrs = [b.data_ptr() for b in held[16]]
+    for M in (8, 512):
+        st.buffers(M)
+        held[M] = [b for buffers in st._split_k[M].values() for b in buffers]
+    assert all(len(b) == 1 for b in held.values()) and held[512][0].numel() > 16 << 20 > held[16][0].numel()
+    assert [b.data_ptr() for buffers in st._split_k[16].values() for b in buffers] == ptrs
+    spans = sorted((b.data_ptr(), b.data_ptr() + b.numel()) for b in
+                   [b for buffers in held.values() for b in buffers] + list(L._WORKSPACES.values()))
+    assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
+    del held
+    torch.cuda.empty_cache()
+    others = [torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda") for n in (1 << 20, 1213184, 16 << 20, 20 << 20)]
+    st.buffers(16)["y"].fill_(float("nan"))
+    assert torch.equal(st.forward(x, "y"), first) and torch.equal(first, want)
+    assert all(bool((o == 0xFF).all()) for o in others)
+
+
+def test_captured_call_takes_a_workspace_that_its_graph_owns():
+    """torch.cuda.graph around a layer: every graph holds a workspace of its own, zeroed by a node of its own, until it
+    is destroyed; the eager calls' buffer is not used."""
+    import gc
+    import time
+
+    from gemmlib_b200 import ms_blkq4linear as L
+    from gemmlib_b200 import ms_blkq4linear_ext as ext
+
+    layer = _balanced_layer()
+    eager = dict(L._WORKSPACES)
+    for M in (16, 40):
+        x = gaussian_act(M, 1216, seed=M).cuda()
+        want, out = layer(x), [torch.empty(M, 28672, dtype=torch.float16, device="cuda") for _ in range(2)]
+        before, eager = ext.graph_workspaces(), dict(L._WORKSPACES)
+        graphs = []
+        for o in out:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                layer(x, out=o)
+                layer(x, out=o)  # the same buffer again
+            graphs.append(g)
+        assert ext.graph_workspaces() == before + 2
+        assert {k: v.data_ptr() for k, v in L._WORKSPACES.items()} == {k: v.data_ptr() for k, v in eager.items()}
+        for g, o in list(zip(graphs, out))[::-1]:  # the later graph first
+            o.fill_(float("nan"))
+            g.replay()
+            assert torch.equal(o, want)
+        torch.cuda.synchronize()
+        del g, graphs
+        gc.collect()
+        deadline = time.time() + 10  # user objects may be released a little later
+        while ext.graph_workspaces() != before and time.time() < deadline:
+            time.sleep(0.05)
+        assert ext.graph_workspaces() == before
+    assert torch.equal(layer(x), want)
