@@ -157,7 +157,8 @@ class BlkQ4Linear(nn.Module):
         if not settled:
             self._settled = True
         if bias is not None and fused is None:
-            output += bias
+            rows = output.view(-1, N)
+            rows += bias  # broadcast against [rows, out_features], whatever the input's leading dimensions
         return output
 
     def extra_repr(self):

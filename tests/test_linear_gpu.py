@@ -250,3 +250,27 @@ def test_captured_call_takes_a_workspace_that_its_graph_owns():
             time.sleep(0.05)
         assert ext.graph_workspaces() == before
     assert torch.equal(layer(x), want)
+
+
+def test_bias_broadcasts_against_flattened_rows():
+    """A bias that cannot be fused is added to the [rows, out_features] result, as in the reference's two-dimensional
+    `output += bias`: its shape has nothing to do with the leading dimensions of the input."""
+    from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
+
+    K, N = 256, 160
+    m = BlkQ4Linear(64, True, False, gaussian_weight(N, K, seed=4).cuda())
+    x = gaussian_act(6, K, seed=5).cuda()
+    plain = m(x)
+    g = torch.Generator().manual_seed(6)
+    for shape in [(1, N), (6, N), (6, 1), (1,), (N,)]:
+        m.bias = torch.randn(shape, generator=g).cuda()  # float32: not fused
+        want = plain.clone().add_(m.bias)
+        assert torch.equal(m(x), want)
+        assert torch.equal(m(x.view(2, 3, K)), want.view(2, 3, N))
+        out = torch.empty(3, 2, N, dtype=torch.float16, device="cuda")
+        assert m(x.view(3, 2, K), out=out).data_ptr() == out.data_ptr() and torch.equal(out.view(6, N), want)
+    m.bias = torch.randn((1, N), generator=g).cuda()
+    assert torch.equal(m(x[0]), plain[:1].clone().add_(m.bias).view(N))
+    m.bias = torch.randn((3, N), generator=g).cuda()
+    with pytest.raises(RuntimeError):
+        m(x.view(2, 3, K))  # three rows against six
