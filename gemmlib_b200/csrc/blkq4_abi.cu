@@ -146,11 +146,14 @@ extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blockin
       reinterpret_cast<uintptr_t>(scales_ptr) % 2 != 0)
     return fail(err, "Kernel execution failed: Error Misaligned Operand");
 
-  // The tensor-core kernel fetches scales and zero points with TMA (16-byte aligned bases; the skinny
-  // kernels fall back to plain loads instead).
-  if (m > 16 && (reinterpret_cast<uintptr_t>(scales_ptr) % 16 != 0 ||
-                 (has_offsets && reinterpret_cast<uintptr_t>(offsets_ptr) % 16 != 0)))
+  // The tensor-core kernel fetches scales and zero points with TMA (16-byte aligned bases), and the generic skinny
+  // kernel reads those of row-wise blocks 16 bytes at a time; column-wise ones it reads one by one.
+  const bool meta_aligned = reinterpret_cast<uintptr_t>(scales_ptr) % 16 == 0 &&
+                            (!has_offsets || reinterpret_cast<uintptr_t>(offsets_ptr) % 16 == 0);
+  if (m > 16 && !meta_aligned)
     return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets must be 16-byte aligned for m > 16)");
+  if (!column_wise_blocking && !meta_aligned)
+    return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets of row-wise blocks must be 16-byte aligned)");
 
   // Up to 16 rows blkq4_gemm_workspace_size is 0, so a caller may pass its prefill workspace along with decode calls
   // that run on another stream; only BLKQ4_GEMM_SKINNY_WORKSPACE says that the workspace is this call's.

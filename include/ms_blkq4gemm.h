@@ -122,6 +122,9 @@ int blkq4_fp16_quant_size_sm80(
  * across the launches of a decode stack.  Activations are read, and the output written, only
  * after the preceding work has completed, so stream order holds for both (and for the split-K
  * workspace).  Both the skinny and the tensor-core kernel honour it.
+ *
+ * Pointers: activations, weights and output 16-byte aligned; scales and offsets too for m > 16 and for row-wise
+ * blocks (a misaligned one is refused with an error), else of their element's alignment.
  */
 #define BLKQ4_GEMM_EARLY_WEIGHT_FETCH 1u
 int blkq4_fp16_gemm_sm100(

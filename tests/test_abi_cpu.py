@@ -111,6 +111,11 @@ def test_extension_entry_points_validate_on_the_host(lib_built):
     with pytest.raises(capi.BlkQ4Error, match="Bias tensor must be 4-byte aligned"):
         capi.gemm(32, True, M, N, K, fake(2 * M * K), fake(K * N // 2), fake(2 * 2 * N), None, fake(2 * M * N),
                   bias=(0x1002, 2 * N))
+    # row-wise meta is read 16 bytes at a time at every row count: refused, not read at a misaligned address
+    for m in (1, 9, 16, 17):
+        for scales, offsets in [((0x1008, 2 * 64), (0x1000, 64)), ((0x1000, 2 * 64), (0x1002, 64))]:
+            with pytest.raises(capi.BlkQ4Error, match="must be 16-byte aligned"):
+                capi.gemm(32, False, m, N, K, fake(2 * m * K), fake(K * N // 2), scales, offsets, fake(2 * m * N))
     # split-K planning is a pure host function (it falls back to 148 SMs without a device)
     assert capi.gemm_workspace_size(512, 4096, 4096) == 256 + 64 * 256 * 128 * 4
     assert capi.gemm_workspace_size(2048, 4096, 4096) == 0
