@@ -716,6 +716,69 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   return best;
 }
 
+// The one-CTA kernel for tiles of BM rows.
+using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params);
+struct KernelChoice {
+  Kern kern;
+  int threads, which;  // which: index of the per-device caches
+  SmemPlan plan;
+  size_t max_smem;     // of the largest tile the kernel takes
+};
+std::atomic<int> g_granted_smem[6][64];
+
+KernelChoice choose_kernel(bool colwise, int BM) {
+  KernelChoice c;
+  auto pick = [&](auto shape, int idx, int max_rows) {
+    using S = decltype(shape);
+    c.kern = colwise ? (Kern)gemm_tc_kernel<true, S> : (Kern)gemm_tc_kernel<false, S>;
+    c.threads = S::kThreads;
+    c.which = 2 * idx + (colwise ? 1 : 0);
+    c.plan = make_plan(BM, S::WS, S::ACT, S::KSUB);
+    c.max_smem = make_plan(max_rows, S::WS, S::ACT, S::KSUB).total;
+  };
+  if (BM <= 64) pick(ShapeSmall{}, 0, 64);
+  else if (BM <= 128) pick(ShapeMid{}, 1, 128);
+  else pick(ShapeLarge{}, 2, 256);
+  return c;
+}
+
+// Clusters of `split` CTAs of the kernel that are resident at once on the current device, 0 when it cannot say.
+// Asked with the largest shared-memory plan of the kernel, so that the answer holds for every BM.
+int resident_clusters(const KernelChoice& kc, int split) {
+  static std::atomic<int> cache[6][kMaxSplit + 1][64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const bool cached = dev >= 0 && dev < 64;
+  int n = cached ? cache[kc.which][split][dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count() / split * split);
+  cfg.blockDim = dim3(kc.threads);
+  cfg.dynamicSmemBytes = kc.max_smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (ensure_dynamic_smem(kc.kern, kc.max_smem, g_granted_smem[kc.which]) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kc.kern, &cfg) != cudaSuccess || n < 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (cached && n > 0) cache[kc.which][split][dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// A group of SMs holds whole clusters only, so fewer than SMs / split may fit: cut in fewer parts until all
+// clusters of the problem run in one round.
+void fit_split(const KernelChoice& kc, int tiles, int k_steps, SplitPlan& sp) {
+  while (sp.split > 1 && resident_clusters(kc, sp.split) < tiles) {
+    sp.k_per_item = (k_steps + sp.split - 2) / (sp.split - 1);
+    sp.split = (k_steps + sp.k_per_item - 1) / sp.k_per_item;
+  }
+}
+
 }  // namespace
 
 namespace {
@@ -940,75 +1003,35 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     return std::string();
   }
   const int num_tiles = p.m_tiles * p.n_tiles;
-  const SplitPlan sp = plan_split(M, N, K, ws_ok ? workspace_bytes : 0);
-  p.split = sp.split;  // split > 1: at most one item per SM
+  const KernelChoice kc = choose_kernel(colwise, p.BM);
   p.k_steps = (K + sk - 1) / sk;
+  SplitPlan sp = plan_split(M, N, K, ws_ok ? workspace_bytes : 0);
+  fit_split(kc, num_tiles, p.k_steps, sp);
+  p.split = sp.split;  // split > 1: at most one item per SM
   p.k_per_item = sp.k_per_item;
   p.min_part = min_part(sk);
   p.balanced = sp.balanced;
   p.total_steps = sp.balanced ? num_tiles * p.k_steps : 0;
   p.ws_flags = reinterpret_cast<unsigned*>(workspace);
   p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + sp.flags_bytes);
-  using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params);
-  static std::atomic<int> granted[6][64];
-  Kern kern;
-  int threads, which;
-  size_t max_smem;
-  SmemPlan plan;
-  auto pick = [&](auto shape, int idx) {
-    using S = decltype(shape);
-    kern = colwise ? (Kern)gemm_tc_kernel<true, S> : (Kern)gemm_tc_kernel<false, S>;
-    threads = S::kThreads;
-    which = 2 * idx + (colwise ? 1 : 0);
-    plan = make_plan(p.BM, S::WS, S::ACT, S::KSUB);
-    max_smem = make_plan(idx == 0 ? 64 : idx == 1 ? 128 : 256, S::WS, S::ACT, S::KSUB).total;
-  };
-  if (p.BM <= 64) pick(ShapeSmall{}, 0);
-  else if (p.BM <= 128) pick(ShapeMid{}, 1);
-  else pick(ShapeLarge{}, 2);
-  cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[which]);
+  cudaError_t e = ensure_dynamic_smem(kc.kern, kc.plan.total, g_granted_smem[kc.which]);
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = plan.total;
+  cfg.blockDim = dim3(kc.threads);
+  cfg.dynamicSmemBytes = kc.plan.total;
   cfg.stream = stream;
   // BLKQ4_GEMM_EARLY_WEIGHT_FETCH: programmatic stream serialization, see the kernel's entry
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)p.split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  while (p.split > 1) {
-    // all clusters in one round, or fewer parts: an SM group holds whole clusters only
-    attr[0].val.clusterDim.x = (unsigned)p.split;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(num_tiles * p.split);
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    static std::atomic<int> fit[6][kMaxSplit + 1][64];  // clusters of this size that are resident at once
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const bool cached = dev >= 0 && dev < 64;
-    int n = cached ? fit[which][p.split][dev].load(std::memory_order_relaxed) : 0;
-    if (n <= 0) {
-      // asked with the largest shared-memory plan of the kernel, so that the answer holds for every BM
-      cfg.dynamicSmemBytes = max_smem;
-      e = ensure_dynamic_smem(kern, max_smem, granted[which]);
-      if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 0) {
-        cudaGetLastError();
-        n = 0;
-      }
-      cfg.dynamicSmemBytes = plan.total;
-      if (cached && n > 0) fit[which][p.split][dev].store(n, std::memory_order_relaxed);
-    }
-    if (n >= num_tiles) break;
-    p.k_per_item = (p.k_steps + p.split - 2) / (p.split - 1);
-    p.split = (p.k_steps + p.k_per_item - 1) / p.k_per_item;
-  }
   p.num_items = num_tiles * p.split;
   cfg.gridDim = dim3(p.num_items < sms ? p.num_items : sms);
   cfg.attrs = p.split > 1 ? attr : attr + 1;
   cfg.numAttrs = (p.split > 1 ? 1 : 0) + ((flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) ? 1 : 0);
-  e = cudaLaunchKernelEx(&cfg, kern, tm_act, tm_pack, tm_scale, tm_zp, p);
+  e = cudaLaunchKernelEx(&cfg, kc.kern, tm_act, tm_pack, tm_scale, tm_zp, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   return std::string();
@@ -1040,9 +1063,14 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
     out6[5] = pp.balanced ? sms / 2 : 0;
     return 0;
   }
-  const blkq4::SplitPlan sp = blkq4::plan_split(m, n, k, workspace_size);
+  blkq4::SplitPlan sp = blkq4::plan_split(m, n, k, workspace_size);
   const int bm = m >= 256 ? 256 : ((m + 15) / 16) * 16;
   out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
+  int devices = 0;
+  if (cudaGetDeviceCount(&devices) != cudaSuccess) cudaGetLastError();
+  // as many clusters fit of the row-wise kernel as of the column-wise one: one CTA per SM, both
+  if (devices > 0)
+    blkq4::fit_split(blkq4::choose_kernel(true, bm), out6[2], (k + blkq4::step_k(bm) - 1) / blkq4::step_k(bm), sp);
   out6[3] = sp.split; out6[4] = sp.balanced; out6[5] = sp.balanced ? sms : 0;
   return 0;
 }

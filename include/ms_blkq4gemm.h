@@ -170,7 +170,8 @@ size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking
 
 /* No counterpart in the reference.  Host-only description of the work plan blkq4_fp16_gemm_ws_sm100 would
  * choose for the problem with a workspace of `workspace_size` bytes: nothing is launched and no device is
- * needed (the plan depends on the current device's SM count; 148 is assumed without a device).
+ * needed (the plan depends on the current device's SM count and on how many clusters of a split's size it holds at
+ * once, as the launch does; 148 SMs and no such limit are assumed without a device).
  *   out6[0]  kernel: 0 = m <= 16 (skinny kernels; some blockings and sizes run on kernel 1), 1 = tensor-core kernel with one CTA per tile,
  *            2 = tensor-core kernel with CTA pairs
  *   out6[1]  activation rows per tile        out6[2]  output tiles

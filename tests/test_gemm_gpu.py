@@ -397,3 +397,31 @@ def test_workspace_up_to_16_rows(M, block, colwise, has_zp):
     assert not ws[:flag_bytes].any()
     written = (ws[flag_bytes:].view(sms, 16, 512) != 0xFF).any(-1)  # [cta][row]
     assert written[:, :M].all(-1).sum() >= sms // 2 and not written[:, M:].any()
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 2304, 8192), (17, 2304, 4096), (128, 1024, 4096), (200, 640, 4160), (512, 4096, 4096),
+                                   (100, 384, 8064), (256, 4096, 4096), (40, 6144, 4096), (512, 1024, 2048)])
+def test_plan_names_the_split_that_is_launched(M, N, K):
+    """The parts of a tile form a cluster, and a group of SMs holds whole clusters only: 18 tiles in eight parts need
+    no more than 144 SMs and still do not all fit.  The grid of the captured launch is tiles x parts."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    from gemmlib_b200 import capi
+
+    need = capi.gemm_workspace_size(M, N, K)
+    plan = capi.gemm_plan(M, N, K, need)
+    assert plan["kernel"] == "one-cta" and need > 0 and not plan["balanced"]
+    a = torch.zeros(M, K, dtype=torch.float16, device="cuda")
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    for block, colwise in ((64, True), (32, False)):
+        qw = torch.zeros(K * N // 2, dtype=torch.uint8, device="cuda")
+        qs = torch.zeros(K * N // block, dtype=torch.float16, device="cuda")
+        out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        stream = torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            capi.gemm(block, colwise, M, N, K, a, qw, qs, None, out, stream=stream.cuda_stream, workspace=ws)
+        handle = driver.CUgraph(int(graph.raw_cuda_graph()))
+        err, nodes, count = driver.cuGraphGetNodes(handle, 8)
+        assert int(err) == 0 and count == 1
+        err, params = driver.cuGraphKernelNodeGetParams(nodes[0])
+        assert int(err) == 0 and params.gridDimX == plan["tiles"] * plan["split"], (params.gridDimX, plan)
