@@ -20,7 +20,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import BlkQ4Linear, split_k_workspace, workspaces_owned_by
+from .ms_blkq4linear import BlkQ4Linear, workspaces_owned_by
 
 
 class LinearStack:
@@ -67,12 +67,16 @@ class LinearStack:
 
     def _capture(self, M: int):
         bufs = self._workspace(M)
+        # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
+        # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
+        need = max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)), default=0)
+        split_k = {}
+        if need > 0:
+            split_k[self.device.index, self.stream.cuda_stream] = [
+                torch.zeros(need, dtype=torch.uint8, device=self.device)]
         self.stream.wait_stream(torch.cuda.current_stream(self.device))
-        with workspaces_owned_by({}) as split_k:
+        with workspaces_owned_by(split_k):
             with torch.cuda.stream(self.stream):
-                # the largest at once: the layers do not outgrow one buffer after another
-                split_k_workspace(self.device, max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps
-                                                    if isinstance(lyr, BlkQ4Linear)), default=0))
                 for _ in range(2):  # the first pass settles every layer (plain launches), the second warms up
                     self._run_eager(bufs)
             self.stream.synchronize()
