@@ -845,20 +845,30 @@ size_t gemm_tc_workspace_bytes(int M, int N, int K) {
 // Which problems of up to 16 rows run here rather than on the generic skinny kernel (blkq4_gemv.cu): both convert
 // the weights to fp16 by the same formula and sum in fp32.  Only those whose blocking no other skinny kernel takes
 // (row-wise, or blocks of 16 and 32): the others scale fp32 sums instead, which is more accurate.
-// The generic kernel splits K over the eight warps of a CTA and streams its weights through registers; it is good for
-// about 1.6 TB/s and a short launch.  Measured on B200, generic against this one, us, block 32 column-wise with
-// zero points (row-wise):
-//   M = 8:  1024 x 4096 3.8 / 5.3 (4.4 / 5.4);  2048 x 8192 8.1 / 8.3 (9.6 / 9.8);  4096 x 4096 7.3 / 8.5 (8.8 / 10.1);
-//           4096 x 8192 13.1 / 11.3 (15.6 / 14.1);  4096 x 11008 18.4 / 13.7 (20.9 / 18.8);  11008 x 512 13.3 / 7.1
-//           (16.7 / 8.5);  8192 x 28672 75.3 / 42.0 (86.0 / 57.9)
-//   M = 16: 512 x 2048 5.5 / 3.4 (5.4 / 3.5);  1024 x 4096 5.6 / 5.4 (5.3 / 5.5);  2048 x 8192 7.8 / 8.5 (8.2 / 9.9);
-//           4096 x 4096 10.5 / 8.7 (11.0 / 10.4);  4096 x 8192 12.8 / 11.5 (13.3 / 14.2);  4096 x 11008 21.6 / 13.8
-//           (23.7 / 18.8);  11008 x 2048 24.9 / 10.8 (25.8 / 13.4);  8192 x 28672 79.2 / 42.3 (84.3 / 58.4)
+// Measured on B200 (graphs of launches over 512 MB of weights), generic against this one, us, K x N, block 32 column-wise
+// with zero points (row-wise).  Blocks of 16, and row-wise blocks of 128, lie within 5 % of these.
+//   M = 1:  4096 x 8192 13.4 / 10.9 (15.3 / 13.7);  8192 x 512 10.0 / 6.1 (13.1 / 7.0);  8192 x 4096 12.2 / 11.3 (14.8 / 14.1);
+//           2048 x 16384 13.7 / 8.8 (16.2 / 11.5);  4096 x 11008 16.9 / 13.5 (20.7 / 18.5);  8192 x 28672 66.6 / 39.7
+//           (80.0 / 55.4);  not taken: 2048 x 4096 5.0 / 6.6 (5.5 / 7.3);  4096 x 4096 7.5 / 8.1 (8.7 / 9.6)
+//           M = 2, 4 and 8: within 8 % of M = 1 on either side, the generic kernel slower with M (8192 x 28672: 77.4 / 40.1)
+//   M = 16: 512 x 2048 5.7 / 3.3 (5.7 / 3.3);  1536 x 4096 8.0 / 6.5 (8.7 / 7.0);  2048 x 2048 6.3 / 5.3 (7.0 / 5.6);
+//           4096 x 4096 10.9 / 8.5 (11.7 / 10.0);  2048 x 11008 12.7 / 8.1 (13.8 / 10.3, not taken);
+//           4096 x 11008 22.2 / 13.6 (25.3 / 18.6);  8192 x 28672 81.1 / 40.3 (88.2 / 55.8);  M = 9, 12: within 3 % of M = 16
+// The generic kernel is at its best at K = 1024 and 2048, where each of its warps has its minimum of four 64-k steps and no
+// more, and where N just fills its rounds of 32 columns per SM; there the cluster exchange here costs more than it
+// gains.  M = 16:
+//   2048 x 4096 6.6 / 7.0 (7.4 / 7.8);  4608 6.7 / 7.4 (7.5 / 8.4);  5120 8.1 / 7.5 (8.4 / 8.7);  7168 8.2 / 8.0 (8.6 / 9.3)
+//   1024 x 512 5.0 / 5.2 (5.0 / 5.2);  1024 5.2 / 5.2 (5.1 / 5.3);  8192 6.6 / 6.8 (7.3 / 7.4);  9216 6.7 / 7.1 (7.3 / 7.8);
+//   11008 7.3 / 5.2 (7.9 / 6.0)
+// Elsewhere the slower side is taken by 7 % at most (row-wise 2560 x 7168 10.0 / 10.5, with blocks of 128 9.7 / 10.4).
 bool gemm_tc_takes_skinny(int block, bool colwise, int M, int N, int K, const void* scales, const void* zp) {
   if (M > 16 || (colwise && block >= 64)) return false;
   if (reinterpret_cast<uintptr_t>(scales) % 16 != 0 || reinterpret_cast<uintptr_t>(zp) % 16 != 0) return false;
   const long long kn = (long long)K * N;
   if (M <= 8) return K >= 8192 || kn >= (1ll << 25);
+  const int round = 32 * (sm_count() > 0 ? sm_count() : 148);  // columns per round of the generic kernel
+  if (K == 2048 && N > round * 4 / 5 && (N <= round || !colwise)) return false;
+  if (K == 1024 && ((N > round * 17 / 10 && N <= 2 * round) || (N <= 1024 && !colwise))) return false;
   return !(N >= 8192 && K >= 2048 && kn <= (colwise ? 1ll << 24 : 1ll << 25));
 }
 

@@ -399,6 +399,16 @@ def test_workspace_up_to_16_rows(M, block, colwise, has_zp):
     assert written[:, :M].all(-1).sum() >= sms // 2 and not written[:, M:].any()
 
 
+def only_kernel_node(driver, graph):
+    """Launch parameters of the one kernel of a torch.cuda.CUDAGraph(keep_graph=True)."""
+    handle = driver.CUgraph(int(graph.raw_cuda_graph()))
+    err, nodes, count = driver.cuGraphGetNodes(handle, 8)
+    assert int(err) == 0 and count == 1
+    err, params = driver.cuGraphKernelNodeGetParams(nodes[0])
+    assert int(err) == 0
+    return params
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 2304, 8192), (17, 2304, 4096), (128, 1024, 4096), (200, 640, 4160), (512, 4096, 4096),
                                    (100, 384, 8064), (256, 4096, 4096), (40, 6144, 4096), (512, 1024, 2048)])
 def test_plan_names_the_split_that_is_launched(M, N, K):
@@ -420,8 +430,31 @@ def test_plan_names_the_split_that_is_launched(M, N, K):
         stream = torch.cuda.Stream()
         with torch.cuda.graph(graph, stream=stream):
             capi.gemm(block, colwise, M, N, K, a, qw, qs, None, out, stream=stream.cuda_stream, workspace=ws)
-        handle = driver.CUgraph(int(graph.raw_cuda_graph()))
-        err, nodes, count = driver.cuGraphGetNodes(handle, 8)
-        assert int(err) == 0 and count == 1
-        err, params = driver.cuGraphKernelNodeGetParams(nodes[0])
-        assert int(err) == 0 and params.gridDimX == plan["tiles"] * plan["split"], (params.gridDimX, plan)
+        params = only_kernel_node(driver, graph)
+        assert params.gridDimX == plan["tiles"] * plan["split"], (params.gridDimX, plan)
+
+
+@pytest.mark.parametrize("block,colwise,M,K,N,kernel", [
+    (32, True, 9, 2048, 4096, "gemv"), (32, True, 16, 2048, 4608, "gemv"), (32, True, 16, 2048, 5120, "gemm_tc"),
+    (32, True, 16, 2048, 3584, "gemm_tc"), (16, True, 12, 1024, 9216, "gemv"), (32, True, 16, 1024, 11008, "gemm_tc"),
+    (32, False, 9, 1024, 512, "gemv"), (32, False, 16, 1024, 2048, "gemm_tc"), (128, False, 16, 2048, 7168, "gemv"),
+    (32, False, 16, 1792, 4096, "gemm_tc"), (32, True, 8, 4096, 4096, "gemv"), (32, True, 1, 8192, 512, "gemm_tc"),
+    (64, True, 16, 8192, 4096, "gemv"), (64, True, 1, 8192, 28672, "gemv")])
+def test_which_kernel_takes_a_skinny_problem(block, colwise, M, K, N, kernel):
+    """The rule beside gemm_tc_takes_skinny, on both sides of its lines: the name of the kernel that is captured."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    from gemmlib_b200 import capi
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines lie at the rounds of 148 SMs")
+    a = torch.zeros(M, K, dtype=torch.float16, device="cuda")
+    qw = torch.zeros(K * N // 2, dtype=torch.uint8, device="cuda")
+    qs = torch.zeros(K * N // block, dtype=torch.float16, device="cuda")
+    out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    stream = torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):
+        capi.gemm(block, colwise, M, N, K, a, qw, qs, None, out, stream=stream.cuda_stream)
+    params = only_kernel_node(driver, graph)
+    err, name = driver.cuKernelGetName(params.kern) if int(params.kern) else driver.cuFuncGetName(params.func)
+    assert int(err) == 0 and (b"gemm_tc" in name) == (kernel == "gemm_tc"), name
