@@ -147,6 +147,22 @@ def test_leading_dimension_and_unaligned_source():
         assert_same(got, want, f"ld={ld} off={off}")
 
 
+@pytest.mark.parametrize("pad", [0, 1, 2, 3])
+@pytest.mark.parametrize("offset", [1, 2, 3, 8])
+@pytest.mark.parametrize("block,colwise", [(16, True), (128, True), (32, False)])
+def test_unaligned_rows(block, colwise, offset, pad):
+    """Rows at every even address modulo 16, of one alignment or of two in turn (odd leading dimension).  What lies
+    before, between and behind the rows is NaN and must not reach the result."""
+    K, N = 192 if block < 128 else 256, 96
+    ld = K + pad
+    base = torch.full((N * ld + 16,), float("nan"), dtype=torch.float16)
+    view = base[offset : offset + N * ld].view(N, ld)
+    view[:, :K] = gaussian_weight(N, K, seed=offset)
+    want = O.quant_prepack(block, colwise, np.ascontiguousarray(view[:, :K].numpy()), True)
+    dview = base.cuda()[offset : offset + N * ld].view(N, ld)[:, :K]
+    assert_same(gpu_quant(block, colwise, dview, True, ld=ld), want, f"ld={ld} offset={offset}")
+
+
 @pytest.mark.parametrize("cfg", [(32, True, True, 4096, 4096), (64, True, False, 4096, 11008)])
 def test_benchmark_shapes_bit_exact(cfg):
     """Full-size benchmark shapes (c3 / c2 weights) against the oracle."""
