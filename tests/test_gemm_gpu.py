@@ -171,18 +171,18 @@ def test_fused_bias_equals_separate_add(case):
                                   (128, True, False, 48, 1024, 4096), (16, True, True, 700, 256, 1024)],
                          ids=lambda c: "-".join(map(str, c)))
 def test_split_k_with_workspace(case):
-    """blkq4_fp16_gemm_ws_sm100: few output tiles, so K is split over several SMs through the
-    caller's workspace.  Same parity bars as the unsplit kernel; the flags part of the workspace
-    is back to zero afterwards; two runs agree bit for bit (partials are added in part order)."""
+    """blkq4_fp16_gemm_ws_sm100: few output tiles, so K is split over the CTAs of a cluster.  Same parity bars as the
+    unsplit kernel; two runs agree bit for bit (partials are added in part order).  The workspace is the caller's
+    opt-in only: the parts meet in distributed shared memory, and what lies in it stays."""
     from gemmlib_b200 import capi
 
     block, colwise, has_zp, M, N, K = case
     need = capi.gemm_workspace_size(M, N, K)
     assert need > 0, "the shape is meant to split"
-    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    assert capi.gemm_plan(M, N, K, need)["split"] > 1  # what the launch uses: test_plan_names_the_split_that_is_launched
+    ws = torch.full((need,), 0xA5, dtype=torch.uint8, device="cuda")
     check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
-    tiles = -(-M // min(256, -(-M // 16) * 16)) * -(-N // 128)
-    assert int(ws[: 4 * tiles].view(torch.int32).abs().sum()) == 0
+    assert (ws == 0xA5).all()
     w = gaussian_weight(N, K, seed=K + N)
     a = gaussian_act(M, K, seed=M).numpy()
     pw, ps, pz = O.quant_prepack(block, colwise, w.numpy(), has_zp)
@@ -302,12 +302,15 @@ def test_output_canaries_untouched():
 @pytest.mark.parametrize("M", [17, 64, 65, 128, 129])
 def test_half_filled_last_step(M, block, colwise, has_zp):
     """Tiles of up to 128 rows run in steps of 128 k: K an odd multiple of 64 leaves the last step half empty
-    (zero-filled), in whole rounds, split over K (17 steps of 128 k do not split, 20 do), and a single step."""
+    (zero-filled), split over K evenly (20 steps) and unevenly (17), in whole rounds (six steps make no two parts of
+    512 k), and a single step."""
     import torch
 
     from gemmlib_b200 import capi
 
-    for N, K in [(384, 2112), (256, 2496), (128, 64)]:
+    for N, K in [(384, 2112), (256, 2496), (384, 704), (128, 64)]:
+        split = capi.gemm_plan(M, N, K, max(256, capi.gemm_workspace_size(M, N, K)))["split"]
+        assert (split > 1) == (K > 2000)
         a, pw, ps, pz = kat_problem(block, colwise, has_zp, M, N, K)
         want = O.dequant_gemm(block, colwise, a, N, pw, ps, pz)
         nbytes = capi.gemm_workspace_size(M, N, K)
@@ -326,13 +329,13 @@ def test_half_filled_last_step(M, block, colwise, has_zp):
     (32, True, False, 19200, 1792)])                               # more tiles than SMs
 def test_skinny_problems_on_the_tensor_core_kernel(M, block, colwise, has_zp, N, K):
     """Up to 16 rows, blockings of the generic skinny kernel: the larger problems run on the tensor-core kernel.
-    Both sides of the rule, with and without a workspace, and with scales that are not 16-byte aligned (those
-    stay on the generic kernel), against the same bars."""
+    Both sides of the rule, with and without a workspace (which they leave alone: no SKINNY_WORKSPACE), and with scales
+    that are not 16-byte aligned (those stay on the generic kernel), against the same bars."""
     from gemmlib_b200 import capi
 
-    for ws in (None, torch.zeros(16 << 20, dtype=torch.uint8, device="cuda")):
+    for ws in (None, torch.full((16 << 20,), 0xA5, dtype=torch.uint8, device="cuda")):
         check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
-        assert ws is None or not ws[:512].any()
+        assert ws is None or (ws == 0xA5).all()
     if not colwise:
         return  # the generic kernel reads row-wise meta 16 bytes at a time
     w = gaussian_weight(N, K, seed=1)
@@ -359,9 +362,9 @@ def test_uneven_split(case):
     block, colwise, has_zp, M, N, K = case
     need = capi.gemm_workspace_size(M, N, K)
     assert need > 0 and capi.gemm_plan(M, N, K, need)["split"] > 1
-    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    ws = torch.full((need,), 0xA5, dtype=torch.uint8, device="cuda")
     check_gaussian(block, colwise, has_zp, M, N, K, workspace=ws)
-    assert not ws.any()
+    assert (ws == 0xA5).all()  # asked for, not used
     assert capi.gemm_plan(M, N, K, 0)["split"] == 1
 
 

@@ -29,6 +29,21 @@ def test_which_kernel_takes_which_problem():
     assert capi.gemm_workspace_size(256, 4096, 4096) > capi.static_scratch_size()  # the shape the static entry refuses
 
 
+def test_workspace_up_to_16_rows():
+    """gemm_workspace_size is 0 there (such calls use none); the size of a call that brings one all the same follows
+    the blocking: one flag word per SM and a 16 x 128 fp32 partial tile per CTA where the tiles are cut in ranges."""
+    ranges = 768 + 148 * 16 * 128 * 4
+    for m in (1, 8, 9, 16):
+        assert capi.gemm_workspace_size(m, 28672, 8192) == 0
+        assert capi.gemm_workspace_size_blocked(32, True, m, 28672, 8192) == ranges
+        assert capi.gemm_workspace_size_blocked(128, False, m, 28672, 1216) == ranges
+        assert capi.gemm_workspace_size_blocked(64, True, m, 28672, 8192) == 0  # the skinny kernels
+        assert capi.gemm_workspace_size_blocked(32, True, m, 4096, 8192) == 0   # a cluster split needs none
+    for m in (17, 64, 512):
+        assert capi.gemm_workspace_size_blocked(32, True, m, 28672, 8192) == capi.gemm_workspace_size(m, 28672, 8192) > 0
+    assert capi.gemm_workspace_size_blocked(48, True, 8, 28672, 8192) == 0
+
+
 @pytest.mark.parametrize("tiles,k_steps,units", [(224, 128, 148), (172, 64, 148), (86, 64, 74), (112, 128, 74),
                                                  (160, 16, 74), (448, 128, 74), (151, 8, 148), (300, 172, 148),
                                                  (32, 64, 74), (40, 172, 74)])
