@@ -1,4 +1,4 @@
-// Tensor-core W4A16 GEMM for sm_100a (M > 16): out[M,N] = A[M,K] x dequant(W4[K,N]).
+// Tensor-core W4A16 GEMM for sm_100a: out[M,N] = A[M,K] x dequant(W4[K,N]).
 //
 // Blackwell-native design: TMA-staged operands, in-kernel dequantization to fp16,
 // tcgen05.mma with fp32 accumulators in tensor memory (TMEM).  The product is
@@ -13,12 +13,13 @@
 // Measured with the operand staged in shared memory instead, the 16 KB written plus 16 KB
 // re-read per step, on top of the TMA traffic, cost a third of the step time.
 //
-// Two kernels share this design.  gemm_tc_kernel (this file; 16 < M < 256) gives every tile to one
-// CTA; gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
+// Two kernels share this design.  gemm_tc_kernel (this file) gives every tile to one CTA, or its K range to a
+// cluster of CTAs: M < 256, the larger skinny problems of gemm_tc_takes_skinny among them, and larger M with few
+// tiles.  gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
 //
 // Persistent CTAs (one per SM) walk the tile list.  Warp roles:
 //   warp 0      TMA producer of the activation tiles (128-byte swizzle)
-//   warp 1      MMA issuer (one elected lane); owns the TMEM allocation
+//   warp 1      MMA issuer (one elected thread); owns the TMEM allocation
 //   warps 2-5   epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
 //               through a second TMEM accumulator buffer where two fit
 //   warps 6-17  dequantizers, three groups of four warps on steps in turn: thread = one
@@ -26,8 +27,9 @@
 //   warp 18     TMA producer of the packed int4 weight tiles
 //   warp 19     TMA producer of their scales and zero points
 // A step is 64 k, or 128 k for tiles of up to 128 rows (struct Shape).
-// Stages are handed over with mbarriers; every wait is bounded and, on expiry, sets
-// an error word and drains the CTA instead of hanging the GPU.
+// Stages are handed over with mbarriers; every such wait, and every wait for another CTA's flag word, is bounded
+// and, on expiry, sets an error word and drains the CTA instead of hanging the GPU.  The cluster barriers of
+// a split have no limit of their own: every CTA of the cluster is resident and reaches them after bounded waits.
 //
 // The packed weight layout was designed for mma.sync register fragments (reference
 // src/mickey/blk_q4/f16_quant_sm80.cuh:362-417); a 16-byte run of a packed column
@@ -107,7 +109,7 @@ struct Params {
   //     count; a tile that straddles two ranges has its tail computed FIRST by the later CTA
   //     (partial tile, slot = that CTA) and its head LAST by the earlier CTA, which adds the partial.
   int split;
-  int k_per_item;      // 64-k steps per work item
+  int k_per_item;      // steps per work item
   int num_items;       // tiles * split
   int balanced;
   int k_steps;         // steps of a tile: K / 64, or / 128 rounded up for tiles of up to 128 rows
@@ -668,11 +670,14 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   const int sms = sm_count() > 0 ? sm_count() : 148;
   SplitPlan best{1, k_steps, 0, 0, 0};
   if (tiles > sms) {
-    // balanced ranges: every range longer than a tile (a cut tile then has exactly two parts), and
-    // only when whole rounds would leave more than a fifth of the SM time idle.  Measured on B200:
-    // 224 tiles of K = 8192 at M = 64: 98 -> 83 us; 172 tiles (M = 512, 4096 -> 11008): 55 -> 49 us;
-    // 256 tiles (M = 2048, N = K = 4096; 86 % busy in whole rounds): 62 -> 66 us, the extra work item
-    // and the fp32 exchange cost more than the balance gains, hence the threshold.
+    // balanced ranges: every range longer than a tile (a cut tile then has exactly two parts), and only when whole
+    // rounds would leave more than a fifth of the SM time idle.  The extra work item and the fp32 exchange cost about
+    // 4.5 us, whatever the balance gains.  Measured on B200, whole rounds / balanced, us (K x N):
+    //   M = 64, block 128: 8192 x 22528 (176 tiles, 59 % busy) 46.6 / 35.7; 25600 46.7 / 40.4; 28672 (76 %) 47.4 / 44.9;
+    //           above the line 32768 (86 %) 50.5 / 52.7; 36864 (97 %) 53.7 / 58.2; 4096 x 22528 24.7 / 20.6; 28672 25.4 / 24.4
+    //   M = 128: 8192 x 22528 56.2 / 48.3; 28672 60.5 / 58.9; 32768 65.9 / 66.3
+    //   M = 16, block 32: 8192 x 22528 44.4 / 31.5; 28672 44.8 / 38.5; 30720 (81 %, not taken) 45.1 / 40.7
+    // With few steps a tile the line comes too late: K = 2048, M = 64, N = 28672 14.7 / 15.8; M = 128, 4096 x 28672 31.3 / 32.4.
     const int rounds = (tiles + sms - 1) / sms;
     const long long total_steps = (long long)tiles * k_steps;
     static const bool off = getenv("BLKQ4_TC_NO_BALANCE") != nullptr;
@@ -686,10 +691,11 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
   }
   // Split only when every work item still gets an SM of its own (one round).  The parts exchange their partial tiles
   // through distributed shared memory, so they may be uneven and as many (of at least 512 k) as there are SMs for.
-  // The workspace stays the caller's opt-in (a split changes the order of the fp32 sums), of the size it has always
-  // been: that of the fp32 partial tiles of an even two- or four-way split, or one page of flags where K does not
-  // divide evenly.  A smaller one gets the split it would hold.  Up to 16 rows no opt-in is asked for: those
-  // calls never needed one.
+  // The workspace is the caller's opt-in (a split changes the order of the fp32 sums) and is not touched.  Its size is
+  // part of the interface - which calls split, and which the static-scratch entry refuses - and stays what it was
+  // when the parts met there: the fp32 partial tiles of an even two- or four-way split, or one page of flags where K
+  // does not divide evenly.  A smaller one gets the split it would hold.  Up to 16 rows no opt-in is asked for:
+  // those calls never needed one.
   auto even_split = [&](size_t avail, size_t* bytes) {
     int split = 1;
     *bytes = 0;
@@ -788,10 +794,11 @@ namespace {
 // M >= 256 when the pair tiles fill at least one round of the device's pairs (the pair kernel has no
 // split-K: M = 512 on a 4096-wide layer, 32 pair tiles, runs faster split over single CTAs).  With a
 // workspace, and when whole rounds would idle more than a fifth of the pairs' time, the work is cut in
-// balanced ranges.  Measured on B200: 86 pair tiles on 74 pairs (M = 512, 4096 -> 11008) 52 -> 43 us;
-// 112 tiles (M = 256, K = 8192, N = 28672) 103 -> 100 us; 128 tiles (c3, 86 % busy in whole rounds)
-// 57 -> 61 us and 448 tiles (M = 1024) unchanged: one more accumulator hand-over per pair and the fp32
-// exchange of a 128 KB partial tile per CTA cost what the balance gains there.
+// balanced ranges.  Measured on B200, whole rounds / balanced: 86 pair tiles on 74 pairs (M = 512, 4096 -> 11008)
+// 45.3 / 42.5 us; 156 tiles (M = 512, N = 19968) 78 / 70; 100 tiles (N = 12800) 46.5 / 47.8; 112 tiles (M = 256,
+// K = 8192, N = 28672) 96.2 / 96.7; above the line 128 tiles (M = 2048, N = K = 4096, 86 % busy in whole rounds)
+// 51.8 / 60.4 and 448 tiles (M = 1024, K = 8192, N = 28672) 332 / 338: one more accumulator hand-over per pair and the
+// fp32 exchange of a 128 KB partial tile per CTA cost what the balance gains there.
 struct PairPlan {
   bool use;
   int BM, m_tiles, items, balanced;
@@ -816,7 +823,7 @@ PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
   static const bool balance_off = getenv("BLKQ4_TC_NO_BALANCE") != nullptr;
   // Fewer tiles than pairs: the one-CTA kernel splits K.  (The pair kernel can do it too - ranges shorter
   // than a tile, a tile finished from several partial tiles - but measured slower: M = 512, K = N = 4096
-  // 35.8 vs 28.7 us, K = 11008 54.0 vs 48.6 us; a 128 KB fp32 partial tile per CTA is a dear exchange.)
+  // 34.5 vs 20.9 us, K = 11008 50.9 vs 40.1 us; a 128 KB fp32 partial tile per CTA is a dear exchange.)
   if (pl.items < pairs) return pl;
   // Balanced ranges need a workspace (one flag word and one fp32 partial tile per CTA), ranges of at least
   // eight steps, and pay when whole rounds would idle more than a fifth of the pairs' time.
@@ -939,7 +946,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   // neighbouring packed columns would otherwise all fall on the same banks.
   // No swizzle on 64-byte rows: the dequantizers' 16-byte loads of eight neighbouring packed
   // columns (64 bytes apart) do conflict four ways, but a 64-byte TMA swizzle that removes the
-  // conflicts measured 1-2 % SLOWER on the same GPU (c3 59.2 vs 58.2 us): those loads are not on
+  // conflicts measured 1-2 % SLOWER on the same GPU (M = 2048, 4096 x 4096: 59.2 vs 58.2 us): those loads are not on
   // the critical path, the extra XOR per load is.
   ok = ok && encode_tensor_map_2d(&tm_pack, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)K, (uint64_t)(N / 2),
                        (uint32_t)sk, TILE_N / 2, sk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);

@@ -276,7 +276,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     w_producer_done:;
     }
   } else if (warp == 1) {
-    // =============================== MMA issuer: the leader's lane 0 =================================
+    // =============================== MMA issuer: one elected thread of the leader =================================
     if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_f16(2 * TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);

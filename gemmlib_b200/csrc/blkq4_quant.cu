@@ -13,11 +13,12 @@
 // 16 columns (128 k of 8 columns for column-wise blocks of 128), so that a load instruction covers whole
 // 128-byte lines and the meta entries of a warp share sectors.
 //
-// What the arithmetic may cost: at HBM's rate an SM has to finish a weight every 1/13 of a cycle, so the budget is
-// ~9 instructions per weight.  One weight takes ~5: see quantize_pair and assemble_word.  Measured on B200
-// (4096 x 11008, block 64, zero points, 114 MB): 27.9 us before, with 14 instructions per weight, four of them
-// float-to-integer conversions and min / max on quarter- and half-rate pipes and the scale's divisions repeated by
-// every lane of a block.
+// What the arithmetic may cost: at HBM's rate an SM moves 22 bytes a cycle (6.5 TB/s, 148 SMs, 1.97 GHz), i.e. finishes
+// 9 weights of 2.5 bytes, so with every issue slot used (128 threads a cycle) the budget is 14 instructions per
+// weight.  The column-wise kernel executes 9.7 (13.7 M warp instructions for 45 M weights), ~5 of them in quantize_pair
+// and assemble_word, and issues in 65 % of the cycles.  Measured on B200 (4096 x 11008, block 64, zero points, 114 MB):
+// 28.5 us with 14 in the conversion alone - float-to-integer conversions and min / max on quarter- and half-rate pipes,
+// the scale's divisions repeated by every lane of a block - and 22.8 us now (0.77 of the measured copy bandwidth).
 #include "blkq4_common.cuh"
 
 namespace blkq4 {

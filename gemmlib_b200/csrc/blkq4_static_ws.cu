@@ -1,7 +1,8 @@
-// blkq4_fp16_gemm_static_ws_sm100: the split-K tensor-core GEMM with its workspace taken from a
-// file-scope device array instead of from the caller.  Nothing on this path allocates: the array
-// is part of the loaded module, its address is looked up once per device, and problems whose
-// workspace would not fit are refused.  The reference has no counterpart.
+// blkq4_fp16_gemm_static_ws_sm100: the tensor-core GEMM with its workspace taken from a file-scope device array
+// instead of from the caller.  Nothing on this path allocates: the array is part of the loaded module and its
+// address is looked up once per device.  Only balanced ranges read and write it; a K split exchanges its
+// partial tiles in shared memory, but its workspace size remains the interface's measure of what this entry takes:
+// problems whose split-K workspace would not fit are refused.  The reference has no counterpart.
 #include <cstddef>
 #include <cstdint>
 #include <atomic>
@@ -14,9 +15,9 @@
 
 namespace {
 
-// 12 MiB.  Covers, e.g., M = 512 on 4096-wide layers (64 tiles, two-way split: 8.4 MB) and a 148-SM
-// part's largest two-way split at BM = 256 (74 tiles x 128 KB = 9.7 MB).  A problem whose preferred
-// plan needs more - e.g. M = 256, N = K = 4096: 32 tiles split four ways, 12.6 MB - is refused; call
+// 12 MiB.  Holds the balanced ranges of tiles of up to 160 rows (148 x 80 KB); larger ones run in whole rounds.
+// By the size of its split-K workspace a problem is taken - e.g. M = 512 on 4096-wide layers (64 tiles, two-way
+// split: 8.4 MB) - or, like M = 256, N = K = 4096 (32 tiles, four-way: 12.6 MB), refused; call
 // blkq4_fp16_gemm_sm100 (no split) or blkq4_fp16_gemm_ws_sm100 with memory of your own for those.
 constexpr size_t kStaticScratchBytes = 12u << 20;
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
@@ -63,7 +64,7 @@ int reset_static_scratch(cudaStream_t stream) {
   std::string why;
   void* scratch = static_scratch(why);
   if (!scratch) return -1;
-  // flags: one word per output tile, at most one tile per SM and split; 64 KB is far beyond any plan
+  // flags: one word per SM; 64 KB is far beyond any plan
   return cudaMemsetAsync(scratch, 0, 64 * 1024, stream) == cudaSuccess ? 0 : -1;
 }
 }  // namespace blkq4

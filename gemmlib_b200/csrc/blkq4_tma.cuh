@@ -92,11 +92,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 // True in exactly one lane of the (converged) warp.  Single-thread roles must be entered through this and
-// not through `lane == 0`: under elect.sync the compiler knows that one thread is active and moves the
-// operands of tcgen05.mma, tcgen05.commit and the bulk-tensor copies straight into uniform registers;
-// under an ordinary lane test it has to assume that they differ between lanes and wraps every such
-// instruction in a loop over their values.  Measured on B200: 54 against 9 cycles per tcgen05.mma
-// (N = 16, issue-bound), 370 cycles per iteration of a wait + expect_tx + copy loop under the lane test.
+// not through `lane == 0`.  Measured on B200: 9 against 54 cycles per tcgen05.mma (N = 16, issue-bound), and 370
+// cycles per iteration of a wait + expect_tx + copy loop under the lane test.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
