@@ -153,7 +153,17 @@ std::vector<torch::Tensor>& g_dropped = *new std::vector<torch::Tensor>;  // out
 std::atomic<bool> g_any_dropped{false};
 std::atomic<int> g_graph_workspaces{0};
 
-// A user object's destructor may not call CUDA, so it leaves the buffer to the next call of graph_workspace.
+// Gives the buffers of graphs that are gone back to the allocator.
+int free_dropped_workspaces(void*) {
+  std::vector<torch::Tensor> dropped;
+  std::lock_guard<std::mutex> lock(g_dropped_mutex);
+  dropped.swap(g_dropped);
+  g_any_dropped.store(false);
+  return 0;  // the lock goes first, then the tensors
+}
+
+// A user object's destructor may run on any thread and may not call CUDA, so it leaves the buffer to the
+// interpreter's next pending calls, or, should that queue be full, to the next call of graph_workspace.
 void drop_graph_workspace(void* held) {
   auto* buffer = static_cast<torch::Tensor*>(held);
   {
@@ -163,17 +173,13 @@ void drop_graph_workspace(void* held) {
   }
   delete buffer;
   --g_graph_workspaces;
+  if (Py_IsInitialized()) Py_AddPendingCall(free_dropped_workspaces, nullptr);
 }
 
 // The workspace of at least `nbytes` for the capture that is under way on the device's current stream (`stream`);
 // nothing when none is, an empty tensor when the graph cannot take one.  Called with the GIL held.
 c10::optional<torch::Tensor> graph_workspace(int device, uintptr_t stream_handle, int64_t nbytes) {
-  if (g_any_dropped.load()) {
-    std::vector<torch::Tensor> dropped;
-    std::lock_guard<std::mutex> lock(g_dropped_mutex);
-    dropped.swap(g_dropped);
-    g_any_dropped.store(false);
-  }
+  if (g_any_dropped.load()) free_dropped_workspaces(nullptr);
   const auto stream = reinterpret_cast<cudaStream_t>(stream_handle);
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
