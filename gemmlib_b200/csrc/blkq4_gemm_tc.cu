@@ -18,14 +18,14 @@
 // tiles.  gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
 //
 // Persistent CTAs (one per SM) walk the tile list.  Warp roles:
-//   warp 0      TMA producer of the activation tiles (128-byte swizzle)
-//   warp 1      MMA issuer (one elected thread); owns the TMEM allocation
-//   warps 2-5   epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
+//   warps 0-3   epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
 //               through a second TMEM accumulator buffer where two fit
-//   warps 6-17  dequantizers, three groups of four warps on steps in turn: thread = one
+//   warps 4-15  dequantizers, three groups of four warps on steps in turn: thread = one
 //               weight column n of the tile (TMEM lane n), 64 k = 32 TMEM columns
-//   warp 18     TMA producer of the packed int4 weight tiles
-//   warp 19     TMA producer of their scales and zero points
+//   warp 16     TMA producer of the activation tiles (128-byte swizzle)
+//   warp 17     TMA producer of the packed int4 weight tiles
+//   warp 18     TMA producer of their scales and zero points
+//   warp 19     MMA issuer (one elected thread); owns the TMEM allocation
 // A step is 64 k, or 128 k for tiles of up to 128 rows (struct Shape).
 // Stages are handed over with mbarriers; every such wait, and every wait for another CTA's flag word, is bounded
 // and, on expiry, sets an error word and drains the CTA instead of hanging the GPU.  The cluster barriers of
@@ -58,21 +58,27 @@ using namespace tc;
 // (TMA -> shared memory -> MMA) is short but its stages are up to 32 KB.
 constexpr int kWarpsPerDeqGroup = 4;  // one warp per quarter of the TMEM lanes
 constexpr int kNumEpiWarps = 4;
-constexpr int kFirstDeqWarp = 2 + kNumEpiWarps;
 
 // Shape of the one-CTA kernel, by activation rows per tile.
+//   MAXM    most activation rows of a tile: the pitch of the activation stages, so that the MMA thread's
+//           operand addresses are constants
 //   KSUB    64-k sub-steps per pipeline step: what the roles hand to one another at a time
-//   ACT/WS  shared-memory stages of the activations / of the packed weights and meta
-//   DS      stages of dequantized weights in tensor memory (32 * KSUB columns each)
+//   RING    stages of the activations in shared memory and of dequantized weights in tensor memory (32 * KSUB
+//           columns each): one ring, so that one barrier collects everything the MMAs of a step read
+//   WS      shared-memory stages of the packed weights and meta
 //   NG      dequantizer groups of four warps, on steps in turn
-template <int KSUB_, int ACT_, int WS_, int DS_, int NG_>
+template <int MAXM_, int KSUB_, int RING_, int WS_, int NG_>
 struct Shape {
-  static constexpr int KSUB = KSUB_, ACT = ACT_, WS = WS_, DS = DS_, NG = NG_;
+  static constexpr int MAXM = MAXM_, KSUB = KSUB_, RING = RING_, WS = WS_, NG = NG_;
   static constexpr int kStepK = BLOCK_K * KSUB;
-  static constexpr int kWeightProducerWarp = kFirstDeqWarp + 4 * NG;
-  static constexpr int kMetaProducerWarp = kWeightProducerWarp + 1;
-  static constexpr int kThreads = 32 * (kMetaProducerWarp + 1);
-  static_assert(ACT <= DS, "an activation stage is released by the MMA_DONE barrier of its step");
+  static constexpr int kActSubBytes = MAXM * 128, kActBytes = kActSubBytes * KSUB;
+  static constexpr int kDeqTmemCols = RING * KSUB * kDeqCols;
+  static constexpr int kFirstDeqWarp = kNumEpiWarps;
+  static constexpr int kActProducerWarp = kFirstDeqWarp + 4 * NG;
+  static constexpr int kWeightProducerWarp = kActProducerWarp + 1;
+  static constexpr int kMetaProducerWarp = kActProducerWarp + 2;
+  static constexpr int kMmaWarp = kActProducerWarp + 3;
+  static constexpr int kThreads = 32 * (kMmaWarp + 1);
 };
 // Up to 128 rows the math of a 64-k step is shorter than its hand-overs (three barriers, a commit, the polls
 // of five roles: ~400 cycles with loads, conversion and MMAs all left out), so a step carries 128 k.  Measured on
@@ -80,9 +86,9 @@ struct Shape {
 // M = 17 50.2 vs 40.3, M = 128 67.2 vs 58.0; M = 100, 4096 -> 11008 20.5 vs 16.3; M = 32, 4096 x 4096 10.1 vs 9.5.
 // Above 128 rows two 64-k steps of activations per stage leave three stages only (rowwise M = 333: 24.8 vs 27.4 us).
 // Groups: two / three / four at M = 64: 47.3 / 43.9 / 44.5 us; M = 32, 4096 x 4096: 9.7 / 9.5 / 10.3 us.
-using ShapeSmall = Shape<2, 6, 10, 6, 3>;  // BM <= 64:  two accumulators + six stages of 64 TMEM columns = 512
-using ShapeMid = Shape<2, 4, 8, 4, 3>;     // BM <= 128: two accumulators + four stages = 512
-using ShapeLarge = Shape<1, 6, 6, 8, 3>;   // BM <= 256
+using ShapeSmall = Shape<64, 2, 6, 10, 3>;  // two accumulators + six stages of 64 TMEM columns = 512
+using ShapeMid = Shape<128, 2, 4, 8, 3>;    // two accumulators + four stages = 512
+using ShapeLarge = Shape<256, 1, 6, 6, 3>;
 // k per pipeline step of the kernel that takes tiles of BM rows
 inline int step_k(int BM) { return BM <= 64 ? ShapeSmall::kStepK : BM <= 128 ? ShapeMid::kStepK : ShapeLarge::kStepK; }
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s: far beyond any legitimate wait
@@ -189,13 +195,12 @@ __device__ __forceinline__ bool next_item(const Params& p, ItemCursor& c, Item& 
 
 struct SmemPlan {
   uint32_t act, pack, scale, zp, out, bars, total;
-  uint32_t act_bytes;
 };
-__host__ __device__ inline SmemPlan make_plan(int BM, int kStages, int act_stages, int ksub, uint32_t out_bytes = 0) {
-  SmemPlan p;
-  p.act_bytes = (uint32_t)(BM * 128 * ksub);  // BM is a multiple of 16: 1024-aligned sub-tiles of 64 k
+// rows: activation rows a stage has room for (a multiple of 8: 1024-aligned sub-tiles of 64 k)
+__host__ __device__ constexpr SmemPlan make_plan(int rows, int kStages, int act_stages, int ksub, uint32_t out_bytes = 0) {
+  SmemPlan p{};
   uint32_t o = 0;
-  p.act = o;   o += act_stages * p.act_bytes;
+  p.act = o;   o += act_stages * (uint32_t)(rows * 128 * ksub);
   p.pack = o;  o += kStages * kPackTileBytes * ksub;
   p.scale = o; o += kStages * kScaleTileBytes * ksub;
   p.zp = o;    o += kStages * kZpTileBytes * ksub;
@@ -205,16 +210,16 @@ __host__ __device__ inline SmemPlan make_plan(int BM, int kStages, int act_stage
   return p;
 }
 
-// Barrier slots (8 bytes each) inside the barrier block.  An "MMA done" barrier frees the activation stage and
-// the stage of dequantized weights of its step.
-#define BLKQ4_TC_BARRIER_SLOTS(WS, ACT, DS, DONE)                                                     \
+// Barrier slots (8 bytes each) inside the barrier block.  A "step full" barrier collects what the MMAs of a step
+// read: the bytes of its activation tile and the arrivals of its dequantizer warps.  An "MMA done" barrier frees the
+// activation stage and the stage of dequantized weights of its step.
+#define BLKQ4_TC_BARRIER_SLOTS(WS, RING)                                                                            \
   constexpr int kStages = (WS);                                                                                    \
-  constexpr int BAR_ACT_FULL = 0;                        /* [kActStages] activation tile landed (-> MMA issuer) */  \
-  constexpr int BAR_FULL = BAR_ACT_FULL + (ACT);         /* [kStages] packed weights + meta landed (-> dequantizers) */ \
+  constexpr int BAR_FULL = 0;                            /* [kStages] packed weights + meta landed (-> dequantizers) */ \
   constexpr int BAR_PACK_FREE = BAR_FULL + kStages;      /* [kStages] packed weights / meta read (-> producer) */   \
-  constexpr int BAR_DEQ_FULL = BAR_PACK_FREE + kStages;  /* [kDeqStages] dequantized stage in TMEM (-> MMA issuer) */ \
-  constexpr int BAR_MMA_DONE = BAR_DEQ_FULL + (DS);  /* MMAs of step it retired, index it % count */ \
-  constexpr int BAR_ACC_FULL = BAR_MMA_DONE + (DONE);    /* [2] accumulator complete */                             \
+  constexpr int BAR_STEP_FULL = BAR_PACK_FREE + kStages; /* [ring] operands of the step are there (-> MMA issuer) */ \
+  constexpr int BAR_MMA_DONE = BAR_STEP_FULL + (RING);   /* [ring] MMAs of the step retired */                      \
+  constexpr int BAR_ACC_FULL = BAR_MMA_DONE + (RING);    /* [2] accumulator complete */                             \
   constexpr int BAR_ACC_EMPTY = BAR_ACC_FULL + 2;        /* [2] accumulator drained by the epilogue */              \
   constexpr int BAR_COUNT = BAR_ACC_EMPTY + 2;                                                                      \
   static_assert(BAR_COUNT * 8 + 16 <= 512, "barrier block too small");
@@ -224,14 +229,14 @@ __global__ void __launch_bounds__(S::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_pack,
                const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
                const Params p) {
-  constexpr int KSUB = S::KSUB, kActStages = S::ACT, kDeqStages = S::DS, kStepK = S::kStepK;
+  constexpr int KSUB = S::KSUB, kRing = S::RING, kStepK = S::kStepK;
   constexpr int kStepCols = kDeqCols * KSUB, kStepPackBytes = kPackTileBytes * KSUB;
   constexpr int kStepScaleBytes = kScaleTileBytes * KSUB, kStepZpBytes = kZpTileBytes * KSUB;
-  BLKQ4_TC_BARRIER_SLOTS(S::WS, kActStages, kDeqStages, kDeqStages)
+  BLKQ4_TC_BARRIER_SLOTS(S::WS, kRing)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const SmemPlan plan = make_plan(p.BM, kStages, kActStages, KSUB);
+  constexpr SmemPlan plan = make_plan(S::MAXM, kStages, kRing, KSUB);
   const uint32_t bars = base + plan.bars;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + plan.bars + BAR_COUNT * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + plan.bars + BAR_COUNT * 8 + 8);
@@ -247,13 +252,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   asm volatile("griddepcontrol.launch_dependents;");
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kActStages; ++i) mbar_init(bar(BAR_ACT_FULL + i), 1);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bar(BAR_FULL + i), 2);  // the packed-tile producer and the meta producer, each with its bytes
       mbar_init(bar(BAR_PACK_FREE + i), kWarpsPerDeqGroup);
     }
-    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_DEQ_FULL + i), kWarpsPerDeqGroup);
-    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(bar(BAR_STEP_FULL + i), kWarpsPerDeqGroup + 1);  // the dequantizer warps; the activation producer, with its bytes
+      mbar_init(bar(BAR_MMA_DONE + i), 1);
+    }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(BAR_ACC_FULL + i), 1);
       mbar_init(bar(BAR_ACC_EMPTY + i), kNumEpiWarps);
@@ -261,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     *abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 1) {
+  if (warp == S::kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
                  "r"(tmem_cols)
@@ -273,29 +279,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
+  if (warp == S::kActProducerWarp) {
     // ========================= TMA producer: activations ========================
-    // Stage sa = it % kActStages is free once the commit group of step it - kActStages retired.
+    // A stage is free once the MMAs of the step that used it last have retired.
     if (elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // activations belong to stream order
-      uint32_t it = 0;
+      const uint32_t tx = (uint32_t)(p.BM * 128 * KSUB);
+      uint32_t s = 0, free_par = 1;  // (the first round finds fresh barriers: the phase before their first one is complete)
       ItemCursor cur = first_item(p);
       Item item;
       while (next_item(p, cur, item)) {
         const int m_tile = item.tile % p.m_tiles;
-        for (int ks = item.ks0; ks < item.ks0 + item.count; ++ks, ++it) {
-          const int sa = it % kActStages;
-          if (it >= (uint32_t)kActStages) {
-            const uint32_t g = it - kActStages;  // the stage's last user
-            if (!mbar_wait(bar(BAR_MMA_DONE + g % kDeqStages), (g / kDeqStages) & 1, abort_flag, 0x100 | sa))
-              goto act_producer_done;
-          }
-          const uint32_t fb = bar(BAR_ACT_FULL + sa);
-          mbar_arrive_expect_tx(fb, plan.act_bytes);
+        for (int ks = item.ks0; ks < item.ks0 + item.count; ++ks) {
+          if (!mbar_wait(bar(BAR_MMA_DONE + s), free_par, abort_flag, 0x100 | s)) goto act_producer_done;
+          const uint32_t fb = bar(BAR_STEP_FULL + s);
+          mbar_arrive_expect_tx(fb, tx);
 #pragma unroll
           for (int u = 0; u < KSUB; ++u)  // past the end of K the copy fills zeros
-            tma_load_2d(base + plan.act + sa * plan.act_bytes + u * (p.BM * 128), &tm_act, ks * kStepK + u * BLOCK_K,
+            tma_load_2d(base + plan.act + s * S::kActBytes + u * S::kActSubBytes, &tm_act, ks * kStepK + u * BLOCK_K,
                         m_tile * p.BM, fb);
+          if (++s == kRing) { s = 0; free_par ^= 1u; }
         }
       }
     act_producer_done:;
@@ -339,75 +342,59 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       }
     w_producer_done:;
     }
-  } else if (warp == 1) {
+  } else if (warp == S::kMmaWarp) {
     // =============================== MMA issuer =================================
-    // One thread drives the tensor pipe; a 128x256x16 MMA takes 128 cycles, so the waits, address
-    // arithmetic, four issues and the commit of a 64-k step must fit in 512 cycles of
-    // dependent scalar code.  Hence: ring indices and parities are carried incrementally
-    // (no division), the four MMAs of 64 k are one asm block, and the barrier polls take
-    // the slow (bounded, instrumented) path only when the first poll fails.
+    // One thread drives the tensor pipe: eight 128 x BM x 16 MMAs of a 128-k step take 130 cycles at BM = 16, 260 at
+    // 64.  The dequantizer warps of the thread's scheduler compete with it for issue slots, so what the step holds besides
+    // its MMAs sets the pace up to 128 rows.  Hence: one barrier per step; the ring unrolled, so that operand
+    // and barrier addresses are constants; the poll of step i + 1 (non-blocking) ahead of the MMAs of step i; the
+    // bounded, instrumented wait only where a poll fails; the last warp of the CTA (the scheduler favours it).  Measured on
+    // B200, the loop alone beside three warps of dependent FMAs per scheduler, cycles a step at N = 16: two barriers and
+    // ring indices 321, one barrier 262, the ring unrolled 143, as the last warp 131.
     if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
       const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);  // LBO field
       const uint32_t act_lo0 = desc_lo_flags | (((base + plan.act) >> 4) & 0x3FFFu);
-      const uint32_t act_lo_step = plan.act_bytes >> 4, act_lo_sub = (uint32_t)p.BM * 128u >> 4;
       const uint32_t a_tmem0 = tmem_base + (uint32_t)p.a_col0;
-      uint32_t s = 0, sa = 0, par_s = 0, par_sa = 0, tcount = 0;
-      uint32_t ab = 0, par_acc = 0;
-      // The barriers of step i + 1 are polled (without blocking) BEFORE the MMAs of step i are
-      // issued, so that the poll's round trip to shared memory overlaps the issue instead of
-      // extending the dependent chain of the next step.
-      bool ready_a = false, ready_d = false;
-#define BLKQ4_TC_MMA_ITEM(COUNT)                                                                                    \
-  {                                                                                                                 \
-    if (tcount >= (uint32_t)p.acc_bufs &&                                                                           \
-        !mbar_wait(bar(BAR_ACC_EMPTY + ab), par_acc ^ 1u, abort_flag, 0x200 | ab))                                  \
-      goto mma_done;                                                                                                \
-    tc_fence_after();                                                                                               \
-    const uint32_t d_tmem = tmem_base + ab * (uint32_t)p.BM;                                                        \
-    for (int ks = 0; ks < (COUNT); ++ks) {                                                                          \
-      const uint32_t bar_a = bar(BAR_ACT_FULL) + 8u * sa, bar_d = bar(BAR_DEQ_FULL) + 8u * s;                       \
-      if (!ready_a && !mbar_try_wait(bar_a, par_sa) && !mbar_wait(bar_a, par_sa, abort_flag, 0x210 | sa))           \
-        goto mma_done;                                                                                              \
-      if (!ready_d && !mbar_try_wait(bar_d, par_s) && !mbar_wait(bar_d, par_s, abort_flag, 0x220 | s))              \
-        goto mma_done;                                                                                              \
-      tc_fence_after();                                                                                             \
-      /* 16 k = 8 TMEM columns of the weights, 32 bytes (2 descriptor units) of the activation row */              \
-      const uint32_t a_tmem = a_tmem0 + s * kStepCols, b_lo = act_lo0 + sa * act_lo_step;                           \
-      const uint32_t done_bar = bar(BAR_MMA_DONE) + 8u * s;                                                         \
-      if (++s == kDeqStages) { s = 0; par_s ^= 1u; }                                                                \
-      if (++sa == kActStages) { sa = 0; par_sa ^= 1u; }                                                             \
-      ready_a = mbar_test_wait(bar(BAR_ACT_FULL) + 8u * sa, par_sa);                                                \
-      ready_d = mbar_test_wait(bar(BAR_DEQ_FULL) + 8u * s, par_s);                                                  \
-      umma_f16_ts_x4(d_tmem, a_tmem, b_lo, desc_hi, idesc, ks > 0 ? 1u : 0u);                                       \
-      _Pragma("unroll") for (int u = 1; u < KSUB; ++u)                                                              \
-        umma_f16_ts_x4(d_tmem, a_tmem + u * kDeqCols, b_lo + u * act_lo_sub, desc_hi, idesc, 1u);                   \
-      umma_commit(done_bar);                                                                                        \
-    }                                                                                                               \
-    umma_commit(bar(BAR_ACC_FULL + ab));                                                                            \
-    if (++ab == (uint32_t)p.acc_bufs) { ab = 0; par_acc ^= 1u; }                                                    \
-  }
-      if (!p.balanced) {
-        for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++tcount) {
-          const int count = min(p.k_per_item, p.k_steps - item % p.split * p.k_per_item);
-          BLKQ4_TC_MMA_ITEM(count)
-        }
-      } else {
-        int pos = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x, p.min_part);
-        const int end = range_bound(p.total_steps, p.k_steps, (int)gridDim.x, (int)blockIdx.x + 1, p.min_part);
-        int to_tile_end = p.k_steps - pos % p.k_steps;
-        for (; pos < end; ++tcount) {
-          const int count = min(to_tile_end, end - pos);
-          BLKQ4_TC_MMA_ITEM(count)
-          pos += count;
-          to_tile_end = p.k_steps;
+      ItemCursor cur = first_item(p);
+      Item item;
+      uint32_t tcount = 0, ab = 0, par_acc = 0, par = 0;
+      bool ready = false;
+      if (!next_item(p, cur, item)) goto mma_done;
+      {
+      uint32_t left = (uint32_t)item.count, accumulate = 0, d_tmem = tmem_base;
+      for (;; par ^= 1u) {
+#pragma unroll
+        for (int s = 0; s < kRing; ++s) {
+          const uint32_t full = bar(BAR_STEP_FULL + s);
+          if (!ready && !mbar_try_wait(full, par) && !mbar_wait(full, par, abort_flag, 0x220 | s)) goto mma_done;
+          tc_fence_after();
+          ready = s + 1 < kRing ? mbar_test_wait(full + 8u, par) : mbar_test_wait(bar(BAR_STEP_FULL), par ^ 1u);
+          // 16 k = 8 TMEM columns of the weights, 32 bytes (2 descriptor units) of the activation row
+#pragma unroll
+          for (int u = 0; u < KSUB; ++u)
+            umma_f16_ts_x4(d_tmem, a_tmem0 + s * kStepCols + u * kDeqCols,
+                           act_lo0 + ((s * S::kActBytes + u * S::kActSubBytes) >> 4), desc_hi, idesc, u > 0 ? 1u : accumulate);
+          umma_commit(bar(BAR_MMA_DONE + s));
+          accumulate = 1;
+          if (--left == 0) {
+            umma_commit(bar(BAR_ACC_FULL + ab));
+            if (!next_item(p, cur, item)) goto mma_done;
+            left = (uint32_t)item.count;
+            accumulate = 0;
+            if (++ab == (uint32_t)p.acc_bufs) { ab = 0; par_acc ^= 1u; }
+            if (++tcount >= (uint32_t)p.acc_bufs && !mbar_wait(bar(BAR_ACC_EMPTY + ab), par_acc ^ 1u, abort_flag, 0x200 | ab))
+              goto mma_done;
+            tc_fence_after();
+            d_tmem = tmem_base + ab * (uint32_t)p.BM;
+          }
         }
       }
-#undef BLKQ4_TC_MMA_ITEM
+      }
     mma_done:;
     }
-  } else if (warp < 2 + kNumEpiWarps) {
+  } else if (warp < kNumEpiWarps) {
     // =============================== epilogue ===================================
     // A warp reads the TMEM lanes of its quarter (warp id % 4): lane = weight column n of
     // the tile, TMEM column = activation row m.  For one m the 32 lanes hold 32
@@ -517,7 +504,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           p.ws_flags[item.slot] = 0u;
       }
     }
-  } else if (warp < S::kWeightProducerWarp) {
+  } else {
     // =============================== dequantizers ===============================
     // The groups of four warps take steps in turn, so that a group has as many step times as there are
     // groups for the dependent chain wait -> load -> convert -> tcgen05.st -> arrive of one step.
@@ -527,7 +514,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     // nibble positions when n % 16 < 8 and 8 bits further up otherwise (the thread of n +- 8
     // reads the same bytes).  Per 64 k it reads the column's 64 bytes and writes 32 TMEM
     // columns: column j = fp16 pair k = (2j, 2j + 1).
-    const int group = (warp - kFirstDeqWarp) / kWarpsPerDeqGroup;
+    const int group = (warp - S::kFirstDeqWarp) / kWarpsPerDeqGroup;
     const int n_l = 32 * (warp & 3) + lane;
     const int np_l = 8 * (n_l >> 4) + (n_l & 7);
     const uint32_t rot_lo = (n_l & 8) ? 30u : 6u, rot_hi = (n_l & 8) ? 26u : 2u;
@@ -540,11 +527,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     }
     with_block_shift(p.block_shift, p.has_zp, [&](auto bsh, auto zp) {
     for (uint32_t it = group; it < total_its; it += S::NG) {
-      const int s = it % kStages, d = it % kDeqStages;
-      if (it >= (uint32_t)kDeqStages) {
-        const uint32_t g = it - kDeqStages;  // the TMEM stage's last user
-        if (!mbar_wait(bar(BAR_MMA_DONE + d), (g / kDeqStages) & 1, abort_flag, 0x410 | d)) break;
-      }
+      const int s = it % kStages, d = it % kRing;
+      // the TMEM stage's last user has retired (nobody's in the first round, which finds fresh barriers)
+      if (!mbar_wait(bar(BAR_MMA_DONE + d), ((it / kRing) & 1) ^ 1u, abort_flag, 0x410 | d)) break;
       if (!mbar_wait(bar(BAR_FULL + s), (it / kStages) & 1, abort_flag, 0x400 | s)) break;
       tc_fence_after();
       const uint8_t* pk = base_ptr + plan.pack + s * kStepPackBytes + np_l * kStepK;
@@ -563,7 +548,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(bar(BAR_DEQ_FULL + d));
+        mbar_arrive(bar(BAR_STEP_FULL + d));
         mbar_arrive(bar(BAR_PACK_FREE + s));
       }
     }
@@ -588,11 +573,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     const int rows = min(p.BM, p.M - m0);
     const int slice = 2 * ((p.BM + 2 * split - 1) / (2 * split));
     const uint32_t region = base + plan.act;  // [part][slice][128] fp32
-    if (warp >= 2 && warp < S::kWeightProducerWarp) {
+    if (warp < S::kActProducerWarp) {
       // a warp may read the TMEM lanes of its quarter: the epilogue and dequantizer warps share the columns
       const int n_l = 32 * (warp & 3) + lane;
       const uint32_t lane_base = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
-      for (int c0 = 32 * ((warp - 2) >> 2); c0 < rows; c0 += 32 * (S::NG + 1)) {
+      for (int c0 = 32 * (warp >> 2); c0 < rows; c0 += 32 * (S::NG + 1)) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(lane_base + (uint32_t)c0, v);
         tmem_ld_wait();
@@ -635,7 +620,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) __nanosleep(50000);  // let copies in flight land
   __syncthreads();
-  if (warp == 1) {
+  if (warp == S::kMmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols)
                  : "memory");
@@ -727,29 +712,28 @@ using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params
 struct KernelChoice {
   Kern kern;
   int threads, which;  // which: index of the per-device caches
-  SmemPlan plan;
-  size_t max_smem;     // of the largest tile the kernel takes
+  size_t smem;
+  int deq_cols;        // tensor memory of the dequantized stages
 };
 std::atomic<int> g_granted_smem[6][64];
 
 KernelChoice choose_kernel(bool colwise, int BM) {
   KernelChoice c;
-  auto pick = [&](auto shape, int idx, int max_rows) {
+  auto pick = [&](auto shape, int idx) {
     using S = decltype(shape);
     c.kern = colwise ? (Kern)gemm_tc_kernel<true, S> : (Kern)gemm_tc_kernel<false, S>;
     c.threads = S::kThreads;
     c.which = 2 * idx + (colwise ? 1 : 0);
-    c.plan = make_plan(BM, S::WS, S::ACT, S::KSUB);
-    c.max_smem = make_plan(max_rows, S::WS, S::ACT, S::KSUB).total;
+    c.smem = make_plan(S::MAXM, S::WS, S::RING, S::KSUB).total;
+    c.deq_cols = S::kDeqTmemCols;
   };
-  if (BM <= 64) pick(ShapeSmall{}, 0, 64);
-  else if (BM <= 128) pick(ShapeMid{}, 1, 128);
-  else pick(ShapeLarge{}, 2, 256);
+  if (BM <= ShapeSmall::MAXM) pick(ShapeSmall{}, 0);
+  else if (BM <= ShapeMid::MAXM) pick(ShapeMid{}, 1);
+  else pick(ShapeLarge{}, 2);
   return c;
 }
 
 // Clusters of `split` CTAs of the kernel that are resident at once on the current device, 0 when it cannot say.
-// Asked with the largest shared-memory plan of the kernel, so that the answer holds for every BM.
 int resident_clusters(const KernelChoice& kc, int split) {
   static std::atomic<int> cache[6][kMaxSplit + 1][64];
   int dev = 0;
@@ -764,10 +748,10 @@ int resident_clusters(const KernelChoice& kc, int split) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(sm_count() / split * split);
   cfg.blockDim = dim3(kc.threads);
-  cfg.dynamicSmemBytes = kc.max_smem;
+  cfg.dynamicSmemBytes = kc.smem;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (ensure_dynamic_smem(kc.kern, kc.max_smem, g_granted_smem[kc.which]) != cudaSuccess ||
+  if (ensure_dynamic_smem(kc.kern, kc.smem, g_granted_smem[kc.which]) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, kc.kern, &cfg) != cudaSuccess || n < 0) {
     cudaGetLastError();
     return 0;
@@ -916,9 +900,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   p.out = out;
   p.bias = bias;
   // tensor memory: accumulators first, then the dequantized stages
-  const int deq_cols = p.BM <= 64 ? ShapeSmall::DS * ShapeSmall::KSUB * kDeqCols
-                       : p.BM <= 128 ? ShapeMid::DS * ShapeMid::KSUB * kDeqCols
-                                     : ShapeLarge::DS * ShapeLarge::KSUB * kDeqCols;
+  const int deq_cols = choose_kernel(colwise, p.BM).deq_cols;
   p.acc_bufs = (2 * p.BM + deq_cols <= 512) ? 2 : 1;
   p.a_col0 = p.acc_bufs * p.BM;
   {
@@ -1031,11 +1013,11 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   p.total_steps = sp.balanced ? num_tiles * p.k_steps : 0;
   p.ws_flags = reinterpret_cast<unsigned*>(workspace);
   p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + sp.flags_bytes);
-  cudaError_t e = ensure_dynamic_smem(kc.kern, kc.plan.total, g_granted_smem[kc.which]);
+  cudaError_t e = ensure_dynamic_smem(kc.kern, kc.smem, g_granted_smem[kc.which]);
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kc.threads);
-  cfg.dynamicSmemBytes = kc.plan.total;
+  cfg.dynamicSmemBytes = kc.smem;
   cfg.stream = stream;
   // BLKQ4_GEMM_EARLY_WEIGHT_FETCH: programmatic stream serialization, see the kernel's entry
   cudaLaunchAttribute attr[2];

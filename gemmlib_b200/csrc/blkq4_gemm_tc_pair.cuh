@@ -11,15 +11,15 @@
 // step: 16 KB of activations written, 16 KB read.
 //
 // Protocol (leader = cluster rank 0; every barrier the MMA thread waits on lives in the leader):
-//   STEP_FULL[s]  (the slots named DEQ_FULL) count 9: the leader's activation producer arrives with
+//   STEP_FULL[s]  count 9: the leader's activation producer arrives with
 //                 expect_tx of BOTH halves of the step's activations, and the four dequantizer warps of
 //                 each CTA arrive once their part of the step's weights is in tensor memory (the peer's
 //                 remotely).  Both activation producers issue their TMA load with .cta_group::2, which
 //                 lets the copy into the peer's own shared memory complete its bytes on the leader's
 //                 barrier.
-//   MMA_DONE[g]   tcgen05.commit with a two-CTA multicast: the copy in each CTA frees that CTA's
+//   MMA_DONE[s]   tcgen05.commit with a two-CTA multicast: the copy in each CTA frees that CTA's
 //                 activation stage and dequantized stage.
-//   ACC_FULL      same multicast commit, to both epilogues; ACC_EMPTY count 8, like DEQ_FULL.
+//   ACC_FULL      same multicast commit, to both epilogues; ACC_EMPTY count 8, arrivals as on STEP_FULL.
 //   FULL / PACK_FREE (weight ring) stay local to each CTA.
 // The loads here carry no cluster multicast: every CTA copies its own rows.  All waits are bounded;
 // the two CTAs meet at a cluster barrier before either frees its tensor memory or exits.
@@ -39,16 +39,13 @@ constexpr int kPairActStages = 8;     // 16 KB each
 constexpr int kDeqStages = 8;         // dequantized weights in tensor memory, 32 columns each
 constexpr int kDeqGroups = 2;         // warp groups taking k steps in turn (three or four measured slower)
 constexpr int kNumDeqWarps = 4 * kDeqGroups;
+constexpr int kFirstDeqWarp = 2 + kNumEpiWarps;
 constexpr int kWeightProducerWarp = kFirstDeqWarp + kNumDeqWarps;  // last warp
 constexpr int kPairWeightStages = 6;  // 5.5 KB each; deeper rings measured no faster
-constexpr int kPairCommitSteps = 1;   // a commit per two steps measured no faster
 // fp16 staging of a CTA's 128 x 256 output tile: the epilogue empties the accumulator into it, hands
 // the accumulator back, and only then writes global memory, under the next tile's MMAs
 constexpr uint32_t kPairOutBytes = 128u * 256u * 2u;
-// one "MMAs retired" barrier per commit group a waiter may look back to: the deeper of the two rings
-constexpr int kPairDoneBars = (kPairActStages > kDeqStages ? kPairActStages : kDeqStages) / kPairCommitSteps + 1;
 static_assert(kPairActStages == kDeqStages, "one barrier per step serves both rings");
-static_assert(kDeqStages % kPairCommitSteps == 0, "rings are released per commit group");
 
 // Arrival on a barrier of the peer CTA.  What it publishes lives in tensor memory and is ordered by
 // tcgen05.wait::st / tcgen05.fence::before_thread_sync, so the arrive carries no cluster-scope release
@@ -164,13 +161,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_pack,
                     const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
                     const Params p) {
-  constexpr int kActStages = kPairActStages, kDoneBars = kPairDoneBars, kCommitSteps = kPairCommitSteps;
-  BLKQ4_TC_BARRIER_SLOTS(WS, kPairActStages, kDeqStages, kPairDoneBars)
+  constexpr int kActStages = kPairActStages;
+  BLKQ4_TC_BARRIER_SLOTS(WS, kDeqStages)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const SmemPlan plan = make_plan(kPairRows, kStages, kActStages, 1, kPairOutBytes);
-  const uint32_t act_stride = (plan.act_bytes + 1023u) & ~1023u;
+  constexpr SmemPlan plan = make_plan(kPairRows, kStages, kActStages, 1, kPairOutBytes);
+  constexpr uint32_t act_stride = kPairRows * 128;
   const uint32_t bars = base + plan.bars;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + plan.bars + BAR_COUNT * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + plan.bars + BAR_COUNT * 8 + 8);
@@ -188,13 +185,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
   asm volatile("griddepcontrol.launch_dependents;");
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kActStages; ++i) mbar_init(bar(BAR_ACT_FULL + i), 1);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bar(BAR_FULL + i), 1);
       mbar_init(bar(BAR_PACK_FREE + i), kWarpsPerDeqGroup);
     }
-    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_DEQ_FULL + i), 1 + 2 * kWarpsPerDeqGroup);  // "step full"
-    for (int i = 0; i < kDoneBars; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
+    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_STEP_FULL + i), 1 + 2 * kWarpsPerDeqGroup);  // "step full"
+    for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(BAR_ACC_FULL + i), 1);
       mbar_init(bar(BAR_ACC_EMPTY + i), 2 * kNumEpiWarps);
@@ -228,13 +224,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       while (walk.next(item, ks0, count, role)) {
         const int m_tile = p.n_fastest ? item / p.n_pairs : item % p.m_tiles;
         for (int ks = ks0; ks < ks0 + count; ++ks, ++it) {
-          const int sa = it % kActStages;
-          if (it >= (uint32_t)kActStages) {
-            const uint32_t g = (it - kActStages) / kCommitSteps;
-            if (!mbar_wait(bar(BAR_MMA_DONE + g % kDoneBars), (g / kDoneBars) & 1, abort_flag, 0x100 | sa))
-              goto act_producer_done;
-          }
-          const uint32_t fb = bar(BAR_DEQ_FULL + sa);  // the step's one barrier
+          const int sa = it % kActStages;  // (the first round finds fresh barriers: the phase before their first one is complete)
+          if (!mbar_wait(bar(BAR_MMA_DONE + sa), ((it / kActStages) & 1) ^ 1u, abort_flag, 0x100 | sa)) goto act_producer_done;
+          const uint32_t fb = bar(BAR_STEP_FULL + sa);  // the step's one barrier
           if (rank == 0) mbar_arrive_expect_tx(fb, 2u * (uint32_t)half * 128u);
           tma_load_2d_pair(base + plan.act + sa * act_stride, &tm_act, ks * BLOCK_K,
                            m_tile * p.BM + (int)rank * half, map_to_cta(fb, 0));
@@ -277,50 +269,44 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     }
   } else if (warp == 1) {
     // =============================== MMA issuer: one elected thread of the leader =================================
+    // The ring is unrolled, so that operand and barrier addresses are constants (see the one-CTA kernel).
     if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_f16(2 * TILE_N, p.BM);
       const uint32_t desc_hi = (uint32_t)(make_sw128_kmajor_desc(0) >> 32);
       const uint32_t desc_lo_flags = (uint32_t)(make_sw128_kmajor_desc(0) & 0xFFFFFFFFu);
       const uint32_t act_lo0 = desc_lo_flags | (((base + plan.act) >> 4) & 0x3FFFu);
-      const uint32_t act_lo_step = act_stride >> 4;
       const uint32_t a_tmem0 = tmem_base + kAcol0;
-      uint32_t s = 0, par_s = 0, gdone = 0, it = 0, tcount = 0;
+      PairWalk walk(p, pair, num_pairs);
+      int item, ks0, count, role;
+      uint32_t par = 0, par_acc = 0;
       // the barrier of step i + 1 is polled (without blocking) before the MMAs of step i are issued, so
       // that the poll's round trip overlaps the issue
       bool ready = false;
-#define BLKQ4_TC_PAIR_MMA_ITEM(COUNT)                                                                              \
-  {                                                                                                                 \
-    if (tcount >= 1u && !mbar_wait_cluster(bar(BAR_ACC_EMPTY), (tcount - 1u) & 1u, abort_flag, 0x200)) goto mma_done; \
-    tc_fence_after();                                                                                               \
-    for (int ks = 0; ks < (COUNT); ++ks, ++it) {                                                                    \
-      const uint32_t bar_d = bar(BAR_DEQ_FULL) + 8u * s;                                                            \
-      if (!ready && !mbar_try_wait(bar_d, par_s) && !mbar_wait(bar_d, par_s, abort_flag, 0x220 | s)) goto mma_done; \
-      tc_fence_after();                                                                                             \
-      const uint32_t a_tmem = a_tmem0 + s * kDeqCols, b_lo = act_lo0 + s * act_lo_step;                             \
-      if (++s == kDeqStages) { s = 0; par_s ^= 1u; }                                                                \
-      ready = mbar_test_wait(bar(BAR_DEQ_FULL) + 8u * s, par_s);                                                    \
-      umma_f16_ts_x4_pair(tmem_base, a_tmem, b_lo, desc_hi, idesc, ks > 0 ? 1u : 0u);                               \
-      if (it % kCommitSteps == kCommitSteps - 1) {                                                                  \
-        umma_commit_pair(bar(BAR_MMA_DONE) + 8u * gdone);                                                           \
-        if (++gdone == kDoneBars) gdone = 0;                                                                        \
-      }                                                                                                             \
-    }                                                                                                               \
-    umma_commit_pair(bar(BAR_ACC_FULL));                                                                            \
-  }
-      if (!p.balanced) {
-        for (int item = pair; item < p.num_items; item += num_pairs, ++tcount) BLKQ4_TC_PAIR_MMA_ITEM(k_steps)
-      } else {
-        int pos = range_bound(p.total_steps, k_steps, num_pairs, pair);
-        const int end = range_bound(p.total_steps, k_steps, num_pairs, pair + 1);
-        int to_tile_end = k_steps - pos % k_steps;
-        for (; pos < end; ++tcount) {
-          const int count = min(to_tile_end, end - pos);
-          BLKQ4_TC_PAIR_MMA_ITEM(count)
-          pos += count;
-          to_tile_end = k_steps;
+      if (!walk.next(item, ks0, count, role)) goto mma_done;
+      {
+      uint32_t left = (uint32_t)count, accumulate = 0;
+      for (;; par ^= 1u) {
+#pragma unroll
+        for (int s = 0; s < kDeqStages; ++s) {
+          const uint32_t full = bar(BAR_STEP_FULL + s);
+          if (!ready && !mbar_try_wait(full, par) && !mbar_wait(full, par, abort_flag, 0x220 | s)) goto mma_done;
+          tc_fence_after();
+          ready = s + 1 < kDeqStages ? mbar_test_wait(full + 8u, par) : mbar_test_wait(bar(BAR_STEP_FULL), par ^ 1u);
+          umma_f16_ts_x4_pair(tmem_base, a_tmem0 + s * kDeqCols, act_lo0 + s * (act_stride >> 4), desc_hi, idesc, accumulate);
+          umma_commit_pair(bar(BAR_MMA_DONE + s));
+          accumulate = 1;
+          if (--left == 0) {
+            umma_commit_pair(bar(BAR_ACC_FULL));
+            if (!walk.next(item, ks0, count, role)) goto mma_done;
+            left = (uint32_t)count;
+            accumulate = 0;
+            if (!mbar_wait_cluster(bar(BAR_ACC_EMPTY), par_acc, abort_flag, 0x200)) goto mma_done;
+            par_acc ^= 1u;
+            tc_fence_after();
+          }
         }
       }
-#undef BLKQ4_TC_PAIR_MMA_ITEM
+      }
     mma_done:;
     }
   } else if (warp < 2 + kNumEpiWarps) {
@@ -579,7 +565,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int np_l = 8 * (n_l >> 4) + (n_l & 7);
     const uint32_t rot_lo = (n_l & 8) ? 30u : 6u, rot_hi = (n_l & 8) ? 26u : 2u;
     const uint32_t tmem_row = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + kAcol0;
-    const uint32_t deq_full_leader = map_to_cta(bar(BAR_DEQ_FULL), 0);
+    const uint32_t deq_full_leader = map_to_cta(bar(BAR_STEP_FULL), 0);
     uint32_t total_its = 0;
     {
       PairWalk walk(p, pair, num_pairs);
@@ -589,10 +575,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     with_block_shift(p.block_shift, p.has_zp, [&](auto bsh, auto zp) {
     for (uint32_t it = group; it < total_its; it += kDeqGroups) {
       const int s = it % kStages, d = it % kDeqStages;
-      if (it >= (uint32_t)kDeqStages) {
-        const uint32_t g = (it - kDeqStages) / kCommitSteps;
-        if (!mbar_wait(bar(BAR_MMA_DONE + g % kDoneBars), (g / kDoneBars) & 1, abort_flag, 0x410 | d)) break;
-      }
+      if (!mbar_wait(bar(BAR_MMA_DONE + d), ((it / kDeqStages) & 1) ^ 1u, abort_flag, 0x410 | d)) break;
       if (!mbar_wait(bar(BAR_FULL + s), (it / kStages) & 1, abort_flag, 0x400 | s)) break;
       tc_fence_after();
       const uint8_t* pk = base_ptr + plan.pack + s * kPackTileBytes + np_l * 64;
@@ -607,7 +590,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if (rank == 0) mbar_arrive(bar(BAR_DEQ_FULL + d));
+        if (rank == 0) mbar_arrive(bar(BAR_STEP_FULL + d));
         else mbar_arrive_remote(deq_full_leader + 8u * (uint32_t)d);
         mbar_arrive(bar(BAR_PACK_FREE + s));
       }
