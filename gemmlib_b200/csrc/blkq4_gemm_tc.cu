@@ -89,6 +89,13 @@ struct Shape {
 using ShapeSmall = Shape<64, 2, 6, 10, 3>;  // two accumulators + six stages of 64 TMEM columns = 512
 using ShapeMid = Shape<128, 2, 4, 8, 3>;    // two accumulators + four stages = 512
 using ShapeLarge = Shape<256, 1, 6, 6, 3>;
+// Activation rows of a tile, a multiple of `unit`: as few tiles of up to 256 rows as there can be, all of one height.
+// Measured on B200 against tiles of 256 and a remainder, whose MMAs multiply rows that are not there, us: M = 300, 4096 x 28672
+// 88.1 / 73.3; M = 333, 1024 x 28672 34.0 / 31.9; M = 400, 8192 x 22528 135.3 / 125.6.
+inline int tile_rows(int M, int unit) {
+  const int tiles = (M + 255) / 256, rows = (M + tiles - 1) / tiles;
+  return (rows + unit - 1) / unit * unit;
+}
 // k per pipeline step of the kernel that takes tiles of BM rows
 inline int step_k(int BM) { return BM <= 64 ? ShapeSmall::kStepK : BM <= 128 ? ShapeMid::kStepK : ShapeLarge::kStepK; }
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s: far beyond any legitimate wait
@@ -190,6 +197,18 @@ __device__ __forceinline__ bool next_item(const Params& p, ItemCursor& c, Item& 
   }
   return true;
 }
+
+// Owner of row group r4 of a split tile whose parts own `slice4` groups each: r4 / slice4 for r4 < 64 (a tile has at
+// most 256 rows) without a division.
+__host__ __device__ constexpr int slice_inverse(int slice4) { return 65536 / slice4 + 1; }
+__host__ __device__ constexpr int slice_owner(int r4, int inv) { return (r4 * inv) >> 16; }
+constexpr bool slice_owner_is_exact() {
+  for (int s = 1; s <= 64; ++s)
+    for (int r = 0; r < 64; ++r)
+      if (slice_owner(r, slice_inverse(s)) != r / s) return false;
+  return true;
+}
+static_assert(slice_owner_is_exact());
 
 // ---- shared-memory plan ---------------------------------------------------------------------
 
@@ -458,21 +477,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       }
       const float* src_ws = p.ws_partials + (size_t)item.slot * tile_floats + n_l;
       const int n = n_tile * TILE_N + quarter * 32 + lane;
-      const int m0 = m_tile * p.BM;
+      const int m0 = m_tile * p.BM, m_end = min(p.M, m0 + p.BM);  // a chunk of 32 rows may reach into the next tile
       // Lanes pair up (n even / odd) so that every store carries two adjacent n (4 bytes per
       // lane, 128 contiguous bytes per warp): the even lane writes the even rows m of a
       // 32-row chunk, the odd lane the odd rows, each with its partner's value alongside.
       const int odd = lane & 1;
       const bool n_ok = (n | 1) < p.N;  // N is a multiple of 16: the pair is in or out together
       for (int c0 = 0; c0 < p.BM; c0 += 32) {
-        if (m0 + c0 >= p.M) break;  // warp-uniform
+        if (m0 + c0 >= m_end) break;  // warp-uniform
         uint32_t r[32];
         load_acc(c0, r);
         if (item.role == 2) {
           const float* sq = src_ws + (size_t)c0 * TILE_N;
           float f[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = (m0 + c0 + j < p.M) ? __ldcg(sq + (size_t)j * TILE_N) : 0.0f;
+          for (int j = 0; j < 32; ++j) f[j] = (m0 + c0 + j < m_end) ? __ldcg(sq + (size_t)j * TILE_N) : 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + f[j]);
         }
@@ -490,7 +509,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           const float got = __shfl_xor_sync(0xffffffffu, give, 1);          // partner's n, my row
           __half2 v = odd ? __floats2half2_rn(got, mine) : __floats2half2_rn(mine, got);
           if (add_bias) v = __hadd2(v, bias2);
-          if (n_ok && m < p.M) *reinterpret_cast<__half2*>(dst) = v;
+          if (n_ok && m < m_end) *reinterpret_cast<__half2*>(dst) = v;
           dst += row_step;
           m += 2;
         }
@@ -556,13 +575,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   }
 
   if (p.split > 1) {
-    // ---- split K: the cluster's CTAs hold one fp32 partial tile each.  Part q owns rows [q slice, (q + 1) slice): every
+    // ---- split K: the cluster's CTAs hold one fp32 partial tile each.  Part q owns `slice4` groups of four rows: every
     //      CTA stores the other parts' rows of its partial tile into THEIR shared memory (over the activation
     //      ring, idle once the MMAs of all parts have retired) and then adds up its own rows, in part order, with
-    //      all its threads.  With the partial tiles in global memory and one finishing CTA, which read them chunk by
-    //      chunk from L2 (one round trip per 32 rows and part), more parts cost more than they gave; 4096 x 4096,
-    //      us: M = 128, four parts 16.7 -> 11.0; M = 256, four parts 28.0 -> 15.7; M = 512, two parts 24.9 -> 20.9;
-    //      K = 4096, N = 1024, M = 128: four parts through memory 15.4, eight 21.7, eight in a cluster 8.2.
+    //      all its threads.  Four rows of a column travel as one 16-byte store, laid out [part][row group][column]
+    //      so that the lanes of a warp are contiguous on both sides; each part starts with its own rows, so that the parts
+    //      of a cluster write to different CTAs at a time; the loops are rolled, because they run a few times per launch from
+    //      a cold instruction cache.  Measured on B200 against 4-byte stores from an unrolled loop with a branch per row, us:
+    //      M = 16, 4096 x 4096, four parts 8.8 / 7.8; M = 48, 2048 x 1024 6.0 / 4.9; M = 256, 4096 x 4096, four parts 15.6 / 14.8
+    //      (16.3 where all parts start with row 0); M = 512, two parts 21.4 / 18.6; M = 300, 8192 x 1024, five parts 16.5 / 12.5.
+    //      With the partial tiles in global memory and one finishing CTA, which read them chunk by
+    //      chunk from L2 (one round trip per 32 rows and part), more parts cost more than they gave: K = 4096, N = 1024,
+    //      M = 128: four parts through memory 15.4 us, eight 21.7.
     //      A cluster's CTAs are co-resident by construction, so nobody waits for a CTA that is not running.
     asm volatile("griddepcontrol.wait;" ::: "memory");  // all warps store to the output
     __syncwarp();
@@ -571,47 +595,61 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     const int split = p.split, part = (int)blockIdx.x % split, tile = (int)blockIdx.x / split;
     const int n_tile = tile / p.m_tiles, m0 = (tile % p.m_tiles) * p.BM;
     const int rows = min(p.BM, p.M - m0);
-    const int slice = 2 * ((p.BM + 2 * split - 1) / (2 * split));
-    const uint32_t region = base + plan.act;  // [part][slice][128] fp32
+    const int slice4 = (p.BM / 4 + split - 1) / split;
+    const uint32_t region = base + plan.act;
     if (warp < S::kActProducerWarp) {
       // a warp may read the TMEM lanes of its quarter: the epilogue and dequantizer warps share the columns
       const int n_l = 32 * (warp & 3) + lane;
       const uint32_t lane_base = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
-      for (int c0 = 32 * (warp >> 2); c0 < rows; c0 += 32 * (S::NG + 1)) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(lane_base + (uint32_t)c0, v);
+      const int inv = slice_inverse(slice4);
+      const int chunks = (rows + 15) / 16, first = chunks * part / split;  // BM is a multiple of 16
+#pragma unroll 1
+      for (int i = warp >> 2; i < chunks; i += S::NG + 1) {
+        const int c0 = 16 * (first + i < chunks ? first + i : first + i - chunks);
+        uint32_t v[16];
+        tmem_ld_32x32b_x16(lane_base + (uint32_t)c0, v);
         tmem_ld_wait();
-        int owner = c0 / slice, rr = c0 - owner * slice;
-        uint32_t dst = map_to_cta(region + (uint32_t)(((part * slice + rr) * TILE_N + n_l) * 4), (uint32_t)owner);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (c0 + j < rows) {
-            st_shared_cluster_f32(dst, v[j]);
-            dst += TILE_N * 4;
-            if (++rr == slice) {
-              rr = 0;
-              if (++owner < split) dst = map_to_cta(region + (uint32_t)((part * slice * TILE_N + n_l) * 4), (uint32_t)owner);
-            }
-          }
+        for (int g = 0; g < 4; ++g) {
+          const int r4 = c0 / 4 + g, owner = slice_owner(r4, inv), rg = r4 - owner * slice4;
+          st_shared_cluster_v4(map_to_cta(region + (uint32_t)(((part * slice4 + rg) * TILE_N + n_l) * 16), (uint32_t)owner),
+                               v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
         }
       }
     }
     cluster_sync_all();
-    const int r0 = part * slice, mine = min(slice, rows - r0);
-    const float* src = reinterpret_cast<const float*>(base_ptr + plan.act);
-    for (int idx = threadIdx.x; idx < mine * (TILE_N / 2); idx += S::kThreads) {
-      const int rr = idx / (TILE_N / 2), n2 = 2 * (idx % (TILE_N / 2)), n = n_tile * TILE_N + n2;
-      if (n >= p.N) continue;
-      float2 sum = make_float2(0.0f, 0.0f);
+    const int g0 = part * slice4, mine = min(slice4, (rows + 3) / 4 - g0);
+    const float4* src = reinterpret_cast<const float4*>(base_ptr + plan.act);
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < mine * TILE_N; idx += S::kThreads) {  // whole warps
+      const int n = n_tile * TILE_N + (idx % TILE_N);
+      float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
       for (int q = 0; q < split; ++q) {
-        const float2 f = *reinterpret_cast<const float2*>(src + (size_t)(q * slice + rr) * TILE_N + n2);
+        const float4 f = src[q * slice4 * TILE_N + idx];
         sum.x += f.x;
         sum.y += f.y;
+        sum.z += f.z;
+        sum.w += f.w;
       }
-      __half2 v = __floats2half2_rn(sum.x, sum.y);
-      // the bias is added to the rounded result in fp16, as above
-      if (p.bias) v = __hadd2(v, *reinterpret_cast<const __half2*>(p.bias + n));
-      *reinterpret_cast<__half2*>(p.out + (size_t)(m0 + r0 + rr) * p.N + n) = v;
+      // lanes pair up (n even / odd): the even one stores rows 0 and 1 of both columns, the odd one rows 2 and 3
+      const int odd = lane & 1;
+      const float got0 = __shfl_xor_sync(0xffffffffu, odd ? sum.x : sum.z, 1);
+      const float got1 = __shfl_xor_sync(0xffffffffu, odd ? sum.y : sum.w, 1);
+      __half2 h0 = odd ? __floats2half2_rn(got0, sum.z) : __floats2half2_rn(sum.x, got0);
+      __half2 h1 = odd ? __floats2half2_rn(got1, sum.w) : __floats2half2_rn(sum.y, got1);
+      const int m = m0 + 4 * (g0 + idx / TILE_N) + 2 * odd;
+      if (n < p.N) {  // N is a multiple of 16: the pair is in or out together
+        // the bias is added to the rounded result in fp16, as above
+        if (p.bias) {
+          const __half2 b = *reinterpret_cast<const __half2*>(p.bias + (n & ~1));
+          h0 = __hadd2(h0, b);
+          h1 = __hadd2(h1, b);
+        }
+        __half* dst = p.out + (size_t)m * p.N + (n & ~1);
+        if (m < p.M) *reinterpret_cast<__half2*>(dst) = h0;
+        if (m + 1 < p.M) *reinterpret_cast<__half2*>(dst + p.N) = h1;
+      }
     }
   }
 
@@ -649,9 +687,10 @@ struct SplitPlan {
 };
 
 SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
-  const int BM = M >= 256 ? 256 : ((M + 15) / 16) * 16;
+  const int BM = tile_rows(M, 16);
   const int tiles = ((M + BM - 1) / BM) * ((N + TILE_N - 1) / TILE_N);
   const int k_steps = (K + step_k(BM) - 1) / step_k(BM);
+  const int ws_rows = M >= 256 ? 256 : BM;  // of a partial tile in the workspace: its size is part of the interface
   const int sms = sm_count() > 0 ? sm_count() : 148;
   SplitPlan best{1, k_steps, 0, 0, 0};
   if (tiles > sms) {
@@ -669,7 +708,7 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
     if (!off && total_steps < (1ll << 30) / sms && total_steps / sms >= k_steps + 2 * min_part(step_k(BM)) &&
         (double)tiles < 0.80 * rounds * sms) {
       const size_t flags = ((size_t)sms * sizeof(unsigned) + 255) & ~(size_t)255;
-      const size_t total = flags + (size_t)sms * BM * TILE_N * sizeof(float);
+      const size_t total = flags + (size_t)sms * ws_rows * TILE_N * sizeof(float);
       if (total <= ws_bytes_available) best = SplitPlan{1, k_steps, 1, flags, total};
     }
     return best;
@@ -686,7 +725,7 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
     *bytes = 0;
     for (int parts = 2; parts <= 4; parts *= 2) {
       const size_t flags = ((size_t)tiles * sizeof(unsigned) + 255) & ~(size_t)255;
-      const size_t total = flags + (size_t)tiles * (parts - 1) * BM * TILE_N * sizeof(float);
+      const size_t total = flags + (size_t)tiles * (parts - 1) * ws_rows * TILE_N * sizeof(float);
       if (k_steps % parts != 0 || (k_steps / parts) * step_k(BM) < 512 || tiles * parts > sms || total > avail) continue;
       split = parts;
       *bytes = total;
@@ -798,7 +837,7 @@ PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
   if (M < pair_min_m || pair_off) return pl;
   const int sms = sm_count() > 0 ? sm_count() : 148;
   const int pairs = sms / 2;
-  pl.BM = M >= 256 ? 256 : ((M + 31) / 32) * 32;
+  pl.BM = tile_rows(M, 32);
   pl.m_tiles = (M + pl.BM - 1) / pl.BM;
   pl.items = pl.m_tiles * (((N + TILE_N - 1) / TILE_N + 1) / 2);
   const int k_steps = K / BLOCK_K;
@@ -812,7 +851,7 @@ PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
   // Balanced ranges need a workspace (one flag word and one fp32 partial tile per CTA), ranges of at least
   // eight steps, and pay when whole rounds would idle more than a fifth of the pairs' time.
   const size_t flags = ((size_t)sms * sizeof(unsigned) + 255) & ~(size_t)255;
-  const size_t total = flags + (size_t)sms * pl.BM * TILE_N * sizeof(float);
+  const size_t total = flags + (size_t)sms * (M >= 256 ? 256 : pl.BM) * TILE_N * sizeof(float);  // part of the interface
   const bool can_balance = !balance_off && total_steps < (1ll << 30) / pairs && total_steps / pairs >= 8 &&
                            (double)pl.items < balance_below * rounds * pairs && total <= ws_bytes_available;
   pl.use = true;
@@ -893,13 +932,13 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   if (gt) p.gt = *gt;
   p.M = M; p.N = N; p.K = K; p.block = block;
   p.block_shift = block == 16 ? 4 : block == 32 ? 5 : block == 64 ? 6 : 7;
-  p.BM = M >= 256 ? 256 : ((M + 15) / 16) * 16;
+  p.BM = tile_rows(M, 16);
   p.m_tiles = (M + p.BM - 1) / p.BM;
   p.n_tiles = (N + TILE_N - 1) / TILE_N;
   p.has_zp = zp != nullptr;
   p.out = out;
   p.bias = bias;
-  // tensor memory: accumulators first, then the dequantized stages
+  // tensor memory of the one-CTA kernel: accumulators first, then the dequantized stages
   const int deq_cols = choose_kernel(colwise, p.BM).deq_cols;
   p.acc_bufs = (2 * p.BM + deq_cols <= 512) ? 2 : 1;
   p.a_col0 = p.acc_bufs * p.BM;
@@ -1063,7 +1102,7 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
     return 0;
   }
   blkq4::SplitPlan sp = blkq4::plan_split(m, n, k, workspace_size);
-  const int bm = m >= 256 ? 256 : ((m + 15) / 16) * 16;
+  const int bm = blkq4::tile_rows(m, 16);
   out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
   int devices = 0;
   if (cudaGetDeviceCount(&devices) != cudaSuccess) cudaGetLastError();
