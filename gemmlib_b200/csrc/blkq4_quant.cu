@@ -28,6 +28,15 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr unsigned kMaxGridY = 32768;
 
+// Both kernels are launched with programmatic stream serialization: their CTAs become resident, and the launch's own
+// latency passes, while the last CTAs of the preceding kernel still run; nothing is read or written before that kernel
+// has completed.  Measured on B200, the seven weights of a decoder block (4096, 11008; block 64, zero points) 117.1 us
+// without it, 101.2 with; row-wise 11008 x 4096, block 32 29.0 / 27.4.
+__device__ __forceinline__ void start_in_stream_order() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Scale and zero point from a block's range.  Same float operation sequence as
 // the reference's range2scalezp (f16_quant_sm80.cuh:96-122): IEEE division,
 // roundf (halves away from zero), clamp to [0, 15], fp32 -> fp16 round-to-nearest.
@@ -166,6 +175,7 @@ quant_colwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   constexpr int G = BLOCK / 16;          // lanes per quantization block: 1, 2, 4, 8
   constexpr int KL = G > 4 ? G : 4;      // lanes of a warp along k
   constexpr int NL = 32 / KL;            // packed columns of a warp
+  start_in_stream_order();
   const int lane = threadIdx.x & 31;
   const int kblk = blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (kblk * (16 * KL) >= K) return;     // whole warps
@@ -267,6 +277,7 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   __shared__ __align__(16) float s_recip[NB][64];  // -1 / scale
   __shared__ __align__(16) float s_zp[NB][64];     // -zero point
 
+  start_in_stream_order();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kl = lane & 3, npl = lane >> 2;   // chunk along k, packed column of the group
   const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 128;
@@ -356,17 +367,24 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
 }
 
 template <int BLOCK, bool ALIGNED>
-void launch_T(bool colwise, int K, int N, int ld, cudaStream_t stream, const __half* w, uint8_t* packed,
+cudaError_t launch_T(bool colwise, int K, int N, int ld, cudaStream_t stream, const __half* w, uint8_t* packed,
               __half* scales, uint8_t* zp) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (colwise) {
     constexpr int KL = BLOCK == 128 ? 8 : 4;
     const unsigned kblks = K / (16 * KL), groups = N / 2 / (32 / KL);
-    const dim3 grid((kblks + kWarps - 1) / kWarps, groups < kMaxGridY ? groups : kMaxGridY, (groups + kMaxGridY - 1) / kMaxGridY);
-    quant_colwise_kernel<BLOCK, ALIGNED><<<grid, kThreads, 0, stream>>>(w, K, N, ld, packed, scales, zp);
-  } else {
-    const dim3 grid(K / 64, (N + 127) / 128);
-    quant_rowwise_kernel<BLOCK, ALIGNED><<<grid, kThreads, 0, stream>>>(w, K, N, ld, packed, scales, zp);
+    cfg.gridDim = dim3((kblks + kWarps - 1) / kWarps, groups < kMaxGridY ? groups : kMaxGridY, (groups + kMaxGridY - 1) / kMaxGridY);
+    return cudaLaunchKernelEx(&cfg, quant_colwise_kernel<BLOCK, ALIGNED>, w, K, N, ld, packed, scales, zp);
   }
+  cfg.gridDim = dim3(K / 64, (N + 127) / 128);
+  return cudaLaunchKernelEx(&cfg, quant_rowwise_kernel<BLOCK, ALIGNED>, w, K, N, ld, packed, scales, zp);
 }
 
 }  // namespace
@@ -375,12 +393,11 @@ std::string launch_quant_prepack(int block, bool colwise, int K, int N, int ld,
                                  cudaStream_t stream, const __half* w, uint8_t* packed,
                                  __half* scales, uint8_t* zp) {
   const bool aligned = (reinterpret_cast<uintptr_t>(w) % 16 == 0) && (ld % 8 == 0);
-#define BLKQ4_CASE(B)                                                            \
-  case B:                                                                        \
-    if (aligned)                                                                 \
-      launch_T<B, true>(colwise, K, N, ld, stream, w, packed, scales, zp);       \
-    else                                                                         \
-      launch_T<B, false>(colwise, K, N, ld, stream, w, packed, scales, zp);      \
+  cudaError_t e = cudaSuccess;
+#define BLKQ4_CASE(B)                                                                         \
+  case B:                                                                                     \
+    e = aligned ? launch_T<B, true>(colwise, K, N, ld, stream, w, packed, scales, zp)         \
+                : launch_T<B, false>(colwise, K, N, ld, stream, w, packed, scales, zp);       \
     break;
   switch (block) {
     BLKQ4_CASE(16)
@@ -391,7 +408,8 @@ std::string launch_quant_prepack(int block, bool colwise, int K, int N, int ld,
       return "Unsupported block size: " + std::to_string(block);
   }
 #undef BLKQ4_CASE
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t last = cudaGetLastError();
+  if (e == cudaSuccess) e = last;
   if (e != cudaSuccess) return std::string("Kernel launch failed: ") + cudaGetErrorString(e);
   return std::string();
 }
