@@ -37,6 +37,9 @@ SYMBOLS = (
     "blkq4_gather_destroy",
     "blkq4_gather_reset",
     "blkq4_gather_supported_sm100",
+    "blkq4_fp16_gemm_group_sm100",
+    "blkq4_gemm_group_supported_sm100",
+    "blkq4_gemm_group_workspace_size_sm100",
     "blkq4_gemm_plan",
     "blkq4_gemm_plan_range_bound",
     "blkq4_reset",
@@ -46,6 +49,16 @@ SYMBOLS = (
 
 class BlkQ4Error(RuntimeError):
     pass
+
+
+class GemmPart(ctypes.Structure):
+    """``blkq4_gemm_part``."""
+
+    _fields_ = [("n", ctypes.c_int), ("weights", ctypes.c_void_p), ("weights_size", ctypes.c_size_t),
+                ("scales", ctypes.c_void_p), ("scales_size", ctypes.c_size_t),
+                ("offsets", ctypes.c_void_p), ("offsets_size", ctypes.c_size_t),
+                ("output", ctypes.c_void_p), ("output_size", ctypes.c_size_t),
+                ("bias", ctypes.c_void_p), ("bias_size", ctypes.c_size_t)]
 
 
 def _load() -> ctypes.CDLL:
@@ -63,6 +76,13 @@ def _load() -> ctypes.CDLL:
     lib.blkq4_fp16_gemm_ws_sm100.argtypes = [i, b, i, i, i, vp, vp, sz, vp, sz, vp, sz, vp, sz, vp, sz, vp, sz,
                                              ctypes.c_uint, vp, sz, vp]
     lib.blkq4_fp16_gemm_ws_sm100.restype = i
+    lib.blkq4_fp16_gemm_group_sm100.argtypes = [i, b, i, i, vp, vp, sz, i, ctypes.POINTER(GemmPart), ctypes.c_uint,
+                                                vp, sz, vp]
+    lib.blkq4_fp16_gemm_group_sm100.restype = i
+    lib.blkq4_gemm_group_supported_sm100.argtypes = [i, b, i, i, i, ctypes.POINTER(i)]
+    lib.blkq4_gemm_group_supported_sm100.restype = i
+    lib.blkq4_gemm_group_workspace_size_sm100.argtypes = [i, b, i, i, i, ctypes.POINTER(i)]
+    lib.blkq4_gemm_group_workspace_size_sm100.restype = sz
     lib.blkq4_gemm_workspace_size.argtypes = [i, i, i]
     lib.blkq4_gemm_workspace_size.restype = sz
     lib.blkq4_gemm_workspace_size_sm100.argtypes = [i, b, i, i, i]
@@ -182,6 +202,27 @@ def gemm_workspace_size(m: int, n: int, k: int) -> int:
 def gemm_workspace_size_blocked(block_size: int, col_wise: bool, m: int, n: int, k: int) -> int:
     """Bytes of zeroed workspace of a call with SKINNY_WORKSPACE (0: it would not use one)."""
     return int(lib.blkq4_gemm_workspace_size_sm100(block_size, col_wise, m, n, k))
+
+
+def gemm_group_supported(block_size: int, col_wise: bool, m: int, k: int, n) -> bool:
+    """Whether ``gemm_group`` takes the weight matrices of ``n`` columns each in one launch."""
+    return bool(lib.blkq4_gemm_group_supported_sm100(block_size, col_wise, m, k, len(n), (ctypes.c_int * len(n))(*n)))
+
+
+def gemm_group_workspace_size(block_size: int, col_wise: bool, m: int, k: int, n) -> int:
+    """Bytes of zeroed workspace with which ``gemm_group`` would split K over the tiles of all matrices (0: it would not)."""
+    return int(lib.blkq4_gemm_group_workspace_size_sm100(block_size, col_wise, m, k, len(n), (ctypes.c_int * len(n))(*n)))
+
+
+def gemm_group(block_size, col_wise, m, k, act, parts, flags=0, stream=0, workspace=None):
+    """One launch for several weight matrices with the same activations; ``parts`` = [(n, weights, scales, offsets or
+    None, output, bias or None), ...]."""
+    arr = (GemmPart * len(parts))(*(GemmPart(n, *(x for t in tensors for x in _ptr_size(t))) for n, *tensors in parts))
+    ap, asz = _ptr_size(act)
+    with _ErrMsg() as e:
+        if lib.blkq4_fp16_gemm_group_sm100(block_size, col_wise, m, k, stream, ap, asz, len(parts), arr, flags,
+                                           *_ptr_size(workspace), e.p) != 0:
+            raise BlkQ4Error(e.text())
 
 
 def gather_supported(block_size: int, col_wise: bool, m: int, n_shard: int, k: int) -> bool:

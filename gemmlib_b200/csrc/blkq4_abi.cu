@@ -93,13 +93,11 @@ extern "C" int blkq4_fp16_quant_sm80(int block_size, bool column_wise_blocking, 
   return 0;
 }
 
-extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blocking, int m, int n, int k,
-                                        void* stream_ptr, void const* act_ptr, size_t a_size,
-                                        void const* weights_ptr, size_t weights_size,
-                                        void const* scales_ptr, size_t scales_size,
-                                        void const* offsets_ptr, size_t offsets_size, void* output_ptr,
-                                        size_t output_size, void const* bias_ptr, size_t bias_size,
-                                        unsigned flags, void* workspace, size_t workspace_size, void* err) {
+// Every rule on sizes and pointers of one GEMM; 0 if it holds them all, else -1 and the reason in `err`.
+static int check_gemm(int block_size, bool column_wise_blocking, int m, int n, int k, void const* act_ptr, size_t a_size,
+                      void const* weights_ptr, size_t weights_size, void const* scales_ptr, size_t scales_size,
+                      void const* offsets_ptr, size_t offsets_size, void* output_ptr, size_t output_size,
+                      void const* bias_ptr, size_t bias_size, void* err) {
   if (!blkq4::supported_block(block_size))
     return fail(err, "Unsupported block size: " + std::to_string(block_size));
   if (m <= 0 || n <= 0 || k <= 0)
@@ -154,6 +152,20 @@ extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blockin
     return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets must be 16-byte aligned for m > 16)");
   if (!column_wise_blocking && !meta_aligned)
     return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets of row-wise blocks must be 16-byte aligned)");
+  return 0;
+}
+
+extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blocking, int m, int n, int k,
+                                        void* stream_ptr, void const* act_ptr, size_t a_size,
+                                        void const* weights_ptr, size_t weights_size,
+                                        void const* scales_ptr, size_t scales_size,
+                                        void const* offsets_ptr, size_t offsets_size, void* output_ptr,
+                                        size_t output_size, void const* bias_ptr, size_t bias_size,
+                                        unsigned flags, void* workspace, size_t workspace_size, void* err) {
+  if (check_gemm(block_size, column_wise_blocking, m, n, k, act_ptr, a_size, weights_ptr, weights_size, scales_ptr, scales_size,
+                 offsets_ptr, offsets_size, output_ptr, output_size, bias_ptr, bias_size, err) != 0)
+    return -1;
+  const bool has_offsets = offsets_ptr && offsets_size > 0, has_bias = bias_ptr && bias_size > 0;
 
   // Up to 16 rows blkq4_gemm_workspace_size is 0, so a caller may pass its prefill workspace along with decode calls
   // that run on another stream; only BLKQ4_GEMM_SKINNY_WORKSPACE says that the workspace is this call's.
@@ -176,6 +188,77 @@ extern "C" int blkq4_fp16_gemm_ws_sm100(int block_size, bool column_wise_blockin
           ? blkq4::launch_gemv(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, flags)
           : blkq4::launch_gemm_tc(block_size, column_wise_blocking, m, n, k, stream, a, w, s, z, o, bias, workspace,
                                           workspace_size, flags);
+  if (!e.empty()) return fail(err, "Kernel execution failed: " + e);
+  return 0;
+}
+
+// One launch for several weight matrices: see the header.
+static bool group_supported(int block_size, bool column_wise_blocking, int m, int k, int count, const int* n) {
+  if (count < 2 || count > blkq4::kMaxGroup || !n || m < 1 || k <= 0 || !blkq4::supported_block(block_size)) return false;
+  long long total = 0;
+  for (int i = 0; i < count; ++i) {
+    if (n[i] <= 0 || n[i] % 16 != 0) return false;
+    total += n[i];
+  }
+  if (total > (1 << 30)) return false;
+  if (m <= 16) return m <= 8 && blkq4::gemv_stream_takes(block_size, column_wise_blocking, m, (int)total, k);
+  const blkq4::Blocking b(block_size, column_wise_blocking);
+  if (k % 64 != 0 || k % b.bk != 0) return false;
+  for (int i = 0; i < count; ++i)
+    if (n[i] % b.bn != 0) return false;
+  return true;
+}
+
+extern "C" int blkq4_gemm_group_supported_sm100(int block_size, bool column_wise_blocking, int m, int k, int count,
+                                                int const* n) {
+  return group_supported(block_size, column_wise_blocking, m, k, count, n) ? 1 : 0;
+}
+
+extern "C" size_t blkq4_gemm_group_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int k, int count,
+                                                        int const* n) {
+  if (m <= 16 || !group_supported(block_size, column_wise_blocking, m, k, count, n)) return 0;
+  return blkq4::gemm_tc_group_workspace_bytes(m, k, count, n);
+}
+
+extern "C" int blkq4_fp16_gemm_group_sm100(int block_size, bool column_wise_blocking, int m, int k, void* stream_ptr,
+                                           void const* act_ptr, size_t a_size, int count, blkq4_gemm_part const* parts,
+                                           unsigned flags, void* workspace, size_t workspace_size, void* err) {
+  if (!parts || count < 2 || count > blkq4::kMaxGroup)
+    return fail(err, "A group has 2 to " + std::to_string(blkq4::kMaxGroup) + " parts, not " + std::to_string(count));
+  int n[blkq4::kMaxGroup];
+  for (int i = 0; i < count; ++i) {
+    const blkq4_gemm_part& q = parts[i];
+    if (check_gemm(block_size, column_wise_blocking, m, q.n, k, act_ptr, a_size, q.weights, q.weights_size, q.scales,
+                   q.scales_size, q.offsets, q.offsets_size, q.output, q.output_size, q.bias, q.bias_size, err) != 0)
+      return -1;
+    if (reinterpret_cast<uintptr_t>(q.scales) % 16 != 0 || reinterpret_cast<uintptr_t>(q.offsets) % 16 != 0)
+      return fail(err, "Kernel execution failed: Error Misaligned Operand (scales and offsets of a group must be 16-byte aligned)");
+    if ((q.offsets && q.offsets_size > 0) != (parts[0].offsets && parts[0].offsets_size > 0))
+      return fail(err, "The parts of a group have offsets all or none");
+    n[i] = q.n;
+  }
+  if (!group_supported(block_size, column_wise_blocking, m, k, count, n))
+    return fail(err, "Unsupported group: see blkq4_gemm_group_supported_sm100");
+  blkq4::GemmGroup g{};
+  g.count = count;
+  int total = 0;
+  for (int i = 0; i < count; ++i) {
+    const blkq4_gemm_part& q = parts[i];
+    g.n[i] = q.n;
+    total += q.n;
+    g.tile_end[i] = total / 16;
+    g.packed[i] = reinterpret_cast<const uint8_t*>(q.weights);
+    g.scales[i] = reinterpret_cast<const __half*>(q.scales);
+    g.zp[i] = q.offsets && q.offsets_size > 0 ? reinterpret_cast<const uint8_t*>(q.offsets) : nullptr;
+    g.out[i] = reinterpret_cast<__half*>(q.output);
+    g.bias[i] = q.bias && q.bias_size > 0 ? reinterpret_cast<const __half*>(q.bias) : nullptr;
+  }
+  const auto stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  const auto a = reinterpret_cast<const __half*>(act_ptr);
+  const std::string e =
+      m <= 16 ? blkq4::launch_gemv_stream(block_size, column_wise_blocking, m, total, k, stream, a, g.packed[0], g.scales[0],
+                                          g.zp[0], g.out[0], nullptr, flags, nullptr, &g)
+              : blkq4::launch_gemm_tc_group(block_size, column_wise_blocking, m, k, stream, a, g, workspace, workspace_size, flags);
   if (!e.empty()) return fail(err, "Kernel execution failed: " + e);
   return 0;
 }

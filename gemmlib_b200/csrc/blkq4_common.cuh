@@ -33,15 +33,42 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
 // cp.async rings, two launches resident per SM.  Returns kStreamUnsupported for other shapes.
 extern const char* const kStreamUnsupported;
 struct GatherTable;
+struct GemmGroup;
 std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
                                const __half* a, const uint8_t* packed, const __half* scales,
                                const uint8_t* zp, __half* out, const __half* bias, unsigned flags,
-                               const GatherTable* gt = nullptr);
+                               const GatherTable* gt = nullptr, const GemmGroup* grp = nullptr);
+
+// Whether it takes the problem (with 16-byte aligned scales and zero points), alone or as a group of N columns in all.
+bool gemv_stream_takes(int block, bool colwise, int M, int N, int K);
 
 // The same weight stream for 9 <= M <= 16 (two row groups, two tiles per pass, activations from L2).
 std::string launch_gemv_wide(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
                              const __half* a, const uint8_t* packed, const __half* scales,
                              const uint8_t* zp, __half* out, const __half* bias, unsigned flags);
+
+// Up to four weight matrices of one K, block size and kind of zero points that one launch multiplies with the same
+// activations.  Their tiles (of 16 columns in the decode kernel, of 128 or 256 in the tensor-core kernels) are numbered one
+// matrix after the other.
+constexpr int kMaxGroup = 4;
+struct GemmGroup {
+  int count;
+  int n[kMaxGroup];
+  int tile_end[kMaxGroup];  // tiles of the matrices up to and including this one
+  const uint8_t* packed[kMaxGroup];
+  const __half* scales[kMaxGroup];
+  const uint8_t* zp[kMaxGroup];
+  __half* out[kMaxGroup];
+  const __half* bias[kMaxGroup];
+#ifdef __CUDACC__
+  __device__ __forceinline__ int of_tile(int tile) const {
+    int i = 0;
+    while (i + 1 < count && tile >= tile_end[i]) ++i;
+    return i;
+  }
+  __device__ __forceinline__ int first_tile(int i) const { return i == 0 ? 0 : tile_end[i - 1]; }
+#endif
+};
 
 // Multiprocessor count of the CURRENT device (cached per device index).
 int sm_count();
@@ -81,6 +108,10 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
                            const __half* a, const uint8_t* packed, const __half* scales,
                            const uint8_t* zp, __half* out, const __half* bias, void* workspace,
                            size_t workspace_bytes, unsigned flags, const GatherTable* gt = nullptr);
+// The weight matrices of a group (more than 16 rows), and the workspace that such a launch would use.
+std::string launch_gemm_tc_group(int block, bool colwise, int M, int K, cudaStream_t stream, const __half* a,
+                                 const GemmGroup& grp, void* workspace, size_t workspace_bytes, unsigned flags);
+size_t gemm_tc_group_workspace_bytes(int M, int K, int count, const int* n);
 // True when launch_gemm_tc takes the problem with a GatherTable (the CTA-pair kernel's fused all-gather).
 bool gemm_tc_gather_supported(int M, int N, int K);
 // Bytes of zero-initialised workspace with which launch_gemm_tc would split K for this problem

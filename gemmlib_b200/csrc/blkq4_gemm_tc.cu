@@ -131,9 +131,33 @@ struct Params {
   float* ws_partials;  // balanced: [cta][BM][128] fp32
   int gather_bulk;         // pair kernel, gather mode: peer copies as cp.async.bulk of whole rows
   int n_fastest, n_pairs;  // pair kernel: tile order (0: the m tiles of a pair of weight columns run together; 1: the column pairs of an m tile)
+  GemmGroup grp;       // kernels with G > 1: the weight matrices whose column tiles (pairs of tiles) follow one another
   GatherTable gt;      // pair kernel, gt.world > 0: the result goes to every rank's gathered buffer instead of `out`
   unsigned* ws_flags;  // balanced: [cta]: arrivals (self-resetting)
 };
+
+// Tensor maps of the G weight matrices of a launch.
+template <int G>
+struct WeightMaps {
+  CUtensorMap pack[G], scale[G], zp[G];
+};
+// The matrix that column tile `t` of a launch belongs to, and what the epilogue needs of it.  A unit is one tile of
+// 128 columns, or in the pair kernel two.
+struct Columns {
+  int matrix, unit;  // unit: of the matrix
+  int N;
+  __half* out;
+  const __half* bias;
+};
+template <int G>
+__device__ __forceinline__ Columns columns_of(const Params& p, int unit) {
+  if constexpr (G == 1) {
+    return Columns{0, unit, p.N, p.out, p.bias};
+  } else {
+    const int i = p.grp.of_tile(unit);
+    return Columns{i, unit - p.grp.first_tile(i), p.grp.n[i], p.grp.out[i], p.grp.bias[i]};
+  }
+}
 
 // ---- PTX wrappers ---------------------------------------------------------------------------
 
@@ -243,11 +267,9 @@ __host__ __device__ constexpr SmemPlan make_plan(int rows, int kStages, int act_
   constexpr int BAR_COUNT = BAR_ACC_EMPTY + 2;                                                                      \
   static_assert(BAR_COUNT * 8 + 16 <= 512, "barrier block too small");
 
-template <bool COLWISE, class S>
+template <bool COLWISE, class S, int G>
 __global__ void __launch_bounds__(S::kThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_pack,
-               const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
-               const Params p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ WeightMaps<G> wm, const Params p) {
   constexpr int KSUB = S::KSUB, kRing = S::RING, kStepK = S::kStepK;
   constexpr int kStepCols = kDeqCols * KSUB, kStepPackBytes = kPackTileBytes * KSUB;
   constexpr int kStepScaleBytes = kScaleTileBytes * KSUB, kStepZpBytes = kZpTileBytes * KSUB;
@@ -335,7 +357,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       ItemCursor cur = first_item(p);
       Item item;
       while (next_item(p, cur, item)) {
-        const int n_tile = item.tile / p.m_tiles;
+        const Columns col = columns_of<G>(p, item.tile / p.m_tiles);
+        const int n_tile = col.unit;
         for (int ks = item.ks0; ks < item.ks0 + item.count; ++ks, ++it) {
           const int s = it % kStages;
           if (it >= (uint32_t)kStages &&
@@ -345,17 +368,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           mbar_arrive_expect_tx(fb, tx);
           const int k0 = ks * kStepK;
           if (!meta) {
-            tma_load_2d(base + plan.pack + s * kStepPackBytes, &tm_pack, k0, n_tile * (TILE_N / 2), fb);
+            tma_load_2d(base + plan.pack + s * kStepPackBytes, &wm.pack[col.matrix], k0, n_tile * (TILE_N / 2), fb);
           } else if (COLWISE) {
             // meta row-major [K/block, N]: box = meta_rows x 128 columns
             const int mrow = k0 >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &tm_scale, n_tile * TILE_N, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &tm_zp, n_tile * TILE_N, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &wm.scale[col.matrix], n_tile * TILE_N, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &wm.zp[col.matrix], n_tile * TILE_N, mrow, fb);
           } else {
             // meta column-major [K, N/block]: box = meta_rows (n blocks) x 64 k
             const int mrow = (n_tile * TILE_N) >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &tm_scale, k0, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &tm_zp, k0, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kStepScaleBytes, &wm.scale[col.matrix], k0, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kStepZpBytes, &wm.zp[col.matrix], k0, mrow, fb);
           }
         }
       }
@@ -425,7 +448,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     ItemCursor cur = first_item(p);
     Item item;
     for (; next_item(p, cur, item); ++tcount) {
-      const int n_tile = item.tile / p.m_tiles, m_tile = item.tile % p.m_tiles;
+      const Columns col = columns_of<G>(p, item.tile / p.m_tiles);
+      const int n_tile = col.unit, m_tile = item.tile % p.m_tiles;
       const int ab = tcount % p.acc_bufs;
       if (!mbar_wait(bar(BAR_ACC_FULL + ab), (tcount / p.acc_bufs) & 1, abort_flag, 0x300 | ab)) break;
       tc_fence_after();
@@ -482,7 +506,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       // lane, 128 contiguous bytes per warp): the even lane writes the even rows m of a
       // 32-row chunk, the odd lane the odd rows, each with its partner's value alongside.
       const int odd = lane & 1;
-      const bool n_ok = (n | 1) < p.N;  // N is a multiple of 16: the pair is in or out together
+      const bool n_ok = (n | 1) < col.N;  // N is a multiple of 16: the pair is in or out together
       for (int c0 = 0; c0 < p.BM; c0 += 32) {
         if (m0 + c0 >= m_end) break;  // warp-uniform
         uint32_t r[32];
@@ -496,12 +520,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + f[j]);
         }
         int m = m0 + c0 + odd;
-        __half* dst = p.out + (size_t)m * p.N + (n & ~1);
+        __half* dst = col.out + (size_t)m * col.N + (n & ~1);
         // The bias is added to the ROUNDED result in fp16, which is what a separate
         // `output += bias` on the fp16 tensor computes.
-        const bool add_bias = p.bias != nullptr && n_ok;
-        const __half2 bias2 = add_bias ? *reinterpret_cast<const __half2*>(p.bias + (n & ~1)) : __half2();
-        const size_t row_step = 2 * (size_t)p.N;
+        const bool add_bias = col.bias != nullptr && n_ok;
+        const __half2 bias2 = add_bias ? *reinterpret_cast<const __half2*>(col.bias + (n & ~1)) : __half2();
+        const size_t row_step = 2 * (size_t)col.N;
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float mine = __uint_as_float(odd ? r[j + 1] : r[j]);       // my n, my row
@@ -593,7 +617,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     cluster_sync_all();  // every part's epilogue warps have seen their accumulator complete
     tc_fence_after();
     const int split = p.split, part = (int)blockIdx.x % split, tile = (int)blockIdx.x / split;
-    const int n_tile = tile / p.m_tiles, m0 = (tile % p.m_tiles) * p.BM;
+    const Columns col = columns_of<G>(p, tile / p.m_tiles);
+    const int n_tile = col.unit, m0 = (tile % p.m_tiles) * p.BM;
     const int rows = min(p.BM, p.M - m0);
     const int slice4 = (p.BM / 4 + split - 1) / split;
     const uint32_t region = base + plan.act;
@@ -639,16 +664,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       __half2 h0 = odd ? __floats2half2_rn(got0, sum.z) : __floats2half2_rn(sum.x, got0);
       __half2 h1 = odd ? __floats2half2_rn(got1, sum.w) : __floats2half2_rn(sum.y, got1);
       const int m = m0 + 4 * (g0 + idx / TILE_N) + 2 * odd;
-      if (n < p.N) {  // N is a multiple of 16: the pair is in or out together
+      if (n < col.N) {  // N is a multiple of 16: the pair is in or out together
         // the bias is added to the rounded result in fp16, as above
-        if (p.bias) {
-          const __half2 b = *reinterpret_cast<const __half2*>(p.bias + (n & ~1));
+        if (col.bias) {
+          const __half2 b = *reinterpret_cast<const __half2*>(col.bias + (n & ~1));
           h0 = __hadd2(h0, b);
           h1 = __hadd2(h1, b);
         }
-        __half* dst = p.out + (size_t)m * p.N + (n & ~1);
+        __half* dst = col.out + (size_t)m * col.N + (n & ~1);
         if (m < p.M) *reinterpret_cast<__half2*>(dst) = h0;
-        if (m + 1 < p.M) *reinterpret_cast<__half2*>(dst + p.N) = h1;
+        if (m + 1 < p.M) *reinterpret_cast<__half2*>(dst + col.N) = h1;
       }
     }
   }
@@ -686,9 +711,12 @@ struct SplitPlan {
   size_t flags_bytes, total_bytes;  // workspace: [flags, 256-byte aligned][partials]
 };
 
-SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
+inline int column_tiles(int N) { return (N + TILE_N - 1) / TILE_N; }
+inline int column_pairs(int N) { return (column_tiles(N) + 1) / 2; }
+
+SplitPlan plan_split(int M, int n_tiles, int K, size_t ws_bytes_available) {
   const int BM = tile_rows(M, 16);
-  const int tiles = ((M + BM - 1) / BM) * ((N + TILE_N - 1) / TILE_N);
+  const int tiles = ((M + BM - 1) / BM) * n_tiles;
   const int k_steps = (K + step_k(BM) - 1) / step_k(BM);
   const int ws_rows = M >= 256 ? 256 : BM;  // of a partial tile in the workspace: its size is part of the interface
   const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -747,22 +775,25 @@ SplitPlan plan_split(int M, int N, int K, size_t ws_bytes_available) {
 }
 
 // The one-CTA kernel for tiles of BM rows.
-using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params);
+template <int G>
+using Kern = void (*)(CUtensorMap, WeightMaps<G>, Params);
+template <int G>
 struct KernelChoice {
-  Kern kern;
+  Kern<G> kern;
   int threads, which;  // which: index of the per-device caches
   size_t smem;
   int deq_cols;        // tensor memory of the dequantized stages
 };
-std::atomic<int> g_granted_smem[6][64];
+std::atomic<int> g_granted_smem[12][64];
 
-KernelChoice choose_kernel(bool colwise, int BM) {
-  KernelChoice c;
+template <int G>
+KernelChoice<G> choose_kernel(bool colwise, int BM) {
+  KernelChoice<G> c;
   auto pick = [&](auto shape, int idx) {
     using S = decltype(shape);
-    c.kern = colwise ? (Kern)gemm_tc_kernel<true, S> : (Kern)gemm_tc_kernel<false, S>;
+    c.kern = colwise ? (Kern<G>)gemm_tc_kernel<true, S, G> : (Kern<G>)gemm_tc_kernel<false, S, G>;
     c.threads = S::kThreads;
-    c.which = 2 * idx + (colwise ? 1 : 0);
+    c.which = 4 * idx + (G > 1 ? 2 : 0) + (colwise ? 1 : 0);
     c.smem = make_plan(S::MAXM, S::WS, S::RING, S::KSUB).total;
     c.deq_cols = S::kDeqTmemCols;
   };
@@ -773,8 +804,9 @@ KernelChoice choose_kernel(bool colwise, int BM) {
 }
 
 // Clusters of `split` CTAs of the kernel that are resident at once on the current device, 0 when it cannot say.
-int resident_clusters(const KernelChoice& kc, int split) {
-  static std::atomic<int> cache[6][kMaxSplit + 1][64];
+template <int G>
+int resident_clusters(const KernelChoice<G>& kc, int split) {
+  static std::atomic<int> cache[12][kMaxSplit + 1][64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   const bool cached = dev >= 0 && dev < 64;
@@ -801,7 +833,8 @@ int resident_clusters(const KernelChoice& kc, int split) {
 
 // A group of SMs holds whole clusters only, so fewer than SMs / split may fit: cut in fewer parts until all
 // clusters of the problem run in one round.
-void fit_split(const KernelChoice& kc, int tiles, int k_steps, SplitPlan& sp) {
+template <int G>
+void fit_split(const KernelChoice<G>& kc, int tiles, int k_steps, SplitPlan& sp) {
   while (sp.split > 1 && resident_clusters(kc, sp.split) < tiles) {
     sp.k_per_item = (k_steps + sp.split - 2) / (sp.split - 1);
     sp.split = (k_steps + sp.k_per_item - 1) / sp.k_per_item;
@@ -828,7 +861,7 @@ struct PairPlan {
   size_t flags_bytes, total_bytes;
 };
 
-PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
+PairPlan plan_pair(int M, int n_pairs, int K, size_t ws_bytes_available) {
   static const bool pair_off = getenv("BLKQ4_TC_NO_PAIR") != nullptr;
   static const int pair_min_m = getenv("BLKQ4_TC_PAIR_MIN_M") ? atoi(getenv("BLKQ4_TC_PAIR_MIN_M")) : 256;
   static const double balance_below =
@@ -839,7 +872,7 @@ PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
   const int pairs = sms / 2;
   pl.BM = tile_rows(M, 32);
   pl.m_tiles = (M + pl.BM - 1) / pl.BM;
-  pl.items = pl.m_tiles * (((N + TILE_N - 1) / TILE_N + 1) / 2);
+  pl.items = pl.m_tiles * n_pairs;
   const int k_steps = K / BLOCK_K;
   const long long total_steps = (long long)pl.items * k_steps;
   const int rounds = (pl.items + pairs - 1) / pairs;
@@ -867,9 +900,9 @@ PairPlan plan_pair(int M, int N, int K, size_t ws_bytes_available) {
 
 size_t gemm_tc_workspace_bytes(int M, int N, int K) {
   if (M <= 16) return 0;
-  const PairPlan pp = plan_pair(M, N, K, ~(size_t)0);
+  const PairPlan pp = plan_pair(M, column_pairs(N), K, ~(size_t)0);
   if (pp.use) return pp.total_bytes;
-  return plan_split(M, N, K, ~(size_t)0).total_bytes;
+  return plan_split(M, column_tiles(N), K, ~(size_t)0).total_bytes;
 }
 
 // Which problems of up to 16 rows run here rather than on the generic skinny kernel (blkq4_gemv.cu): both convert
@@ -904,42 +937,51 @@ bool gemm_tc_takes_skinny(int block, bool colwise, int M, int N, int K, const vo
 
 size_t gemm_tc_workspace_bytes_any(int block, bool colwise, int M, int N, int K) {
   if (M > 16) return gemm_tc_workspace_bytes(M, N, K);
-  return gemm_tc_takes_skinny(block, colwise, M, N, K, nullptr, nullptr) ? plan_split(M, N, K, ~(size_t)0).total_bytes : 0;
+  return gemm_tc_takes_skinny(block, colwise, M, N, K, nullptr, nullptr) ? plan_split(M, column_tiles(N), K, ~(size_t)0).total_bytes : 0;
 }
 
 bool gemm_tc_split_plan_refusable(int M, int N, int K, size_t capacity) {
   if (M <= 16) return false;
-  const SplitPlan sp = plan_split(M, N, K, ~(size_t)0);
+  const SplitPlan sp = plan_split(M, column_tiles(N), K, ~(size_t)0);
   return sp.total_bytes > capacity && sp.balanced == 0;
 }
 
 bool gemm_tc_gather_supported(int M, int N, int K) {
-  return M > 16 && plan_pair(M, N, K, 0).use;
+  return M > 16 && plan_pair(M, column_pairs(N), K, 0).use;
 }
 
 bool gemm_tc_plan_balanced(int M, int N, int K) {
   if (M <= 16) return false;
-  const PairPlan pp = plan_pair(M, N, K, ~(size_t)0);
+  const PairPlan pp = plan_pair(M, column_pairs(N), K, ~(size_t)0);
   if (pp.use) return pp.balanced != 0;
-  return plan_split(M, N, K, ~(size_t)0).balanced != 0;
+  return plan_split(M, column_tiles(N), K, ~(size_t)0).balanced != 0;
 }
 
-std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
-                           const __half* a, const uint8_t* packed, const __half* scales,
-                           const uint8_t* zp, __half* out, const __half* bias, void* workspace,
-                           size_t workspace_bytes, unsigned flags, const GatherTable* gt) {
+namespace {
+
+// G == 1: one weight matrix.  G > 1: the `grp` of them, whose tiles the plans see as those of one wide matrix.
+template <int G>
+std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t stream, const __half* a, const GemmGroup& grp,
+                           void* workspace, size_t workspace_bytes, unsigned flags, const GatherTable* gt) {
   Params p{};
   if (gt) p.gt = *gt;
+  const int N = grp.n[0];
+  const uint8_t* zp = grp.zp[0];
+  int n_tiles = 0, n_pairs = 0;
+  for (int i = 0; i < grp.count; ++i) {
+    n_tiles += column_tiles(grp.n[i]);
+    n_pairs += column_pairs(grp.n[i]);
+  }
   p.M = M; p.N = N; p.K = K; p.block = block;
   p.block_shift = block == 16 ? 4 : block == 32 ? 5 : block == 64 ? 6 : 7;
   p.BM = tile_rows(M, 16);
   p.m_tiles = (M + p.BM - 1) / p.BM;
-  p.n_tiles = (N + TILE_N - 1) / TILE_N;
+  p.n_tiles = n_tiles;
   p.has_zp = zp != nullptr;
-  p.out = out;
-  p.bias = bias;
+  p.out = grp.out[0];
+  p.bias = grp.bias[0];
   // tensor memory of the one-CTA kernel: accumulators first, then the dequantized stages
-  const int deq_cols = choose_kernel(colwise, p.BM).deq_cols;
+  const int deq_cols = choose_kernel<G>(colwise, p.BM).deq_cols;
   p.acc_bufs = (2 * p.BM + deq_cols <= 512) ? 2 : 1;
   p.a_col0 = p.acc_bufs * p.BM;
   {
@@ -950,43 +992,53 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
 
   const bool ws_ok = workspace && reinterpret_cast<uintptr_t>(workspace) % 256 == 0;
   // the fused exchange lives in the pair kernel's epilogue and runs in whole rounds
-  const PairPlan pp = plan_pair(M, N, K, (ws_ok && !gt) ? workspace_bytes : 0);
+  const PairPlan pp = plan_pair(M, n_pairs, K, (ws_ok && !gt) ? workspace_bytes : 0);
   const bool pair = pp.use;
   if (gt && !pair) return "unsupported shape for the fused all-gather";
   if (pair) {
     p.BM = pp.BM;
     p.m_tiles = pp.m_tiles;
   }
+  if constexpr (G > 1) {
+    p.grp = grp;
+    int end = 0;
+    for (int i = 0; i < grp.count; ++i) {
+      end += pair ? column_pairs(grp.n[i]) : column_tiles(grp.n[i]);
+      p.grp.tile_end[i] = end;
+    }
+  }
 
   // k per pipeline step: the box of the weights and of the meta spans it, the activations come in 64-k tiles
   const int sk = pair ? BLOCK_K : step_k(p.BM);
-  CUtensorMap tm_act, tm_pack, tm_scale, tm_zp;
+  CUtensorMap tm_act;
+  WeightMaps<G> wm;
   bool ok = encode_tensor_map_2d(&tm_act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a, (uint64_t)K, (uint64_t)M, BLOCK_K,
                       pair ? (uint32_t)(p.BM / 2) : (uint32_t)p.BM, CU_TENSOR_MAP_SWIZZLE_128B);
-  // Packed tiles of 128-byte rows carry the 128-byte swizzle: the dequantizers' 16-byte loads of eight
-  // neighbouring packed columns would otherwise all fall on the same banks.
-  // No swizzle on 64-byte rows: the dequantizers' 16-byte loads of eight neighbouring packed
-  // columns (64 bytes apart) do conflict four ways, but a 64-byte TMA swizzle that removes the
-  // conflicts measured 1-2 % SLOWER on the same GPU (M = 2048, 4096 x 4096: 59.2 vs 58.2 us): those loads are not on
-  // the critical path, the extra XOR per load is.
-  ok = ok && encode_tensor_map_2d(&tm_pack, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)K, (uint64_t)(N / 2),
-                       (uint32_t)sk, TILE_N / 2, sk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
   if (colwise) {
     p.meta_rows = block >= sk ? 1 : sk / block;
     p.meta_row_bytes_s = TILE_N * 2;
     p.meta_row_bytes_z = TILE_N;
-    ok = ok && encode_tensor_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, (uint64_t)N,
-                         (uint64_t)(K / block), TILE_N, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
-    ok = ok && encode_tensor_map_2d(&tm_zp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, zp ? zp : packed, (uint64_t)N,
-                         (uint64_t)(K / block), TILE_N, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
   } else {
     p.meta_rows = block >= TILE_N ? 1 : TILE_N / block;
     p.meta_row_bytes_s = (uint32_t)sk * 2;
     p.meta_row_bytes_z = (uint32_t)sk;
-    ok = ok && encode_tensor_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, (uint64_t)K,
-                         (uint64_t)(N / block), (uint32_t)sk, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
-    ok = ok && encode_tensor_map_2d(&tm_zp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, zp ? zp : packed, (uint64_t)K,
-                         (uint64_t)(N / block), (uint32_t)sk, (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+  }
+  for (int i = 0; i < grp.count; ++i) {
+    const int Ni = grp.n[i];
+    // Packed tiles of 128-byte rows carry the 128-byte swizzle: the dequantizers' 16-byte loads of eight
+    // neighbouring packed columns would otherwise all fall on the same banks.
+    // No swizzle on 64-byte rows: the dequantizers' 16-byte loads of eight neighbouring packed
+    // columns (64 bytes apart) do conflict four ways, but a 64-byte TMA swizzle that removes the
+    // conflicts measured 1-2 % SLOWER on the same GPU (M = 2048, 4096 x 4096: 59.2 vs 58.2 us): those loads are not on
+    // the critical path, the extra XOR per load is.
+    ok = ok && encode_tensor_map_2d(&wm.pack[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, grp.packed[i], (uint64_t)K, (uint64_t)(Ni / 2),
+                         (uint32_t)sk, TILE_N / 2, sk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
+    const uint64_t cols = colwise ? (uint64_t)Ni : (uint64_t)K, rows = (uint64_t)((colwise ? K : Ni) / block);
+    const uint32_t box = colwise ? (uint32_t)TILE_N : (uint32_t)sk;
+    ok = ok && encode_tensor_map_2d(&wm.scale[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, grp.scales[i], cols, rows, box,
+                                    (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+    ok = ok && encode_tensor_map_2d(&wm.zp[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, zp ? grp.zp[i] : grp.packed[i], cols, rows, box,
+                                    (uint32_t)p.meta_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
   }
   if (!ok) return "cuTensorMapEncodeTiled failed";
 
@@ -994,7 +1046,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   if (pair) {
     p.k_steps = K / BLOCK_K;
     p.num_items = pp.items;
-    p.n_pairs = (p.n_tiles + 1) / 2;
+    p.n_pairs = n_pairs;
     // fused all-gather: walk the column pairs of one m tile together, so that at any moment the stores of all
     // ranks fall into a few hundred rows of every destination
     static const bool nf_off = getenv("BLKQ4_TC_GATHER_M_FASTEST") != nullptr;
@@ -1005,7 +1057,7 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     p.total_steps = pp.balanced ? pp.items * p.k_steps : 0;
     p.ws_flags = reinterpret_cast<unsigned*>(workspace);
     p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + pp.flags_bytes);
-    auto kern = colwise ? gemm_tc_pair_kernel<true, kPairWeightStages> : gemm_tc_pair_kernel<false, kPairWeightStages>;
+    auto kern = colwise ? gemm_tc_pair_kernel<true, kPairWeightStages, G> : gemm_tc_pair_kernel<false, kPairWeightStages, G>;
     const SmemPlan plan = make_plan(kPairRows, kPairWeightStages, kPairActStages, 1, kPairOutBytes);
     static std::atomic<int> granted[2][64];
     cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[colwise ? 1 : 0]);
@@ -1035,15 +1087,15 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
     cfg.numAttrs = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) ? 1 : 0;
     // balanced ranges use every resident pair, whole rounds at most one pair per tile
     cfg.gridDim = dim3(2 * ((p.balanced || p.num_items >= pairs) ? pairs : p.num_items));
-    e = cudaLaunchKernelEx(&cfg, kern, tm_act, tm_pack, tm_scale, tm_zp, p);
+    e = cudaLaunchKernelEx(&cfg, kern, tm_act, wm, p);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
     return std::string();
   }
   const int num_tiles = p.m_tiles * p.n_tiles;
-  const KernelChoice kc = choose_kernel(colwise, p.BM);
+  const KernelChoice<G> kc = choose_kernel<G>(colwise, p.BM);
   p.k_steps = (K + sk - 1) / sk;
-  SplitPlan sp = plan_split(M, N, K, ws_ok ? workspace_bytes : 0);
+  SplitPlan sp = plan_split(M, n_tiles, K, ws_ok ? workspace_bytes : 0);
   fit_split(kc, num_tiles, p.k_steps, sp);
   p.split = sp.split;  // split > 1: at most one item per SM
   p.k_per_item = sp.k_per_item;
@@ -1069,10 +1121,42 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
   cfg.gridDim = dim3(p.num_items < sms ? p.num_items : sms);
   cfg.attrs = p.split > 1 ? attr : attr + 1;
   cfg.numAttrs = (p.split > 1 ? 1 : 0) + ((flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) ? 1 : 0);
-  e = cudaLaunchKernelEx(&cfg, kc.kern, tm_act, tm_pack, tm_scale, tm_zp, p);
+  e = cudaLaunchKernelEx(&cfg, kc.kern, tm_act, wm, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
   return std::string();
+}
+
+}  // namespace
+
+std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
+                           const __half* a, const uint8_t* packed, const __half* scales,
+                           const uint8_t* zp, __half* out, const __half* bias, void* workspace,
+                           size_t workspace_bytes, unsigned flags, const GatherTable* gt) {
+  GemmGroup one{};
+  one.count = 1;
+  one.n[0] = N;
+  one.packed[0] = packed;
+  one.scales[0] = scales;
+  one.zp[0] = zp;
+  one.out[0] = out;
+  one.bias[0] = bias;
+  return launch_weights<1>(block, colwise, M, K, stream, a, one, workspace, workspace_bytes, flags, gt);
+}
+
+std::string launch_gemm_tc_group(int block, bool colwise, int M, int K, cudaStream_t stream, const __half* a,
+                                 const GemmGroup& grp, void* workspace, size_t workspace_bytes, unsigned flags) {
+  return launch_weights<kMaxGroup>(block, colwise, M, K, stream, a, grp, workspace, workspace_bytes, flags, nullptr);
+}
+
+size_t gemm_tc_group_workspace_bytes(int M, int K, int count, const int* n) {
+  int n_tiles = 0, n_pairs = 0;
+  for (int i = 0; i < count; ++i) {
+    n_tiles += column_tiles(n[i]);
+    n_pairs += column_pairs(n[i]);
+  }
+  const PairPlan pp = plan_pair(M, n_pairs, K, ~(size_t)0);
+  return pp.use ? pp.total_bytes : plan_split(M, n_tiles, K, ~(size_t)0).total_bytes;
 }
 
 int clear_gemm_tc_error(cudaStream_t stream) {
@@ -1095,20 +1179,20 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
   for (int i = 0; i < 6; ++i) out6[i] = 0;
   if (m <= 16) return 0;
   const int sms = blkq4::sm_count() > 0 ? blkq4::sm_count() : 148;
-  const blkq4::PairPlan pp = blkq4::plan_pair(m, n, k, workspace_size);
+  const blkq4::PairPlan pp = blkq4::plan_pair(m, blkq4::column_pairs(n), k, workspace_size);
   if (pp.use) {
     out6[0] = 2; out6[1] = pp.BM; out6[2] = pp.items; out6[3] = 1; out6[4] = pp.balanced;
     out6[5] = pp.balanced ? sms / 2 : 0;
     return 0;
   }
-  blkq4::SplitPlan sp = blkq4::plan_split(m, n, k, workspace_size);
+  blkq4::SplitPlan sp = blkq4::plan_split(m, blkq4::column_tiles(n), k, workspace_size);
   const int bm = blkq4::tile_rows(m, 16);
   out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
   int devices = 0;
   if (cudaGetDeviceCount(&devices) != cudaSuccess) cudaGetLastError();
   // as many clusters fit of the row-wise kernel as of the column-wise one: one CTA per SM, both
   if (devices > 0)
-    blkq4::fit_split(blkq4::choose_kernel(true, bm), out6[2], (k + blkq4::step_k(bm) - 1) / blkq4::step_k(bm), sp);
+    blkq4::fit_split(blkq4::choose_kernel<1>(true, bm), out6[2], (k + blkq4::step_k(bm) - 1) / blkq4::step_k(bm), sp);
   out6[3] = sp.split; out6[4] = sp.balanced; out6[5] = sp.balanced ? sms : 0;
   return 0;
 }

@@ -156,11 +156,9 @@ struct PairWalk {
   }
 };
 
-template <bool COLWISE, int WS>
+template <bool COLWISE, int WS, int G>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_pack,
-                    const __grid_constant__ CUtensorMap tm_scale, const __grid_constant__ CUtensorMap tm_zp,
-                    const Params p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ WeightMaps<G> wm, const Params p) {
   constexpr int kActStages = kPairActStages;
   BLKQ4_TC_BARRIER_SLOTS(WS, kDeqStages)
   extern __shared__ uint8_t smem_raw[];
@@ -244,7 +242,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       PairWalk walk(p, pair, num_pairs);
       int item, ks0, count, role;
       while (walk.next(item, ks0, count, role)) {
-        const int n_tile = 2 * (p.n_fastest ? item % p.n_pairs : item / p.m_tiles) + (int)rank;
+        const Columns col = columns_of<G>(p, p.n_fastest ? item % p.n_pairs : item / p.m_tiles);
+        const int n_tile = 2 * col.unit + (int)rank;
         for (int ks = ks0; ks < ks0 + count; ++ks, ++it) {
           const int s = it % kStages;
           if (it >= (uint32_t)kStages &&
@@ -253,15 +252,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
           const uint32_t fb = bar(BAR_FULL + s);
           mbar_arrive_expect_tx(fb, tx);
           const int k0 = ks * BLOCK_K;
-          tma_load_2d(base + plan.pack + s * kPackTileBytes, &tm_pack, k0, n_tile * (TILE_N / 2), fb);
+          tma_load_2d(base + plan.pack + s * kPackTileBytes, &wm.pack[col.matrix], k0, n_tile * (TILE_N / 2), fb);
           if (COLWISE) {
             const int mrow = k0 >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &tm_scale, n_tile * TILE_N, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &tm_zp, n_tile * TILE_N, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &wm.scale[col.matrix], n_tile * TILE_N, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &wm.zp[col.matrix], n_tile * TILE_N, mrow, fb);
           } else {
             const int mrow = (n_tile * TILE_N) >> p.block_shift;
-            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &tm_scale, k0, mrow, fb);
-            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &tm_zp, k0, mrow, fb);
+            tma_load_2d(base + plan.scale + s * kScaleTileBytes, &wm.scale[col.matrix], k0, mrow, fb);
+            if (p.has_zp) tma_load_2d(base + plan.zp + s * kZpTileBytes, &wm.zp[col.matrix], k0, mrow, fb);
           }
         }
       }
@@ -357,7 +356,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     PairWalk walk(p, pair, num_pairs);
     int item, ks0, count, role;
     for (; walk.next(item, ks0, count, role); ++tcount) {
-      const int n_tile = 2 * (p.n_fastest ? item % p.n_pairs : item / p.m_tiles) + (int)rank;
+      const Columns col = columns_of<G>(p, p.n_fastest ? item % p.n_pairs : item / p.m_tiles);
+      const int n_tile = 2 * col.unit + (int)rank;
       const int m_tile = p.n_fastest ? item / p.n_pairs : item % p.m_tiles;
       if (!mbar_wait_cluster(bar(BAR_ACC_FULL), tcount & 1u, abort_flag, 0x300)) break;
       tc_fence_after();
@@ -454,15 +454,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       }
       // staging -> global: one instruction moves four rows' 64-byte pieces
       const int n4 = n_tile * TILE_N + quarter * 32 + (lane & 7) * 4;  // first of this lane's 4 columns
-      const bool n_ok = n4 + 3 < p.N;                                    // N is a multiple of 16
+      const bool n_ok = n4 + 3 < col.N;                                  // N is a multiple of 16
       __half2 b01 = __half2(), b23 = __half2();
-      const bool add_bias = p.bias != nullptr && n_ok;
+      const bool add_bias = col.bias != nullptr && n_ok;
       if (add_bias) {
-        b01 = *reinterpret_cast<const __half2*>(p.bias + n4);
-        b23 = *reinterpret_cast<const __half2*>(p.bias + n4 + 2);
+        b01 = *reinterpret_cast<const __half2*>(col.bias + n4);
+        b23 = *reinterpret_cast<const __half2*>(col.bias + n4 + 2);
       }
       if (p.gt.world == 0) {
-        __half* gdst = p.out + (size_t)(m0 + (lane >> 3)) * p.N + n4;
+        __half* gdst = col.out + (size_t)(m0 + (lane >> 3)) * col.N + n4;
         for (int r0 = 0; r0 < rows; r0 += 4) {
           uint2 v = *reinterpret_cast<const uint2*>(stage + r0 * 64 + lane * 8);
           if (add_bias) {
@@ -472,7 +472,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             v.y = *reinterpret_cast<uint32_t*>(&hi);
           }
           if (n_ok && r0 + (lane >> 3) < rows) *reinterpret_cast<uint2*>(gdst) = v;
-          gdst += 4 * (size_t)p.N;
+          gdst += 4 * (size_t)col.N;
         }
       } else if (bulk) {
         // Fused all-gather with bulk copies (the default): every row of the CTA's tile (256 contiguous

@@ -144,6 +144,61 @@ torch::Tensor blkq4linear_linear(int block_size, bool col_wise, int in_features,
   return output.view(shape);
 }
 
+// Layers that read the same activations, as one launch (blkq4_fp16_gemm_group_sm100): their packed tensors, zero points
+// (all or none), fp16 biases or None, and the [rows, out_features] outputs to write.
+void blkq4linear_group(int block_size, bool col_wise, int in_features, const torch::Tensor& input,
+                       const std::vector<torch::Tensor>& q_weights, const std::vector<torch::Tensor>& q_scales,
+                       const std::vector<torch::Tensor>& q_zp, const std::vector<c10::optional<torch::Tensor>>& bias,
+                       const std::vector<torch::Tensor>& outputs, int64_t flags,
+                       const c10::optional<torch::Tensor>& workspace) {
+  const size_t count = q_weights.size();
+  TORCH_CHECK(count >= 2 && count <= 4 && q_scales.size() == count && q_zp.size() == count && bias.size() == count &&
+                  outputs.size() == count,
+              "A group has two to four layers");
+  TORCH_CHECK(input.scalar_type() == torch::kFloat16 && input.dim() == 2 && input.size(1) == in_features &&
+                  input.is_contiguous() && input.device().type() == torch::kCUDA,
+              "Activations must be a contiguous float16 CUDA tensor [rows, in_features]");
+  const auto dev = input.device();
+  blkq4_gemm_part parts[4] = {};
+  for (size_t i = 0; i < count; ++i) {
+    const bool has_bias = bias[i].has_value() && bias[i]->defined() && bias[i]->numel() > 0;
+    TORCH_CHECK(q_weights[i].device() == dev && q_scales[i].device() == dev && outputs[i].device() == dev &&
+                    (q_zp[i].numel() == 0 || q_zp[i].device() == dev) && (!has_bias || bias[i]->device() == dev),
+                "A group requires all tensors on the same device");
+    TORCH_CHECK(outputs[i].scalar_type() == torch::kFloat16 && outputs[i].is_contiguous() && outputs[i].dim() == 2 &&
+                    outputs[i].size(0) == input.size(0),
+                "Outputs must be contiguous float16 [rows, out_features] tensors");
+    TORCH_CHECK(!has_bias || (bias[i]->scalar_type() == torch::kFloat16 && bias[i]->is_contiguous()),
+                "Fused biases must be contiguous float16 tensors");
+    auto& p = parts[i];
+    p.n = int(outputs[i].size(1));
+    p.weights = q_weights[i].data_ptr();
+    p.weights_size = size_t(q_weights[i].numel());
+    p.scales = q_scales[i].data_ptr();
+    p.scales_size = size_t(q_scales[i].numel()) * kHalfBytes;
+    if (q_zp[i].numel() > 0) {
+      p.offsets = q_zp[i].data_ptr();
+      p.offsets_size = size_t(q_zp[i].numel());
+    }
+    p.output = outputs[i].data_ptr();
+    p.output_size = size_t(outputs[i].numel()) * kHalfBytes;
+    if (has_bias) {
+      p.bias = bias[i]->data_ptr();
+      p.bias_size = size_t(bias[i]->numel()) * kHalfBytes;
+    }
+  }
+  const bool has_ws = workspace.has_value() && workspace->defined() && workspace->numel() > 0;
+  TORCH_CHECK(!has_ws || (workspace->device() == dev && workspace->is_contiguous()),
+              "The split-K workspace must be a contiguous tensor on the input's device");
+  const c10::cuda::CUDAGuard guard(dev);
+  std::string err;
+  const int rc = blkq4_fp16_gemm_group_sm100(block_size, col_wise, int(input.size(0)), in_features,
+                                             c10::cuda::getCurrentCUDAStream().stream(), input.data_ptr(),
+                                             size_t(input.numel()) * kHalfBytes, int(count), parts, unsigned(flags),
+                                             has_ws ? workspace->data_ptr() : nullptr, has_ws ? workspace->nbytes() : 0, &err);
+  TORCH_CHECK(rc == 0, err);
+}
+
 // ---- workspaces of calls that are being captured into a CUDA graph ----
 // The graph keeps the buffer's address, so the graph keeps the buffer: a user object of the graph holds the tensor
 // until the graph and everything instantiated from it are gone.  One buffer per capture and stream, its flag words
@@ -230,6 +285,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("block_size"), py::arg("col_wise"), py::arg("in_features"), py::arg("out_features"),
         py::arg("input"), py::arg("q_weights"), py::arg("q_scales"), py::arg("q_zp"), py::arg("bias"), py::arg("flags"),
         py::arg("workspace"), py::arg("out"));
+  m.def("linear_group", &blkq4linear_group, "Layers that read the same activations, as one launch");
+  m.def("linear_group_supported",
+        [](int block, bool col_wise, int m_, int k_, const std::vector<int>& n_) {
+          return blkq4_gemm_group_supported_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()) != 0;
+        },
+        "Whether one launch takes layers of these widths");
+  m.def("linear_group_workspace_size",
+        [](int block, bool col_wise, int m_, int k_, const std::vector<int>& n_) {
+          return int64_t(blkq4_gemm_group_workspace_size_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()));
+        },
+        "Bytes of zeroed workspace with which linear_group splits K (0: it does not)");
   m.def("gemm_workspace_size_blocked",
         [](int block, bool col_wise, int m_, int n_, int k_) {
           return int64_t(blkq4_gemm_workspace_size_sm100(block, col_wise, m_, n_, k_));

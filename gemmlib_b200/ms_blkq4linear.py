@@ -31,6 +31,9 @@ from . import ms_blkq4linear_ext
 _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
 _SKINNY_WS = ms_blkq4linear_ext.SKINNY_WORKSPACE
 _linear = ms_blkq4linear_ext.linear
+_linear_group = ms_blkq4linear_ext.linear_group
+_group_supported = ms_blkq4linear_ext.linear_group_supported
+_group_workspace_size = ms_blkq4linear_ext.linear_group_workspace_size
 _graph_workspace = ms_blkq4linear_ext.graph_workspace
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
@@ -75,6 +78,47 @@ def split_k_workspace(device, nbytes: int):
         ws = torch.zeros(max(nbytes, 16 << 20), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
     return ws
+
+
+MAX_GROUP = 4  # layers of one launch
+
+
+def can_share_launch(layers, rows) -> bool:
+    """Whether one launch computes all ``layers`` (two to four) from the same ``rows`` activation rows, with the results
+    their ``forward`` calls give: layers of one shape of blocks, with nothing hooked into their calls."""
+    first = layers[0]
+    for l in layers:
+        if not isinstance(l, BlkQ4Linear):
+            return False
+        q = l.q_weights
+        if (type(l).forward is not BlkQ4Linear.forward or "forward" in l.__dict__
+                or l._forward_hooks or l._forward_pre_hooks or nn.modules.module._has_any_global_hook()
+                or (l.block_size, l.col_wise, l.in_features) != (first.block_size, first.col_wise, first.in_features)
+                or (l.q_zp.numel() > 0) != (first.q_zp.numel() > 0) or q.device != first.q_weights.device
+                or (l.bias is not None and l._fusable_bias(q) is None)
+                or l.q_scales.data_ptr() % 16 or l.q_zp.data_ptr() % 16):
+            return False
+    return _group_supported(first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers])
+
+
+def shared_workspace_bytes(layers, rows):
+    """Split-K workspace that ``run_as_one`` uses for ``rows`` activation rows (0: none)."""
+    first = layers[0]
+    if not all(l.split_k for l in layers):
+        return 0
+    return _group_workspace_size(first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers])
+
+
+def run_as_one(layers, input, outputs):
+    """One launch for layers that ``can_share_launch``: ``outputs[i] = layers[i](input)``."""
+    first = layers[0]
+    ws = split_k_workspace(input.device, shared_workspace_bytes(layers, input.size(0)))
+    early = all(l._settled and l.early_weight_fetch for l in layers)
+    _linear_group(first.block_size, first.col_wise, first.in_features, input, [l.q_weights for l in layers],
+                  [l.q_scales for l in layers], [l.q_zp for l in layers], [l.bias for l in layers], list(outputs),
+                  _EARLY if early else 0, ws)
+    for l in layers:
+        l._settled = True
 
 
 class BlkQ4Linear(nn.Module):

@@ -8,7 +8,8 @@ persistent workspace (one buffer per named activation), wires each layer to an i
 an output buffer, captures the whole pass once per row count M on its own stream, and
 replays it.  Inside the graph the skinny kernels are launched with
 ``BLKQ4_GEMM_EARLY_WEIGHT_FETCH``: the weights of layer i+1 stream in while layer i
-drains.
+drains.  Consecutive layers that read the same buffer (q, k and v; gate and up) are one launch where a kernel
+takes them together.
 
 It runs the linears only: what sits between them in a model (attention, activation
 functions, norms) is the caller's and can be captured into the same graph by passing
@@ -20,7 +21,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import BlkQ4Linear, workspaces_owned_by
+from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, run_as_one, shared_workspace_bytes, workspaces_owned_by
 
 
 class LinearStack:
@@ -58,18 +59,42 @@ class LinearStack:
                 raise ValueError(f"buffer {dst!r} has width {bufs[dst].size(1)}, layer writes {lyr.out_features}")
         return bufs
 
-    def _run_eager(self, bufs):
+    def _groups(self, M: int) -> List[range]:
+        """The steps in runs that one launch takes at this row count: up to four that follow one another, read the same
+        buffer, write others, and have no hook between them."""
+        runs: List[range] = []
         for i, (lyr, src, dst) in enumerate(self.steps):
-            lyr(bufs[src], out=bufs[dst])
-            hook = self.between.get(i)
+            if runs and len(runs[-1]) < MAX_GROUP and (i - 1) not in self.between:
+                run = runs[-1]
+                members = [self.steps[j] for j in run] + [(lyr, src, dst)]
+                outputs = [d for _, _, d in members]
+                if (all(s == src for _, s, _ in members) and src not in outputs and len(set(outputs)) == len(outputs)
+                        and can_share_launch([m for m, _, _ in members], M)):
+                    runs[-1] = range(run.start, i + 1)
+                    continue
+            runs.append(range(i, i + 1))
+        return runs
+
+    def _run_eager(self, bufs, groups):
+        for run in groups:
+            members = [self.steps[i] for i in run]
+            if len(members) > 1:
+                run_as_one([lyr for lyr, _, _ in members], bufs[members[0][1]], [bufs[dst] for _, _, dst in members])
+            else:
+                lyr, src, dst = members[0]
+                lyr(bufs[src], out=bufs[dst])
+            hook = self.between.get(run[-1])
             if hook is not None:
                 hook(bufs)
 
     def _capture(self, M: int):
         bufs = self._workspace(M)
+        groups = self._groups(M)
         # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
         # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
-        need = max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)), default=0)
+        need = max((shared_workspace_bytes(layers, M) if len(layers) > 1 else layers[0].workspace_bytes(M)
+                    for layers in ([self.steps[i][0] for i in run] for run in groups)
+                    if isinstance(layers[0], BlkQ4Linear)), default=0)
         split_k = {}
         if need > 0:
             split_k[self.device.index, self.stream.cuda_stream] = [
@@ -78,13 +103,13 @@ class LinearStack:
         with workspaces_owned_by(split_k):
             with torch.cuda.stream(self.stream):
                 for _ in range(2):  # the first pass settles every layer (plain launches), the second warms up
-                    self._run_eager(bufs)
+                    self._run_eager(bufs, groups)
             self.stream.synchronize()
             for buffers in split_k.values():
                 del buffers[:-1]  # outgrown in the first pass
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=self.stream):
-                self._run_eager(bufs)
+                self._run_eager(bufs, groups)
         self._split_k[M] = split_k
         self._graphs[M] = (graph, bufs)
         return self._graphs[M]

@@ -168,6 +168,41 @@ size_t blkq4_gemm_workspace_size(int m, int n, int k);
  * larger sizes) and would cut it in balanced ranges; for m > 16 equal to blkq4_gemm_workspace_size. */
 size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int n, int k);
 
+/**
+ * Several GEMMs that read the same activations - the q, k and v projections of a decoder block, or its gate and up
+ * projections - as one launch: 2 to 4 weight matrices of one k, block size and orientation, with offsets all or none.
+ * The rules on the sizes and pointers of each part are those of blkq4_fp16_gemm_ws_sm100, with scales and offsets 16-byte
+ * aligned, and the outputs must overlap neither one another nor the activations.  Up to 16 rows, and without a workspace
+ * of blkq4_gemm_group_workspace_size_sm100 bytes, the result of every part is the one its own call gives, bit for bit; with
+ * it K may be split as blkq4_fp16_gemm_ws_sm100 does, over the tiles of all parts together.  Flags:
+ * BLKQ4_GEMM_EARLY_WEIGHT_FETCH.  Shapes that blkq4_gemm_group_supported_sm100 answers 0 for are refused.  No counterpart in
+ * the reference.
+ */
+typedef struct blkq4_gemm_part {
+  int n;
+  void const* weights;
+  size_t weights_size;
+  void const* scales;
+  size_t scales_size;
+  void const* offsets;  /* null / 0: none */
+  size_t offsets_size;
+  void* output;
+  size_t output_size;
+  void const* bias;     /* null / 0: none */
+  size_t bias_size;
+} blkq4_gemm_part;
+size_t blkq4_gemm_group_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int k, int count, int const* n);
+int blkq4_gemm_group_supported_sm100(int block_size, bool column_wise_blocking, int m, int k, int count, int const* n);
+int blkq4_fp16_gemm_group_sm100(
+  int block_size,
+  bool column_wise_blocking,
+  int m, int k, void* stream,
+  void const* act_ptr, size_t a_size,
+  int count, blkq4_gemm_part const* parts,
+  unsigned flags,
+  void* workspace, size_t workspace_size,
+  void* error_message);
+
 /* No counterpart in the reference.  Host-only description of the work plan blkq4_fp16_gemm_ws_sm100 would
  * choose for the problem with a workspace of `workspace_size` bytes: nothing is launched and no device is
  * needed (the plan depends on the current device's SM count and on how many clusters of a split's size it holds at

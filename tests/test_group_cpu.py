@@ -1,0 +1,38 @@
+"""Which groups of weight matrices one launch takes (host only)."""
+import pytest
+
+from gemmlib_b200 import capi
+
+
+def test_supported_groups():
+    assert capi.gemm_group_supported(64, True, 1, 4096, (4096, 4096, 4096))
+    assert capi.gemm_group_supported(128, True, 8, 2048, (16, 28672))
+    assert capi.gemm_group_supported(32, False, 17, 64, (32, 4096))   # the tensor-core kernels: any blocking
+    assert capi.gemm_group_supported(16, True, 4096, 4096, (11008, 11008))
+    for args in ((64, True, 9, 4096, (4096, 4096)),      # more rows than the decode kernel takes
+                 (32, True, 1, 4096, (4096, 4096)),      # another kernel's blocking
+                 (64, False, 1, 4096, (4096, 4096)),
+                 (64, True, 1, 1984, (4096, 4096)),      # K too short, and not in groups of 256
+                 (64, True, 1, 2112, (4096, 4096)),
+                 (64, True, 1, 4096, (4096,)),
+                 (64, True, 1, 4096, (16,) * 5),
+                 (64, True, 1, 4096, (4096, 24)),
+                 (64, True, 1, 4096, (4096, 0)),
+                 (48, True, 1, 4096, (4096, 4096)),
+                 (64, True, 0, 4096, (4096, 4096)),
+                 (64, True, 64, 4064, (4096, 4096)),
+                 (32, False, 64, 4096, (4096, 48))):
+        assert not capi.gemm_group_supported(*args), args
+
+
+@pytest.mark.parametrize("parts,message", [([], "2 to 4"), ([(64, (16, 1), (16, 1), None, (16, 1), None)] * 2, "Unexpected weight")])
+def test_refused_groups(parts, message):
+    with pytest.raises(capi.BlkQ4Error, match=message):
+        capi.gemm_group(64, True, 1, 2048, (16, 4096), parts)
+
+
+def test_workspace_of_a_group():
+    """That of one matrix with the columns of all."""
+    for m, k, widths in ((64, 8192, (14336, 14336)), (512, 4096, (4096, 4096, 4096)), (512, 4096, (11008, 11008)), (64, 4096, (1024, 1024))):
+        assert capi.gemm_group_workspace_size(64, True, m, k, widths) == capi.gemm_workspace_size(m, sum(widths), k) > 0
+    assert capi.gemm_group_workspace_size(64, True, 8, 4096, (4096, 4096)) == 0
