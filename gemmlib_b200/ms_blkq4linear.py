@@ -29,7 +29,6 @@ from torch import nn
 from . import ms_blkq4linear_ext
 
 _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
-_SKINNY_WS = ms_blkq4linear_ext.SKINNY_WORKSPACE
 _linear = ms_blkq4linear_ext.linear
 _linear_group = ms_blkq4linear_ext.linear_group
 _group_supported = ms_blkq4linear_ext.linear_group_supported
@@ -53,9 +52,11 @@ def workspaces_owned_by(workspaces: dict):
     in the block may replay; unlike a graph's own workspace these need no zeroing node."""
     before = getattr(_owner, "workspaces", None)
     _owner.workspaces = workspaces
+    ms_blkq4linear_ext.workspace_owners(1)
     try:
         yield workspaces
     finally:
+        ms_blkq4linear_ext.workspace_owners(-1)
         _owner.workspaces = before
 
 
@@ -79,6 +80,8 @@ def split_k_workspace(device, nbytes: int):
         _WORKSPACES[key] = ws
     return ws
 
+
+ms_blkq4linear_ext.workspace_source(_WORKSPACES, lambda index, nbytes: split_k_workspace(torch.device("cuda", index), nbytes))
 
 MAX_GROUP = 4  # layers of one launch
 
@@ -179,29 +182,20 @@ class BlkQ4Linear(nn.Module):
 
     def forward(self, input, out=None):
         # Few and plain lookups: at decode sizes the host's time per call is what a caller sees.
-        block, col_wise, K, N = self.block_size, self.col_wise, self.in_features, self.out_features
         bias = self.bias
         fused = None if bias is None else self._fusable_bias(input)
         settled = self._settled
-        flags = _EARLY if (settled and self.early_weight_fetch) else 0
-        ws = None
-        if self.split_k:
-            rows = input.numel() // K
-            if rows > 16 or block < 64 or not col_wise:  # the others never use one
-                need = _workspace_size(block, col_wise, rows, N, K)
-                if need > 0:
-                    ws = split_k_workspace(input.device, need)
-                    flags |= _SKINNY_WS
         buf = self._buffers
         if "q_weights" in buf and "q_scales" in buf and "q_zp" in buf:
-            packed = buf["q_weights"], buf["q_scales"], buf["q_zp"]
+            w, s, z = buf["q_weights"], buf["q_scales"], buf["q_zp"]
         else:  # replaced on the module by something other than a buffer
-            packed = self.q_weights, self.q_scales, self.q_zp
-        output = _linear(block, col_wise, K, N, input, *packed, fused, flags, ws, out)
+            w, s, z = self.q_weights, self.q_scales, self.q_zp
+        output = _linear(self.block_size, self.col_wise, self.in_features, self.out_features, input, w, s, z, fused,
+                         _EARLY if settled and self.early_weight_fetch else 0, self.split_k, out)
         if not settled:
             self._settled = True
         if bias is not None and fused is None:
-            rows = output.view(-1, N)
+            rows = output.view(-1, self.out_features)
             rows += bias  # broadcast against [rows, out_features], whatever the input's leading dimensions
         return output
 
