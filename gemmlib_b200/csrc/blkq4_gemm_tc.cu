@@ -506,6 +506,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       // lane, 128 contiguous bytes per warp): the even lane writes the even rows m of a
       // 32-row chunk, the odd lane the odd rows, each with its partner's value alongside.
       const int odd = lane & 1;
+      const uint32_t pick = trade_selector(odd);
       const bool n_ok = (n | 1) < col.N;  // N is a multiple of 16: the pair is in or out together
       for (int c0 = 0; c0 < p.BM; c0 += 32) {
         if (m0 + c0 >= m_end) break;  // warp-uniform
@@ -528,10 +529,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         const size_t row_step = 2 * (size_t)col.N;
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-          const float mine = __uint_as_float(odd ? r[j + 1] : r[j]);       // my n, my row
-          const float give = __uint_as_float(odd ? r[j] : r[j + 1]);       // my n, partner's row
-          const float got = __shfl_xor_sync(0xffffffffu, give, 1);          // partner's n, my row
-          __half2 v = odd ? __floats2half2_rn(got, mine) : __floats2half2_rn(mine, got);
+          const uint32_t traded = trade_rows(r[j], r[j + 1], pick);
+          __half2 v = *reinterpret_cast<const __half2*>(&traded);
           if (add_bias) v = __hadd2(v, bias2);
           if (n_ok && m < m_end) *reinterpret_cast<__half2*>(dst) = v;
           dst += row_step;

@@ -39,7 +39,9 @@ constexpr int kPairActStages = 8;     // 16 KB each
 constexpr int kDeqStages = 8;         // dequantized weights in tensor memory, 32 columns each
 constexpr int kDeqGroups = 2;         // warp groups taking k steps in turn (three or four measured slower)
 constexpr int kNumDeqWarps = 4 * kDeqGroups;
-constexpr int kFirstDeqWarp = 2 + kNumEpiWarps;
+// Epilogue warps: kPairEpiShare of them share a quarter of the TMEM lanes, on 32-row chunks in turn
+constexpr int kPairEpiShare = 2, kPairEpiWarps = 4 * kPairEpiShare;
+constexpr int kFirstDeqWarp = 2 + kPairEpiWarps;
 constexpr int kWeightProducerWarp = kFirstDeqWarp + kNumDeqWarps;  // last warp
 constexpr int kPairWeightStages = 6;  // 5.5 KB each; deeper rings measured no faster
 // fp16 staging of a CTA's 128 x 256 output tile: the epilogue empties the accumulator into it, hands
@@ -191,7 +193,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     for (int i = 0; i < kDeqStages; ++i) mbar_init(bar(BAR_MMA_DONE + i), 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(BAR_ACC_FULL + i), 1);
-      mbar_init(bar(BAR_ACC_EMPTY + i), 2 * kNumEpiWarps);
+      mbar_init(bar(BAR_ACC_EMPTY + i), 2 * kPairEpiWarps);
     }
     *abort_flag = 0;
     *s_done = 0u;
@@ -308,14 +310,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       }
     mma_done:;
     }
-  } else if (warp < 2 + kNumEpiWarps) {
+  } else if (warp < kFirstDeqWarp) {
     // =============================== epilogue: this CTA's 128 weight columns ===================================
-    // A warp owns the 32 weight columns n of its TMEM quarter (lane = n) for all 256 activation rows m
+    // A warp owns the 32 weight columns n of its TMEM quarter (lane = n) for every second chunk of 32 activation rows m
     // (TMEM columns).  With the single 256-column accumulator the next tile's MMAs wait for this drain,
-    // so it is kept short: tensor memory -> fp16 -> the warp's own staging block [256 m][32 n] in shared
+    // so it is kept short: tensor memory -> fp16 -> the quarter's staging block [256 m][32 n] in shared
     // memory, accumulator released, and only then staging -> global memory (64-byte row pieces, 8 bytes
-    // per lane), which overlaps the next tile.  No other warp touches the block: only __syncwarp.
-    const int quarter = warp & 3;
+    // per lane), which overlaps the next tile.  No other warp touches the rows of a chunk: only __syncwarp.
+    // Measured on B200, one warp per quarter and a select, conversion and shuffle per value / two warps and trade_rows, us:
+    // M = 4096, 1024 x 4096 35.9 / 30.7; M = 3000, row-wise 512 x 8192 35.3 / 30.0; M = 300, 4096 x 28672 83.2 / 72.5; M = 4096, 8192 x
+    // 28672 1557 / 1487; M = 2048, 4096 x 4096, one hand-over under way 52.7 / 52.3.
+    const int quarter = warp & 3, epi = warp - 2, chunk0 = 32 * (epi >> 2);
     uint32_t tcount = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the output belongs to stream order
     const uint32_t acc_empty_leader = map_to_cta(bar(BAR_ACC_EMPTY), 0);
@@ -328,7 +333,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       gather_off = kGatherCtrlBytes + (size_t)(gather_epoch & 1u) * p.gt.buf_bytes;
     }
     uint8_t* stage = base_ptr + plan.out + quarter * (256 * 64);
-    // Barrier of the four epilogue warps (gather mode), bounded like every wait here: a counter in
+    // Barrier of the epilogue warps (gather mode), bounded like every wait here: a counter in
     // shared memory that only grows; a warp that sees the CTA's abort flag leaves instead of waiting.
     unsigned epi_calls = 0;
     auto epi_barrier = [&]() -> bool {
@@ -338,7 +343,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         __threadfence_block();
         atomicAdd(s_epi, 1u);
         const long long t0 = clock64();
-        while (*reinterpret_cast<volatile unsigned*>(s_epi) < epi_calls * (unsigned)kNumEpiWarps) {
+        while (*reinterpret_cast<volatile unsigned*>(s_epi) < epi_calls * (unsigned)kPairEpiWarps) {
           if (*abort_flag || clock64() - t0 > kWaitCycles) {
             *abort_flag = 1;
             atomicCAS(&g_gemm_tc_error, 0, 0x330 | quarter);
@@ -351,6 +356,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       return *abort_flag == 0;
     };
     const int odd = lane & 1;
+    const uint32_t pick = trade_selector(odd);
     const bool bulk = p.gt.world > 0 && p.gather_bulk;
     const size_t tile_floats = (size_t)p.BM * TILE_N;
     PairWalk walk(p, pair, num_pairs);
@@ -368,7 +374,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         // ---- the tail of a tile whose head another pair computes: fp32 partial tile [m][n] to this CTA's slot
         //      of the workspace (for a row m the 32 lanes of a warp write 128 contiguous bytes)
         float* dst_ws = p.ws_partials + (size_t)blockIdx.x * tile_floats + n_l;
-        for (int c0 = 0; c0 < rows; c0 += 32) {
+        for (int c0 = chunk0; c0 < rows; c0 += 32 * kPairEpiShare) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
           tmem_ld_wait();
@@ -401,7 +407,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         if (lane == 0) {
           const long long t0 = clock64();
           for (int i = 0; i < nparts; ++i) {
-            while (*reinterpret_cast<volatile unsigned*>(p.ws_flags + src_slot + 2u * i) < (unsigned)kNumEpiWarps) {
+            while (*reinterpret_cast<volatile unsigned*>(p.ws_flags + src_slot + 2u * i) < (unsigned)kPairEpiWarps) {
               if (*abort_flag || clock64() - t0 > kWaitCycles) {
                 *abort_flag = 1;
                 atomicCAS(&g_gemm_tc_error, 0, 0x320 | quarter);
@@ -415,7 +421,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         if (*abort_flag) break;
       }
       const float* src_ws = p.ws_partials + (size_t)src_slot * tile_floats + n_l;
-      for (int c0 = 0; c0 < rows; c0 += 32) {
+      for (int c0 = chunk0; c0 < rows; c0 += 32 * kPairEpiShare) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
         tmem_ld_wait();
@@ -437,10 +443,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         const int pitch = bulk ? 256 : 64;
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-          const float mine = __uint_as_float(odd ? r[j + 1] : r[j]);
-          const float give = __uint_as_float(odd ? r[j] : r[j + 1]);
-          const float got = __shfl_xor_sync(0xffffffffu, give, 1);
-          *reinterpret_cast<__half2*>(dst + j * pitch) = odd ? __floats2half2_rn(got, mine) : __floats2half2_rn(mine, got);
+          *reinterpret_cast<uint32_t*>(dst + j * pitch) = trade_rows(r[j], r[j + 1], pick);
         }
       }
       tc_fence_before();
@@ -448,9 +451,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       if (lane == 0) {
         if (rank == 0) mbar_arrive(bar(BAR_ACC_EMPTY));
         else mbar_arrive_remote(acc_empty_leader);
-        // the warp that completes a slot's count (4 writers + 4 readers) puts the flag back to zero
+        // the warp that completes a slot's count (writers + readers) puts the flag back to zero
         for (int i = 0; i < nparts; ++i)
-          if (atomicAdd(p.ws_flags + src_slot + 2u * i, 1u) == (unsigned)(2 * kNumEpiWarps - 1)) p.ws_flags[src_slot + 2u * i] = 0u;
+          if (atomicAdd(p.ws_flags + src_slot + 2u * i, 1u) == (unsigned)(2 * kPairEpiWarps - 1)) p.ws_flags[src_slot + 2u * i] = 0u;
       }
       // staging -> global: one instruction moves four rows' 64-byte pieces
       const int n4 = n_tile * TILE_N + quarter * 32 + (lane & 7) * 4;  // first of this lane's 4 columns
@@ -462,22 +465,25 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         b23 = *reinterpret_cast<const __half2*>(col.bias + n4 + 2);
       }
       if (p.gt.world == 0) {
-        __half* gdst = col.out + (size_t)(m0 + (lane >> 3)) * col.N + n4;
-        for (int r0 = 0; r0 < rows; r0 += 4) {
-          uint2 v = *reinterpret_cast<const uint2*>(stage + r0 * 64 + lane * 8);
-          if (add_bias) {
-            // the bias is added to the ROUNDED result in fp16, as a separate `output += bias` would
-            __half2 lo = __hadd2(*reinterpret_cast<__half2*>(&v.x), b01), hi = __hadd2(*reinterpret_cast<__half2*>(&v.y), b23);
-            v.x = *reinterpret_cast<uint32_t*>(&lo);
-            v.y = *reinterpret_cast<uint32_t*>(&hi);
+        __syncwarp();
+        for (int c0 = chunk0; c0 < rows; c0 += 32 * kPairEpiShare) {
+          __half* gdst = col.out + (size_t)(m0 + c0 + (lane >> 3)) * col.N + n4;
+          for (int r0 = c0; r0 < min(c0 + 32, rows); r0 += 4) {
+            uint2 v = *reinterpret_cast<const uint2*>(stage + r0 * 64 + lane * 8);
+            if (add_bias) {
+              // the bias is added to the ROUNDED result in fp16, as a separate `output += bias` would
+              __half2 lo = __hadd2(*reinterpret_cast<__half2*>(&v.x), b01), hi = __hadd2(*reinterpret_cast<__half2*>(&v.y), b23);
+              v.x = *reinterpret_cast<uint32_t*>(&lo);
+              v.y = *reinterpret_cast<uint32_t*>(&hi);
+            }
+            if (n_ok && r0 + (lane >> 3) < rows) *reinterpret_cast<uint2*>(gdst) = v;
+            gdst += 4 * (size_t)col.N;
           }
-          if (n_ok && r0 + (lane >> 3) < rows) *reinterpret_cast<uint2*>(gdst) = v;
-          gdst += 4 * (size_t)col.N;
         }
       } else if (bulk) {
         // Fused all-gather with bulk copies (the default): every row of the CTA's tile (256 contiguous
         // bytes in the row-major staging block) goes to every rank's gathered buffer as one
-        // cp.async.bulk of the async proxy - 256 rows x world copies per tile, spread over the 128
+        // cp.async.bulk of the async proxy - 256 rows x world copies per tile, spread over the
         // epilogue threads - instead of 16-byte stores by the threads themselves (the branch below,
         // BLKQ4_TC_GATHER_NO_BULK=1).  Measured at 8 ranks, M = 4096: 778 vs 857 us; the same at 2 ranks.
         fence_proxy_async();  // the staging writes (generic proxy) before the bulk copies read them
@@ -487,7 +493,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
           const uint32_t bytes = (uint32_t)cols * 2u;
           const size_t row_bytes = (size_t)p.gt.n_total * 2;
           const size_t off0 = gather_off + ((size_t)p.gt.rank * p.N + (size_t)n_tile * TILE_N) * 2;
-          for (int row = quarter * 32 + lane; row < rows; row += 32 * kNumEpiWarps) {
+          for (int row = epi * 32 + lane; row < rows; row += 32 * kPairEpiWarps) {
             const uint32_t src = smem_u32(base_ptr + plan.out + row * 256);
             const size_t off = off0 + (size_t)(m0 + row) * row_bytes;
             int r = p.gt.rank;
@@ -505,7 +511,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       } else {
         // Fused all-gather: this rank's columns go straight into EVERY rank's gathered buffer
         // [M, n_total] (plain stores over NVLink for the peers), under the next tile's MMAs.  Peer
-        // stores want long contiguous runs, so here the four warps wait for one another and every warp
+        // stores want long contiguous runs, so here the warps wait for one another and every warp
         // then writes whole 256-byte rows of the CTA's 128 columns (16 bytes per lane, two rows per
         // instruction) instead of its own 64-byte pieces (measured at 4 ranks: 64-byte pieces held the
         // kernel at twice its compute time).
@@ -516,7 +522,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         const size_t row_bytes = (size_t)p.gt.n_total * 2;
         const size_t off0 = gather_off + ((size_t)p.gt.rank * p.N + (size_t)n_tile * TILE_N + c8) * 2;
         const uint8_t* src0 = stage_all + (c8 >> 5) * (256 * 64) + (c8 & 31) * 2;
-        for (int r0 = 2 * quarter; r0 < rows; r0 += 2 * kNumEpiWarps) {
+        for (int r0 = 2 * epi; r0 < rows; r0 += 2 * kPairEpiWarps) {
           const int row = r0 + (lane >> 4);
           if (n_ok8 && row < rows) {
             const uint4 v = *reinterpret_cast<const uint4*>(src0 + row * 64);
@@ -542,7 +548,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
       // rank's flag in every rank's block.  One system-scope fence per CTA.
       __syncwarp();
       if (lane == 0) __threadfence_block();
-      if (lane == 0 && atomicAdd(s_done, 1u) == (unsigned)kNumEpiWarps - 1u) {
+      if (lane == 0 && atomicAdd(s_done, 1u) == (unsigned)kPairEpiWarps - 1u) {
         uint8_t* local = p.gt.base[p.gt.rank];
         __threadfence_system();
         const unsigned arrived = atomicAdd(reinterpret_cast<unsigned*>(local + kGatherDoneOff), 1u);
@@ -559,7 +565,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     }
   } else if (warp < kWeightProducerWarp) {
     // =============================== dequantizers: this CTA's 128 weight columns ===============================
-    const int dw = warp - (2 + kNumEpiWarps);
+    const int dw = warp - kFirstDeqWarp;
     const int group = dw / kWarpsPerDeqGroup;
     const int n_l = 32 * (warp & 3) + lane;
     const int np_l = 8 * (n_l >> 4) + (n_l & 7);

@@ -87,6 +87,16 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Two accumulator values of one weight column n, activation rows m and m + 1, rounded to fp16 and traded with the lane of
+// the other column of the pair (lanes n even / odd): the even lane gets row m of both columns, the odd one row m + 1.
+// `pick` is trade_selector(n odd).  One conversion, shuffle and byte permutation for two values.
+__device__ __forceinline__ uint32_t trade_selector(int odd) { return odd ? 0x3276u : 0x5410u; }
+__device__ __forceinline__ uint32_t trade_rows(uint32_t row0, uint32_t row1, uint32_t pick) {
+  const __half2 own = __floats2half2_rn(__uint_as_float(row0), __uint_as_float(row1));
+  const uint32_t mine = *reinterpret_cast<const uint32_t*>(&own);
+  return __byte_perm(mine, __shfl_xor_sync(0xffffffffu, mine, 1), pick);
+}
+
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
