@@ -18,13 +18,18 @@
 // weight.  The column-wise kernel executes 9.7 (13.7 M warp instructions for 45 M weights), ~5 of them in quantize_pair
 // and assemble_word, and issues in 65 % of the cycles.  Measured on B200 (4096 x 11008, block 64, zero points, 114 MB):
 // 28.5 us with 14 in the conversion alone - float-to-integer conversions and min / max on quarter- and half-rate pipes,
-// the scale's divisions repeated by every lane of a block - and 22.8 us now (0.77 of the measured copy bandwidth).
+// the scale's divisions repeated by every lane of a block - and 21.5 us now (0.81 of the measured copy bandwidth).
+//
+// A CTA is short: it loads, waits, computes and leaves, so small ones keep the SM's slots turning over more evenly.  CTAs of
+// 128 threads, ten of them on an SM (48 registers), against 256, us: column-wise 4096 x 11008 22.0 / 21.5, 8192 x 28672
+// block 128 101.7 / 94.8; row-wise 11008 x 4096 block 32 28.1 / 25.0, 4096 x 11008 block 64 29.0 / 24.8.  Twelve on an SM
+// (40 registers, spills) 21.5, 101.9, 26.7, 25.8.
 #include "blkq4_common.cuh"
 
 namespace blkq4 {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr unsigned kMaxGridY = 32768;
 
@@ -169,7 +174,7 @@ __device__ __forceinline__ float half_bits_to_float(uint32_t h) { return __half2
 // (min, max) pairs.  Where a block has several lanes, the even ones compute the scale of column n0 and the odd
 // ones that of n0 + 8 (two or three IEEE divisions each) and they trade results.
 template <int BLOCK, bool ALIGNED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 10)
 quant_colwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t* __restrict__ packed,
                      __half* __restrict__ scales, uint8_t* __restrict__ zps) {
   constexpr int G = BLOCK / 16;          // lanes per quantization block: 1, 2, 4, 8
@@ -262,25 +267,31 @@ quant_colwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
 // ---- row-wise blocks ----------------------------------------------------------------------------------
 // A block is BLOCK consecutive columns at one k, i.e. one value of each column of one to eight warps.  Each warp
 // reduces its 16 columns (the min / max of eight k pairs across the eight lanes of a k chunk, halving the pairs a
-// lane carries at every exchange), the CTA's eight warps (64 k x 128 columns) meet in shared memory, one thread per
-// block computes the scale, and every thread picks up the parameters of its 16 k.  The weights stay in registers.
+// lane carries at every exchange), the CTA's four warps (64 k x 64 columns; eight for blocks of 128) meet in shared memory,
+// one thread per block computes the scale, and every thread picks up the parameters of its 16 k.  The weights stay in registers.
 // (Measured, 11008 x 4096, block 32, symmetric: 82 us with the whole tile staged in shared memory and scanned in
 // four passes.)
+template <int BLOCK>
+constexpr int kRowWarps = BLOCK == 128 ? 8 : 4;  // 16 columns each: whole blocks
+// Word of shared memory of the parameter of row k: 16 rows and a gap of four words, so that the four k chunks whose
+// parameters a warp reads 16 bytes at a time lie on different banks
+__device__ __forceinline__ int param_word(int k) { return k + (k >> 4) * 4; }
 template <int BLOCK, bool ALIGNED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(32 * kRowWarps<BLOCK>, (kRowWarps<BLOCK> == 4 ? 10 : 5))
 quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t* __restrict__ packed,
                      __half* __restrict__ scales, uint8_t* __restrict__ zps) {
   constexpr int GROUPS = BLOCK / 16;          // 16-column groups (warps) per block
-  constexpr int NB = 128 / BLOCK;             // blocks per k in the tile
-  __shared__ uint2 s_range[kWarps][32];       // [16-column group][k pair] min2, max2
-  __shared__ __align__(16) unsigned short s_first[kWarps][64];  // [group][k] the group's first column
-  __shared__ __align__(16) float s_recip[NB][64];  // -1 / scale
-  __shared__ __align__(16) float s_zp[NB][64];     // -zero point
+  constexpr int W = kRowWarps<BLOCK>;
+  constexpr int NB = 16 * W / BLOCK;          // blocks per k in the tile
+  __shared__ uint2 s_range[W][32];       // [16-column group][k pair] min2, max2
+  __shared__ __align__(16) unsigned short s_first[W][64];  // [group][k] the group's first column
+  __shared__ __align__(16) float s_recip[NB][80];  // -1 / scale
+  __shared__ __align__(16) float s_zp[NB][80];     // -zero point
 
   start_in_stream_order();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kl = lane & 3, npl = lane >> 2;   // chunk along k, packed column of the group
-  const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 128;
+  const int k0 = blockIdx.x * 64, n0 = (blockIdx.z * kMaxGridY + blockIdx.y) * (16 * W);
   const bool valid = n0 + warp * 16 < N;      // whole warps; N is a multiple of 16
   const bool has_zp = zps != nullptr;
   uint32_t va[8], vb[8];
@@ -318,7 +329,7 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   __syncthreads();
 
   // ---- one thread per quantization block ----
-  for (int b = threadIdx.x; b < 64 * NB; b += kThreads) {
+  for (int b = threadIdx.x; b < 64 * NB; b += 32 * W) {
     const int nb = b >> 6, k = b & 63;
     if (n0 + nb * BLOCK >= N) break;
     const int sh = (k & 1) * 16;
@@ -333,8 +344,8 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
     uint8_t z;
     float rc;
     block_params(mn, mx, half_bits_to_float(s_first[nb * GROUPS][k]), has_zp, sc, z, rc);
-    s_recip[nb][k] = -rc;
-    s_zp[nb][k] = -(float)z;
+    s_recip[nb][param_word(k)] = -rc;
+    s_zp[nb][param_word(k)] = -(float)z;
     // meta column-major [K, N / BLOCK], every 16 rows permuted (reference dev_prepack_scales, :457-547): source row
     // 2t + u + 8h goes to 4t + u + 2h (scales) and 4t + 2u + h (zero points)
     const int g16 = k & ~15, u = k & 1, t = (k >> 1) & 3, h = (k >> 3) & 1;
@@ -350,8 +361,8 @@ quant_rowwise_kernel(const __half* __restrict__ w, int K, int N, int ld, uint8_t
   unsigned long long r2[8], z2[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 r = *reinterpret_cast<const float4*>(&s_recip[nb][kl * 16 + 4 * i]);
-    const float4 z = *reinterpret_cast<const float4*>(&s_zp[nb][kl * 16 + 4 * i]);
+    const float4 r = *reinterpret_cast<const float4*>(&s_recip[nb][param_word(kl * 16) + 4 * i]);
+    const float4 z = *reinterpret_cast<const float4*>(&s_zp[nb][param_word(kl * 16) + 4 * i]);
     r2[2 * i] = pack_f32x2(r.x, r.y);
     r2[2 * i + 1] = pack_f32x2(r.z, r.w);
     z2[2 * i] = pack_f32x2(z.x, z.y);
@@ -383,7 +394,10 @@ cudaError_t launch_T(bool colwise, int K, int N, int ld, cudaStream_t stream, co
     cfg.gridDim = dim3((kblks + kWarps - 1) / kWarps, groups < kMaxGridY ? groups : kMaxGridY, (groups + kMaxGridY - 1) / kMaxGridY);
     return cudaLaunchKernelEx(&cfg, quant_colwise_kernel<BLOCK, ALIGNED>, w, K, N, ld, packed, scales, zp);
   }
-  cfg.gridDim = dim3(K / 64, (N + 127) / 128);
+  constexpr int kCols = 16 * kRowWarps<BLOCK>;
+  const unsigned tiles = (N + kCols - 1) / kCols;
+  cfg.gridDim = dim3(K / 64, tiles < kMaxGridY ? tiles : kMaxGridY, (tiles + kMaxGridY - 1) / kMaxGridY);
+  cfg.blockDim = dim3(2 * kCols);
   return cudaLaunchKernelEx(&cfg, quant_rowwise_kernel<BLOCK, ALIGNED>, w, K, N, ld, packed, scales, zp);
 }
 

@@ -37,3 +37,23 @@ def test_quantizer_keeps_stream_order(colwise):
     for a, b in zip(want + [want[-1]], got + [list(q)]):
         for s, t in zip(a, b):
             assert torch.equal(s.view(torch.uint8), t.view(torch.uint8))
+
+
+@pytest.mark.parametrize("block,N", [(32, 64 * 32768 + 32), (128, 128 * 32768 + 128), (16, 64 * 32768 - 32)])
+def test_row_wise_tiles_beyond_one_grid_layer(block, N):
+    """The column tiles fold into the grid's third dimension: what lies behind the fold against the same columns alone."""
+    K, tail = 64, 4096
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w = (torch.randn(N, K, generator=g, device="cuda") * 0.02).half()
+
+    def quant(x):
+        n = x.size(0)
+        q = (torch.empty(K * n // 2, dtype=torch.uint8, device="cuda"), torch.empty(K * n // block, dtype=torch.float16, device="cuda"),
+             torch.empty(K * n // block, dtype=torch.uint8, device="cuda"))
+        capi.quant(block, False, K, n, K, x, *q)
+        torch.cuda.synchronize()
+        return q
+
+    start = (N - tail) // 128 * 128  # a shard of the columns is a contiguous range of bytes
+    for whole, part in zip(quant(w), quant(w[start:].contiguous())):
+        assert torch.equal(whole[-part.numel():].view(torch.uint8), part.view(torch.uint8))
