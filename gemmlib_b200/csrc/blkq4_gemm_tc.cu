@@ -86,7 +86,14 @@ struct Shape {
 // M = 17 50.2 vs 40.3, M = 128 67.2 vs 58.0; M = 100, 4096 -> 11008 20.5 vs 16.3; M = 32, 4096 x 4096 10.1 vs 9.5.
 // Above 128 rows two 64-k steps of activations per stage leave three stages only (rowwise M = 333: 24.8 vs 27.4 us).
 // Groups: two / three / four at M = 64: 47.3 / 43.9 / 44.5 us; M = 32, 4096 x 4096: 9.7 / 9.5 / 10.3 us.
+// Four groups where a CTA has many steps: up to 64 rows the dequantizers' instructions set the pace, and the scheduler has more
+// to choose from; the fourth group's start-up and its share of the ring only pay off after some 16 steps.  Three / four, us, block
+// 64 column-wise with zero points: K = 8192, N = 28672 (97 steps a CTA): M = 17 40.8 / 38.7, M = 64 50.9 / 48.6; 11008 x 4096
+// (22) M = 40 13.2 / 12.8; 4096 x 11008 (32) M = 64 14.1 / 13.4; 2048 x 22528 (19) M = 64 12.9 / 12.7; 1024 x 14336 (8) 6.2 / 6.3;
+// 4096 x 4096 (8) 8.8 / 8.9.
 using ShapeSmall = Shape<64, 2, 6, 10, 3>;  // two accumulators + six stages of 64 TMEM columns = 512
+using ShapeSmallLong = Shape<64, 2, 6, 10, 4>;
+constexpr int kLongSteps = 16;
 using ShapeMid = Shape<128, 2, 4, 8, 3>;    // two accumulators + four stages = 512
 using ShapeLarge = Shape<256, 1, 6, 6, 3>;
 // Activation rows of a tile, a multiple of `unit`: as few tiles of up to 256 rows as there can be, all of one height.
@@ -773,7 +780,7 @@ SplitPlan plan_split(int M, int n_tiles, int K, size_t ws_bytes_available) {
   return best;
 }
 
-// The one-CTA kernel for tiles of BM rows.
+// The one-CTA kernel for tiles of BM rows and `steps` pipeline steps a CTA.
 template <int G>
 using Kern = void (*)(CUtensorMap, WeightMaps<G>, Params);
 template <int G>
@@ -783,10 +790,10 @@ struct KernelChoice {
   size_t smem;
   int deq_cols;        // tensor memory of the dequantized stages
 };
-std::atomic<int> g_granted_smem[12][64];
+std::atomic<int> g_granted_smem[16][64];
 
 template <int G>
-KernelChoice<G> choose_kernel(bool colwise, int BM) {
+KernelChoice<G> choose_kernel(bool colwise, int BM, int steps = 0) {
   KernelChoice<G> c;
   auto pick = [&](auto shape, int idx) {
     using S = decltype(shape);
@@ -796,7 +803,8 @@ KernelChoice<G> choose_kernel(bool colwise, int BM) {
     c.smem = make_plan(S::MAXM, S::WS, S::RING, S::KSUB).total;
     c.deq_cols = S::kDeqTmemCols;
   };
-  if (BM <= ShapeSmall::MAXM) pick(ShapeSmall{}, 0);
+  if (BM <= ShapeSmall::MAXM && steps >= kLongSteps) pick(ShapeSmallLong{}, 3);
+  else if (BM <= ShapeSmall::MAXM) pick(ShapeSmall{}, 0);
   else if (BM <= ShapeMid::MAXM) pick(ShapeMid{}, 1);
   else pick(ShapeLarge{}, 2);
   return c;
@@ -805,7 +813,7 @@ KernelChoice<G> choose_kernel(bool colwise, int BM) {
 // Clusters of `split` CTAs of the kernel that are resident at once on the current device, 0 when it cannot say.
 template <int G>
 int resident_clusters(const KernelChoice<G>& kc, int split) {
-  static std::atomic<int> cache[12][kMaxSplit + 1][64];
+  static std::atomic<int> cache[16][kMaxSplit + 1][64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   const bool cached = dev >= 0 && dev < 64;
@@ -1092,9 +1100,10 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
     return std::string();
   }
   const int num_tiles = p.m_tiles * p.n_tiles;
-  const KernelChoice<G> kc = choose_kernel<G>(colwise, p.BM);
   p.k_steps = (K + sk - 1) / sk;
   SplitPlan sp = plan_split(M, n_tiles, K, ws_ok ? workspace_bytes : 0);
+  const int cta_steps = sp.split > 1 ? sp.k_per_item : (int)((long long)num_tiles * p.k_steps / (num_tiles < sms ? num_tiles : sms));
+  const KernelChoice<G> kc = choose_kernel<G>(colwise, p.BM, cta_steps);
   fit_split(kc, num_tiles, p.k_steps, sp);
   p.split = sp.split;  // split > 1: at most one item per SM
   p.k_per_item = sp.k_per_item;

@@ -29,7 +29,8 @@ def test_workspace_sizes_do_not_follow_the_tile_height():
                                   (16, True, True, 257, 18944, 128), (32, False, True, 513, 9504, 192),  # pairs of CTAs
                                   (128, True, False, 289, 18976, 256),
                                   (64, True, True, 17, 96, 4096), (64, True, True, 66, 128, 4096), (32, True, True, 131, 128, 4096),
-                                  (32, True, True, 13, 4096, 4096)],
+                                  (32, True, True, 13, 4096, 4096),
+                                  (32, False, True, 64, 160, 2048), (16, True, False, 40, 96, 1984)],  # 16 steps a CTA: four groups
                          ids=lambda c: "-".join(map(str, c)))
 def test_ragged_rows(case):
     """Against the oracle, with the split (workspace) and without; both runs of a split agree bit for bit."""
