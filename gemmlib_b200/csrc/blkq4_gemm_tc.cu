@@ -85,7 +85,6 @@ struct Shape {
 // B200, 64-k against 128-k steps with three groups each: K = 8192, N = 28672, block 128: M = 64 54.6 vs 43.9 us,
 // M = 17 50.2 vs 40.3, M = 128 67.2 vs 58.0; M = 100, 4096 -> 11008 20.5 vs 16.3; M = 32, 4096 x 4096 10.1 vs 9.5.
 // Above 128 rows two 64-k steps of activations per stage leave three stages only (rowwise M = 333: 24.8 vs 27.4 us).
-// Groups: two / three / four at M = 64: 47.3 / 43.9 / 44.5 us; M = 32, 4096 x 4096: 9.7 / 9.5 / 10.3 us.
 // Four groups where a CTA has many steps: up to 64 rows the dequantizers' instructions set the pace, and the scheduler has more
 // to choose from; the fourth group's start-up and its share of the ring only pay off after some 16 steps.  Three / four, us, block
 // 64 column-wise with zero points: K = 8192, N = 28672 (97 steps a CTA): M = 17 40.8 / 38.7, M = 64 50.9 / 48.6; 11008 x 4096
