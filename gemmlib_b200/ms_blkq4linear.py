@@ -32,7 +32,6 @@ _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
 _linear = ms_blkq4linear_ext.linear
 _linear_group = ms_blkq4linear_ext.linear_group
 _group_supported = ms_blkq4linear_ext.linear_group_supported
-_group_workspace_size = ms_blkq4linear_ext.linear_group_workspace_size
 _graph_workspace = ms_blkq4linear_ext.graph_workspace
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
@@ -87,8 +86,8 @@ MAX_GROUP = 4  # layers of one launch
 
 
 def can_share_launch(layers, rows) -> bool:
-    """Whether one launch computes all ``layers`` (two to four) from the same ``rows`` activation rows, with the results
-    their ``forward`` calls give: layers of one shape of blocks, with nothing hooked into their calls."""
+    """Whether one launch can compute all ``layers`` (two to four) from the same ``rows`` activation rows: layers of one
+    shape of blocks, with nothing hooked into their calls."""
     first = layers[0]
     for l in layers:
         if not isinstance(l, BlkQ4Linear):
@@ -104,22 +103,25 @@ def can_share_launch(layers, rows) -> bool:
     return _group_supported(first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers])
 
 
-def shared_workspace_bytes(layers, rows):
-    """Split-K workspace that ``run_as_one`` uses for ``rows`` activation rows (0: none)."""
-    first = layers[0]
-    if not all(l.split_k for l in layers):
-        return 0
-    return _group_workspace_size(first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers])
+def one_launch_keeps_bits(layers, rows) -> bool:
+    """Whether one launch for layers that ``can_share_launch`` gives every bit of their ``forward`` calls.  Up to 16 rows it
+    does.  Above, a layer whose own call splits K adds its fp32 sums in the order of that split, which a launch over the tiles
+    of all layers would cut elsewhere, so only layers that run without a split are taken together."""
+    return rows <= 16 or all(l.workspace_bytes(rows) == 0 for l in layers)
 
 
-def run_as_one(layers, input, outputs):
-    """One launch for layers that ``can_share_launch``: ``outputs[i] = layers[i](input)``."""
+def run_group(layers, input, outputs):
+    """``outputs[i] = layers[i](input)``, bit for bit, for layers that ``can_share_launch``: in one launch where that keeps
+    the bits, else in one per layer."""
+    if not one_launch_keeps_bits(layers, input.size(0)):
+        for l, out in zip(layers, outputs):
+            l(input, out=out)
+        return
     first = layers[0]
-    ws = split_k_workspace(input.device, shared_workspace_bytes(layers, input.size(0)))
     early = all(l._settled and l.early_weight_fetch for l in layers)
     _linear_group(first.block_size, first.col_wise, first.in_features, input, [l.q_weights for l in layers],
                   [l.q_scales for l in layers], [l.q_zp for l in layers], [l.bias for l in layers], list(outputs),
-                  _EARLY if early else 0, ws)
+                  _EARLY if early else 0, None)
     for l in layers:
         l._settled = True
 

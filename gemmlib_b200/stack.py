@@ -9,7 +9,7 @@ an output buffer, captures the whole pass once per row count M on its own stream
 replays it.  Inside the graph the skinny kernels are launched with
 ``BLKQ4_GEMM_EARLY_WEIGHT_FETCH``: the weights of layer i+1 stream in while layer i
 drains.  Consecutive layers that read the same buffer (q, k and v; gate and up) are one launch where a kernel
-takes them together.
+takes them together with every bit of their own calls' results.
 
 It runs the linears only: what sits between them in a model (attention, activation
 functions, norms) is the caller's and can be captured into the same graph by passing
@@ -21,7 +21,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, run_as_one, shared_workspace_bytes, workspaces_owned_by
+from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, run_group, workspaces_owned_by
 
 
 class LinearStack:
@@ -60,7 +60,7 @@ class LinearStack:
         return bufs
 
     def _groups(self, M: int) -> List[range]:
-        """The steps in runs that one launch takes at this row count: up to four that follow one another, read the same
+        """The steps in runs that one launch can take at this row count (``run_group`` says whether it does): up to four that follow one another, read the same
         buffer, write others, and have no hook between them."""
         runs: List[range] = []
         for i, (lyr, src, dst) in enumerate(self.steps):
@@ -79,7 +79,7 @@ class LinearStack:
         for run in groups:
             members = [self.steps[i] for i in run]
             if len(members) > 1:
-                run_as_one([lyr for lyr, _, _ in members], bufs[members[0][1]], [bufs[dst] for _, _, dst in members])
+                run_group([lyr for lyr, _, _ in members], bufs[members[0][1]], [bufs[dst] for _, _, dst in members])
             else:
                 lyr, src, dst = members[0]
                 lyr(bufs[src], out=bufs[dst])
@@ -92,9 +92,7 @@ class LinearStack:
         groups = self._groups(M)
         # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
         # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
-        need = max((shared_workspace_bytes(layers, M) if len(layers) > 1 else layers[0].workspace_bytes(M)
-                    for layers in ([self.steps[i][0] for i in run] for run in groups)
-                    if isinstance(layers[0], BlkQ4Linear)), default=0)
+        need = max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)), default=0)
         split_k = {}
         if need > 0:
             split_k[self.device.index, self.stream.cuda_stream] = [

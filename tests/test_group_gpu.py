@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from gemmlib_b200 import capi
-from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
+from gemmlib_b200.ms_blkq4linear import BlkQ4Linear, one_launch_keeps_bits
 from gemmlib_b200.stack import LinearStack, llama_like_stack
 
 pytestmark = pytest.mark.gpu
@@ -89,8 +89,8 @@ def test_prefill_group_equals_its_parts(M, K, block, colwise, zp, widths):
 
 @pytest.mark.parametrize("M", [1, 7, 9, 40, 300])
 def test_stack_equals_its_layers(M):
-    """q, k, v and gate, up go in one launch where a kernel takes them; the buffers are those of one call per layer (above
-    16 rows up to the order of the fp32 sums)."""
+    """q, k, v and gate, up are runs of their own, in one launch up to 16 rows and where no layer splits K; the buffers are
+    those of one call per layer, bit for bit."""
     stack = llama_like_stack(2048, 2304, 2, 64, True, False, torch.device("cuda"))
     x = torch.randn(M, 2048, device="cuda").half()
     stack.forward(x, "h1")
@@ -99,11 +99,21 @@ def test_stack_equals_its_layers(M):
     assert sum(runs) == 14 and max(runs) == (1 if 8 < M <= 16 else 3)
     for lyr, src, dst in stack.steps[7:]:  # the first block's buffers but "h0" were overwritten by the second's
         want = lyr(got[src])
-        if M <= 16:
-            assert torch.equal(got[dst], want), dst
-        else:
-            d = (got[dst].float() - want.float()).abs()
-            assert bool((d <= 2.0 ** -10 * torch.clamp(want.float().abs(), min=1.0)).all()), (dst, float(d.max()))
+        assert torch.equal(got[dst].view(torch.int16), want.view(torch.int16)), dst
+
+
+# (hidden, ffn, rows, launches of a block): layers alone split K; balanced ranges; neither, so q, k, v and gate, up go together
+@pytest.mark.parametrize("hidden,ffn,M,launches", [(2048, 2304, 40, 7), (2048, 2304, 300, 7), (1024, 19200, 300, 7),
+                                                   (512, 768, 17, 4), (512, 768, 333, 4)])
+def test_prefill_stack_keeps_every_bit(hidden, ffn, M, launches):
+    stack = llama_like_stack(hidden, ffn, 1, 64, True, False, torch.device("cuda"))
+    x = torch.randn(M, hidden, device="cuda").half()
+    stack.forward(x, "h0")
+    got = stack.buffers(M)
+    runs = [[stack.steps[i][0] for i in r] for r in stack._groups(M)]
+    assert sum(1 if one_launch_keeps_bits(r, M) else len(r) for r in runs) == launches
+    for lyr, src, dst in stack.steps:
+        assert torch.equal(got[dst].view(torch.int16), lyr(got[src]).view(torch.int16)), dst
 
 
 def test_what_keeps_layers_of_a_stack_apart():
