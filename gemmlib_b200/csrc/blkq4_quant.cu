@@ -34,13 +34,13 @@ constexpr int kWarps = kThreads / 32;
 constexpr unsigned kMaxGridY = 32768;
 
 // Both kernels are launched with programmatic stream serialization: their CTAs become resident, and the launch's own
-// latency passes, while the last CTAs of the preceding kernel still run; nothing is read or written before that kernel
-// has completed.  Measured on B200, the seven weights of a decoder block (4096, 11008; block 64, zero points) 117.1 us
-// without it, 101.2 with; row-wise 11008 x 4096, block 32 29.0 / 27.4.
-__device__ __forceinline__ void start_in_stream_order() {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// latency passes, while the preceding kernel ends (or, where that kernel lets its successor start early, while it still
+// runs); nothing is read or written before it has completed.  Measured on B200, seven weights of a decoder block (4096, 11008;
+// block 64, zero points) 117.1 us without it, 104.9 with; row-wise 11008 x 4096, block 32 29.0 / 26.7.
+// They execute no griddepcontrol.launch_dependents: a GEMM with BLKQ4_GEMM_EARLY_WEIGHT_FETCH right behind a quantizer would
+// then read packed weights that are not written yet.  It would gain nothing either (quantizer behind quantizer, with / without:
+// 106.1 / 104.9 us a block, row-wise 26.7 / 26.7; 4096 x 4096, block 16 10.8 / 10.8).
+__device__ __forceinline__ void start_in_stream_order() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Scale and zero point from a block's range.  Same float operation sequence as
 // the reference's range2scalezp (f16_quant_sm80.cuh:96-122): IEEE division,

@@ -143,7 +143,9 @@ class BlkQ4Linear(nn.Module):
         self.bias = bias_tensor
         self.early_weight_fetch = True
         self.split_k = True  # prefill shapes with few output tiles split K through a shared workspace
-        self._settled = False  # the first forward is a plain launch, ordered after the quantizer
+        # The first forward is a plain launch.  It may run on another stream than the quantizer: no launch starts before
+        # the CTAs of a quantizer ahead of it in its own stream have left.
+        self._settled = False
 
     @classmethod
     def from_packed(cls, block_size, col_wise, in_features, out_features, q_weights, q_scales, q_zp=None,

@@ -1,8 +1,10 @@
-"""The quantizer's launch starts early but keeps stream order with what writes its weights and reads its results."""
+"""The quantizer's launch starts early but keeps stream order with what writes its weights and reads or overwrites its
+results."""
 import pytest
 import torch
 
-from gemmlib_b200 import capi
+from gemmlib_b200 import capi, ms_blkq4linear_ext
+from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +59,42 @@ def test_row_wise_tiles_beyond_one_grid_layer(block, N):
     start = (N - tail) // 128 * 128  # a shard of the columns is a contiguous range of bytes
     for whole, part in zip(quant(w), quant(w[start:].contiguous())):
         assert torch.equal(whole[-part.numel():].view(torch.uint8), part.view(torch.uint8))
+
+
+def weight(N, K, seed):
+    return (torch.randn(N, K, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * 0.02).half()
+
+
+@pytest.mark.parametrize("col_wise,N,K", [(True, 2048, 2048), (False, 1024, 2048), (True, 512, 4096)])
+@pytest.mark.parametrize("M", [1, 12, 40])
+def test_early_weight_fetch_behind_the_quantizer(M, col_wise, N, K):
+    """A layer whose first (plain) call ran on a side stream, and a layer whose packed tensors were replaced, are called with
+    the early weight fetch right behind the quantizer of those tensors, all queued behind a long kernel."""
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(7), device="cuda").half()
+    ws = [weight(N, K, s) for s in range(4)]
+    want = []
+    for w in ws:
+        layer = BlkQ4Linear(64, col_wise, False, w)
+        torch.cuda.synchronize()
+        want.append(layer(x))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = []
+    for w in ws:
+        torch.cuda._sleep(2_000_000)  # about a millisecond: the calls below are queued before the quantizer starts
+        layer = BlkQ4Linear(64, col_wise, False, w)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            layer(x)
+        assert layer._settled and layer.early_weight_fetch
+        got.append(layer(x))
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    replaced = []
+    for w in ws:
+        torch.cuda._sleep(2_000_000)
+        layer.q_weights, layer.q_scales, layer.q_zp = ms_blkq4linear_ext.quant(64, col_wise, True, w)
+        replaced.append(layer(x))
+    torch.cuda.synchronize()
+    for a, b, c in zip(want, got, replaced):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16)) and torch.equal(a.view(torch.int16), c.view(torch.int16))
