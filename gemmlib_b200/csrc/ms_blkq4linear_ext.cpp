@@ -253,14 +253,15 @@ c10::optional<torch::Tensor> graph_workspace(int device, uintptr_t stream_handle
 
 // ---- BlkQ4Linear.forward ----
 // Where split-K workspaces come from: `eager` is the module's dict (device, stream) -> tensor, `provide(device, nbytes)`
-// its function for every other case; `owners` counts the blocks in which somebody else provides them, in any thread.
+// its function for every other case, both null until somebody imports that module; `owners` counts the blocks in which somebody else provides them, in any thread.
 PyObject* g_eager_workspaces = nullptr;
 PyObject* g_provide_workspace = nullptr;
 std::atomic<int> g_workspace_owners{0};
 
-// The workspace of a call on the device's current stream.  The common case, an eager call on a stream that has a
-// buffer of the size, is answered here.
+// The workspace of a call on the device's current stream; none without a source of them.  The common case, an eager call on
+// a stream that has a buffer of the size, is answered here.
 c10::optional<torch::Tensor> split_k_workspace(int device, int64_t nbytes) {
+  if (!g_eager_workspaces || !g_provide_workspace) return c10::nullopt;
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {

@@ -1,5 +1,9 @@
 """Where an eager BlkQ4Linear call takes its split-K workspace from: the device and stream's buffer, grown on demand, or the
 owner's; and what the native call refuses."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -50,3 +54,19 @@ def test_what_the_native_call_refuses():
         layer(torch.zeros(20, 256, dtype=torch.float16, device="cuda"), out=torch.zeros(20, 128, device="cuda"))
     x = torch.randn(3, 256, device="cuda").half()
     assert torch.equal(layer(x), layer(x, out=torch.empty(3, 128, dtype=torch.float16, device="cuda")))
+
+
+def test_native_call_without_the_module():
+    """The extension alone, in a process of its own: no source of workspaces, so a shape that would split K runs whole."""
+    code = """
+import torch
+from gemmlib_b200 import ms_blkq4linear_ext as ext
+q = ext.quant(64, True, True, (torch.randn(1024, 1024, device="cuda") * 0.02).half())
+x = torch.randn(64, 1024, device="cuda").half()
+assert ext.gemm_workspace_size_blocked(64, True, 64, 1024, 1024) > 0
+got = ext.linear(64, True, 1024, 1024, x, *q, None, 0, True, None)
+assert torch.equal(got.view(torch.int16), ext.forward(64, True, 1024, 1024, x, *q).view(torch.int16))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
