@@ -287,26 +287,56 @@ c10::optional<torch::Tensor> split_k_workspace(int device, int64_t nbytes) {
 // because at decode sizes the Python calls around the launch took longer than the kernel, and with CPython's vectorcall
 // signature because pybind11 took about 1 us to convert the arguments.  Measured, host time per call: one token 7.1 -> 6.4 us,
 // with a split-K workspace (M = 333) 13.4 -> 9.0.
-PyObject* linear_fastcall(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+constexpr int kLinearArgs = 12;
+constexpr const char* kLinearNames[kLinearArgs] = {"block_size", "col_wise", "in_features", "out_features", "input", "q_weights",
+                                                   "q_scales", "q_zp", "bias", "flags", "workspace", "out"};
+
+PyObject* linear_fastcall(PyObject*, PyObject* const* given, Py_ssize_t nargs, PyObject* kwnames) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK_TYPE(nargs == 12,
-                   "linear(block_size, col_wise, in_features, out_features, input, q_weights, q_scales, q_zp, bias, flags, split_k, out)");
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  PyObject* const* args = given;
+  PyObject* named[kLinearArgs] = {};
+  if (nkw > 0 && nargs + nkw == kLinearArgs) {  // all of them, each once
+    std::copy(given, given + nargs, named);
+    for (Py_ssize_t k = 0; k < nkw; ++k) {
+      int i = 0;
+      while (i < kLinearArgs && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, k), kLinearNames[i]) != 0) ++i;
+      TORCH_CHECK_TYPE(i < kLinearArgs && !named[i], "linear: a keyword that it does not have, or an argument given twice");
+      named[i] = given[nargs + k];
+    }
+    args = named;
+  }
+  TORCH_CHECK_TYPE(nargs + nkw == kLinearArgs,
+                   "linear(block_size, col_wise, in_features, out_features, input, q_weights, q_scales, q_zp, bias, flags, workspace, out)");
   auto integer = [&](int i) {
     const long v = PyLong_AsLong(args[i]);
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
   };
+  auto small = [&](int i) {
+    const long v = integer(i);
+    TORCH_CHECK_TYPE(v == long(int(v)), "linear: ", kLinearNames[i], " = ", v, " is out of range");
+    return int(v);
+  };
+  auto truth = [&](int i) {
+    const int v = PyObject_IsTrue(args[i]);
+    if (v < 0) throw python_error();
+    return v == 1;
+  };
   auto tensor = [&](int i) -> const torch::Tensor& {
-    TORCH_CHECK_TYPE(THPVariable_Check(args[i]), "linear: argument ", i, " must be a tensor");
+    TORCH_CHECK_TYPE(THPVariable_Check(args[i]), "linear: ", kLinearNames[i], " must be a tensor");
     return THPVariable_Unpack(args[i]);
   };
-  const int block_size = int(integer(0)), in_features = int(integer(2)), out_features = int(integer(3));
-  const bool col_wise = PyObject_IsTrue(args[1]) == 1;
+  const int block_size = small(0), in_features = small(2), out_features = small(3);
+  const bool col_wise = truth(1);
   const torch::Tensor &input = tensor(4), &q_weights = tensor(5), &q_scales = tensor(6), &q_zp = tensor(7);
   c10::optional<torch::Tensor> bias, workspace;
   if (args[8] != Py_None) bias = tensor(8);
   int64_t flags = integer(9);
-  const bool split_k = PyObject_IsTrue(args[10]) == 1;
+  // the caller's workspace, or whether to find one
+  bool split_k = false;
+  if (THPVariable_Check(args[10])) workspace = tensor(10);
+  else split_k = truth(10);
   torch::Tensor output;
   {
     const bool flat = input.dim() == 2 && input.size(1) == in_features && input.is_contiguous();
@@ -336,8 +366,8 @@ PyObject* linear_fastcall(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 PyMethodDef g_methods[] = {
-    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear_fastcall)), METH_FASTCALL,
-     "BlkQ4Linear.forward: any leading dimensions, the output allocated unless given"},
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear_fastcall)), METH_FASTCALL | METH_KEYWORDS,
+     "BlkQ4Linear.forward: any leading dimensions, the output allocated unless given; workspace: a tensor, or whether to find one"},
     {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace

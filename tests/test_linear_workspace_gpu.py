@@ -70,3 +70,12 @@ assert torch.equal(got.view(torch.int16), ext.forward(64, True, 1024, 1024, x, *
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_native_call_with_the_callers_workspace():
+    layer = L.BlkQ4Linear(64, True, False, (torch.randn(1024, 1024, device="cuda") * 0.02).half())
+    x = torch.randn(64, 1024, device="cuda").half()
+    ws = torch.zeros(layer.workspace_bytes(64), dtype=torch.uint8, device="cuda")
+    got = L._linear(block_size=64, col_wise=True, in_features=1024, out_features=1024, input=x, q_weights=layer.q_weights,
+                    q_scales=layer.q_scales, q_zp=layer.q_zp, bias=None, flags=0, workspace=ws, out=None)
+    assert torch.equal(got.view(torch.int16), layer(x).view(torch.int16))
