@@ -87,13 +87,14 @@ MAX_GROUP = 4  # layers of one launch
 
 def can_share_launch(layers, rows) -> bool:
     """Whether one launch can compute all ``layers`` (two to four) from the same ``rows`` activation rows: layers of one
-    shape of blocks, with nothing hooked into their calls."""
+    shape of blocks, with nothing of the user's in their calls (hooks, another ``forward`` or ``__call__``, ``compile``)."""
     first = layers[0]
     for l in layers:
         if not isinstance(l, BlkQ4Linear):
             return False
         q = l.q_weights
         if (type(l).forward is not BlkQ4Linear.forward or "forward" in l.__dict__
+                or type(l).__call__ is not nn.Module.__call__ or getattr(l, "_compiled_call_impl", None) is not None
                 or l._forward_hooks or l._forward_pre_hooks or nn.modules.module._has_any_global_hook()
                 or (l.block_size, l.col_wise, l.in_features) != (first.block_size, first.col_wise, first.in_features)
                 or (l.q_zp.numel() > 0) != (first.q_zp.numel() > 0) or q.device != first.q_weights.device

@@ -1,7 +1,9 @@
 """Which groups of weight matrices one launch takes (host only)."""
 import pytest
+import torch
 
 from gemmlib_b200 import capi
+from gemmlib_b200.ms_blkq4linear import BlkQ4Linear, can_share_launch
 
 
 def test_supported_groups():
@@ -36,3 +38,29 @@ def test_workspace_of_a_group():
     for m, k, widths in ((64, 8192, (14336, 14336)), (512, 4096, (4096, 4096, 4096)), (512, 4096, (11008, 11008)), (64, 4096, (1024, 1024))):
         assert capi.gemm_group_workspace_size(64, True, m, k, widths) == capi.gemm_workspace_size(m, sum(widths), k) > 0
     assert capi.gemm_group_workspace_size(64, True, 8, 4096, (4096, 4096)) == 0
+
+
+def test_layers_with_calls_of_their_own_stay_apart():
+    def layer(cls=BlkQ4Linear):
+        n, k = 64, 2048
+        return cls.from_packed(64, True, k, n, torch.zeros(n * k // 2, dtype=torch.uint8), torch.zeros(n * k // 64, dtype=torch.float16))
+
+    class OwnCall(BlkQ4Linear):
+        def __call__(self, *args, **kwargs):
+            return super().__call__(*args, **kwargs)
+
+    class OwnForward(BlkQ4Linear):
+        def forward(self, input, out=None):
+            return super().forward(input, out)
+
+    class Plain(BlkQ4Linear):
+        pass
+
+    compiled, hooked, patched = layer(), layer(), layer()
+    compiled.compile(backend="eager")
+    hooked.register_forward_pre_hook(lambda *_: None)
+    patched.forward = lambda x, out=None: x
+    for other in (layer(), layer(Plain)):
+        assert can_share_launch([layer(), other], 1)
+    for other in (layer(OwnCall), layer(OwnForward), compiled, hooked, patched):
+        assert not can_share_launch([layer(), other], 1) and not can_share_launch([other, layer()], 1)
