@@ -201,7 +201,7 @@ static bool group_supported(int block_size, bool column_wise_blocking, int m, in
     total += n[i];
   }
   if (total > (1 << 30)) return false;
-  if (m <= 16) return m <= 8 && blkq4::gemv_stream_takes(block_size, column_wise_blocking, m, (int)total, k);
+  if (m <= 16) return m <= 8 && !blkq4::gemv_stream_off() && blkq4::gemv_stream_takes(block_size, column_wise_blocking, m, (int)total, k);
   const blkq4::Blocking b(block_size, column_wise_blocking);
   if (k % 64 != 0 || k % b.bk != 0) return false;
   for (int i = 0; i < count; ++i)

@@ -41,6 +41,8 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
 
 // Whether it takes the problem (with 16-byte aligned scales and zero points), alone or as a group of N columns in all.
 bool gemv_stream_takes(int block, bool colwise, int M, int N, int K);
+// True when the environment (BLKQ4_GEMV_NO_STREAM, BLKQ4_GEMV_GENERIC) keeps calls of up to 16 rows off it.
+bool gemv_stream_off();
 
 // The same weight stream for 9 <= M <= 16 (two row groups, two tiles per pass, activations from L2).
 std::string launch_gemv_wide(int block, bool colwise, int M, int N, int K, cudaStream_t stream,

@@ -784,6 +784,16 @@ int read_gemv_error() {
   return v;
 }
 
+// Both are read once: a group of layers has to take the same kernel as its layers' own calls.
+static int generic_only() {
+  static const int v = env_int("BLKQ4_GEMV_GENERIC");
+  return v;
+}
+bool gemv_stream_off() {
+  static const int v = env_int("BLKQ4_GEMV_NO_STREAM");
+  return v != 0 || generic_only() != 0;
+}
+
 std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
                         const __half* a, const uint8_t* packed, const __half* scales,
                         const uint8_t* zp, __half* out, const __half* bias, unsigned flags) {
@@ -797,16 +807,15 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
   if (env_warps >= 1 && env_warps <= kMaxWarps) warps = env_warps;
   const int u = env_u ? env_u : 4;
   cudaError_t e;
-  static const int env_generic = env_int("BLKQ4_GEMV_GENERIC"), env_no_stream = env_int("BLKQ4_GEMV_NO_STREAM");
   // Decode shapes first: the cp.async stream kernel (blkq4_gemv_stream.cu).
-  if (!env_generic && !env_no_stream) {
+  if (!gemv_stream_off()) {
     const std::string r = M <= 8 ? launch_gemv_stream(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags)
                                  : launch_gemv_wide(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
     if (r != kStreamUnsupported) return r;
   }
   // Fast path: one scale per 64-k step; at least one 512-k unit (the last one may be partial), meta
   // rows and pointers 16-byte aligned (TMA), shared memory for the per-step terms within reach.
-  if (colwise && block >= 64 && !env_generic && K >= kUnitKBytes && K <= 32768 &&
+  if (colwise && block >= 64 && !generic_only() && K >= kUnitKBytes && K <= 32768 &&
       reinterpret_cast<uintptr_t>(scales) % 16 == 0 && (!zp || reinterpret_cast<uintptr_t>(zp) % 16 == 0)) {
     const std::string r =
         (M <= 8) ? (zp ? launch_persistent_T<1, true>(M, N, K, block, stream, a, packed, scales, zp, out, bias, early)

@@ -1,4 +1,8 @@
 """Which groups of weight matrices one launch takes (host only)."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -64,3 +68,15 @@ def test_layers_with_calls_of_their_own_stay_apart():
         assert can_share_launch([layer(), other], 1)
     for other in (layer(OwnCall), layer(OwnForward), compiled, hooked, patched):
         assert not can_share_launch([layer(), other], 1) and not can_share_launch([other, layer()], 1)
+
+
+@pytest.mark.parametrize("switch", ["BLKQ4_GEMV_NO_STREAM", "BLKQ4_GEMV_GENERIC"])
+def test_no_decode_groups_where_the_decode_kernel_is_off(switch):
+    """Its layers' own calls take another kernel there, with other bits."""
+    code = ("from gemmlib_b200 import capi; w = (4096, 4096)\n"
+            "print(*[int(capi.gemm_group_supported(64, True, m, 4096, w)) for m in (1, 8, 17, 512)])")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for value, want in (("0", "1 1 1 1"), ("1", "0 0 1 1")):
+        r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300,
+                           env={**os.environ, switch: value})
+        assert r.returncode == 0 and r.stdout.split("\n")[0] == want, (r.stdout, r.stderr[-1000:])
