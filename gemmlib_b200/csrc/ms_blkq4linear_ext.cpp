@@ -394,6 +394,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           return blkq4_gemm_group_supported_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()) != 0;
         },
         "Whether one launch takes layers of these widths");
+  m.def("gemm_plan",
+        [](int m_, int n_, int k_) {
+          int plan[6];
+          blkq4_gemm_plan(m_, n_, k_, 0, plan);
+          return py::make_tuple(plan[0], plan[2]);
+        },
+        "Kernel and output tiles of a call without a workspace (blkq4_gemm_plan)");
   m.def("linear_group_workspace_size",
         [](int block, bool col_wise, int m_, int k_, const std::vector<int>& n_) {
           return int64_t(blkq4_gemm_group_workspace_size_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()));

@@ -32,6 +32,7 @@ _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
 _linear = ms_blkq4linear_ext.linear
 _linear_group = ms_blkq4linear_ext.linear_group
 _group_supported = ms_blkq4linear_ext.linear_group_supported
+_gemm_plan = ms_blkq4linear_ext.gemm_plan
 _graph_workspace = ms_blkq4linear_ext.graph_workspace
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
 
@@ -83,6 +84,7 @@ def split_k_workspace(device, nbytes: int):
 ms_blkq4linear_ext.workspace_source(_WORKSPACES, lambda index, nbytes: split_k_workspace(torch.device("cuda", index), nbytes))
 
 MAX_GROUP = 4  # layers of one launch
+_PAIR_KERNEL = 2  # of blkq4_gemm_plan
 
 
 def can_share_launch(layers, rows) -> bool:
@@ -111,10 +113,35 @@ def one_launch_keeps_bits(layers, rows) -> bool:
     return rows <= 16 or all(l.workspace_bytes(rows) == 0 for l in layers)
 
 
+def one_launch_is_faster(layers, rows) -> bool:
+    """Whether layers that run without a split of K are at least as fast in one launch.  They are, by up to half, but where
+    layers that fill the one-CTA kernel alone become tiles of the CTA-pair kernel of fewer than 256 rows: that kernel's
+    step does not get shorter with its rows as the other's does.  Only fewer rounds make up for it.  Measured on B200, blocks
+    of 64 with zero points, separate / together, us: two layers of 5632 columns (two rounds either way), K = 4096: M = 300
+    40.9 / 44.6, M = 400 42.4 / 45.8, M = 512 49.8 / 48.4; K = 11008, M = 333 93.9 / 105.0; K = 2048, M = 333 27.2 / 27.7; K = 1024,
+    M = 333 19.2 / 19.2; four of them (four rounds / three), K = 3072, M = 300 62.2 / 50.3; three of 9472 (pairs alone too),
+    K = 4096, M = 300 74.4 / 64.2."""
+    first = layers[0]
+    k = first.in_features
+    if not 256 < rows < 512 or k <= 1024:
+        return True
+    alone = [_gemm_plan(rows, l.out_features, k) for l in layers]
+    kernel, tiles = _gemm_plan(rows, sum(-(-l.out_features // 256) * 256 for l in layers), k)  # whole pairs of tiles, as in a group
+    if kernel != _PAIR_KERNEL or any(kern == _PAIR_KERNEL for kern, _ in alone):
+        return True
+    sms = torch.cuda.get_device_properties(first.q_weights.device).multi_processor_count
+    return -(-tiles // (sms // 2)) < sum(-(-t // sms) for _, t in alone)
+
+
+def shares_launch(layers, rows) -> bool:
+    """Whether ``run_group`` takes one launch."""
+    return one_launch_keeps_bits(layers, rows) and one_launch_is_faster(layers, rows)
+
+
 def run_group(layers, input, outputs):
     """``outputs[i] = layers[i](input)``, bit for bit, for layers that ``can_share_launch``: in one launch where that keeps
-    the bits, else in one per layer."""
-    if not one_launch_keeps_bits(layers, input.size(0)):
+    the bits and is not slower, else in one per layer."""
+    if not shares_launch(layers, input.size(0)):
         for l, out in zip(layers, outputs):
             l(input, out=out)
         return

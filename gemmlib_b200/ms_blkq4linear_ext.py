@@ -36,6 +36,7 @@ gemm_workspace_size_blocked = _mod.gemm_workspace_size_blocked
 linear = _mod.linear
 workspace_source = _mod.workspace_source
 workspace_owners = _mod.workspace_owners
+gemm_plan = _mod.gemm_plan
 linear_group = _mod.linear_group
 linear_group_supported = _mod.linear_group_supported
 linear_group_workspace_size = _mod.linear_group_workspace_size

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from gemmlib_b200 import capi
-from gemmlib_b200.ms_blkq4linear import BlkQ4Linear, one_launch_keeps_bits
+from gemmlib_b200.ms_blkq4linear import BlkQ4Linear, shares_launch
 from gemmlib_b200.stack import LinearStack, llama_like_stack
 
 pytestmark = pytest.mark.gpu
@@ -102,16 +102,18 @@ def test_stack_equals_its_layers(M):
         assert torch.equal(got[dst].view(torch.int16), want.view(torch.int16)), dst
 
 
-# (hidden, ffn, rows, launches of a block): layers alone split K; balanced ranges; neither, so q, k, v and gate, up go together
+# (hidden, ffn, rows, launches of a block): layers alone split K; balanced ranges; neither, so q, k, v and gate, up go together, but
+# not gate and up where short tiles would change to the pair kernel without saving a round
 @pytest.mark.parametrize("hidden,ffn,M,launches", [(2048, 2304, 40, 7), (2048, 2304, 300, 7), (1024, 19200, 300, 7),
-                                                   (512, 768, 17, 4), (512, 768, 333, 4)])
+                                                   (512, 768, 17, 4), (512, 768, 333, 4), (2048, 5632, 333, 7),
+                                                   (2048, 5632, 512, 6), (2048, 9472, 300, 6), (1024, 5632, 333, 6)])
 def test_prefill_stack_keeps_every_bit(hidden, ffn, M, launches):
     stack = llama_like_stack(hidden, ffn, 1, 64, True, False, torch.device("cuda"))
     x = torch.randn(M, hidden, device="cuda").half()
     stack.forward(x, "h0")
     got = stack.buffers(M)
     runs = [[stack.steps[i][0] for i in r] for r in stack._groups(M)]
-    assert sum(1 if one_launch_keeps_bits(r, M) else len(r) for r in runs) == launches
+    assert sum(1 if shares_launch(r, M) else len(r) for r in runs) == launches
     for lyr, src, dst in stack.steps:
         assert torch.equal(got[dst].view(torch.int16), lyr(got[src]).view(torch.int16)), dst
 
