@@ -56,7 +56,10 @@ def test_misaligned_scales_of_a_group_are_refused():
 PREFILL = [(17, 512, 32, True, True, (96, 32, 2080)), (64, 1024, 64, True, False, (1024, 1024, 1024)),
            (100, 4096, 128, True, True, (11008, 11008)), (200, 960, 32, False, True, (2080, 4128)),
            (333, 2048, 16, True, False, (7200, 544)), (300, 1024, 64, False, True, (9536, 192, 2048, 64)),
-           (512, 1024, 64, True, True, (4096, 4096, 4096))]
+           (512, 1024, 64, True, True, (4096, 4096, 4096)),
+           # up to 64 rows and 16 steps a CTA or more (four dequantizer groups): whole rounds, balanced ranges, row-wise blocks
+           (64, 4096, 64, True, True, (4096, 4096, 4096)), (33, 4096, 32, True, False, (11008, 11008)),
+           (48, 2048, 32, False, True, (2080, 4128))]
 
 
 @pytest.mark.parametrize("M,K,block,colwise,zp,widths", PREFILL)

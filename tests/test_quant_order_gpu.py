@@ -65,6 +65,87 @@ def weight(N, K, seed):
     return (torch.randn(N, K, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * 0.02).half()
 
 
+def packed(K, N, block):
+    meta = K * N // block
+    return (torch.empty(K * N // 2, dtype=torch.uint8, device="cuda"), torch.empty(meta, dtype=torch.float16, device="cuda"),
+            torch.empty(meta, dtype=torch.uint8, device="cuda"))
+
+
+def same(a, b):
+    return torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
+def long_gemm(M, N, K):
+    """Activations, and a function that multiplies them into a tensor: a kernel of about 100 us that lets its successor start at once."""
+    layer = BlkQ4Linear(64, True, False, weight(N, K, 11))
+    a = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(12), device="cuda").half()
+    stream = torch.cuda.current_stream().cuda_stream
+    return a, lambda out: capi.gemm(64, True, M, N, K, a, layer.q_weights, layer.q_scales, layer.q_zp, out, stream=stream)
+
+
+@pytest.mark.parametrize("col_wise", [True, False])
+def test_quantizer_waits_for_the_kernel_that_writes_its_weights(col_wise):
+    """The weights are the result of a GEMM, which lets the quantizer start before it has written anything."""
+    M, N, K = 2048, 4096, 8192
+    _, gemm = long_gemm(M, N, K)
+    out, want = torch.empty(M, N, dtype=torch.float16, device="cuda"), packed(N, M, 64)
+    gemm(out)
+    torch.cuda.synchronize()
+    capi.quant(64, col_wise, N, M, N, out, *want)
+    for _ in range(5):
+        got = packed(N, M, 64)
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        torch.cuda._sleep(400_000)  # both launches are queued before the first starts
+        gemm(out)
+        capi.quant(64, col_wise, N, M, N, out, *got)
+        torch.cuda.synchronize()
+        assert all(same(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("col_wise", [True, False])
+def test_quantizer_waits_for_the_kernel_that_reads_what_it_overwrites(col_wise):
+    """The scales of the quantizer take the place of the activations of the GEMM before it."""
+    M, N, K = 256, 28672, 8192
+    n, k, block = 8192, 4096, 16  # as many scales as activations
+    a, gemm = long_gemm(M, N, K)
+    w, keep = weight(n, k, 13), a.clone()
+    out, want = torch.empty(M, N, dtype=torch.float16, device="cuda"), torch.empty(M, N, dtype=torch.float16, device="cuda")
+    gemm(want)
+    q = packed(k, n, block)
+    assert q[1].numel() == a.numel()
+    for _ in range(5):
+        a.copy_(keep)
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        torch.cuda._sleep(400_000)
+        gemm(out)
+        capi.quant(block, col_wise, k, n, k, w, q[0], a.view(-1), q[2])
+        torch.cuda.synchronize()
+        assert same(out, want) and not same(a, keep)
+
+
+def test_captured_copy_quantizer_and_gemm():
+    """Replays of one graph that copies new weights in, quantizes them and multiplies with the early weight fetch."""
+    N, K, M = 2048, 2048, 4
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(7), device="cuda").half()
+    src, w = weight(N, K, 0), torch.empty(N, K, dtype=torch.float16, device="cuda")
+    layer = BlkQ4Linear(64, True, False, src)
+    layer(x)
+    graph, stream, out = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.empty(M, N, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        w.copy_(src)
+        capi.quant(64, True, K, N, K, w, layer.q_weights, layer.q_scales, layer.q_zp, stream=stream.cuda_stream)
+        layer(x, out=out)
+    for seed in range(1, 5):
+        new = weight(N, K, seed)
+        src.copy_(new)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert same(out, BlkQ4Linear(64, True, False, new)(x))
+
+
 @pytest.mark.parametrize("col_wise,N,K", [(True, 2048, 2048), (False, 1024, 2048), (True, 512, 4096)])
 @pytest.mark.parametrize("M", [1, 12, 40])
 def test_early_weight_fetch_behind_the_quantizer(M, col_wise, N, K):
