@@ -17,15 +17,16 @@
 // cluster of CTAs: M < 256, the larger skinny problems of gemm_tc_takes_skinny among them, and larger M with few
 // tiles.  gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
 //
-// Persistent CTAs (one per SM) walk the tile list.  Warp roles:
-//   warps 0-3   epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
-//               through a second TMEM accumulator buffer where two fit
-//   warps 4-15  dequantizers, three groups of four warps on steps in turn: thread = one
-//               weight column n of the tile (TMEM lane n), 64 k = 32 TMEM columns
-//   warp 16     TMA producer of the activation tiles (128-byte swizzle)
-//   warp 17     TMA producer of the packed int4 weight tiles
-//   warp 18     TMA producer of their scales and zero points
-//   warp 19     MMA issuer (one elected thread); owns the TMEM allocation
+// Persistent CTAs (one per SM) walk the tile list.  Warp roles of the one-CTA kernel, in the order of the warps (struct Shape:
+// NG dequantizer groups, three or four):
+//   0 to 3              epilogue: tcgen05.ld -> fp16 -> global, overlapped with the next tile
+//                       through a second TMEM accumulator buffer where two fit
+//   kFirstDeqWarp (4)   dequantizers, NG groups of four warps on steps in turn: thread = one
+//                       weight column n of the tile (TMEM lane n), 64 k = 32 TMEM columns
+//   kActProducerWarp    TMA producer of the activation tiles (128-byte swizzle); 4 + 4 NG
+//   kWeightProducerWarp TMA producer of the packed int4 weight tiles
+//   kMetaProducerWarp   TMA producer of their scales and zero points
+//   kMmaWarp            MMA issuer (one elected thread), the last warp; owns the TMEM allocation
 // A step is 64 k, or 128 k for tiles of up to 128 rows (struct Shape).
 // Stages are handed over with mbarriers; every such wait, and every wait for another CTA's flag word, is bounded
 // and, on expiry, sets an error word and drains the CTA instead of hanging the GPU.  The cluster barriers of
@@ -87,9 +88,9 @@ struct Shape {
 // Above 128 rows two 64-k steps of activations per stage leave three stages only (rowwise M = 333: 24.8 vs 27.4 us).
 // Four groups where a CTA has many steps: up to 64 rows the dequantizers' instructions set the pace, and the scheduler has more
 // to choose from; the fourth group's start-up and its share of the ring only pay off after some 16 steps.  Three / four, us, block
-// 64 column-wise with zero points: K = 8192, N = 28672 (97 steps a CTA): M = 17 40.8 / 38.7, M = 64 50.9 / 48.6; 11008 x 4096
-// (22) M = 40 13.2 / 12.8; 4096 x 11008 (32) M = 64 14.1 / 13.4; 2048 x 22528 (19) M = 64 12.9 / 12.7; 1024 x 14336 (8) 6.2 / 6.3;
-// 4096 x 4096 (8) 8.8 / 8.9.
+// 64 column-wise with zero points: K = 8192, N = 28672 (97 steps a CTA): M = 17 43.0 / 41.6, M = 64 46.7 / 45.7 (block 128,
+// symmetric 45.7 / 45.1); 11008 x 4096 (22) M = 40 13.6 / 13.3; 4096 x 11008 (32) M = 64 14.4 / 14.0; 2048 x 22528 (19) M = 64
+// 13.5 / 13.2; 1024 x 14336 (8) 6.4 / 6.4; 4096 x 4096 (8) 8.9 / 9.0.
 using ShapeSmall = Shape<64, 2, 6, 10, 3>;  // two accumulators + six stages of 64 TMEM columns = 512
 using ShapeSmallLong = Shape<64, 2, 6, 10, 4>;
 constexpr int kLongSteps = 16;
@@ -97,7 +98,7 @@ using ShapeMid = Shape<128, 2, 4, 8, 3>;    // two accumulators + four stages = 
 using ShapeLarge = Shape<256, 1, 6, 6, 3>;
 // Activation rows of a tile, a multiple of `unit`: as few tiles of up to 256 rows as there can be, all of one height.
 // Measured on B200 against tiles of 256 and a remainder, whose MMAs multiply rows that are not there, us: M = 300, 4096 x 28672
-// 88.1 / 73.3; M = 333, 1024 x 28672 34.0 / 31.9; M = 400, 8192 x 22528 135.3 / 125.6.
+// 85.3 / 75.1; M = 333, 1024 x 28672 36.4 / 32.3; M = 400, 8192 x 22528 137.2 / 128.5.
 inline int tile_rows(int M, int unit) {
   const int tiles = (M + 255) / 256, rows = (M + tiles - 1) / tiles;
   return (rows + unit - 1) / unit * unit;
@@ -611,8 +612,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     //      so that the lanes of a warp are contiguous on both sides; each part starts with its own rows, so that the parts
     //      of a cluster write to different CTAs at a time; the loops are rolled, because they run a few times per launch from
     //      a cold instruction cache.  Measured on B200 against 4-byte stores from an unrolled loop with a branch per row, us:
-    //      M = 16, 4096 x 4096, four parts 8.8 / 7.8; M = 48, 2048 x 1024 6.0 / 4.9; M = 256, 4096 x 4096, four parts 15.6 / 14.8
-    //      (16.3 where all parts start with row 0); M = 512, two parts 21.4 / 18.6; M = 300, 8192 x 1024, five parts 16.5 / 12.5.
+    //      M = 16, 4096 x 4096, four parts 8.8 / 7.9; M = 48, 2048 x 1024 6.0 / 4.9; M = 256, 4096 x 4096, four parts 15.7 / 14.9
+    //      (16.3 where all parts start with row 0); M = 512, two parts 21.3 / 19.2; M = 300, 8192 x 1024, five parts (and tiles
+    //      of one height) 16.9 / 12.8.
     //      With the partial tiles in global memory and one finishing CTA, which read them chunk by
     //      chunk from L2 (one round trip per 32 rows and part), more parts cost more than they gave: K = 4096, N = 1024,
     //      M = 128: four parts through memory 15.4 us, eight 21.7.

@@ -19,7 +19,8 @@
 //                 barrier.
 //   MMA_DONE[s]   tcgen05.commit with a two-CTA multicast: the copy in each CTA frees that CTA's
 //                 activation stage and dequantized stage.
-//   ACC_FULL      same multicast commit, to both epilogues; ACC_EMPTY count 8, arrivals as on STEP_FULL.
+//   ACC_FULL      same multicast commit, to both epilogues; ACC_EMPTY count 2 * kPairEpiWarps, the epilogue warps of both
+//                 CTAs (the peer's remotely, as on STEP_FULL).
 //   FULL / PACK_FREE (weight ring) stay local to each CTA.
 // The loads here carry no cluster multicast: every CTA copies its own rows.  All waits are bounded;
 // the two CTAs meet at a cluster barrier before either frees its tensor memory or exits.
@@ -318,8 +319,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     // memory, accumulator released, and only then staging -> global memory (64-byte row pieces, 8 bytes
     // per lane), which overlaps the next tile.  No other warp touches the rows of a chunk: only __syncwarp.
     // Measured on B200, one warp per quarter and a select, conversion and shuffle per value / two warps and trade_rows, us:
-    // M = 4096, 1024 x 4096 35.9 / 30.7; M = 3000, row-wise 512 x 8192 35.3 / 30.0; M = 300, 4096 x 28672 83.2 / 72.5; M = 4096, 8192 x
-    // 28672 1557 / 1487; M = 2048, 4096 x 4096, one hand-over under way 52.7 / 52.3.
+    // M = 4096, 1024 x 4096 34.0 / 32.2; M = 3000, row-wise 512 x 8192 35.2 / 32.0; M = 333, 1024 x 28672 32.3 / 28.8; M = 300, 4096 x
+    // 28672 74.8 / 73.0; M = 2048, 4096 x 4096, one hand-over under way 52.3 / 51.5; M = 4096, 8192 x 28672 1337 / 1329 (a cool GPU;
+    // at the power cap, 1550 to 1590, no difference).
     const int quarter = warp & 3, epi = warp - 2, chunk0 = 32 * (epi >> 2);
     uint32_t tcount = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the output belongs to stream order

@@ -83,8 +83,8 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 // GROUP: several weight matrices of one K read the same activations (the q, k and v projections of a decoder block, or its
 // gate and up projections): the tiles of all of them are one sequence, so one launch takes the place of two to four, with
 // one ramp, one wait for the preceding launch and one staging of the activations, and its tiles fill the SMs more evenly.
-// Measured on B200, graph of two decoder blocks (hidden 4096, 11008; block 64, zero points; 14 layers, 8 launches), M = 1: 106.1 us in
-// one launch per layer, 81.0 in groups.
+// Measured on B200, graph of two decoder blocks (hidden 4096, 11008; block 64, zero points; 14 layers, 8 launches), M = 1: 102.5 us in
+// one launch per layer, 76.5 in groups; M = 4 134.0 / 95.1.
 //
 // BS: steps of a quantization block, as a shift (0: blocks of 64, 1: of 128).  The two steps of a 128-k block share scale and
 // zero point: one load and conversion of them, two accumulators with independent mma chains, one scaling of their sum.

@@ -23,7 +23,9 @@
 // A CTA is short: it loads, waits, computes and leaves, so small ones keep the SM's slots turning over more evenly.  CTAs of
 // 128 threads, ten of them on an SM (48 registers), against 256, us: column-wise 4096 x 11008 22.0 / 21.5, 8192 x 28672
 // block 128 101.7 / 94.8; row-wise 11008 x 4096 block 32 28.1 / 25.0, 4096 x 11008 block 64 29.0 / 24.8.  Twelve on an SM
-// (40 registers, spills) 21.5, 101.9, 26.7, 25.8.
+// (40 registers, spills) 21.5, 101.9, 26.7, 25.8.  Of the kernels with 48 registers only column-wise block 16 spills, 4 bytes
+// (8 with unaligned rows); 256 threads and 42 registers against that: 4096 x 11008 22.7 / 22.2, symmetric 20.9 / 20.4, 8192 x 28672
+// 106.8 / 105.7.
 #include "blkq4_common.cuh"
 
 namespace blkq4 {

@@ -285,8 +285,8 @@ c10::optional<torch::Tensor> split_k_workspace(int device, int64_t nbytes) {
 // The whole of BlkQ4Linear.forward but a bias that cannot be fused: leading dimensions flattened, the split-K workspace
 // found, the output allocated unless the caller brought one, the launch, the leading dimensions restored.  In one call
 // because at decode sizes the Python calls around the launch took longer than the kernel, and with CPython's vectorcall
-// signature because pybind11 took about 1 us to convert the arguments.  Measured, host time per call: one token 7.1 -> 6.4 us,
-// with a split-K workspace (M = 333) 13.4 -> 9.0.
+// signature because pybind11 took about 1 us to convert the arguments.  Measured, host time per call: one token 6.7 -> 6.1 us,
+// with a split-K workspace (M = 333) 12.7 -> 7.8.
 constexpr int kLinearArgs = 12;
 constexpr const char* kLinearNames[kLinearArgs] = {"block_size", "col_wise", "in_features", "out_features", "input", "q_weights",
                                                    "q_scales", "q_zp", "bias", "flags", "workspace", "out"};
