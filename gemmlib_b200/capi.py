@@ -40,6 +40,7 @@ SYMBOLS = (
     "blkq4_fp16_gemm_group_sm100",
     "blkq4_gemm_group_supported_sm100",
     "blkq4_gemm_group_workspace_size_sm100",
+    "blkq4_gemm_group_keeps_bits_sm100",
     "blkq4_gemm_plan",
     "blkq4_gemm_plan_range_bound",
     "blkq4_reset",
@@ -81,6 +82,8 @@ def _load() -> ctypes.CDLL:
     lib.blkq4_fp16_gemm_group_sm100.restype = i
     lib.blkq4_gemm_group_supported_sm100.argtypes = [i, b, i, i, i, ctypes.POINTER(i)]
     lib.blkq4_gemm_group_supported_sm100.restype = i
+    lib.blkq4_gemm_group_keeps_bits_sm100.argtypes = [i, b, i, i, i, ctypes.POINTER(i)]
+    lib.blkq4_gemm_group_keeps_bits_sm100.restype = i
     lib.blkq4_gemm_group_workspace_size_sm100.argtypes = [i, b, i, i, i, ctypes.POINTER(i)]
     lib.blkq4_gemm_group_workspace_size_sm100.restype = sz
     lib.blkq4_gemm_workspace_size.argtypes = [i, i, i]
@@ -212,6 +215,11 @@ def gemm_group_supported(block_size: int, col_wise: bool, m: int, k: int, n) -> 
 def gemm_group_workspace_size(block_size: int, col_wise: bool, m: int, k: int, n) -> int:
     """Bytes of zeroed workspace with which ``gemm_group`` would split K over the tiles of all matrices (0: it would not)."""
     return int(lib.blkq4_gemm_group_workspace_size_sm100(block_size, col_wise, m, k, len(n), (ctypes.c_int * len(n))(*n)))
+
+
+def gemm_group_keeps_bits(block_size: int, col_wise: bool, m: int, k: int, n) -> bool:
+    """Whether ``gemm_group`` with the workspace it asks for gives every bit of the parts' own calls with theirs."""
+    return bool(lib.blkq4_gemm_group_keeps_bits_sm100(block_size, col_wise, m, k, len(n), (ctypes.c_int * len(n))(*n)))
 
 
 def gemm_group(block_size, col_wise, m, k, act, parts, flags=0, stream=0, workspace=None):

@@ -220,6 +220,12 @@ extern "C" size_t blkq4_gemm_group_workspace_size_sm100(int block_size, bool col
   return blkq4::gemm_tc_group_workspace_bytes(m, k, count, n);
 }
 
+extern "C" int blkq4_gemm_group_keeps_bits_sm100(int block_size, bool column_wise_blocking, int m, int k, int count,
+                                                 int const* n) {
+  if (!group_supported(block_size, column_wise_blocking, m, k, count, n)) return 0;
+  return m <= 16 || blkq4::gemm_tc_group_keeps_bits(column_wise_blocking, m, k, count, n) ? 1 : 0;
+}
+
 extern "C" int blkq4_fp16_gemm_group_sm100(int block_size, bool column_wise_blocking, int m, int k, void* stream_ptr,
                                            void const* act_ptr, size_t a_size, int count, blkq4_gemm_part const* parts,
                                            unsigned flags, void* workspace, size_t workspace_size, void* err) {

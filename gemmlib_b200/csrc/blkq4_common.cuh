@@ -114,6 +114,8 @@ std::string launch_gemm_tc(int block, bool colwise, int M, int N, int K, cudaStr
 std::string launch_gemm_tc_group(int block, bool colwise, int M, int K, cudaStream_t stream, const __half* a,
                                  const GemmGroup& grp, void* workspace, size_t workspace_bytes, unsigned flags);
 size_t gemm_tc_group_workspace_bytes(int M, int K, int count, const int* n);
+// True when that launch adds every value's fp32 sums in the order of the matrix's own launch, each with the workspace it asks for.
+bool gemm_tc_group_keeps_bits(bool colwise, int M, int K, int count, const int* n);
 // True when launch_gemm_tc takes the problem with a GatherTable (the CTA-pair kernel's fused all-gather).
 bool gemm_tc_gather_supported(int M, int N, int K);
 // Bytes of zero-initialised workspace with which launch_gemm_tc would split K for this problem

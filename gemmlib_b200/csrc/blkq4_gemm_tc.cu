@@ -849,6 +849,22 @@ void fit_split(const KernelChoice<G>& kc, int tiles, int k_steps, SplitPlan& sp)
   }
 }
 
+// Whether there is a device to ask for its clusters.
+bool have_device() {
+  int devices = 0;
+  if (cudaGetDeviceCount(&devices) != cudaSuccess) cudaGetLastError();
+  return devices > 0;
+}
+
+// The kernel of a planned launch; the plan's split as this device can run it.
+template <int G>
+KernelChoice<G> fit_plan(bool colwise, int BM, int tiles, int k_steps, int sms, SplitPlan& sp) {
+  const int cta_steps = sp.split > 1 ? sp.k_per_item : (int)((long long)tiles * k_steps / (tiles < sms ? tiles : sms));
+  const KernelChoice<G> kc = choose_kernel<G>(colwise, BM, cta_steps);
+  fit_split(kc, tiles, k_steps, sp);
+  return kc;
+}
+
 }  // namespace
 
 namespace {
@@ -1103,9 +1119,7 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
   const int num_tiles = p.m_tiles * p.n_tiles;
   p.k_steps = (K + sk - 1) / sk;
   SplitPlan sp = plan_split(M, n_tiles, K, ws_ok ? workspace_bytes : 0);
-  const int cta_steps = sp.split > 1 ? sp.k_per_item : (int)((long long)num_tiles * p.k_steps / (num_tiles < sms ? num_tiles : sms));
-  const KernelChoice<G> kc = choose_kernel<G>(colwise, p.BM, cta_steps);
-  fit_split(kc, num_tiles, p.k_steps, sp);
+  const KernelChoice<G> kc = fit_plan<G>(colwise, p.BM, num_tiles, p.k_steps, sms, sp);
   p.split = sp.split;  // split > 1: at most one item per SM
   p.k_per_item = sp.k_per_item;
   p.min_part = min_part(sk);
@@ -1168,6 +1182,37 @@ size_t gemm_tc_group_workspace_bytes(int M, int K, int count, const int* n) {
   return pp.use ? pp.total_bytes : plan_split(M, n_tiles, K, ~(size_t)0).total_bytes;
 }
 
+namespace {
+
+// K split of a launch with all the workspace that it asks for; k_per_item 0 where balanced ranges would cut its tiles.
+template <int G>
+SplitPlan launched_split(bool colwise, int M, int K, int n_tiles, int n_pairs) {
+  const PairPlan pp = plan_pair(M, n_pairs, K, ~(size_t)0);
+  if (pp.use) return SplitPlan{1, pp.balanced ? 0 : K, 0, 0, 0};
+  SplitPlan sp = plan_split(M, n_tiles, K, ~(size_t)0);
+  if (sp.balanced) return SplitPlan{1, 0, 0, 0, 0};
+  const int BM = tile_rows(M, 16), k_steps = (K + step_k(BM) - 1) / step_k(BM);
+  if (have_device()) fit_plan<G>(colwise, BM, (M + BM - 1) / BM * n_tiles, k_steps, sm_count() > 0 ? sm_count() : 148, sp);
+  return SplitPlan{sp.split, sp.split > 1 ? sp.k_per_item : K, 0, 0, 0};
+}
+
+}  // namespace
+
+bool gemm_tc_group_keeps_bits(bool colwise, int M, int K, int count, const int* n) {
+  int n_tiles = 0, n_pairs = 0;
+  for (int i = 0; i < count; ++i) {
+    n_tiles += column_tiles(n[i]);
+    n_pairs += column_pairs(n[i]);
+  }
+  const SplitPlan all = launched_split<kMaxGroup>(colwise, M, K, n_tiles, n_pairs);
+  if (all.k_per_item == 0) return false;
+  for (int i = 0; i < count; ++i) {
+    const SplitPlan one = launched_split<1>(colwise, M, K, column_tiles(n[i]), column_pairs(n[i]));
+    if (one.split != all.split || one.k_per_item != all.k_per_item) return false;
+  }
+  return true;
+}
+
 int clear_gemm_tc_error(cudaStream_t stream) {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_gemm_tc_error) != cudaSuccess) return -1;
@@ -1197,10 +1242,8 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
   blkq4::SplitPlan sp = blkq4::plan_split(m, blkq4::column_tiles(n), k, workspace_size);
   const int bm = blkq4::tile_rows(m, 16);
   out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
-  int devices = 0;
-  if (cudaGetDeviceCount(&devices) != cudaSuccess) cudaGetLastError();
   // as many clusters fit of the row-wise kernel as of the column-wise one: one CTA per SM, both
-  if (devices > 0)
+  if (blkq4::have_device())
     blkq4::fit_split(blkq4::choose_kernel<1>(true, bm), out6[2], (k + blkq4::step_k(bm) - 1) / blkq4::step_k(bm), sp);
   out6[3] = sp.split; out6[4] = sp.balanced; out6[5] = sp.balanced ? sms : 0;
   return 0;

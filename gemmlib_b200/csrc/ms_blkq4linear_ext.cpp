@@ -394,6 +394,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           return blkq4_gemm_group_supported_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()) != 0;
         },
         "Whether one launch takes layers of these widths");
+  m.def("linear_group_keeps_bits",
+        [](int block, bool col_wise, int m_, int k_, const std::vector<int>& n_) {
+          return blkq4_gemm_group_keeps_bits_sm100(block, col_wise, m_, k_, int(n_.size()), n_.data()) != 0;
+        },
+        "Whether linear_group with its workspace gives every bit of the layers' own calls with theirs");
   m.def("gemm_plan",
         [](int m_, int n_, int k_) {
           int plan[6];

@@ -32,6 +32,8 @@ _EARLY = ms_blkq4linear_ext.EARLY_WEIGHT_FETCH
 _linear = ms_blkq4linear_ext.linear
 _linear_group = ms_blkq4linear_ext.linear_group
 _group_supported = ms_blkq4linear_ext.linear_group_supported
+_group_workspace_size = ms_blkq4linear_ext.linear_group_workspace_size
+_group_keeps_bits = ms_blkq4linear_ext.linear_group_keeps_bits
 _gemm_plan = ms_blkq4linear_ext.gemm_plan
 _graph_workspace = ms_blkq4linear_ext.graph_workspace
 _workspace_size = ms_blkq4linear_ext.gemm_workspace_size_blocked
@@ -106,15 +108,22 @@ def can_share_launch(layers, rows) -> bool:
     return _group_supported(first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers])
 
 
-def one_launch_keeps_bits(layers, rows) -> bool:
-    """Whether one launch for layers that ``can_share_launch`` gives every bit of their ``forward`` calls.  Up to 16 rows it
-    does.  Above, a layer whose own call splits K adds its fp32 sums in the order of that split, which a launch over the tiles
-    of all layers would cut elsewhere, so only layers that run without a split are taken together."""
-    return rows <= 16 or all(l.workspace_bytes(rows) == 0 for l in layers)
+def group_workspace_bytes(layers, rows):
+    """Split-K workspace with which one launch for layers that ``can_share_launch`` gives every bit of their ``forward`` calls;
+    None where it would not.  Up to 16 rows, and where no layer splits K alone, it does without any.  Otherwise the layers' own
+    fp32 sums are added in the order of their splits, and a launch over the tiles of all layers has to cut K in the same
+    places."""
+    if rows <= 16 or all(l.workspace_bytes(rows) == 0 for l in layers):
+        return 0
+    first = layers[0]
+    shape = first.block_size, first.col_wise, rows, first.in_features, [l.out_features for l in layers]
+    if all(l.split_k for l in layers) and _group_keeps_bits(*shape):
+        return _group_workspace_size(*shape)
+    return None
 
 
 def one_launch_is_faster(layers, rows) -> bool:
-    """Whether layers that run without a split of K are at least as fast in one launch.  They are, by up to half, but where
+    """Whether layers that can share a launch are at least as fast in one.  They are, by up to half, but where
     layers that fill the one-CTA kernel alone become tiles of the CTA-pair kernel of fewer than 256 rows: that kernel's
     step does not get shorter with its rows as the other's does.  Only fewer rounds make up for it.  Measured on B200, blocks
     of 64 with zero points, separate / together, us: two layers of 5632 columns (two rounds either way), K = 4096: M = 300
@@ -135,7 +144,7 @@ def one_launch_is_faster(layers, rows) -> bool:
 
 def shares_launch(layers, rows) -> bool:
     """Whether ``run_group`` takes one launch."""
-    return one_launch_keeps_bits(layers, rows) and one_launch_is_faster(layers, rows)
+    return group_workspace_bytes(layers, rows) is not None and one_launch_is_faster(layers, rows)
 
 
 def run_group(layers, input, outputs):
@@ -146,10 +155,11 @@ def run_group(layers, input, outputs):
             l(input, out=out)
         return
     first = layers[0]
+    ws = split_k_workspace(input.device, group_workspace_bytes(layers, input.size(0)))
     early = all(l._settled and l.early_weight_fetch for l in layers)
     _linear_group(first.block_size, first.col_wise, first.in_features, input, [l.q_weights for l in layers],
                   [l.q_scales for l in layers], [l.q_zp for l in layers], [l.bias for l in layers], list(outputs),
-                  _EARLY if early else 0, None)
+                  _EARLY if early else 0, ws)
     for l in layers:
         l._settled = True
 

@@ -37,6 +37,7 @@ linear = _mod.linear
 workspace_source = _mod.workspace_source
 workspace_owners = _mod.workspace_owners
 gemm_plan = _mod.gemm_plan
+linear_group_keeps_bits = _mod.linear_group_keeps_bits
 linear_group = _mod.linear_group
 linear_group_supported = _mod.linear_group_supported
 linear_group_workspace_size = _mod.linear_group_workspace_size

@@ -21,7 +21,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, run_group, workspaces_owned_by
+from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, group_workspace_bytes, run_group, workspaces_owned_by
 
 
 class LinearStack:
@@ -93,6 +93,7 @@ class LinearStack:
         # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
         # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
         need = max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)), default=0)
+        need = max([need] + [group_workspace_bytes([self.steps[i][0] for i in run], M) or 0 for run in groups if len(run) > 1])
         split_k = {}
         if need > 0:
             split_k[self.device.index, self.stream.cuda_stream] = [

@@ -174,7 +174,9 @@ size_t blkq4_gemm_workspace_size_sm100(int block_size, bool column_wise_blocking
  * The rules on the sizes and pointers of each part are those of blkq4_fp16_gemm_ws_sm100, with scales and offsets 16-byte
  * aligned, and the outputs must overlap neither one another nor the activations.  Up to 16 rows, and without a workspace
  * of blkq4_gemm_group_workspace_size_sm100 bytes, the result of every part is the one its own call gives, bit for bit; with
- * it K may be split as blkq4_fp16_gemm_ws_sm100 does, over the tiles of all parts together.  Flags:
+ * it K may be split as blkq4_fp16_gemm_ws_sm100 does, over the tiles of all parts together.  That is another order of the fp32
+ * sums than that of the parts' own calls with the workspaces they ask for, except where
+ * blkq4_gemm_group_keeps_bits_sm100 answers 1.  Flags:
  * BLKQ4_GEMM_EARLY_WEIGHT_FETCH.  Shapes that blkq4_gemm_group_supported_sm100 answers 0 for are refused.  No counterpart in
  * the reference.
  */
@@ -193,6 +195,7 @@ typedef struct blkq4_gemm_part {
 } blkq4_gemm_part;
 size_t blkq4_gemm_group_workspace_size_sm100(int block_size, bool column_wise_blocking, int m, int k, int count, int const* n);
 int blkq4_gemm_group_supported_sm100(int block_size, bool column_wise_blocking, int m, int k, int count, int const* n);
+int blkq4_gemm_group_keeps_bits_sm100(int block_size, bool column_wise_blocking, int m, int k, int count, int const* n);
 int blkq4_fp16_gemm_group_sm100(
   int block_size,
   bool column_wise_blocking,

@@ -80,3 +80,21 @@ def test_no_decode_groups_where_the_decode_kernel_is_off(switch):
         r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300,
                            env={**os.environ, switch: value})
         assert r.returncode == 0 and r.stdout.split("\n")[0] == want, (r.stdout, r.stderr[-1000:])
+
+
+def test_groups_that_keep_every_bit():
+    """Those whose launch cuts K where the parts' own launches do (148 SMs without a device)."""
+    for m, k, widths, keeps in ((8, 4096, (4096, 4096), True),           # the decode kernel
+                                (512, 512, (4096, 4096, 4096), True),    # K too short to split
+                                (40, 1024, (1024, 1024, 1024), True),    # two parts, one or three matrices
+                                (40, 1024, (1024, 2816), True),          # of any widths
+                                (64, 4096, (1024, 1024), True),          # eight parts of 16 tiles too
+                                (64, 8192, (1024, 2048), True),          # eight parts each, six of 24 tiles
+                                (512, 4096, (4096, 4096, 4096), False),  # two parts of 64 tiles, ranges of 96 pair tiles
+                                (512, 4096, (11008, 11008), False),      # other ranges of 86 and of 172 pair tiles
+                                (2048, 4096, (4096, 4096), True)):       # whole rounds of pair tiles
+        plans = [capi.gemm_plan(m, n, k, 1 << 30) for n in widths + (sum(widths),)]
+        same = m <= 16 or len({p["split"] for p in plans}) == 1 and not any(p["balanced"] for p in plans)
+        assert capi.gemm_group_keeps_bits(64, True, m, k, widths) == same, (m, k, widths, plans)
+    assert not capi.gemm_group_keeps_bits(64, True, 64, 4096, (4096,))
+    assert not capi.gemm_group_keeps_bits(32, True, 1, 4096, (4096, 4096))

@@ -105,11 +105,12 @@ def test_stack_equals_its_layers(M):
         assert torch.equal(got[dst].view(torch.int16), want.view(torch.int16)), dst
 
 
-# (hidden, ffn, rows, launches of a block): layers alone split K; balanced ranges; neither, so q, k, v and gate, up go together, but
-# not gate and up where short tiles would change to the pair kernel without saving a round
-@pytest.mark.parametrize("hidden,ffn,M,launches", [(2048, 2304, 40, 7), (2048, 2304, 300, 7), (1024, 19200, 300, 7),
+# (hidden, ffn, rows, launches of a block): layers split K otherwise than a group; balanced ranges; no split, or the same one, so q, k, v
+# and gate, up go together, but not gate and up where short tiles would change to the pair kernel without saving a round
+@pytest.mark.parametrize("hidden,ffn,M,launches", [(2048, 2304, 40, 7), (2048, 2304, 300, 7), (1024, 19200, 300, 5),
                                                    (512, 768, 17, 4), (512, 768, 333, 4), (2048, 5632, 333, 7),
-                                                   (2048, 5632, 512, 6), (2048, 9472, 300, 6), (1024, 5632, 333, 6)])
+                                                   (2048, 5632, 512, 6), (2048, 9472, 300, 6), (1024, 5632, 333, 4),
+                                                   (1024, 2816, 40, 4), (1024, 2816, 128, 4), (1536, 2816, 100, 4)])
 def test_prefill_stack_keeps_every_bit(hidden, ffn, M, launches):
     stack = llama_like_stack(hidden, ffn, 1, 64, True, False, torch.device("cuda"))
     x = torch.randn(M, hidden, device="cuda").half()
