@@ -333,10 +333,12 @@ PyObject* linear_fastcall(PyObject*, PyObject* const* given, Py_ssize_t nargs, P
   c10::optional<torch::Tensor> bias, workspace;
   if (args[8] != Py_None) bias = tensor(8);
   int64_t flags = integer(9);
-  // the caller's workspace, or whether to find one
-  bool split_k = false;
-  if (THPVariable_Check(args[10])) workspace = tensor(10);
-  else split_k = truth(10);
+  // the caller's workspace, or whether to find one (a bool first: asking whether one is a tensor takes 0.1 us)
+  bool split_k = args[10] == Py_True;
+  if (!split_k && args[10] != Py_False && args[10] != Py_None) {
+    if (THPVariable_Check(args[10])) workspace = tensor(10);
+    else split_k = truth(10);
+  }
   torch::Tensor output;
   {
     const bool flat = input.dim() == 2 && input.size(1) == in_features && input.is_contiguous();
