@@ -291,23 +291,8 @@ constexpr int kLinearArgs = 12;
 constexpr const char* kLinearNames[kLinearArgs] = {"block_size", "col_wise", "in_features", "out_features", "input", "q_weights",
                                                    "q_scales", "q_zp", "bias", "flags", "workspace", "out"};
 
-PyObject* linear_fastcall(PyObject*, PyObject* const* given, Py_ssize_t nargs, PyObject* kwnames) {
+PyObject* linear_positional(PyObject* const* args) {
   HANDLE_TH_ERRORS
-  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
-  PyObject* const* args = given;
-  PyObject* named[kLinearArgs] = {};
-  if (nkw > 0 && nargs + nkw == kLinearArgs) {  // all of them, each once
-    std::copy(given, given + nargs, named);
-    for (Py_ssize_t k = 0; k < nkw; ++k) {
-      int i = 0;
-      while (i < kLinearArgs && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, k), kLinearNames[i]) != 0) ++i;
-      TORCH_CHECK_TYPE(i < kLinearArgs && !named[i], "linear: a keyword that it does not have, or an argument given twice");
-      named[i] = given[nargs + k];
-    }
-    args = named;
-  }
-  TORCH_CHECK_TYPE(nargs + nkw == kLinearArgs,
-                   "linear(block_size, col_wise, in_features, out_features, input, q_weights, q_scales, q_zp, bias, flags, workspace, out)");
   auto integer = [&](int i) {
     const long v = PyLong_AsLong(args[i]);
     if (v == -1 && PyErr_Occurred()) throw python_error();
@@ -364,6 +349,29 @@ PyObject* linear_fastcall(PyObject*, PyObject* const* given, Py_ssize_t nargs, P
     }
   }
   return THPVariable_Wrap(output);
+  END_HANDLE_TH_ERRORS
+}
+
+// The arguments by position; `named`: where those given by keyword are put.
+PyObject* const* linear_arguments(PyObject* const* given, Py_ssize_t nargs, PyObject* kwnames, PyObject** named) {
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  TORCH_CHECK_TYPE(nargs + nkw == kLinearArgs,
+                   "linear(block_size, col_wise, in_features, out_features, input, q_weights, q_scales, q_zp, bias, flags, workspace, out)");
+  std::copy(given, given + nargs, named);
+  for (Py_ssize_t k = 0; k < nkw; ++k) {
+    int i = 0;
+    while (i < kLinearArgs && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, k), kLinearNames[i]) != 0) ++i;
+    TORCH_CHECK_TYPE(i < kLinearArgs && !named[i], "linear: a keyword that it does not have, or an argument given twice");
+    named[i] = given[nargs + k];
+  }
+  return named;
+}
+
+PyObject* linear_fastcall(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  if (nargs == kLinearArgs && !kwnames) return linear_positional(args);
+  HANDLE_TH_ERRORS
+  PyObject* named[kLinearArgs] = {};
+  return linear_positional(linear_arguments(args, nargs, kwnames, named));
   END_HANDLE_TH_ERRORS
 }
 
