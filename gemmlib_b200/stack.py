@@ -60,8 +60,8 @@ class LinearStack:
         return bufs
 
     def _groups(self, M: int) -> List[range]:
-        """The steps in runs that one launch can take at this row count (``run_group`` says whether it does): up to four that follow one another, read the same
-        buffer, write others, and have no hook between them."""
+        """The steps in runs that one launch can take at this row count (``run_group`` decides whether it does): up to four
+        that follow one another, read the same buffer, write others, and have no hook between them."""
         runs: List[range] = []
         for i, (lyr, src, dst) in enumerate(self.steps):
             if runs and len(runs[-1]) < MAX_GROUP and (i - 1) not in self.between:
@@ -92,8 +92,8 @@ class LinearStack:
         groups = self._groups(M)
         # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
         # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
-        need = max((lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)), default=0)
-        need = max([need] + [group_workspace_bytes([self.steps[i][0] for i in run], M) or 0 for run in groups if len(run) > 1])
+        need = max([0] + [lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)]
+                   + [group_workspace_bytes([self.steps[i][0] for i in run], M) or 0 for run in groups if len(run) > 1])
         split_k = {}
         if need > 0:
             split_k[self.device.index, self.stream.cuda_stream] = [
