@@ -143,17 +143,12 @@ def one_launch_is_faster(layers, rows) -> bool:
 
 
 def shares_launch(layers, rows) -> bool:
-    """Whether ``run_group`` takes one launch."""
+    """Whether one launch for layers that ``can_share_launch`` keeps every bit of their calls and is not slower."""
     return group_workspace_bytes(layers, rows) is not None and one_launch_is_faster(layers, rows)
 
 
-def run_group(layers, input, outputs):
-    """``outputs[i] = layers[i](input)``, bit for bit, for layers that ``can_share_launch``: in one launch where that keeps
-    the bits and is not slower, else in one per layer."""
-    if not shares_launch(layers, input.size(0)):
-        for l, out in zip(layers, outputs):
-            l(input, out=out)
-        return
+def run_as_one(layers, input, outputs):
+    """One launch for layers that ``shares_launch``: ``outputs[i] = layers[i](input)``, bit for bit."""
     first = layers[0]
     ws = split_k_workspace(input.device, group_workspace_bytes(layers, input.size(0)))
     early = all(l._settled and l.early_weight_fetch for l in layers)

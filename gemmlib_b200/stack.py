@@ -21,7 +21,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
-from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, group_workspace_bytes, run_group, workspaces_owned_by
+from .ms_blkq4linear import MAX_GROUP, BlkQ4Linear, can_share_launch, group_workspace_bytes, run_as_one, shares_launch, workspaces_owned_by
 
 
 class LinearStack:
@@ -60,8 +60,8 @@ class LinearStack:
         return bufs
 
     def _groups(self, M: int) -> List[range]:
-        """The steps in runs that one launch can take at this row count (``run_group`` decides whether it does): up to four
-        that follow one another, read the same buffer, write others, and have no hook between them."""
+        """The steps in runs that one launch can take at this row count: up to four that follow one another, read the same
+        buffer, write others, and have no hook between them."""
         runs: List[range] = []
         for i, (lyr, src, dst) in enumerate(self.steps):
             if runs and len(runs[-1]) < MAX_GROUP and (i - 1) not in self.between:
@@ -75,11 +75,19 @@ class LinearStack:
             runs.append(range(i, i + 1))
         return runs
 
-    def _run_eager(self, bufs, groups):
-        for run in groups:
+    def _launches(self, M: int) -> List[range]:
+        """The steps of each launch: the runs that share one, every other step by itself."""
+        launches: List[range] = []
+        for run in self._groups(M):
+            together = len(run) > 1 and shares_launch([self.steps[i][0] for i in run], M)
+            launches += [run] if together else [range(i, i + 1) for i in run]
+        return launches
+
+    def _run_eager(self, bufs, launches):
+        for run in launches:
             members = [self.steps[i] for i in run]
             if len(members) > 1:
-                run_group([lyr for lyr, _, _ in members], bufs[members[0][1]], [bufs[dst] for _, _, dst in members])
+                run_as_one([lyr for lyr, _, _ in members], bufs[members[0][1]], [bufs[dst] for _, _, dst in members])
             else:
                 lyr, src, dst = members[0]
                 lyr(bufs[src], out=bufs[dst])
@@ -89,11 +97,12 @@ class LinearStack:
 
     def _capture(self, M: int):
         bufs = self._workspace(M)
-        groups = self._groups(M)
+        launches = self._launches(M)
         # The layers' split-K workspace, like the buffers, from the caller's stream: its allocator pool has the blocks of
         # stacks that are gone, a new stream's is empty.  The largest at once, so that the layers do not outgrow it.
-        need = max([0] + [lyr.workspace_bytes(M) for lyr, _, _ in self.steps if isinstance(lyr, BlkQ4Linear)]
-                   + [group_workspace_bytes([self.steps[i][0] for i in run], M) or 0 for run in groups if len(run) > 1])
+        need = max((group_workspace_bytes(layers, M) if len(layers) > 1 else layers[0].workspace_bytes(M)
+                    for layers in ([self.steps[i][0] for i in run] for run in launches)
+                    if isinstance(layers[0], BlkQ4Linear)), default=0)
         split_k = {}
         if need > 0:
             split_k[self.device.index, self.stream.cuda_stream] = [
@@ -102,13 +111,13 @@ class LinearStack:
         with workspaces_owned_by(split_k):
             with torch.cuda.stream(self.stream):
                 for _ in range(2):  # the first pass settles every layer (plain launches), the second warms up
-                    self._run_eager(bufs, groups)
+                    self._run_eager(bufs, launches)
             self.stream.synchronize()
             for buffers in split_k.values():
                 del buffers[:-1]  # outgrown in the first pass
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=self.stream):
-                self._run_eager(bufs, groups)
+                self._run_eager(bufs, launches)
         self._split_k[M] = split_k
         self._graphs[M] = (graph, bufs)
         return self._graphs[M]

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from gemmlib_b200 import capi
-from gemmlib_b200.ms_blkq4linear import BlkQ4Linear, shares_launch
+from gemmlib_b200.ms_blkq4linear import BlkQ4Linear
 from gemmlib_b200.stack import LinearStack, llama_like_stack
 
 pytestmark = pytest.mark.gpu
@@ -116,8 +116,7 @@ def test_prefill_stack_keeps_every_bit(hidden, ffn, M, launches):
     x = torch.randn(M, hidden, device="cuda").half()
     stack.forward(x, "h0")
     got = stack.buffers(M)
-    runs = [[stack.steps[i][0] for i in r] for r in stack._groups(M)]
-    assert sum(1 if shares_launch(r, M) else len(r) for r in runs) == launches
+    assert len(stack._launches(M)) == launches
     for lyr, src, dst in stack.steps:
         assert torch.equal(got[dst].view(torch.int16), lyr(got[src]).view(torch.int16)), dst
 
