@@ -15,7 +15,7 @@
 //
 // Two kernels share this design.  gemm_tc_kernel (this file) gives every tile to one CTA, or its K range to a
 // cluster of CTAs: M < 256, the larger skinny problems of gemm_tc_takes_skinny among them, and larger M with few
-// tiles.  gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
+// tiles or short K (plan_tc).  gemm_tc_pair_kernel (blkq4_gemm_tc_pair.cuh; M >= 256) gives a 256 x 256 tile to a CTA pair.
 //
 // Persistent CTAs (one per SM) walk the tile list.  Warp roles of the one-CTA kernel, in the order of the warps (struct Shape:
 // NG dequantizer groups, three or four):
@@ -41,6 +41,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "blkq4_common.cuh"
 #include "blkq4_tc.cuh"
@@ -920,6 +921,115 @@ PairPlan plan_pair(int M, int n_pairs, int K, size_t ws_bytes_available) {
   return pl;
 }
 
+// What a problem is launched as.
+//
+// plan_pair and plan_split make tiles as high as they can be (each weight is dequantized once per 256 rows) and then cut K
+// until the SMs are busy.  That is right for long K.  With fewer than 48 steps a tile is short, and what it costs besides
+// its steps - filling the pipeline, draining the accumulator by four warps, above all a cluster's or two ranges' exchange of fp32
+// partial tiles - outweighs the second conversion of the weights: more and lower tiles, each with all or more of K, are faster.
+// Below kCostK the parts of K follow short_k_parts and the height of the tiles is the one that promises the largest gain, where
+// both column-wise and row-wise blocks gain (the conversion of row-wise ones takes longer, and a plan serves all blockings).
+// Measured on B200 (block 64, zero points), tiles as high and parts as many as possible / as planned here, us (M, K x N): 256,
+// 512 x 512 6.4 / 3.5 (64 rows); 256, 1024 x 1024 9.6 / 4.4 (64); 512, 1024 x 4096 11.2 / 7.4 (128); 23, 1024 x 7328 0.71 of the
+// time in one part instead of two; 128, 1024 x 28672 14.9 / 10.6; 469, 960 x 576 9.3 / 6.1; 320, 512 x 22528 18.2 / 12.8 (tiles
+// of the one-CTA kernel instead of balanced ranges of pairs); 512, 2048 x 2048 11.9 / 8.8.  Over 394 random problems of 17 to 1100
+// rows and 512 to 3008 k the planned launch takes 0.90 of the time, 0.93 with row-wise blocks of 32 (the best candidate of each 0.85
+// and 0.90); two and five of them are slower by more than 3 %.  From 3072 to 4095 k the gain was 2.6 %, above 2 %, within
+// the prediction's error: plans stay as they are there.  Pair tiles in whole rounds are not questioned: one-CTA tiles took
+// 0.82 to 1.13 of their time.
+constexpr int kCostK = 3072, kMinPlannedRows = 48;
+
+// Parts of K of a problem that plan_split would cut in `parts`.  Up to 64 rows, where lower tiles do not help, a split in two
+// costs more than it gains below 2048 k (whole / in two: K = 832 to 1088 0.68 to 0.90, 1856 0.83, 2048 0.92, 2496 1.00), one in
+// four does not (1.0 to 1.4); above, only five or more parts say that the SMs would stay idle with low tiles too.  Fewer than eight
+// column tiles leave them idle in any case: those keep their parts.
+// Apart from that the answer does not depend on the columns, so that layers cut alike alone are mostly cut alike in a group.
+inline int short_k_parts(int M, int n_tiles, int K, int parts) {
+  if (n_tiles < 8) return parts;
+  if (M <= 64) return parts >= 3 || K >= 2048 ? parts : 1;
+  return parts >= 5 ? 4 : 1;
+}
+
+// Predicted time in us, by least squares over the candidates of the problems above (rms error 10 %): start-up, then per round of
+// tiles the 64-k steps of one and its end, then the exchange between the parts of a cluster or of balanced ranges.
+struct TileCost {
+  double start, step, step_row, end, end_row;
+};
+struct CostModel {
+  TileCost small, mid, large, pair;
+  double split, split_row, split_part, balanced;
+  double us(const TileCost& c, int BM, double rounds, int steps64) const {
+    return c.start + rounds * (steps64 * (c.step + c.step_row * BM) + c.end + c.end_row * BM);
+  }
+  double one_cta(int BM, int tiles, const SplitPlan& sp, int sms) const {
+    const TileCost& c = BM <= ShapeSmall::MAXM ? small : BM <= ShapeMid::MAXM ? mid : large;
+    const double rounds = sp.balanced ? (double)tiles / sms : (double)((tiles * sp.split + sms - 1) / sms);
+    return us(c, BM, rounds, sp.k_per_item * (step_k(BM) / BLOCK_K)) +
+           (sp.balanced ? balanced : sp.split > 1 ? split + split_row * BM + split_part * sp.split : 0.0);
+  }
+  double balanced_pairs(int BM, int items, int pairs, int steps64) const {
+    return us(pair, BM, items / (double)pairs, steps64) + balanced;
+  }
+};
+constexpr CostModel kColumnWise{{1.5869, 0.165, 0, 0.6429, 0}, {2.272, 0.1311, 0.0004, 0, 0.0083}, {1.4118, 0.1161, 0.0009, 0, 0.0098}, {5.4188, 0.1224, 0.0009, 0, 0.003}, 1.13, 0.0071, 0.21, 6.6},
+    kRowWise{{0.8339, 0.2595, 0, 0.5351, 0}, {1.6446, 0.219, 0.0004, 0, 0.0074}, {1.2523, 0.2433, 0.0005, 0, 0.0096}, {5.7228, 0.2428, 0.0007, 0, 0.0019}, 1.42, 0.0048, 0.29, 6.3};
+
+struct TcPlan {
+  bool pair;
+  PairPlan pp;   // pair
+  int BM;        // rows of a tile, either kernel
+  int m_tiles;
+  SplitPlan sp;  // !pair
+};
+
+// plan_pair and plan_split as they are.
+TcPlan plan_high_tiles(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available) {
+  TcPlan pl{};
+  pl.pp = plan_pair(M, n_pairs, K, ws_bytes_available);
+  pl.pair = pl.pp.use;
+  pl.BM = pl.pair ? pl.pp.BM : tile_rows(M, 16);
+  pl.m_tiles = (M + pl.BM - 1) / pl.BM;
+  if (!pl.pair) pl.sp = plan_split(M, n_tiles, K, ws_bytes_available);
+  return pl;
+}
+
+// gather: the fused exchange, which lives in the pair kernel's epilogue and runs in whole rounds.
+TcPlan plan_tc(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available, bool gather = false) {
+  TcPlan pl = plan_high_tiles(M, n_tiles, n_pairs, K, gather ? 0 : ws_bytes_available);
+  if (gather || M <= 16 || K >= kCostK || (pl.pair && !pl.pp.balanced)) return pl;
+  const int sms = sm_count() > 0 ? sm_count() : 148;
+  const int parts = pl.pair ? 1 : short_k_parts(M, n_tiles, K, pl.sp.split);
+  auto high_us = [&](const CostModel& c) {
+    return pl.pair ? c.balanced_pairs(pl.BM, pl.pp.items, sms / 2, K / BLOCK_K) : c.one_cta(pl.BM, pl.m_tiles * n_tiles, pl.sp, sms);
+  };
+  const double high_col = high_us(kColumnWise), high_row = high_us(kRowWise);
+  // the gain has to exceed the prediction's error: against the same kernel, and against the other one
+  double best = pl.pair ? 0.88 : 0.96;
+  int last_rows = 0;
+  for (int m_tiles = (M + 255) / 256;; ++m_tiles) {
+    const int BM = ((M + m_tiles - 1) / m_tiles + 15) / 16 * 16;
+    if (BM < kMinPlannedRows && last_rows > 0) break;
+    if (BM == last_rows) {
+      if (BM <= kMinPlannedRows) break;
+      continue;
+    }
+    last_rows = BM;
+    const int tiles = (M + BM - 1) / BM * n_tiles, k_steps = (K + step_k(BM) - 1) / step_k(BM);
+    const int per = (k_steps + parts - 1) / parts;
+    if ((k_steps + per - 1) / per != parts || (parts > 1 && tiles * parts > sms)) continue;
+    const SplitPlan sp{parts, per, 0, 0, 0};
+    const double col = kColumnWise.one_cta(BM, tiles, sp, sms) / high_col, row = kRowWise.one_cta(BM, tiles, sp, sms) / high_row;
+    const double ratio = col > row ? col : row;
+    if (ratio >= best) continue;
+    best = ratio;
+    pl.pair = false;
+    pl.BM = BM;
+    pl.m_tiles = (M + BM - 1) / BM;
+    pl.sp = sp;
+  }
+  return pl;
+}
+
 }  // namespace
 
 size_t gemm_tc_workspace_bytes(int M, int N, int K) {
@@ -998,8 +1108,13 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
   }
   p.M = M; p.N = N; p.K = K; p.block = block;
   p.block_shift = block == 16 ? 4 : block == 32 ? 5 : block == 64 ? 6 : 7;
-  p.BM = tile_rows(M, 16);
-  p.m_tiles = (M + p.BM - 1) / p.BM;
+  const bool ws_ok = workspace && reinterpret_cast<uintptr_t>(workspace) % 256 == 0;
+  // the fused exchange lives in the pair kernel's epilogue and runs in whole rounds
+  const TcPlan plan = plan_tc(M, n_tiles, n_pairs, K, ws_ok ? workspace_bytes : 0, gt != nullptr);
+  const bool pair = plan.pair;
+  if (gt && !pair) return "unsupported shape for the fused all-gather";
+  p.BM = plan.BM;
+  p.m_tiles = plan.m_tiles;
   p.n_tiles = n_tiles;
   p.has_zp = zp != nullptr;
   p.out = grp.out[0];
@@ -1014,15 +1129,6 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
     while (p.tmem_cols < need) p.tmem_cols <<= 1;
   }
 
-  const bool ws_ok = workspace && reinterpret_cast<uintptr_t>(workspace) % 256 == 0;
-  // the fused exchange lives in the pair kernel's epilogue and runs in whole rounds
-  const PairPlan pp = plan_pair(M, n_pairs, K, (ws_ok && !gt) ? workspace_bytes : 0);
-  const bool pair = pp.use;
-  if (gt && !pair) return "unsupported shape for the fused all-gather";
-  if (pair) {
-    p.BM = pp.BM;
-    p.m_tiles = pp.m_tiles;
-  }
   if constexpr (G > 1) {
     p.grp = grp;
     int end = 0;
@@ -1069,6 +1175,7 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
   const int sms = sm_count();
   if (pair) {
     p.k_steps = K / BLOCK_K;
+    const PairPlan& pp = plan.pp;
     p.num_items = pp.items;
     p.n_pairs = n_pairs;
     // fused all-gather: walk the column pairs of one m tile together, so that at any moment the stores of all
@@ -1082,13 +1189,13 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
     p.ws_flags = reinterpret_cast<unsigned*>(workspace);
     p.ws_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + pp.flags_bytes);
     auto kern = colwise ? gemm_tc_pair_kernel<true, kPairWeightStages, G> : gemm_tc_pair_kernel<false, kPairWeightStages, G>;
-    const SmemPlan plan = make_plan(kPairRows, kPairWeightStages, kPairActStages, 1, kPairOutBytes);
+    const SmemPlan smem = make_plan(kPairRows, kPairWeightStages, kPairActStages, 1, kPairOutBytes);
     static std::atomic<int> granted[2][64];
-    cudaError_t e = ensure_dynamic_smem(kern, plan.total, granted[colwise ? 1 : 0]);
+    cudaError_t e = ensure_dynamic_smem(kern, smem.total, granted[colwise ? 1 : 0]);
     if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kPairThreads);
-    cfg.dynamicSmemBytes = plan.total;
+    cfg.dynamicSmemBytes = smem.total;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1118,7 +1225,7 @@ std::string launch_weights(int block, bool colwise, int M, int K, cudaStream_t s
   }
   const int num_tiles = p.m_tiles * p.n_tiles;
   p.k_steps = (K + sk - 1) / sk;
-  SplitPlan sp = plan_split(M, n_tiles, K, ws_ok ? workspace_bytes : 0);
+  SplitPlan sp = plan.sp;
   const KernelChoice<G> kc = fit_plan<G>(colwise, p.BM, num_tiles, p.k_steps, sms, sp);
   p.split = sp.split;  // split > 1: at most one item per SM
   p.k_per_item = sp.k_per_item;
@@ -1184,31 +1291,40 @@ size_t gemm_tc_group_workspace_bytes(int M, int K, int count, const int* n) {
 
 namespace {
 
-// K split of a launch with all the workspace that it asks for; k_per_item 0 where balanced ranges would cut its tiles.
+// K split of a plan as the device runs it, k_per_item in k; 0 where balanced ranges would cut its tiles.
 template <int G>
-SplitPlan launched_split(bool colwise, int M, int K, int n_tiles, int n_pairs) {
-  const PairPlan pp = plan_pair(M, n_pairs, K, ~(size_t)0);
-  if (pp.use) return SplitPlan{1, pp.balanced ? 0 : K, 0, 0, 0};
-  SplitPlan sp = plan_split(M, n_tiles, K, ~(size_t)0);
+SplitPlan launched_split(bool colwise, int K, int n_tiles, const TcPlan& pl) {
+  if (pl.pair) return SplitPlan{1, pl.pp.balanced ? 0 : K, 0, 0, 0};
+  SplitPlan sp = pl.sp;
   if (sp.balanced) return SplitPlan{1, 0, 0, 0, 0};
-  const int BM = tile_rows(M, 16), k_steps = (K + step_k(BM) - 1) / step_k(BM);
-  if (have_device()) fit_plan<G>(colwise, BM, (M + BM - 1) / BM * n_tiles, k_steps, sm_count() > 0 ? sm_count() : 148, sp);
-  return SplitPlan{sp.split, sp.split > 1 ? sp.k_per_item : K, 0, 0, 0};
+  const int k_steps = (K + step_k(pl.BM) - 1) / step_k(pl.BM);
+  if (have_device()) fit_plan<G>(colwise, pl.BM, pl.m_tiles * n_tiles, k_steps, sm_count() > 0 ? sm_count() : 148, sp);
+  return SplitPlan{sp.split, sp.split > 1 ? sp.k_per_item * step_k(pl.BM) : K, 0, 0, 0};
 }
 
 }  // namespace
 
+// With all the workspace that is asked for.  Layers that high tiles would cut in balanced ranges, or in other parts than their
+// group, stay apart although lower tiles may cut all of them alike: which layers share a launch is part of the interface.
 bool gemm_tc_group_keeps_bits(bool colwise, int M, int K, int count, const int* n) {
   int n_tiles = 0, n_pairs = 0;
   for (int i = 0; i < count; ++i) {
     n_tiles += column_tiles(n[i]);
     n_pairs += column_pairs(n[i]);
   }
-  const SplitPlan all = launched_split<kMaxGroup>(colwise, M, K, n_tiles, n_pairs);
+  auto split_of = [&](auto g, int tiles, int pairs, bool high) {
+    const TcPlan pl = high ? plan_high_tiles(M, tiles, pairs, K, ~(size_t)0) : plan_tc(M, tiles, pairs, K, ~(size_t)0);
+    return launched_split<decltype(g)::value>(colwise, K, tiles, pl);
+  };
+  const std::integral_constant<int, kMaxGroup> group{};
+  const std::integral_constant<int, 1> alone{};
+  const SplitPlan all = split_of(group, n_tiles, n_pairs, false), all_high = split_of(group, n_tiles, n_pairs, true);
   if (all.k_per_item == 0) return false;
   for (int i = 0; i < count; ++i) {
-    const SplitPlan one = launched_split<1>(colwise, M, K, column_tiles(n[i]), column_pairs(n[i]));
+    const int tiles = column_tiles(n[i]), pairs = column_pairs(n[i]);
+    const SplitPlan one = split_of(alone, tiles, pairs, false), one_high = split_of(alone, tiles, pairs, true);
     if (one.split != all.split || one.k_per_item != all.k_per_item) return false;
+    if (one_high.split != all_high.split || one_high.k_per_item == 0) return false;
   }
   return true;
 }
@@ -1233,15 +1349,15 @@ extern "C" int blkq4_gemm_plan(int m, int n, int k, size_t workspace_size, int* 
   for (int i = 0; i < 6; ++i) out6[i] = 0;
   if (m <= 16) return 0;
   const int sms = blkq4::sm_count() > 0 ? blkq4::sm_count() : 148;
-  const blkq4::PairPlan pp = blkq4::plan_pair(m, blkq4::column_pairs(n), k, workspace_size);
-  if (pp.use) {
-    out6[0] = 2; out6[1] = pp.BM; out6[2] = pp.items; out6[3] = 1; out6[4] = pp.balanced;
-    out6[5] = pp.balanced ? sms / 2 : 0;
+  const blkq4::TcPlan pl = blkq4::plan_tc(m, blkq4::column_tiles(n), blkq4::column_pairs(n), k, workspace_size);
+  if (pl.pair) {
+    out6[0] = 2; out6[1] = pl.BM; out6[2] = pl.pp.items; out6[3] = 1; out6[4] = pl.pp.balanced;
+    out6[5] = pl.pp.balanced ? sms / 2 : 0;
     return 0;
   }
-  blkq4::SplitPlan sp = blkq4::plan_split(m, blkq4::column_tiles(n), k, workspace_size);
-  const int bm = blkq4::tile_rows(m, 16);
-  out6[0] = 1; out6[1] = bm; out6[2] = ((m + bm - 1) / bm) * ((n + blkq4::tc::TILE_N - 1) / blkq4::tc::TILE_N);
+  blkq4::SplitPlan sp = pl.sp;
+  const int bm = pl.BM;
+  out6[0] = 1; out6[1] = bm; out6[2] = pl.m_tiles * blkq4::column_tiles(n);
   // as many clusters fit of the row-wise kernel as of the column-wise one: one CTA per SM, both
   if (blkq4::have_device())
     blkq4::fit_split(blkq4::choose_kernel<1>(true, bm), out6[2], (k + blkq4::step_k(bm) - 1) / blkq4::step_k(bm), sp);
