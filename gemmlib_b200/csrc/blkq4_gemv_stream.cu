@@ -18,8 +18,9 @@
 //     16-row operand and the activations as its 8-column operand, the accumulator of a 64-k step
 //     starts at minus the activation-only term of that step, and the step's sum is scaled in fp32:
 //         total += scale * (sum_k a_k (magic + q_k) - sum_k a_k (magic + 8)).
-//     With zero points the term zp * scale * sum_k a_k is accumulated separately, one (step, column)
-//     pair per lane, instead of inside the per-step code of every lane.
+//     With zero points the term zp * scale * sum_k a_k is accumulated separately for one or two rows, one (step, column)
+//     pair per lane, instead of inside the per-step code of every lane.  For more rows it is subtracted
+//     from the step's sum (ZFOLD): the separate terms would be 16 rows x columns more partial sums per warp and as many shuffles.
 //   * At the end of a tile the warps leave their partial sums in shared memory, the CTA meets at one
 //     barrier, and one warp (rotating) adds them in a fixed order, rounds to fp16 and stores.
 //
@@ -47,6 +48,7 @@ namespace blkq4 {
 namespace {
 
 using namespace stream;
+__device__ __forceinline__ float2 add_f2(const float2& a, const float2& b) { return make_float2(a.x + b.x, a.y + b.y); }
 constexpr int kCorrStep = 4 * 16;    // bytes of mma-initialising terms per step: four row pairs, float4 each
 
 struct StreamParams {
@@ -68,7 +70,7 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 
 // Shared memory: rings [kWarps][D][kSlotBytes] | s_corr [steps][4] float4 | s_asum [steps][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
-// MZ: rows of the zero-point accumulators kept in registers (2 for M <= 2, else 8).
+// MZ: 2 for M <= 2, whose zero-point terms have accumulators of their own, else 8.
 //
 // GATHER (N-sharded layer, one process per GPU).  The exchange is latency-bound (a few tens of KB per
 // rank), so it carries its own flags: the adding warp stores the tile's results into EVERY rank's
@@ -86,6 +88,13 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 // Measured on B200, graph of two decoder blocks (hidden 4096, 11008; block 64, zero points; 14 layers, 8 launches), M = 1: 102.5 us in
 // one launch per layer, 76.5 in groups; M = 4 134.0 / 95.1.
 //
+// ZFOLD (zero points, three rows and more): zp * sum_k a_k is subtracted from the step's sum before it is scaled, four FMAs and three
+// loads a step, instead of sums of their own: eight FMAs and four loads for two steps, but a shuffle, an addition and a store per row and
+// 16 more terms per output at the tile's end.  Measured on B200, block 64, own sums / subtracted, us: M = 8: 2048 x 2048 4.1 / 3.5,
+// 4096 x 4096 7.9 / 6.8, 4096 x 11008 13.5 / 10.8, 8192 x 28672 43.0 / 38.1; M = 4: 3.2 / 3.0, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 34.9; M = 1 and 2
+// keep theirs (two FMAs for two steps).  (As part of the accumulator's initial value, which is a thousand times larger than the sum, the
+// term would be rounded there: relative error against 64 bits 2.0853e-4, with sums of their own 2.0841e-4.)
+//
 // BS: steps of a quantization block, as a shift (0: blocks of 64, 1: of 128).  The two steps of a 128-k block share scale and
 // zero point: one load and conversion of them, two accumulators with independent mma chains, one scaling of their sum.
 // (One chain of eight mma from the sum of both activation-only terms is faster still, but the larger partial sums cost
@@ -96,7 +105,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 gemv_stream_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint8_t s_raw[];
   constexpr int W = kWarps, GS = kGroupSteps;
-  constexpr int PW = HAS_ZP ? 2 * W : W;  // partial-sum entries per tile: the warps (+ their zero-point terms)
+  constexpr bool ZFOLD = HAS_ZP && MZ > 2;       // zero points are subtracted step by step (see above)
+  constexpr bool ZSEP = HAS_ZP && !ZFOLD;
+  constexpr int PW = ZSEP ? 2 * W : W;  // partial-sum entries per tile: the warps (+ their zero-point terms)
   const int MS = (p.M + 1) & ~1;
   uint8_t* s_ring = s_raw;
   float* s_corr = reinterpret_cast<float*>(s_ring + W * D * kSlotBytes);
@@ -266,9 +277,7 @@ gemv_stream_kernel(const StreamParams p) {
   const uint32_t asum_base = smem_u32(s_asum) + (uint32_t)(gb * GS) * 32u;
 
   float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  float ztot[MZ];  // zero-point terms of column (lane & 15), rows m, over the steps of half (lane >> 4)
-#pragma unroll
-  for (int m = 0; m < MZ; ++m) ztot[m] = 0.0f;
+  float ztot[2] = {0.0f, 0.0f};  // ZSEP: zero-point terms of column (lane & 15), rows m, over the steps of half (lane >> 4)
 
   uint32_t src = ring_addr;
   for (int tl = 0; tl < my_tiles; ++tl) {
@@ -278,7 +287,8 @@ gemv_stream_kernel(const StreamParams p) {
       __syncwarp();  // the scales / zero points of the slot were copied by other lanes
       const uint32_t src_w = src + lane * 16;
       const uint32_t src_s = src + kSlotW + g * 2;
-      if (HAS_ZP) {
+      const uint32_t src_z = src + kSlotW + kSlotS + g, as_t = as_addr + t * 8;
+      if (ZSEP) {
         const uint32_t col = lane & 15, u0 = (lane >> 4) * (GS / 2);
 #pragma unroll
         for (int uu = 0; uu < GS / 2; uu += 1 << BS) {
@@ -288,13 +298,10 @@ gemv_stream_kernel(const StreamParams p) {
           const float nsz = -s * z;
 #pragma unroll
           for (int v = 0; v < (1 << BS); ++v) {
-#pragma unroll
-            for (int m = 0; m < MZ; m += 2) {
-              if (m < M) {
-                const float2 as = lds_f2(as_addr + (u + v) * 32 + m * 4);
-                ztot[m] = fmaf(nsz, as.x, ztot[m]);
-                ztot[m + 1] = fmaf(nsz, as.y, ztot[m + 1]);
-              }
+            if (M > 0) {  // always: without the branch the compiler's schedule is 1 to 2 % slower (M = 1, 4096 x 11008 8.5 / 8.6)
+              const float2 as = lds_f2<0>(as_addr + (u + v) * 32);
+              ztot[0] = fmaf(nsz, as.x, ztot[0]);
+              ztot[1] = fmaf(nsz, as.y, ztot[1]);
             }
           }
         }
@@ -310,6 +317,15 @@ gemv_stream_kernel(const StreamParams p) {
           hi_a##U[r] = lop3_and_or(x, kHiMask, kHiMagic); /* (n;     k 2r+8, 2r+9)   64 + q */  \
           lo_b##U[r] = lop3_and_or(y, kLoMask, kLoMagic); /* (n + 8; k 2r, 2r+1)            */  \
           hi_b##U[r] = lop3_and_or(y, kHiMask, kHiMagic); /* (n + 8; k 2r+8, 2r+9)          */  \
+        }
+#define BLKQ4_STREAM_ZP(U, ACC, AS)                                                             \
+        {                                                                                       \
+          const float za = lds_u8_by_mantissa<(U) * 16>(src_z), zb = lds_u8_by_mantissa<(U) * 16 + 8>(src_z); \
+          const float2 as = AS;                                                                 \
+          ACC[0] = fmaf(-za, as.x, ACC[0]);                                                     \
+          ACC[1] = fmaf(-za, as.y, ACC[1]);                                                     \
+          ACC[2] = fmaf(-zb, as.x, ACC[2]);                                                     \
+          ACC[3] = fmaf(-zb, as.y, ACC[3]);                                                     \
         }
 #define BLKQ4_STREAM_MMA(U)                                                                     \
         float acc##U[4];                                                                        \
@@ -332,6 +348,7 @@ gemv_stream_kernel(const StreamParams p) {
       {                                                                                         \
         BLKQ4_STREAM_UNPACK(U)                                                                  \
         BLKQ4_STREAM_MMA(U)                                                                     \
+        if (ZFOLD) BLKQ4_STREAM_ZP(U, acc##U, lds_f2<(U) * 32>(as_t))                           \
         BLKQ4_STREAM_SCALE(U, acc##U[0], acc##U[1], acc##U[2], acc##U[3])                       \
       }
 #define BLKQ4_STREAM_BLOCK128(U, V)                                                             \
@@ -340,7 +357,10 @@ gemv_stream_kernel(const StreamParams p) {
         BLKQ4_STREAM_UNPACK(V)                                                                  \
         BLKQ4_STREAM_MMA(U)                                                                     \
         BLKQ4_STREAM_MMA(V)                                                                     \
-        BLKQ4_STREAM_SCALE(U, acc##U[0] + acc##V[0], acc##U[1] + acc##V[1], acc##U[2] + acc##V[2], acc##U[3] + acc##V[3]) \
+        float sum[4];                                                                           \
+        _Pragma("unroll") for (int e = 0; e < 4; ++e) sum[e] = acc##U[e] + acc##V[e];           \
+        if (ZFOLD) BLKQ4_STREAM_ZP(U, sum, add_f2(lds_f2<(U) * 32>(as_t), lds_f2<(V) * 32>(as_t))) \
+        BLKQ4_STREAM_SCALE(U, sum[0], sum[1], sum[2], sum[3])                                   \
       }
       if constexpr (BS == 1) {
         BLKQ4_STREAM_BLOCK128(0, 1)
@@ -355,6 +375,7 @@ gemv_stream_kernel(const StreamParams p) {
 #undef BLKQ4_STREAM_STEP
 #undef BLKQ4_STREAM_SCALE
 #undef BLKQ4_STREAM_MMA
+#undef BLKQ4_STREAM_ZP
 #undef BLKQ4_STREAM_UNPACK
       issue_group(src);  // refill the slot just consumed
       src = (src == ring_last) ? ring_addr : src + kSlotBytes;
@@ -372,9 +393,9 @@ gemv_stream_kernel(const StreamParams p) {
       *reinterpret_cast<float2*>(d0 + 8 * MS) = make_float2(total[2], total[3]);
     }
     total[0] = total[1] = total[2] = total[3] = 0.0f;
-    if (HAS_ZP) {
+    if (ZSEP) {
 #pragma unroll
-      for (int m = 0; m < MZ; ++m) {
+      for (int m = 0; m < 2; ++m) {
         if (m < MS) {
           const float z = ztot[m] + __shfl_xor_sync(0xffffffffu, ztot[m], 16);
           if (lane < 16) buf[((size_t)(W + warp) * 16 + lane) * MS + m] = z;
@@ -481,7 +502,7 @@ std::string launch_T(const StreamParams& p, size_t smem, int grid, cudaStream_t 
 }
 
 size_t stream_smem_bytes(int M, int K, bool has_zp, int D) {
-  const int MS = (M + 1) & ~1, PW = has_zp ? 2 * kWarps : kWarps, steps = K / 64;
+  const int MS = (M + 1) & ~1, PW = has_zp && M <= 2 ? 2 * kWarps : kWarps, steps = K / 64;
   return (size_t)kWarps * D * kSlotBytes + (size_t)steps * 64 + (has_zp ? (size_t)steps * 32 : 0) +
          (size_t)2 * PW * 16 * MS * 4 + 256 + (size_t)M * (K + 8) * 2;
 }
@@ -492,8 +513,10 @@ const char* const kStreamUnsupported = "unsupported by the stream kernel";
 
 bool gemv_stream_takes(int block, bool colwise, int M, int N, int K) {
   const int group_k = kGroupSteps * 64;
+  // what the partial sums of the zero points once took: which layers share a launch is part of the interface
+  const size_t zp_partials = M > 2 ? (size_t)2 * kWarps * 16 * ((M + 1) & ~1) * 4 : 0;
   return colwise && block >= 64 && M >= 1 && M <= 8 && K % group_k == 0 && K / group_k >= kWarps &&
-         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, true, 2) <= (size_t)227 * 1024;
+         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, true, 2) + zp_partials <= (size_t)227 * 1024;
 }
 
 // Returns kStreamUnsupported when the shape is outside this kernel (the caller then takes another one).

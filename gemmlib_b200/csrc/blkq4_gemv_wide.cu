@@ -240,7 +240,7 @@ gemv_wide_kernel(const WideParams p) {
         float2 as[MT];                                                                                   \
         _Pragma("unroll") for (int j = 0; j < MT; ++j) {                                                 \
           c[j] = lds_f4<(U) * kCorrStepW>(c_addr + j * 64);                                              \
-          if (HAS_ZP) as[j] = lds_f2(as_addr + (U) * kAsumStepW + j * 32);                               \
+          if (HAS_ZP) as[j] = lds_f2<0>(as_addr + (U) * kAsumStepW + j * 32);                               \
         }                                                                                                \
         _Pragma("unroll") for (int i = 0; i < NT; ++i) {                                                 \
           const uint4 wv = lds_v4<(U) * 512>(src_w + i * kSlotBytes);                                    \
