@@ -29,8 +29,8 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
                         const __half* a, const uint8_t* packed, const __half* scales,
                         const uint8_t* zp, __half* out, const __half* bias, unsigned flags);
 
-// The decode kernel (M <= 8, column-wise blocks >= 64, K a multiple of 256 and >= 2048): per-warp
-// cp.async rings, two launches resident per SM.  Returns kStreamUnsupported for other shapes.
+// The decode kernel (M <= 8, column-wise blocks >= 64; groups of matrices and the fused exchange only with K a multiple of 256 and
+// >= 2048): per-warp cp.async rings, two launches resident per SM.  Returns kStreamUnsupported for other shapes.
 extern const char* const kStreamUnsupported;
 struct GatherTable;
 struct GemmGroup;
@@ -39,7 +39,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
                                const uint8_t* zp, __half* out, const __half* bias, unsigned flags,
                                const GatherTable* gt = nullptr, const GemmGroup* grp = nullptr);
 
-// Whether it takes the problem (with 16-byte aligned scales and zero points), alone or as a group of N columns in all.
+// Whether it takes a group of N columns in all (with 16-byte aligned scales and zero points).
 bool gemv_stream_takes(int block, bool colwise, int M, int N, int K);
 // True when the environment (BLKQ4_GEMV_NO_STREAM, BLKQ4_GEMV_GENERIC) keeps calls of up to 16 rows off it.
 bool gemv_stream_off();

@@ -3,7 +3,7 @@
 // The weight stream is the only large operand, so the kernel is organised around it.
 //
 //   * Every warp is its own producer and consumer.  A CTA has eight warps; warp w owns a fixed slice
-//     of K (whole groups of four 64-k steps) of EVERY 16-column tile the CTA works on.  It copies its
+//     of K (groups of four 64-k steps, the last one of K perhaps shorter: TAIL) of EVERY 16-column tile the CTA works on.  It copies its
 //     slice of the packed weights, with the scales and zero points of those steps, into a private
 //     ring of shared-memory slots with cp.async (16 bytes per lane, placed as [step][lane], so the
 //     later 128-bit reads are conflict free) and waits with cp.async.wait_group, which, unlike a
@@ -18,9 +18,8 @@
 //     16-row operand and the activations as its 8-column operand, the accumulator of a 64-k step
 //     starts at minus the activation-only term of that step, and the step's sum is scaled in fp32:
 //         total += scale * (sum_k a_k (magic + q_k) - sum_k a_k (magic + 8)).
-//     With zero points the term zp * scale * sum_k a_k is accumulated separately for one or two rows, one (step, column)
-//     pair per lane, instead of inside the per-step code of every lane.  For more rows it is subtracted
-//     from the step's sum (ZFOLD): the separate terms would be 16 rows x columns more partial sums per warp and as many shuffles.
+//     With zero points zp * sum_k a_k is subtracted from the step's sum, or summed separately, one (step, column) pair per lane
+//     (see ZP below).
 //   * At the end of a tile the warps leave their partial sums in shared memory, the CTA meets at one
 //     barrier, and one warp (rotating) adds them in a fixed order, rounds to fp16 and stores.
 //
@@ -51,6 +50,9 @@ using namespace stream;
 __device__ __forceinline__ float2 add_f2(const float2& a, const float2& b) { return make_float2(a.x + b.x, a.y + b.y); }
 constexpr int kCorrStep = 4 * 16;    // bytes of mma-initialising terms per step: four row pairs, float4 each
 
+// Zero points: none; with sums of their own (up to two rows); subtracted from every step's sum.
+enum class Zp { kNone, kOwnSums, kPerStep };
+
 struct StreamParams {
   const __half* a;
   __half* out;
@@ -70,7 +72,7 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 
 // Shared memory: rings [kWarps][D][kSlotBytes] | s_corr [steps][4] float4 | s_asum [steps][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
-// MZ: 2 for M <= 2, whose zero-point terms have accumulators of their own, else 8.
+// MZ: rows whose activations are staged at a time: one after the other for M <= 2 (2), else all together (8).
 //
 // GATHER (N-sharded layer, one process per GPU).  The exchange is latency-bound (a few tens of KB per
 // rank), so it carries its own flags: the adding warp stores the tile's results into EVERY rank's
@@ -88,25 +90,34 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 // Measured on B200, graph of two decoder blocks (hidden 4096, 11008; block 64, zero points; 14 layers, 8 launches), M = 1: 102.5 us in
 // one launch per layer, 76.5 in groups; M = 4 134.0 / 95.1.
 //
-// ZFOLD (zero points, three rows and more): zp * sum_k a_k is subtracted from the step's sum before it is scaled, four FMAs and three
-// loads a step, instead of sums of their own: eight FMAs and four loads for two steps, but a shuffle, an addition and a store per row and
-// 16 more terms per output at the tile's end.  Measured on B200, block 64, own sums / subtracted, us: M = 8: 2048 x 2048 4.1 / 3.5,
-// 4096 x 4096 7.9 / 6.8, 4096 x 11008 13.5 / 10.8, 8192 x 28672 43.0 / 38.1; M = 4: 3.2 / 3.0, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 34.9; M = 1 and 2
-// keep theirs (two FMAs for two steps).  (As part of the accumulator's initial value, which is a thousand times larger than the sum, the
-// term would be rounded there: relative error against 64 bits 2.0853e-4, with sums of their own 2.0841e-4.)
+// ZP: kPerStep subtracts zp * sum_k a_k from a step's sum before it is scaled, four FMAs and three loads a step.  kOwnSums keeps
+// accumulators of their own for these terms, two FMAs and three loads for two steps, but a shuffle, an addition and a store per row
+// and 16 more terms per output at the tile's end.  kPerStep is taken for three rows and more, and for one or two where tiles are
+// short.  Measured on B200, kOwnSums / kPerStep, us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008
+// 13.5 / 10.8, 8192 x 28672 43.0 / 37.9; M = 4: 3.2 / 2.9, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 33.9; M = 1: 512 x 11008 4.3 / 3.5, 4096 x 4096
+// 4.4 / 4.2, 4096 x 11008 8.5 / 7.9, 11008 x 4096 8.5 / 8.4, 8192 x 28672 27.3 / 28.7; block 128 4.2 / 4.2, 8.0 / 8.2, 8.0 / 8.4, 26.0 / 27.3.
+// (As part of the accumulator's initial value, which is a thousand times larger than the sum, the term would be rounded there:
+// relative error against 64 bits 2.0853e-4, with either of these 2.0841e-4.)
+//
+// TAIL: K is not a multiple of 256, or shorter than eight groups of steps.  The steps that are missing from a last group are neither
+// copied nor computed; with fewer groups than warps the other warps only take part in the barriers.  The whole groups of other K
+// need none of these tests (a kernel of its own: 128 registers already).  Measured on B200 against the TMA kernel, which had
+// these shapes (below 512 k the generic kernel), us, symmetric blocks of 128, M = 1, 4 and 8: 256 x 4096 3.4, 3.5, 3.5 / 1.9, 2.3, 3.0;
+// 1024 x 4096 3.1, 4.3, 4.5 / 2.2, 2.7, 3.3; 2176 x 8192 5.7, 7.3, 8.3 / 4.2, 5.4, 6.7; 4224 x 11008 10.5, 12.6, 15.2 / 8.6, 10.6, 12.3;
+// 3200 x 28672 18.7, 20.1, 23.4 / 12.4, 14.0, 15.4.  Slices balanced to the step, every warp's last group short, were 2 to 9 % slower up
+// to 1024 k and equal above: the steps of a short group run one by one.
 //
 // BS: steps of a quantization block, as a shift (0: blocks of 64, 1: of 128).  The two steps of a 128-k block share scale and
 // zero point: one load and conversion of them, two accumulators with independent mma chains, one scaling of their sum.
 // (One chain of eight mma from the sum of both activation-only terms is faster still, but the larger partial sums cost
 // precision: relative error 2.050e-4 against 2.033e-4 on 8192 k; this 2.033e-4.)  Measured on B200 against a load and scaling per
 // step, us: 8192 x 28672 M = 4 28.3 / 28.0, with zero points 36.9 / 36.2, M = 8 33.5 / 32.9; 4096 x 11008, M = 1 7.3 / 7.1.
-template <bool HAS_ZP, int D, int MZ, int BS, bool GATHER, bool GROUP>
+template <Zp ZP, int D, int MZ, int BS, bool GATHER, bool GROUP, bool TAIL>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 gemv_stream_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint8_t s_raw[];
   constexpr int W = kWarps, GS = kGroupSteps;
-  constexpr bool ZFOLD = HAS_ZP && MZ > 2;       // zero points are subtracted step by step (see above)
-  constexpr bool ZSEP = HAS_ZP && !ZFOLD;
+  constexpr bool HAS_ZP = ZP != Zp::kNone, ZFOLD = ZP == Zp::kPerStep, ZSEP = ZP == Zp::kOwnSums;
   constexpr int PW = ZSEP ? 2 * W : W;  // partial-sum entries per tile: the warps (+ their zero-point terms)
   const int MS = (p.M + 1) & ~1;
   uint8_t* s_ring = s_raw;
@@ -121,9 +132,13 @@ gemv_stream_kernel(const StreamParams p) {
   const int K = p.K, M = p.M;
   int N = p.N;  // GROUP: of the tile that is being loaded
   constexpr int bs = BS;
-  const int kgroups = p.steps / GS;
-  const int gb = (int)(((long long)kgroups * warp) / W);
-  const int myg = (int)(((long long)kgroups * (warp + 1)) / W) - gb;  // >= 1: the launcher requires kgroups >= W
+  const int kgroups = (p.steps + GS - 1) / GS;
+  // >= 1 without TAIL: the launcher requires kgroups >= W.  Fewer groups than warps go to the first ones, one each (the formula
+  // would give them to every second warp, which share two of the SM's four schedulers).
+  const bool few = TAIL && kgroups < W;
+  const int gb = few ? min(warp, kgroups) : (int)(((long long)kgroups * warp) / W);
+  const int myg = few ? (warp < kgroups ? 1 : 0) : (int)(((long long)kgroups * (warp + 1)) / W) - gb;
+  const int last_steps = TAIL ? min(GS, p.steps - (gb + myg - 1) * GS) : GS;  // of this warp's last group
   const int my_tiles = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const uint32_t ring_addr = smem_u32(s_ring) + (uint32_t)warp * (D * kSlotBytes);
   const uint32_t ring_last = ring_addr + (D - 1) * kSlotBytes;
@@ -137,6 +152,7 @@ gemv_stream_kernel(const StreamParams p) {
   // lanes 0-7 copy the scales of step lane / 2, column half lane % 2; lanes 8-11 the zero points of step lane - 8
   const uint32_t meta_lane = (lane < 2 * GS || (HAS_ZP && lane < 3 * GS)) ? 1u : 0u;
   const uint32_t m_dst = lane < 2 * GS ? kSlotW + (lane >> 1) * 32 + (lane & 1) * 16 : kSlotW + kSlotS + (lane - 2 * GS) % GS * 16;
+  const int meta_step = lane < 2 * GS ? lane >> 1 : (lane - 2 * GS) % GS;  // step whose scales / zero points this lane copies
   const uint8_t *wp, *mp;
   long long m_step, m_tile_adj;
   // this lane's addresses for the warp's first group of a tile
@@ -167,11 +183,21 @@ gemv_stream_kernel(const StreamParams p) {
   auto issue_group = [&](uint32_t dst) {
     const uint32_t go = ld_left > 0 ? 1u : 0u;
     const uint32_t dw = dst + lane * 16;
-    cp_async16_if<0>(dw, wp, go);
-    cp_async16_if<64>(dw, wp, go);
-    cp_async16_if<128>(dw, wp, go);
-    cp_async16_if<192>(dw, wp, go);
-    cp_async16_if<0>(dst + m_dst, mp, go & meta_lane);
+    if constexpr (TAIL) {
+      // steps past the end of K are neither copied nor computed
+      const int n = go ? (ld_j + 1 == myg ? last_steps : GS) : 0;
+      cp_async16_if<0>(dw, wp, n > 0);
+      cp_async16_if<64>(dw, wp, n > 1);
+      cp_async16_if<128>(dw, wp, n > 2);
+      cp_async16_if<192>(dw, wp, n > 3);
+      cp_async16_if<0>(dst + m_dst, mp, meta_lane && meta_step < n);
+    } else {
+      cp_async16_if<0>(dw, wp, go);
+      cp_async16_if<64>(dw, wp, go);
+      cp_async16_if<128>(dw, wp, go);
+      cp_async16_if<192>(dw, wp, go);
+      cp_async16_if<0>(dst + m_dst, mp, go & meta_lane);
+    }
     cp_async_commit();  // always: the group count per iteration stays fixed
     --ld_left;
     const bool wrap = ++ld_j == myg;
@@ -222,8 +248,13 @@ gemv_stream_kernel(const StreamParams p) {
   {
     const int slice_k0 = gb * (GS * 64);
     const int chunks = myg * (GS * 8);  // a multiple of 32
+    // TAIL: lanes past the end of K run along (the shuffles below are of whole warps) with zeros and store nothing
+    auto load_chunk = [&](int m, int k0) {
+      if (TAIL && k0 >= K) return make_uint4(0u, 0u, 0u, 0u);
+      return __ldg(reinterpret_cast<const uint4*>(p.a + (size_t)m * K + k0));
+    };
     auto finish_row = [&](int m, int k0, const uint4& v) {
-      *reinterpret_cast<uint4*>(s_a + (size_t)m * p.a_pitch + k0) = v;
+      if (!TAIL || k0 < K) *reinterpret_cast<uint4*>(s_a + (size_t)m * p.a_pitch + k0) = v;
       const __half2* h = reinterpret_cast<const __half2*>(&v);
       float s = 0.0f;
 #pragma unroll
@@ -235,7 +266,7 @@ gemv_stream_kernel(const StreamParams p) {
       s += __shfl_xor_sync(0xffffffffu, s, 2);
       s += __shfl_xor_sync(0xffffffffu, s, 4);
       const float other = __shfl_xor_sync(0xffffffffu, s, 1);
-      if ((lane & 7) == 0) {
+      if ((lane & 7) == 0 && (!TAIL || k0 < K)) {
         const float lo = s, hi = other;
         const int step = k0 >> 6;
         // one float4 per row pair (m even, m odd, m even, m odd): the accumulator rows n and n + 8 start alike
@@ -251,7 +282,7 @@ gemv_stream_kernel(const StreamParams p) {
       for (int m = 0; m < M; ++m)
         for (int c0 = 0; c0 < chunks; c0 += 32) {
           const int k0 = slice_k0 + (c0 + lane) * 8;
-          finish_row(m, k0, __ldg(reinterpret_cast<const uint4*>(p.a + (size_t)m * K + k0)));
+          finish_row(m, k0, load_chunk(m, k0));
         }
     } else {
       // several rows: all rows' loads of a chunk first (one L2 round trip per chunk, not one per row)
@@ -260,7 +291,7 @@ gemv_stream_kernel(const StreamParams p) {
         uint4 v[8];
 #pragma unroll
         for (int m = 0; m < 8; ++m)
-          if (m < M) v[m] = __ldg(reinterpret_cast<const uint4*>(p.a + (size_t)m * K + k0));
+          if (m < M) v[m] = load_chunk(m, k0);
 #pragma unroll
         for (int m = 0; m < 8; ++m)
           if (m < M) finish_row(m, k0, v[m]);
@@ -287,12 +318,14 @@ gemv_stream_kernel(const StreamParams p) {
       __syncwarp();  // the scales / zero points of the slot were copied by other lanes
       const uint32_t src_w = src + lane * 16;
       const uint32_t src_s = src + kSlotW + g * 2;
+      const int n_steps = TAIL && j2 + 1 == myg ? last_steps : GS;
       const uint32_t src_z = src + kSlotW + kSlotS + g, as_t = as_addr + t * 8;
       if (ZSEP) {
         const uint32_t col = lane & 15, u0 = (lane >> 4) * (GS / 2);
 #pragma unroll
         for (int uu = 0; uu < GS / 2; uu += 1 << BS) {
           const uint32_t u = u0 + uu;
+          if (TAIL && (int)u >= n_steps) break;
           const float s = lds_half_as_float<0>(src + kSlotW + u * 32 + col * 2);
           const float z = lds_u8_as_float(src + kSlotW + kSlotS + u * 16 + col);
           const float nsz = -s * z;
@@ -364,12 +397,16 @@ gemv_stream_kernel(const StreamParams p) {
       }
       if constexpr (BS == 1) {
         BLKQ4_STREAM_BLOCK128(0, 1)
-        BLKQ4_STREAM_BLOCK128(2, 3)
-      } else {
+        if (n_steps > 2) BLKQ4_STREAM_BLOCK128(2, 3)  // K is a whole number of blocks
+      } else if (n_steps == GS) {
         BLKQ4_STREAM_STEP(0)
         BLKQ4_STREAM_STEP(1)
         BLKQ4_STREAM_STEP(2)
         BLKQ4_STREAM_STEP(3)
+      } else {
+        BLKQ4_STREAM_STEP(0)
+        if (n_steps > 1) BLKQ4_STREAM_STEP(1)
+        if (n_steps > 2) BLKQ4_STREAM_STEP(2)
       }
 #undef BLKQ4_STREAM_BLOCK128
 #undef BLKQ4_STREAM_STEP
@@ -479,9 +516,9 @@ gemv_stream_kernel(const StreamParams p) {
   }
 }
 
-template <bool HAS_ZP, int D, int MZ, int BS, bool GATHER, bool GROUP>
+template <Zp ZP, int D, int MZ, int BS, bool GATHER, bool GROUP, bool TAIL>
 std::string launch_T(const StreamParams& p, size_t smem, int grid, cudaStream_t stream, bool early) {
-  auto kern = gemv_stream_kernel<HAS_ZP, D, MZ, BS, GATHER, GROUP>;
+  auto kern = gemv_stream_kernel<ZP, D, MZ, BS, GATHER, GROUP, TAIL>;
   static std::atomic<int> granted[64];
   cudaError_t e = ensure_dynamic_smem(kern, smem, granted);
   if (e != cudaSuccess) return std::string(cudaGetErrorString(e));
@@ -501,22 +538,22 @@ std::string launch_T(const StreamParams& p, size_t smem, int grid, cudaStream_t 
   return std::string();
 }
 
-size_t stream_smem_bytes(int M, int K, bool has_zp, int D) {
-  const int MS = (M + 1) & ~1, PW = has_zp && M <= 2 ? 2 * kWarps : kWarps, steps = K / 64;
-  return (size_t)kWarps * D * kSlotBytes + (size_t)steps * 64 + (has_zp ? (size_t)steps * 32 : 0) +
+size_t stream_smem_bytes(int M, int K, Zp zp, int D) {
+  const int MS = (M + 1) & ~1, PW = zp == Zp::kOwnSums ? 2 * kWarps : kWarps, steps = K / 64;
+  return (size_t)kWarps * D * kSlotBytes + (size_t)steps * 64 + (zp != Zp::kNone ? (size_t)steps * 32 : 0) +
          (size_t)2 * PW * 16 * MS * 4 + 256 + (size_t)M * (K + 8) * 2;
 }
 
 }  // namespace
 
+
+
 const char* const kStreamUnsupported = "unsupported by the stream kernel";
 
 bool gemv_stream_takes(int block, bool colwise, int M, int N, int K) {
   const int group_k = kGroupSteps * 64;
-  // what the partial sums of the zero points once took: which layers share a launch is part of the interface
-  const size_t zp_partials = M > 2 ? (size_t)2 * kWarps * 16 * ((M + 1) & ~1) * 4 : 0;
   return colwise && block >= 64 && M >= 1 && M <= 8 && K % group_k == 0 && K / group_k >= kWarps &&
-         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, true, 2) + zp_partials <= (size_t)227 * 1024;
+         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, Zp::kOwnSums, 2) <= (size_t)227 * 1024;  // whatever the zero points: part of the interface
 }
 
 // Returns kStreamUnsupported when the shape is outside this kernel (the caller then takes another one).
@@ -525,16 +562,20 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
                                const uint8_t* zp, __half* out, const __half* bias, unsigned flags,
                                const GatherTable* gt, const GemmGroup* grp) {
   const int group_k = kGroupSteps * 64;
-  if (!colwise || block < 64 || M < 1 || M > 8 || K % group_k != 0 || K / group_k < kWarps ||
+  const bool tail = K % group_k != 0 || K / group_k < kWarps;
+  if (!colwise || block < 64 || M < 1 || M > 8 || K % 64 != 0 || (tail && (gt || grp)) ||
       reinterpret_cast<uintptr_t>(scales) % 16 != 0 || (zp && reinterpret_cast<uintptr_t>(zp) % 16 != 0) ||
       (size_t)K * N / 2 >= ((size_t)1 << 40))
     return kStreamUnsupported;
+  // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
+  // (the measurements are beside ZP)
+  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || (block == 64 && K < 8192) ? Zp::kPerStep : Zp::kOwnSums;
   // Two CTAs per SM (this launch's and the next one's) share 227 KB; prefer four groups in flight per warp.
   constexpr size_t kHalfSm = (size_t)(227 * 1024) / 2 - 1024, kWholeSm = (size_t)227 * 1024;
   int D = 4;
-  size_t smem = stream_smem_bytes(M, K, zp != nullptr, 4);
+  size_t smem = stream_smem_bytes(M, K, zp_as, 4);
   if (smem > kHalfSm) {
-    const size_t smem2 = stream_smem_bytes(M, K, zp != nullptr, 2);
+    const size_t smem2 = stream_smem_bytes(M, K, zp_as, 2);
     if (smem2 <= kHalfSm) { D = 2; smem = smem2; }
     else if (smem > kWholeSm) {
       if (smem2 > kWholeSm) return kStreamUnsupported;
@@ -564,21 +605,32 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
   }
   const bool early = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) != 0;
   const bool small_m = M <= 2;
-  auto launch = [&](auto has_zp, auto shift, auto gather, auto group) {
-    constexpr bool Z = decltype(has_zp)::value, GA = decltype(gather)::value, GR = decltype(group)::value;
-    constexpr int BS = decltype(shift)::value;
-    if (D == 4) return small_m ? launch_T<Z, 4, 2, BS, GA, GR>(p, smem, grid, stream, early) : launch_T<Z, 4, 8, BS, GA, GR>(p, smem, grid, stream, early);
-    return small_m ? launch_T<Z, 2, 2, BS, GA, GR>(p, smem, grid, stream, early) : launch_T<Z, 2, 8, BS, GA, GR>(p, smem, grid, stream, early);
+  auto launch = [&](auto zp_kind, auto rows, auto shift, auto gather, auto group, auto short_group) {
+    constexpr Zp Z = decltype(zp_kind)::value;
+    constexpr int MZ = decltype(rows)::value, BS = decltype(shift)::value;
+    constexpr bool GA = decltype(gather)::value, GR = decltype(group)::value, T = decltype(short_group)::value;
+    return D == 4 ? launch_T<Z, 4, MZ, BS, GA, GR, T>(p, smem, grid, stream, early) : launch_T<Z, 2, MZ, BS, GA, GR, T>(p, smem, grid, stream, early);
   };
-  auto with_block = [&](auto gather, auto group) {
-    const std::integral_constant<int, 0> b64{};
-    const std::integral_constant<int, 1> b128{};
-    if (zp) return block == 64 ? launch(std::true_type{}, b64, gather, group) : launch(std::true_type{}, b128, gather, group);
-    return block == 64 ? launch(std::false_type{}, b64, gather, group) : launch(std::false_type{}, b128, gather, group);
+  auto with_kinds = [&](auto shift, auto gather, auto group, auto short_group) {
+    const std::integral_constant<int, 2> two{};
+    const std::integral_constant<int, 8> eight{};
+    const std::integral_constant<Zp, Zp::kNone> none{};
+    const std::integral_constant<Zp, Zp::kPerStep> per_step{};
+    if (!zp) return small_m ? launch(none, two, shift, gather, group, short_group) : launch(none, eight, shift, gather, group, short_group);
+    if (!small_m) return launch(per_step, eight, shift, gather, group, short_group);
+    if constexpr (decltype(short_group)::value) return launch(per_step, two, shift, gather, group, short_group);
+    else if (zp_as == Zp::kPerStep) return launch(per_step, two, shift, gather, group, short_group);
+    else return launch(std::integral_constant<Zp, Zp::kOwnSums>{}, two, shift, gather, group, short_group);
   };
-  if (gt) return with_block(std::true_type{}, std::false_type{});
-  if (grp) return with_block(std::false_type{}, std::true_type{});
-  return with_block(std::false_type{}, std::false_type{});
+  auto with_block = [&](auto gather, auto group, auto short_group) {
+    return block == 64 ? with_kinds(std::integral_constant<int, 0>{}, gather, group, short_group)
+                       : with_kinds(std::integral_constant<int, 1>{}, gather, group, short_group);
+  };
+  const std::true_type yes{};
+  const std::false_type no{};
+  if (gt) return with_block(yes, no, no);
+  if (grp) return with_block(no, yes, no);
+  return tail ? with_block(no, no, yes) : with_block(no, no, no);
 }
 
 }  // namespace blkq4
