@@ -312,13 +312,16 @@ extern "C" int blkq4_last_kernel_status(void* stream_ptr) {
   const int tc = blkq4::read_gemm_tc_error(reinterpret_cast<cudaStream_t>(stream_ptr));
   if (tc != 0) return tc;
   const int gv = blkq4::read_gemv_error();
-  return gv > 0 ? (0x10000 | gv) : gv;
+  if (gv != 0) return gv > 0 ? (0x10000 | gv) : gv;
+  const int sk = blkq4::read_skinny_tc_error();
+  return sk > 0 ? (0x20000 | sk) : sk;
 }
 extern "C" int blkq4_reset(void* stream_ptr) {
   auto stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   int rc = 0;
   rc |= blkq4::clear_gemm_tc_error(stream);
   rc |= blkq4::clear_gemv_error(stream);
+  rc |= blkq4::clear_skinny_tc_error(stream);
   rc |= blkq4::reset_static_scratch(stream);
   return rc == 0 ? 0 : -1;
 }

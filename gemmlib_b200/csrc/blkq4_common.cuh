@@ -44,10 +44,12 @@ bool gemv_stream_takes(int block, bool colwise, int M, int N, int K);
 // True when the environment (BLKQ4_GEMV_NO_STREAM, BLKQ4_GEMV_GENERIC) keeps calls of up to 16 rows off it.
 bool gemv_stream_off();
 
-// The same weight stream for 9 <= M <= 16 (two row groups, two tiles per pass, activations from L2).
-std::string launch_gemv_wide(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
-                             const __half* a, const uint8_t* packed, const __half* scales,
-                             const uint8_t* zp, __half* out, const __half* bias, unsigned flags);
+// Tensor-core kernel of up to 16 rows for column-wise blocks of 64 and 128 (scales and zero points 16-byte aligned).
+// Whether it is faster than the decode kernel for M <= 8.
+bool skinny_tc_is_faster(int M, int N, int K);
+bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* scales, const void* zp);
+std::string launch_skinny_tc(int block, int M, int N, int K, cudaStream_t stream, const __half* a, const uint8_t* packed,
+                             const __half* scales, const uint8_t* zp, __half* out, const __half* bias, unsigned flags);
 
 // Up to four weight matrices of one K, block size and kind of zero points that one launch multiplies with the same
 // activations.  Their tiles (of 16 columns in the decode kernel, of 128 or 256 in the tensor-core kernels) are numbered one
@@ -136,9 +138,11 @@ bool gemm_tc_split_plan_refusable(int M, int N, int K, size_t capacity);
 int read_gemm_tc_error(cudaStream_t stream);
 // The skinny kernel's device error word (call after the stream has been synchronised).
 int read_gemv_error();
+int read_skinny_tc_error();
 // Recovery after an expired wait: clear the kernels' error words / the static scratch's flag words.
 int clear_gemm_tc_error(cudaStream_t stream);
 int clear_gemv_error(cudaStream_t stream);
+int clear_skinny_tc_error(cudaStream_t stream);
 int reset_static_scratch(cudaStream_t stream);
 
 #ifdef __CUDACC__

@@ -1,7 +1,7 @@
 // Skinny W4A16 kernels (M <= 16) for sm_100a: out[M,N] = A[M,K] x dequant(W4[K,N]).
-// This file holds the dispatch (launch_gemv: decode kernel -> wide kernel, both in files of their
-// own, -> the TMA kernel and the generic kernel below) and the two kernels that take every shape
-// the first two refuse.
+// This file holds the dispatch (launch_gemv: decode kernel -> skinny tensor-core kernel, both in files of their
+// own, -> the TMA kernel and the generic kernel below) and the two kernels that take what the first two refuse: the fused
+// exchange of shapes off the decode kernel, other blockings, meta that is not 16-byte aligned.
 //
 // This regime is bound by HBM bandwidth: every packed weight byte is read once
 // and used for at most 16 outputs, so the kernel is organised around the weight
@@ -807,11 +807,15 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
   if (env_warps >= 1 && env_warps <= kMaxWarps) warps = env_warps;
   const int u = env_u ? env_u : 4;
   cudaError_t e;
-  // Decode shapes first: the cp.async stream kernel (blkq4_gemv_stream.cu).
+  // Decode shapes first: the cp.async stream kernel (blkq4_gemv_stream.cu); then the skinny tensor-core kernel (blkq4_skinny_tc.cu),
+  // which has the rest of the column-wise blocks of 64 and 128.
   if (!gemv_stream_off()) {
-    const std::string r = M <= 8 ? launch_gemv_stream(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags)
-                                 : launch_gemv_wide(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
+    const bool tc = skinny_tc_takes(block, colwise, M, N, K, scales, zp);
+    const std::string r = M <= 8 && !(tc && skinny_tc_is_faster(M, N, K))
+                              ? launch_gemv_stream(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags)
+                              : std::string(kStreamUnsupported);
     if (r != kStreamUnsupported) return r;
+    if (tc) return launch_skinny_tc(block, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
   }
   // Fast path: one scale per 64-k step; at least one 512-k unit (the last one may be partial), meta
   // rows and pointers 16-byte aligned (TMA), shared memory for the per-step terms within reach.

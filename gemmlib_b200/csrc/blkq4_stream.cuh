@@ -1,4 +1,4 @@
-// Device helpers shared by the cp.async stream kernels (blkq4_gemv_stream.cu, blkq4_gemv_wide.cu).
+// Device helpers of the decode kernel (blkq4_gemv_stream.cu).
 #pragma once
 
 #include <cuda_fp16.h>

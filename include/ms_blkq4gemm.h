@@ -329,7 +329,8 @@ void blkq4_errmsg_destroy(void* errmsg);      /* delete                         
  * Synchronises `stream` and returns the device-side status word of the kernels: 0 when
  * every in-kernel wait completed.  Waits on mbarriers are bounded; one that expires makes
  * the CTA drain and records (role << 8 | barrier) here instead of hanging the GPU (the
- * skinny kernel's word is reported with bit 16 set).  -1 if the stream itself is in error.
+ * skinny kernel's word is reported with bit 16 set, that of the tensor-core kernel of up to 16 rows
+ * with bit 17).  -1 if the stream itself is in error.
  * No counterpart in the reference, whose kernels have no such waits.
  */
 int blkq4_last_kernel_status(void* stream);
