@@ -72,7 +72,9 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 
 // Shared memory: rings [kWarps][D][kSlotBytes] | s_corr [steps][4] float4 | s_asum [steps][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
-// MZ: rows whose activations are staged at a time: one after the other for M <= 2 (2), else all together (8).
+// MZ: rows whose activations are staged at a time: one after the other (2), or all together (8), which saves a round trip to L2 per
+// row but runs a longer code.  Two rows one after the other / together, us, symmetric blocks of 64: 512 x 512 1.9 / 1.7, 1024 x 4096
+// 2.5 / 2.4, 2048 x 2048 2.7 / 2.5, 4096 x 4096 4.6 / 4.6, 8192 x 28672 26.0 / 26.8, 11008 x 4096 8.7 / 9.8: together below 8192 k.
 //
 // GATHER (N-sharded layer, one process per GPU).  The exchange is latency-bound (a few tens of KB per
 // rank), so it carries its own flags: the adding warp stores the tile's results into EVERY rank's
@@ -92,8 +94,8 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 //
 // ZP: kPerStep subtracts zp * sum_k a_k from a step's sum before it is scaled, four FMAs and three loads a step.  kOwnSums keeps
 // accumulators of their own for these terms, two FMAs and three loads for two steps, but a shuffle, an addition and a store per row
-// and 16 more terms per output at the tile's end.  kPerStep is taken for three rows and more, and for one or two where tiles are
-// short.  Measured on B200, kOwnSums / kPerStep, us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008
+// and 16 more terms per output at the tile's end.  kPerStep is taken for three rows and more, and below 8192 k for two, and for one
+// with blocks of 64.  Measured on B200, kOwnSums / kPerStep, us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008
 // 13.5 / 10.8, 8192 x 28672 43.0 / 37.9; M = 4: 3.2 / 2.9, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 33.9; M = 1: 512 x 11008 4.3 / 3.5, 4096 x 4096
 // 4.4 / 4.2, 4096 x 11008 8.5 / 7.9, 11008 x 4096 8.5 / 8.4, 8192 x 28672 27.3 / 28.7; block 128 4.2 / 4.2, 8.0 / 8.2, 8.0 / 8.4, 26.0 / 27.3.
 // (As part of the accumulator's initial value, which is a thousand times larger than the sum, the term would be rounded there:
@@ -569,7 +571,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
     return kStreamUnsupported;
   // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
   // (the measurements are beside ZP)
-  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || (block == 64 && K < 8192) ? Zp::kPerStep : Zp::kOwnSums;
+  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || (K < 8192 && (block == 64 || M == 2)) ? Zp::kPerStep : Zp::kOwnSums;
   // Two CTAs per SM (this launch's and the next one's) share 227 KB; prefer four groups in flight per warp.
   constexpr size_t kHalfSm = (size_t)(227 * 1024) / 2 - 1024, kWholeSm = (size_t)227 * 1024;
   int D = 4;
@@ -604,7 +606,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
     if (eff2 >= 0.85) grid = p.tiles < 2 * sms ? p.tiles : 2 * sms;
   }
   const bool early = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) != 0;
-  const bool small_m = M <= 2;
+  const bool small_m = M == 1 || (M == 2 && K >= 8192);
   auto launch = [&](auto zp_kind, auto rows, auto shift, auto gather, auto group, auto short_group) {
     constexpr Zp Z = decltype(zp_kind)::value;
     constexpr int MZ = decltype(rows)::value, BS = decltype(shift)::value;
