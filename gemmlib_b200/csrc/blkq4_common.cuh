@@ -29,8 +29,8 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
                         const __half* a, const uint8_t* packed, const __half* scales,
                         const uint8_t* zp, __half* out, const __half* bias, unsigned flags);
 
-// The decode kernel (M <= 8, column-wise blocks >= 64; groups of matrices and the fused exchange only with K a multiple of 256 and
-// >= 2048): per-warp cp.async rings, two launches resident per SM.  Returns kStreamUnsupported for other shapes.
+// The decode kernel (M <= 8, column-wise blocks; groups of matrices and the fused exchange only with blocks of 64 and 128, K a multiple
+// of 256 and >= 2048): per-warp cp.async rings, two launches resident per SM.  Returns kStreamUnsupported for other shapes.
 extern const char* const kStreamUnsupported;
 struct GatherTable;
 struct GemmGroup;

@@ -1,4 +1,4 @@
-// Decode kernel (M <= 8) for column-wise blocks of 64 or 128: out[M,N] = A[M,K] x dequant(W4[K,N]).
+// Decode kernel (M <= 8) for column-wise blocks: out[M,N] = A[M,K] x dequant(W4[K,N]).
 //
 // The weight stream is the only large operand, so the kernel is organised around it.
 //
@@ -53,6 +53,13 @@ constexpr int kCorrStep = 4 * 16;    // bytes of mma-initialising terms per step
 // Zero points: none; with sums of their own (up to two rows); subtracted from every step's sum.
 enum class Zp { kNone, kOwnSums, kPerStep };
 
+// Quantization blocks as a shift: 2^BS steps of 64 k (blocks of 64 and 128), or 2^-BS blocks in a step (of 32 and 16).
+__host__ __device__ constexpr int blocks_per_step(int bs) { return bs < 0 ? 1 << -bs : 1; }
+// A ring slot: four steps of weights, a row of 16 scales and one of 16 zero points per block (blocks of 128: per step).
+__host__ __device__ constexpr int slot_bytes(int bs) { return kSlotW + kGroupSteps * blocks_per_step(bs) * 48; }
+// Halves between the staged activation rows: 16-byte reads of neighbouring rows fall on different banks.
+__host__ __device__ constexpr int a_padding(int bs) { return bs < 0 ? 32 : 8; }
+
 struct StreamParams {
   const __half* a;
   __half* out;
@@ -70,7 +77,7 @@ struct StreamParams {
 
 constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 
-// Shared memory: rings [kWarps][D][kSlotBytes] | s_corr [steps][4] float4 | s_asum [steps][8] (zero points)
+// Shared memory: rings [kWarps][D][slot_bytes] | s_corr [blocks of K, or steps][4] float4 | s_asum [the same][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
 // MZ: rows whose activations are staged at a time: one after the other (2), or all together (8), which saves a round trip to L2 per
 // row but runs a longer code.  Two rows one after the other / together, us, symmetric blocks of 64: 512 x 512 1.9 / 1.7, 1024 x 4096
@@ -109,6 +116,10 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 // 3200 x 28672 18.7, 20.1, 23.4 / 12.4, 14.0, 15.4.  Slices balanced to the step, every warp's last group short, were 2 to 9 % slower up
 // to 1024 k and equal above: the steps of a short group run one by one.
 //
+// BS < 0: blocks of 32 and 16, a row of scales and zero points, an activation-only term and a sum per block.  An mma adds up over the
+// four lanes of a column, so the lanes share a block's 16-byte chunks: 8 bytes each for blocks of 32, 4 for blocks of 16.  The
+// activations are staged in that order, 16 bytes a lane and 32 k, and the chunks lie in the slot so that the reads hit all banks.
+//
 // BS: steps of a quantization block, as a shift (0: blocks of 64, 1: of 128).  The two steps of a 128-k block share scale and
 // zero point: one load and conversion of them, two accumulators with independent mma chains, one scaling of their sum.
 // (One chain of eight mma from the sum of both activation-only terms is faster still, but the larger partial sums cost
@@ -121,11 +132,13 @@ gemv_stream_kernel(const StreamParams p) {
   constexpr int W = kWarps, GS = kGroupSteps;
   constexpr bool HAS_ZP = ZP != Zp::kNone, ZFOLD = ZP == Zp::kPerStep, ZSEP = ZP == Zp::kOwnSums;
   constexpr int PW = ZSEP ? 2 * W : W;  // partial-sum entries per tile: the warps (+ their zero-point terms)
+  constexpr int NB = blocks_per_step(BS), kSlotBytes = slot_bytes(BS);
+  constexpr int kSlotS = GS * NB * 32;      // scales of a slot: rows of 16 fp16; the zero points, rows of 16 bytes, follow
   const int MS = (p.M + 1) & ~1;
   uint8_t* s_ring = s_raw;
   float* s_corr = reinterpret_cast<float*>(s_ring + W * D * kSlotBytes);
-  float* s_asum = s_corr + (size_t)p.steps * 16;
-  float* s_part = s_asum + (HAS_ZP ? (size_t)p.steps * 8 : 0);
+  float* s_asum = s_corr + (size_t)p.steps * NB * 16;
+  float* s_part = s_asum + (HAS_ZP ? (size_t)p.steps * NB * 8 : 0);
   __half* s_stage = reinterpret_cast<__half*>(s_part + (size_t)2 * PW * 16 * MS);
   __half* s_a = s_stage + 128;
 
@@ -133,7 +146,6 @@ gemv_stream_kernel(const StreamParams p) {
   const int g = lane >> 2, t = lane & 3;
   const int K = p.K, M = p.M;
   int N = p.N;  // GROUP: of the tile that is being loaded
-  constexpr int bs = BS;
   const int kgroups = (p.steps + GS - 1) / GS;
   // >= 1 without TAIL: the launcher requires kgroups >= W.  Fewer groups than warps go to the first ones, one each (the formula
   // would give them to every second warp, which share two of the SM's four schedulers).
@@ -151,26 +163,41 @@ gemv_stream_kernel(const StreamParams p) {
 
   // ---- loader: runs D groups ahead of the consumer; all addresses advance incrementally ----
   const long long w_tile_adj = (long long)gridDim.x * 8 * K - (long long)myg * (GS * 64);
-  // lanes 0-7 copy the scales of step lane / 2, column half lane % 2; lanes 8-11 the zero points of step lane - 8
-  const uint32_t meta_lane = (lane < 2 * GS || (HAS_ZP && lane < 3 * GS)) ? 1u : 0u;
-  const uint32_t m_dst = lane < 2 * GS ? kSlotW + (lane >> 1) * 32 + (lane & 1) * 16 : kSlotW + kSlotS + (lane - 2 * GS) % GS * 16;
-  const int meta_step = lane < 2 * GS ? lane >> 1 : (lane - 2 * GS) % GS;  // step whose scales / zero points this lane copies
-  const uint8_t *wp, *mp;
+  // The first 2 R lanes copy the scales of row lane / 2 (blocks of 64: of a step), column half lane % 2, the next R the zero points
+  // of row lane - 2 R; with blocks of 16 (R = 16) the zero points take a copy of their own by lanes 0 to 15.
+  constexpr int R = GS * NB;
+  constexpr bool kZpApart = 3 * R > 32;
+  const int zp_row = BS >= 0 ? (lane - 2 * GS) % GS : lane % R;  // (2 R is a multiple of R)
+  const uint32_t meta_lane = (lane < 2 * R || (HAS_ZP && lane < 3 * R)) ? 1u : 0u;
+  const uint32_t z_dst = kSlotW + kSlotS + zp_row * 16;
+  const uint32_t m_dst = lane < 2 * R ? kSlotW + (lane >> 1) * 32 + (lane & 1) * 16 : z_dst;
+  const int meta_step = lane < 2 * R ? (lane >> 1) / NB : zp_row / NB;  // step whose scales / zero points this lane copies
+  // A weight chunk's place in the slot: chunk t of packed column g at 4 g + t, in another order where lanes read 8 or 4 of its
+  // 16 bytes (blocks of 32 and 16), so that they fall on different banks.
+  const int chunk_xor = BS == -1 ? (g & 2) : BS == -2 ? (g >> 1) & 3 : 0;
+  const uint32_t w_dst = (uint32_t)(BS >= 0 ? lane : 4 * g + (t ^ chunk_xor)) * 16u;
+  const uint8_t *wp, *mp, *zq = nullptr;  // zq: kZpApart
+  long long z_step = 0, z_tile_adj = 0;
   long long m_step, m_tile_adj;
   // this lane's addresses for the warp's first group of a tile
   auto point_at = [&](const uint8_t* packed, const __half* scales, const uint8_t* zp, int tile) {
-    const int rows_per_group = GS >> bs;
     wp = packed + (size_t)(tile * 8 + g) * K + (size_t)gb * (GS * 64) + t * 16;
-    if (lane < 2 * GS) {
-      const int u = lane >> 1, h = lane & 1;
-      mp = reinterpret_cast<const uint8_t*>(scales) + ((size_t)((gb * GS + u) >> bs) * N + tile * 16 + h * 8) * 2;
+    constexpr int rows_per_group = BS > 0 ? GS >> BS : R;
+    auto row_of = [&](int r) { return BS > 0 ? (gb * GS + r) >> BS : gb * R + r; };  // r: of the slot; blocks of 128 have theirs twice
+    if (lane < 2 * R) {
+      const int r = lane >> 1, h = lane & 1;
+      mp = reinterpret_cast<const uint8_t*>(scales) + ((size_t)row_of(r) * N + tile * 16 + h * 8) * 2;
       m_step = (long long)rows_per_group * N * 2;
       m_tile_adj = (long long)gridDim.x * 32 - (long long)myg * m_step;
     } else {
-      const int u = (lane - 2 * GS) % GS;
-      mp = (HAS_ZP ? zp : packed) + (size_t)((gb * GS + u) >> bs) * N + tile * 16;  // only used with zero points
+      mp = (HAS_ZP ? zp : packed) + (size_t)row_of(zp_row) * N + tile * 16;  // only used with zero points
       m_step = (long long)rows_per_group * N;
       m_tile_adj = (long long)gridDim.x * 16 - (long long)myg * m_step;
+    }
+    if (HAS_ZP && kZpApart) {
+      zq = zp + (size_t)row_of(zp_row) * N + tile * 16;
+      z_step = (long long)rows_per_group * N;
+      z_tile_adj = (long long)gridDim.x * 16 - (long long)myg * z_step;
     }
   };
   int ld_tile = blockIdx.x;
@@ -184,7 +211,7 @@ gemv_stream_kernel(const StreamParams p) {
   int ld_left = my_tiles * myg, ld_j = 0;
   auto issue_group = [&](uint32_t dst) {
     const uint32_t go = ld_left > 0 ? 1u : 0u;
-    const uint32_t dw = dst + lane * 16;
+    const uint32_t dw = dst + w_dst;
     if constexpr (TAIL) {
       // steps past the end of K are neither copied nor computed
       const int n = go ? (ld_j + 1 == myg ? last_steps : GS) : 0;
@@ -193,12 +220,14 @@ gemv_stream_kernel(const StreamParams p) {
       cp_async16_if<128>(dw, wp, n > 2);
       cp_async16_if<192>(dw, wp, n > 3);
       cp_async16_if<0>(dst + m_dst, mp, meta_lane && meta_step < n);
+      if (HAS_ZP && kZpApart) cp_async16_if<0>(dst + z_dst, zq, lane < R && zp_row / NB < n);
     } else {
       cp_async16_if<0>(dw, wp, go);
       cp_async16_if<64>(dw, wp, go);
       cp_async16_if<128>(dw, wp, go);
       cp_async16_if<192>(dw, wp, go);
       cp_async16_if<0>(dst + m_dst, mp, go & meta_lane);
+      static_assert(!kZpApart, "blocks of 16: TAIL");
     }
     cp_async_commit();  // always: the group count per iteration stays fixed
     --ld_left;
@@ -218,6 +247,7 @@ gemv_stream_kernel(const StreamParams p) {
     } else {
       wp += (GS * 64) + (wrap ? w_tile_adj : 0);
       mp += m_step + (wrap ? m_tile_adj : 0);
+      if (HAS_ZP && kZpApart) zq += z_step + (wrap ? z_tile_adj : 0);
       if (wrap) ld_j = 0;
     }
   };
@@ -256,7 +286,23 @@ gemv_stream_kernel(const StreamParams p) {
       return __ldg(reinterpret_cast<const uint4*>(p.a + (size_t)m * K + k0));
     };
     auto finish_row = [&](int m, int k0, const uint4& v) {
-      if (!TAIL || k0 < K) *reinterpret_cast<uint4*>(s_a + (size_t)m * p.a_pitch + k0) = v;
+      if (!TAIL || k0 < K) {
+        if constexpr (BS >= 0) {
+          *reinterpret_cast<uint4*>(s_a + (size_t)m * p.a_pitch + k0) = v;
+        } else {
+          // per 32 k, lane t's 16 bytes: of its chunk the k of its two words (blocks of 32: k, then k + 8), or of both chunks
+          // those of its word (blocks of 16)
+          uint8_t* d = reinterpret_cast<uint8_t*>(s_a + (size_t)m * p.a_pitch + (k0 & ~31));
+          const int cb = (k0 >> 4) & 1, hi = (k0 >> 3) & 1;
+          if constexpr (BS == -1) {
+            *reinterpret_cast<uint2*>(d + 32 * cb + 8 * hi) = make_uint2(v.x, v.y);
+            *reinterpret_cast<uint2*>(d + 32 * cb + 16 + 8 * hi) = make_uint2(v.z, v.w);
+          } else {
+            uint32_t* q = reinterpret_cast<uint32_t*>(d + 8 * cb + 4 * hi);
+            q[0] = v.x; q[4] = v.y; q[8] = v.z; q[12] = v.w;
+          }
+        }
+      }
       const __half2* h = reinterpret_cast<const __half2*>(&v);
       float s = 0.0f;
 #pragma unroll
@@ -264,13 +310,13 @@ gemv_stream_kernel(const StreamParams p) {
         const float2 f = __half22float2(h[e]);
         s += f.x + f.y;
       }
-      // the eight lanes of a step: sum the four chunks of equal parity, then pair lo with hi
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      // the lanes of a block (eight of a step, for blocks of 64): sum the chunks of equal parity, then pair lo with hi
+      if (BS >= -1) s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (BS >= 0) s += __shfl_xor_sync(0xffffffffu, s, 4);
       const float other = __shfl_xor_sync(0xffffffffu, s, 1);
-      if ((lane & 7) == 0 && (!TAIL || k0 < K)) {
+      if ((lane & (8 / NB - 1)) == 0 && (!TAIL || k0 < K)) {
         const float lo = s, hi = other;
-        const int step = k0 >> 6;
+        const int step = k0 >> (BS < 0 ? 6 + BS : 6);  // a block where a step holds several
         // one float4 per row pair (m even, m odd, m even, m odd): the accumulator rows n and n + 8 start alike
         float* dst = s_corr + ((size_t)step * 4 + (m >> 1)) * 4 + (m & 1);
         const float nb = -(1024.0f * lo + 64.0f * hi);
@@ -305,12 +351,19 @@ gemv_stream_kernel(const StreamParams p) {
   constexpr uint32_t kLoMask = 0x000f000fu, kHiMask = 0x00f000f0u;
   constexpr uint32_t kLoMagic = 0x64006400u, kHiMagic = 0x54005400u;
   // rows >= M of the activation operand repeat row M - 1; their outputs are never stored
-  const uint32_t a_base = smem_u32(s_a) + (uint32_t)(min(g, M - 1) * p.a_pitch + gb * (GS * 64) + t * 16) * 2u;
-  const uint32_t c_base = smem_u32(s_corr) + (uint32_t)(gb * GS) * kCorrStep + (uint32_t)t * 16u;
-  const uint32_t asum_base = smem_u32(s_asum) + (uint32_t)(gb * GS) * 32u;
+  const uint32_t a_base = smem_u32(s_a) + (uint32_t)(min(g, M - 1) * p.a_pitch + gb * (GS * 64) + t * (BS < 0 ? 8 : 16)) * 2u;
+  const uint32_t c_base = smem_u32(s_corr) + (uint32_t)(gb * R) * kCorrStep + (uint32_t)t * 16u;
+  const uint32_t asum_base = smem_u32(s_asum) + (uint32_t)(gb * R) * 32u;
 
   float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   float ztot[2] = {0.0f, 0.0f};  // ZSEP: zero-point terms of column (lane & 15), rows m, over the steps of half (lane >> 4)
+
+  // where in a slot this lane's weights of a step's blocks lie (BS < 0)
+  uint32_t w_at[NB];
+#pragma unroll
+  for (int b = 0; BS < 0 && b < NB; ++b)
+    w_at[b] = BS == -1 ? (uint32_t)((4 * g + ((2 * b + (t >> 1)) ^ chunk_xor)) * 16 + (t & 1) * 8)
+                       : (uint32_t)((4 * g + (b ^ chunk_xor)) * 16 + t * 4);
 
   uint32_t src = ring_addr;
   for (int tl = 0; tl < my_tiles; ++tl) {
@@ -397,7 +450,51 @@ gemv_stream_kernel(const StreamParams p) {
         if (ZFOLD) BLKQ4_STREAM_ZP(U, sum, add_f2(lds_f2<(U) * 32>(as_t), lds_f2<(V) * 32>(as_t))) \
         BLKQ4_STREAM_SCALE(U, sum[0], sum[1], sum[2], sum[3])                                   \
       }
-      if constexpr (BS == 1) {
+/* Blocks of 32: block J of step U; 8 bytes of weights, two words, per lane. */
+#define BLKQ4_STREAM_BLOCK32(U, J)                                                              \
+      {                                                                                         \
+        const uint2 w = lds_v2<(U) * 512>(src + w_at[J]);                                       \
+        const uint4 v = lds_v4<(U) * 128 + (J) * 64>(a_addr);                                   \
+        const uint32_t y0 = w.x >> 8, y1 = w.y >> 8;                                            \
+        float acc[4];                                                                           \
+        const float4 c = lds_f4<((U) * NB + (J)) * kCorrStep>(c_addr);                          \
+        mma_init(acc, lop3_and_or(w.x, kLoMask, kLoMagic), lop3_and_or(y0, kLoMask, kLoMagic),  \
+                 lop3_and_or(w.y, kLoMask, kLoMagic), lop3_and_or(y1, kLoMask, kLoMagic), v.x, v.y, c); \
+        mma_acc(acc, lop3_and_or(w.x, kHiMask, kHiMagic), lop3_and_or(y0, kHiMask, kHiMagic),   \
+                lop3_and_or(w.y, kHiMask, kHiMagic), lop3_and_or(y1, kHiMask, kHiMagic), v.z, v.w); \
+        if (ZFOLD) BLKQ4_STREAM_ZP((U) * NB + (J), acc, lds_f2<((U) * NB + (J)) * 32>(as_t))    \
+        BLKQ4_STREAM_SCALE((U) * NB + (J), acc[0], acc[1], acc[2], acc[3])                      \
+      }
+/* Blocks of 16: block C of step U; one word per lane.  V: activations of its block pair. */
+#define BLKQ4_STREAM_BLOCK16(U, C, V0, V1)                                                      \
+      {                                                                                         \
+        const uint32_t x = lds_u32<(U) * 512>(src + w_at[C]), y = x >> 8;                       \
+        float acc[4];                                                                           \
+        const float4 c = lds_f4<((U) * NB + (C)) * kCorrStep>(c_addr);                          \
+        mma_init(acc, lop3_and_or(x, kLoMask, kLoMagic), lop3_and_or(y, kLoMask, kLoMagic),     \
+                 lop3_and_or(x, kHiMask, kHiMagic), lop3_and_or(y, kHiMask, kHiMagic), V0, V1, c); \
+        if (ZFOLD) BLKQ4_STREAM_ZP((U) * NB + (C), acc, lds_f2<((U) * NB + (C)) * 32>(as_t))    \
+        BLKQ4_STREAM_SCALE((U) * NB + (C), acc[0], acc[1], acc[2], acc[3])                      \
+      }
+#define BLKQ4_STREAM_SMALL(U)                                                                   \
+      {                                                                                         \
+        if constexpr (BS == -1) {                                                               \
+          BLKQ4_STREAM_BLOCK32(U, 0)                                                            \
+          BLKQ4_STREAM_BLOCK32(U, 1)                                                            \
+        } else {                                                                                \
+          const uint4 p0 = lds_v4<(U) * 128>(a_addr), p1 = lds_v4<(U) * 128 + 64>(a_addr);      \
+          BLKQ4_STREAM_BLOCK16(U, 0, p0.x, p0.y)                                                \
+          BLKQ4_STREAM_BLOCK16(U, 1, p0.z, p0.w)                                                \
+          BLKQ4_STREAM_BLOCK16(U, 2, p1.x, p1.y)                                                \
+          BLKQ4_STREAM_BLOCK16(U, 3, p1.z, p1.w)                                                \
+        }                                                                                       \
+      }
+      if constexpr (BS < 0) {
+        BLKQ4_STREAM_SMALL(0)
+        if (n_steps > 1) BLKQ4_STREAM_SMALL(1)
+        if (n_steps > 2) BLKQ4_STREAM_SMALL(2)
+        if (n_steps > 3) BLKQ4_STREAM_SMALL(3)
+      } else if constexpr (BS == 1) {
         BLKQ4_STREAM_BLOCK128(0, 1)
         if (n_steps > 2) BLKQ4_STREAM_BLOCK128(2, 3)  // K is a whole number of blocks
       } else if (n_steps == GS) {
@@ -410,6 +507,9 @@ gemv_stream_kernel(const StreamParams p) {
         if (n_steps > 1) BLKQ4_STREAM_STEP(1)
         if (n_steps > 2) BLKQ4_STREAM_STEP(2)
       }
+#undef BLKQ4_STREAM_SMALL
+#undef BLKQ4_STREAM_BLOCK16
+#undef BLKQ4_STREAM_BLOCK32
 #undef BLKQ4_STREAM_BLOCK128
 #undef BLKQ4_STREAM_STEP
 #undef BLKQ4_STREAM_SCALE
@@ -419,8 +519,8 @@ gemv_stream_kernel(const StreamParams p) {
       issue_group(src);  // refill the slot just consumed
       src = (src == ring_last) ? ring_addr : src + kSlotBytes;
       a_addr += GS * 128;
-      c_addr += GS * kCorrStep;
-      as_addr += GS * 32;
+      c_addr += R * kCorrStep;
+      as_addr += R * 32;
     }
     // ---- tile end: double-buffered partial sums, one CTA barrier, one warp (rotating) adds them up.
     //      The adder of tile tl reaches the barrier of tile tl + 1 only after it has read the buffer,
@@ -540,22 +640,42 @@ std::string launch_T(const StreamParams& p, size_t smem, int grid, cudaStream_t 
   return std::string();
 }
 
-size_t stream_smem_bytes(int M, int K, Zp zp, int D) {
+size_t stream_smem_bytes(int M, int K, Zp zp, int D, int bs) {
   const int MS = (M + 1) & ~1, PW = zp == Zp::kOwnSums ? 2 * kWarps : kWarps, steps = K / 64;
-  return (size_t)kWarps * D * kSlotBytes + (size_t)steps * 64 + (zp != Zp::kNone ? (size_t)steps * 32 : 0) +
-         (size_t)2 * PW * 16 * MS * 4 + 256 + (size_t)M * (K + 8) * 2;
+  const size_t blocks = (size_t)steps * blocks_per_step(bs);
+  return (size_t)kWarps * D * slot_bytes(bs) + blocks * 64 + (zp != Zp::kNone ? blocks * 32 : 0) + (size_t)2 * PW * 16 * MS * 4 + 256 +
+         (size_t)M * (K + a_padding(bs)) * 2;
 }
 
 }  // namespace
 
 
 
+namespace {
+// Blocks of 32 and 16, against the generic kernel (which scales in fp16; larger problems than these are the tensor-core kernel's, see
+// gemm_tc_takes_skinny).  Every block has a sum to be scaled, with zero points a subtraction too, per eight rows, which the generic
+// kernel's conversion has not: more rows and smaller blocks are its side.  Measured on B200, generic / this, us, M = 1, 2, 4, 8:
+//   block 32, symmetric:   512 x 512 3.1 / 1.7, 1.8, 2.1, 2.7;  1024 x 4096 3.8 / 2.3, 2.5, 2.8, 3.4;  2048 x 2048 3.9 / 2.5, 2.6, 3.0, 3.6;
+//                          2048 x 8192 7.9 / 4.3, 4.6, 5.0, 6.1;  4096 x 4096 7.0 / 4.4, 5.0, 5.9, 7.1;  5632 x 2048 7.9 / 4.5, 5.0, 6.7, 7.2
+//   with zero points:      1024 x 4096 3.8 / 2.5, 2.7, 3.0, 3.6;  1984 x 3008 5.7 / 3.1, 3.3, 3.7, 4.5;  2048 x 2048 4.0 / 2.8, 3.0, 3.6, 4.4;
+//                          4096 x 4096 7.1 / 5.1, 5.6, 6.6, 7.9
+//   block 16, symmetric:   1024 x 4096 3.8 / 2.5, 2.7, 3.1, 3.8;  2048 x 2048 3.9 / 3.0, 3.0, 4.0, 5.4;  4096 x 4096 7.2 / 5.4, 6.2, 7.5, 8.5
+//   with zero points:      1024 x 4096 4.0 / 2.8, 3.0, 3.5, 4.3;  2048 x 2048 4.1 / 3.6, 3.9, 4.8, 6.4;  4096 x 4096 7.9 / 6.6, 7.4, 8.9, 10.0;
+//                          M = 2: 576 x 14720 5.8 / 6.1, 3200 x 3200 to 6656 1.15 of the generic kernel's time
+// Below 512 k or columns nothing was measured: they stay on the generic kernel.
+bool small_blocks_are_faster(int block, int M, int N, int K, bool has_zp) {
+  if (K < 512 || N < 512) return false;
+  if (block == 32) return M <= 4 || !has_zp || K < 2048;
+  return has_zp ? M == 1 || (M <= 4 && K < 2048 && N <= 8192) : M <= 2 || (M <= 4 && K < 2048);
+}
+}  // namespace
+
 const char* const kStreamUnsupported = "unsupported by the stream kernel";
 
 bool gemv_stream_takes(int block, bool colwise, int M, int N, int K) {
   const int group_k = kGroupSteps * 64;
   return colwise && block >= 64 && M >= 1 && M <= 8 && K % group_k == 0 && K / group_k >= kWarps &&
-         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, Zp::kOwnSums, 2) <= (size_t)227 * 1024;  // whatever the zero points: part of the interface
+         (size_t)K * N / 2 < ((size_t)1 << 40) && stream_smem_bytes(M, K, Zp::kOwnSums, 2, 0) <= (size_t)227 * 1024;  // whatever the zero points: part of the interface
 }
 
 // Returns kStreamUnsupported when the shape is outside this kernel (the caller then takes another one).
@@ -565,19 +685,21 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
                                const GatherTable* gt, const GemmGroup* grp) {
   const int group_k = kGroupSteps * 64;
   const bool tail = K % group_k != 0 || K / group_k < kWarps;
-  if (!colwise || block < 64 || M < 1 || M > 8 || K % 64 != 0 || (tail && (gt || grp)) ||
+  const int bs = block == 128 ? 1 : block == 64 ? 0 : block == 32 ? -1 : -2;
+  if (bs < 0 && (gt || grp || !small_blocks_are_faster(block, M, N, K, zp != nullptr))) return kStreamUnsupported;
+  if (!colwise || M < 1 || M > 8 || K % 64 != 0 || (tail && (gt || grp)) ||
       reinterpret_cast<uintptr_t>(scales) % 16 != 0 || (zp && reinterpret_cast<uintptr_t>(zp) % 16 != 0) ||
       (size_t)K * N / 2 >= ((size_t)1 << 40))
     return kStreamUnsupported;
   // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
   // (the measurements are beside ZP)
-  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || (K < 8192 && (block == 64 || M == 2)) ? Zp::kPerStep : Zp::kOwnSums;
+  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || bs < 0 || (K < 8192 && (block == 64 || M == 2)) ? Zp::kPerStep : Zp::kOwnSums;
   // Two CTAs per SM (this launch's and the next one's) share 227 KB; prefer four groups in flight per warp.
   constexpr size_t kHalfSm = (size_t)(227 * 1024) / 2 - 1024, kWholeSm = (size_t)227 * 1024;
   int D = 4;
-  size_t smem = stream_smem_bytes(M, K, zp_as, 4);
+  size_t smem = stream_smem_bytes(M, K, zp_as, 4, bs);
   if (smem > kHalfSm) {
-    const size_t smem2 = stream_smem_bytes(M, K, zp_as, 2);
+    const size_t smem2 = stream_smem_bytes(M, K, zp_as, 2, bs);
     if (smem2 <= kHalfSm) { D = 2; smem = smem2; }
     else if (smem > kWholeSm) {
       if (smem2 > kWholeSm) return kStreamUnsupported;
@@ -589,7 +711,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
   p.M = M; p.N = N; p.K = K;
   p.tiles = N / 16;
   p.steps = K / 64;
-  p.a_pitch = K + 8;
+  p.a_pitch = K + a_padding(bs);
   if (gt) p.gt = *gt;
   if (grp) {
     p.grp = *grp;
@@ -624,6 +746,8 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
     else if (zp_as == Zp::kPerStep) return launch(per_step, two, shift, gather, group, short_group);
     else return launch(std::integral_constant<Zp, Zp::kOwnSums>{}, two, shift, gather, group, short_group);
   };
+  if (bs == -1) return with_kinds(std::integral_constant<int, -1>{}, std::false_type{}, std::false_type{}, std::true_type{});
+  if (bs == -2) return with_kinds(std::integral_constant<int, -2>{}, std::false_type{}, std::false_type{}, std::true_type{});
   auto with_block = [&](auto gather, auto group, auto short_group) {
     return block == 64 ? with_kinds(std::integral_constant<int, 0>{}, gather, group, short_group)
                        : with_kinds(std::integral_constant<int, 1>{}, gather, group, short_group);

@@ -418,8 +418,8 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
 // 8192 x 8192 M = 8 0.95, M = 6 1.03; 5632 x 2048 0.87 to 1.00; 4096 x 4096 M = 4 1.22, M = 8 0.99; 8192 x 28672 M = 8 1.18.
 // K that is a multiple of 256 stays there: layers of such K may share a launch of the decode kernel, with the bits of their own calls.
 bool skinny_tc_is_faster(int M, int N, int K) {
-  const int sms = sm_count();
-  return K >= 8192 && K % 256 != 0 && ((M >= 3 && N <= 16 * sms) || (M >= 6 && N <= 32 * sms));
+  if (K < 8192 || K % 256 == 0 || M < 3) return false;
+  return N <= (M < 6 ? 16 : 32) * sm_count();
 }
 
 std::string launch_skinny_tc(int block, int M, int N, int K, cudaStream_t stream, const __half* a, const uint8_t* packed,

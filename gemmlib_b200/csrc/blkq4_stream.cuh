@@ -10,9 +10,6 @@ namespace stream {
 constexpr int kWarps = 8;            // warps per CTA = K splits
 constexpr int kGroupSteps = 4;       // 64-k steps per group (one ring slot)
 constexpr int kSlotW = kGroupSteps * 512;   // [step][lane] 16 bytes
-constexpr int kSlotS = kGroupSteps * 32;    // [step][16] fp16
-constexpr int kSlotZ = kGroupSteps * 16;    // [step][16] u8
-constexpr int kSlotBytes = kSlotW + kSlotS + kSlotZ;  // 2240
 
 __device__ __forceinline__ uint2 ld_relaxed_sys_v2(const void* p) {
   uint2 v;
@@ -51,6 +48,18 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%5];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr), "n"(OFF));
+  return v;
+}
+template <int OFF>
+__device__ __forceinline__ uint2 lds_v2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(addr), "n"(OFF));
+  return v;
+}
+template <int OFF>
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
   return v;
 }
 template <int OFF>
