@@ -8,7 +8,7 @@
 //     ring of shared-memory slots with cp.async (16 bytes per lane, placed as [step][lane], so the
 //     later 128-bit reads are conflict free) and waits with cp.async.wait_group, which, unlike a
 //     plain load's scoreboard, lets older groups be consumed while younger ones are in flight.
-//     D groups per warp are outstanding: 8 warps x 4 groups x 2 KB = 64 KB per CTA.
+//     D groups per warp are outstanding: 8 warps x 2 groups x 2 KB = 32 KB per CTA, or 64.
 //   * Two CTAs fit on an SM and the grid has one CTA per SM (two when the tile count divides well),
 //     so with programmatic stream serialization the NEXT launch's CTAs become resident beside this
 //     one's, fill their rings, and only then wait for this launch to finish: HBM stays busy across
@@ -26,8 +26,6 @@
 // Instruction economy matters here: with the weight loads left out the kernel still takes 0.93 of its time (M = 1,
 // 4096 x 11008, B200), so the ~58 instructions of a 64-k step and their latencies set its pace and not HBM:
 // immediate-offset shared-memory loads, no predicates, no index math.
-// At 3 to 8 rows and K = 8192 the staged activations (65.6 KB per CTA at M = 4, for each of the two CTAs of an SM) leave
-// rings of two slots instead of four, half the bytes in flight that M = 1 has.
 //
 // Dequantization numerics: exact in fp32 up to the accumulation order (no fp16 rounding of scale * q);
 // equal to the reference kernel's result where that is exact
@@ -694,18 +692,18 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
   // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
   // (the measurements are beside ZP)
   const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || bs < 0 || (K < 8192 && (block == 64 || M == 2)) ? Zp::kPerStep : Zp::kOwnSums;
-  // Two CTAs per SM (this launch's and the next one's) share 227 KB; prefer four groups in flight per warp.
+  // Two CTAs per SM (this launch's and the next one's) share 227 KB.  Where they fit, rings of two groups are enough from 4096 k on:
+  // with four, the first copies of all CTAs, 19 MB, stand before the activations, which everything waits for.  Measured on B200, four
+  // groups / two, us, block 64 with zero points: M = 1: 7168 x 4096 6.2 / 5.7, 11008 x 4096 8.5 / 8.0, 4096 x 11008 7.9 / 7.7, 8192 x 28672
+  // 27.4 / 27.2; M = 4: 4096 x 11008 9.2 / 8.9; M = 8: 4096 x 4096 6.8 / 6.4, 4096 x 11008 10.8 / 10.2; two decoder blocks of 4096 and 11008
+  // as one graph, M = 1, 79.8 / 75.8 (three groups 77.7; five and six as four).  2048 x 2048, M = 1, block 128 2.36 / 2.42: four there.
+  // A CTA alone on its SM takes four: 11008 x 4096, M = 4 11.8 / 12.5; 8192 x 28672, M = 8, symmetric 33.4 / 36.1.
   constexpr size_t kHalfSm = (size_t)(227 * 1024) / 2 - 1024, kWholeSm = (size_t)227 * 1024;
-  int D = 4;
-  size_t smem = stream_smem_bytes(M, K, zp_as, 4, bs);
-  if (smem > kHalfSm) {
-    const size_t smem2 = stream_smem_bytes(M, K, zp_as, 2, bs);
-    if (smem2 <= kHalfSm) { D = 2; smem = smem2; }
-    else if (smem > kWholeSm) {
-      if (smem2 > kWholeSm) return kStreamUnsupported;
-      D = 2; smem = smem2;
-    }
-  }
+  const size_t smem4 = stream_smem_bytes(M, K, zp_as, 4, bs), smem2 = stream_smem_bytes(M, K, zp_as, 2, bs);
+  if (smem2 > kWholeSm) return kStreamUnsupported;
+  const bool two_groups = smem2 <= kHalfSm ? K >= 4096 || smem4 > kHalfSm : smem4 > kWholeSm;
+  const int D = two_groups ? 2 : 4;
+  const size_t smem = two_groups ? smem2 : smem4;
   StreamParams p{};
   p.a = a; p.out = out; p.bias = bias; p.packed = packed; p.scales = scales; p.zp = zp;
   p.M = M; p.N = N; p.K = K;
