@@ -447,7 +447,7 @@ def run_ours(args):
         line["roofline"] = {
             "bound": "hbm", "achieved": round(nbytes / (launch_us * 1e-6) / 1e9, 2), "peak": peaks["hbm_gbs"],
             "unit": "GB/s", "frac": round(nbytes / (launch_us * 1e-6) / 1e9 / peaks["hbm_gbs"], 4),
-            "traffic": TRAFFIC_BYTES_PER_LAUNCH, "kernel": "gemv_stream_kernel<false,4,2,0,false,false>",
+            "traffic": TRAFFIC_BYTES_PER_LAUNCH, "kernel": "gemv_stream_kernel<kNone,2,2,0,false,false,false>",
             "bytes_per_launch": nbytes, "us_per_launch": round(launch_us, 3), "peak_source": peaks["source"],
         }
     if world == 1 and not args.skip_extras:
