@@ -993,8 +993,7 @@ TcPlan plan_high_tiles(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_a
   return pl;
 }
 
-// gather: the fused exchange, which lives in the pair kernel's epilogue and runs in whole rounds.
-TcPlan plan_tc(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available, bool gather = false) {
+TcPlan compute_plan(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available, bool gather) {
   TcPlan pl = plan_high_tiles(M, n_tiles, n_pairs, K, gather ? 0 : ws_bytes_available);
   if (gather || M <= 16 || K >= kCostK || (pl.pair && !pl.pp.balanced)) return pl;
   const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -1028,6 +1027,26 @@ TcPlan plan_tc(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available
     pl.sp = sp;
   }
   return pl;
+}
+
+// gather: the fused exchange, which lives in the pair kernel's epilogue and runs in whole rounds.
+// A plan is a function of the arguments and the number of SMs; a model asks for the same few again and again, and a search takes up to
+// half a microsecond of the launch: the latest ones are kept, per thread and direct-mapped, as the tensor maps are.
+TcPlan plan_tc(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available, bool gather = false) {
+  struct Entry {
+    int M, n_tiles, n_pairs, K, sms;
+    size_t ws;
+    bool gather;
+    TcPlan plan;
+  };
+  constexpr int kEntries = 64;
+  thread_local Entry cache[kEntries];  // M == 0: empty
+  const int sms = sm_count();
+  Entry& e = cache[(uint32_t)(M * 31 + n_tiles * 7 + K / 64) % kEntries];
+  if (M <= 0 || e.M != M || e.n_tiles != n_tiles || e.n_pairs != n_pairs || e.K != K || e.sms != sms || e.ws != ws_bytes_available ||
+      e.gather != gather)
+    e = Entry{M, n_tiles, n_pairs, K, sms, ws_bytes_available, gather, compute_plan(M, n_tiles, n_pairs, K, ws_bytes_available, gather)};
+  return e.plan;
 }
 
 }  // namespace
