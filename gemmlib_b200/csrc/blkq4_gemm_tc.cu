@@ -1060,7 +1060,8 @@ size_t gemm_tc_workspace_bytes(int M, int N, int K) {
 
 // Which problems of up to 16 rows run here rather than on the generic skinny kernel (blkq4_gemv.cu): both convert
 // the weights to fp16 by the same formula and sum in fp32.  Only those whose blocking no other skinny kernel takes
-// (row-wise, or blocks of 16 and 32): the others scale fp32 sums instead, which is more accurate.
+// (row-wise, or blocks of 16 and 32): the others scale fp32 sums instead, which is more accurate.  (Of the problems that stay
+// there, the decode kernel has since taken the column-wise ones of a few rows: small_blocks_are_faster of blkq4_gemv_stream.cu.)
 // Measured on B200 (graphs of launches over 512 MB of weights), generic against this one, us, K x N, block 32 column-wise
 // with zero points (row-wise).  Blocks of 16, and row-wise blocks of 128, lie within 5 % of these.
 //   M = 1:  4096 x 8192 13.4 / 10.9 (15.3 / 13.7);  8192 x 512 10.0 / 6.1 (13.1 / 7.0);  8192 x 4096 12.2 / 11.3 (14.8 / 14.1);
