@@ -1042,7 +1042,7 @@ TcPlan plan_tc(int M, int n_tiles, int n_pairs, int K, size_t ws_bytes_available
   constexpr int kEntries = 64;
   thread_local Entry cache[kEntries];  // M == 0: empty
   const int sms = sm_count();
-  Entry& e = cache[(uint32_t)(M * 31 + n_tiles * 7 + K / 64) % kEntries];
+  Entry& e = cache[((uint32_t)M * 31u + (uint32_t)n_tiles * 7u + (uint32_t)K / 64u) % kEntries];
   if (M <= 0 || e.M != M || e.n_tiles != n_tiles || e.n_pairs != n_pairs || e.K != K || e.sms != sms || e.ws != ws_bytes_available ||
       e.gather != gather)
     e = Entry{M, n_tiles, n_pairs, K, sms, ws_bytes_available, gather, compute_plan(M, n_tiles, n_pairs, K, ws_bytes_available, gather)};
