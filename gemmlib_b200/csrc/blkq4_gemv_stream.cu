@@ -99,10 +99,11 @@ constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 //
 // ZP: kPerStep subtracts zp * sum_k a_k from a step's sum before it is scaled, four FMAs and three loads a step.  kOwnSums keeps
 // accumulators of their own for these terms, two FMAs and three loads for two steps, but a shuffle, an addition and a store per row
-// and 16 more terms per output at the tile's end.  kPerStep is taken for three rows and more, and below 8192 k for two, and for one
-// with blocks of 64.  Measured on B200, kOwnSums / kPerStep, us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008
-// 13.5 / 10.8, 8192 x 28672 43.0 / 37.9; M = 4: 3.2 / 2.9, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 33.9; M = 1: 512 x 11008 4.3 / 3.5, 4096 x 4096
-// 4.4 / 4.2, 4096 x 11008 8.5 / 7.9, 11008 x 4096 8.5 / 8.4, 8192 x 28672 27.3 / 28.7; block 128 4.2 / 4.2, 8.0 / 8.2, 8.0 / 8.4, 26.0 / 27.3.
+// and 16 more terms per output at the tile's end.  kPerStep is taken for three rows and more.  Measured on B200, kOwnSums / kPerStep,
+// us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008 13.5 / 10.8, 8192 x 28672 43.0 / 37.9; M = 4:
+// 3.2 / 2.9, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 33.9.  One and two rows keep kOwnSums whatever it costs (M = 1: 512 x 11008 4.3 / 3.5, 4096 x 4096
+// 4.4 / 4.2, 4096 x 11008 8.5 / 7.9, 8192 x 28672 27.3 / 28.7): the fp32 sums round otherwise in another order, and a model's results
+// would no longer be, to the bit, those it had.  With TAIL it is kPerStep for them too, as the TMA kernel has it.
 // (As part of the accumulator's initial value, which is a thousand times larger than the sum, the term would be rounded there:
 // relative error against 64 bits 2.0853e-4, with either of these 2.0841e-4.)
 //
@@ -690,8 +691,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
       (size_t)K * N / 2 >= ((size_t)1 << 40))
     return kStreamUnsupported;
   // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
-  // (the measurements are beside ZP)
-  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || bs < 0 || (K < 8192 && (block == 64 || M == 2)) ? Zp::kPerStep : Zp::kOwnSums;
+  const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || bs < 0 ? Zp::kPerStep : Zp::kOwnSums;
   // Two CTAs per SM (this launch's and the next one's) share 227 KB.  Where they fit, rings of two groups are enough from 4096 k on:
   // with four, the first copies of all CTAs, 19 MB, stand before the activations, which everything waits for.  Measured on B200, four
   // groups / two, us, block 64 with zero points: M = 1: 7168 x 4096 6.2 / 5.7, 11008 x 4096 8.5 / 8.0, 4096 x 11008 7.9 / 7.7, 8192 x 28672
@@ -739,10 +739,13 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
     const std::integral_constant<Zp, Zp::kNone> none{};
     const std::integral_constant<Zp, Zp::kPerStep> per_step{};
     if (!zp) return small_m ? launch(none, two, shift, gather, group, short_group) : launch(none, eight, shift, gather, group, short_group);
-    if (!small_m) return launch(per_step, eight, shift, gather, group, short_group);
-    if constexpr (decltype(short_group)::value) return launch(per_step, two, shift, gather, group, short_group);
-    else if (zp_as == Zp::kPerStep) return launch(per_step, two, shift, gather, group, short_group);
-    else return launch(std::integral_constant<Zp, Zp::kOwnSums>{}, two, shift, gather, group, short_group);
+    if constexpr (decltype(short_group)::value) {
+      return small_m ? launch(per_step, two, shift, gather, group, short_group) : launch(per_step, eight, shift, gather, group, short_group);
+    } else {
+      const std::integral_constant<Zp, Zp::kOwnSums> own_sums{};
+      if (zp_as == Zp::kPerStep) return launch(per_step, eight, shift, gather, group, short_group);
+      return small_m ? launch(own_sums, two, shift, gather, group, short_group) : launch(own_sums, eight, shift, gather, group, short_group);
+    }
   };
   if (bs == -1) return with_kinds(std::integral_constant<int, -1>{}, std::false_type{}, std::false_type{}, std::true_type{});
   if (bs == -2) return with_kinds(std::integral_constant<int, -2>{}, std::false_type{}, std::false_type{}, std::true_type{});
