@@ -75,6 +75,46 @@ struct StreamParams {
 
 constexpr long long kGatherWaitCycles = 2000000000ll;  // ~1 s
 
+// Where an activation is infinite or NaN the accumulators hold NaN: they start at minus the activation-only terms.  One warp puts the
+// 16 outputs of such a row right: what they are depends only on the weights of those activations, which are rare, and is found from
+// the blocks (of 2^KB k) whose terms in s_corr are not finite.  The weights are those of the other kernels, with two fp16 roundings.
+template <int KB, int BLOCK_SHIFT>
+__device__ __noinline__ void redo_non_finite_rows(const __half* a, const uint8_t* packed, const __half* scales, const uint8_t* zp, __half* out,
+                                                  const __half* bias, int M, int N, int K, const float* s_corr, int tile) {
+  const int lane = threadIdx.x & 31, n = tile * 16 + (lane & 15);
+  const uint8_t* column = packed + (size_t)(tile * 8 + (lane & 7)) * K + ((lane & 8) ? 1 : 0);
+  const int blocks = K >> KB;
+  __syncwarp();  // other lanes have stored these outputs
+  for (int m = 0; m < M; ++m) {
+    float sum = 0.0f;
+    bool found = false, all_nan = false;
+    for (int b0 = 0; b0 < blocks && !all_nan; b0 += 32) {
+      const bool bad = b0 + lane < blocks && !isfinite(s_corr[((size_t)(b0 + lane) * 4 + (m >> 1)) * 4 + (m & 1)]);
+      for (uint32_t todo = __ballot_sync(0xffffffffu, bad); todo && !all_nan; todo &= todo - 1) {
+        found = true;
+        const int first = (b0 + __ffs(todo) - 1) << KB;
+        for (int k0 = first; k0 < first + (1 << KB) && !all_nan; k0 += 32) {
+          const float own = k0 + lane < first + (1 << KB) ? __half2float(a[(size_t)m * K + k0 + lane]) : 0.0f;
+          for (uint32_t ks = __ballot_sync(0xffffffffu, !isfinite(own)); ks && !all_nan; ks &= ks - 1) {
+            const int l = __ffs(ks) - 1, k = k0 + l, r = k & 15;
+            const float v = __shfl_sync(0xffffffffu, own, l);
+            const uint32_t byte = column[(k & ~15) + ((r & 7) >> 1) * 4 + (r & 1) * 2], q = r < 8 ? byte & 15u : byte >> 4;
+            const size_t meta = (size_t)(k >> BLOCK_SHIFT) * N + n;
+            const __half scale = scales[meta];
+            const int z = zp ? (int)zp[meta] : 8;
+            sum += v * __half2float(__hfma(scale, __int2half_rn(16 + (int)q), dequant_offset(scale, z)));
+            all_nan = __all_sync(0xffffffffu, isnan(sum));
+          }
+        }
+      }
+    }
+    if (found && lane < 16) {
+      const __half h = __float2half_rn(sum);
+      out[(size_t)m * N + n] = bias ? __hadd(h, bias[n]) : h;
+    }
+  }
+}
+
 // Shared memory: rings [kWarps][D][slot_bytes] | s_corr [blocks of K, or steps][4] float4 | s_asum [the same][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
 // MZ: rows whose activations are staged at a time: one after the other (2), or all together (8), which saves a round trip to L2 per
@@ -553,6 +593,7 @@ gemv_stream_kernel(const StreamParams p) {
         out = p.grp.out[i];
         bias = p.grp.bias[i];
       }
+      bool not_a_number = false;
       for (int idx = lane; idx < 16 * M; idx += 32) {
         const int row = idx & 15, m = idx >> 4;
         float sum = 0.0f;
@@ -563,7 +604,9 @@ gemv_stream_kernel(const StreamParams p) {
         const __half h = __float2half_rn(sum);
         if (GATHER) s_stage[idx] = h;  // [m][16]
         else out[(size_t)m * n_out + n] = bias ? __hadd(h, bias[n]) : h;
+        if (TAIL) not_a_number |= isnan(sum);
       }
+      if (TAIL && __any_sync(0xffffffffu, not_a_number)) redo_non_finite_rows<(BS < 0 ? 6 + BS : 6), 6 + BS>(p.a, p.packed, p.scales, p.zp, out, bias, M, n_out, K, s_corr, tile);
       if (GATHER) {
         // this rank's 16 columns of row m as eight flagged words, into every rank's buffer
         __syncwarp();

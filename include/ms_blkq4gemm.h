@@ -125,6 +125,12 @@ int blkq4_fp16_quant_size_sm80(
  *
  * Pointers: activations, weights and output 16-byte aligned; scales and offsets too for m > 16 and for row-wise
  * blocks (a misaligned one is refused with an error), else of their element's alignment.
+ *
+ * Infinite and NaN activations: a weight that is not zero times an infinite activation is infinite, so the row's outputs are infinite
+ * or, where the signs differ or a weight is zero, NaN (a zero weight may be what two fp16 roundings leave of it, except for 9 to 16 rows
+ * on column-wise blocks of 64 and 128).  Up to 8 rows on column-wise blocks of 64 and 128 with K a multiple of 256 and >= 2048, and in
+ * the fused exchange up to 16 rows, every output of such a row is NaN: the sums start at minus a multiple of the activations.
+ * Other rows keep every bit.
  */
 #define BLKQ4_GEMM_EARLY_WEIGHT_FETCH 1u
 int blkq4_fp16_gemm_sm100(
