@@ -82,9 +82,13 @@ struct SkinnyParams {
   int split, per_part;   // parts of a tile (1: whole tiles, CTA b takes b, b + grid, ...), steps of a part (the last: what is left)
 };
 
-// q - zp of the 64 k of a column, exact: nibbles become 1024 + q or 64 + q by bit placement, minus 1024 + zp or 64 + zp.
+// q - zp of the 64 k of a column, exact for any byte zp: nibbles become 1024 + q or 64 + q by bit placement, minus 1024 + zp or
+// 64 + zp.
 __device__ __forceinline__ void integers64(const PackedColumn<kSub>& col, uint32_t shift, uint32_t zp, uint32_t (&out)[32]) {
-  const uint32_t lo_off = (0x6400u | zp) * 0x10001u, hi_off = (0x5400u | (zp << 4)) * 0x10001u;
+  const uint32_t lo_off = (0x6400u | zp) * 0x10001u;
+  // A conversion: by bit placement (0x5400 | zp << 4) only zero points below 64 fit, and 1024 + zp minus 960 is 5 % slower (8192 x 28672,
+  // block 128 41.6 / 43.8 us).
+  const uint32_t hi_off = (uint32_t)__half_as_ushort(__uint2half_rn(64u + zp)) * 0x10001u;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint32_t w4[4] = {col.w[c].x, col.w[c].y, col.w[c].z, col.w[c].w};

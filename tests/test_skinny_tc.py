@@ -64,3 +64,18 @@ def test_which_kernel(M, N, K, kernel):
         params = only_kernel_node(driver, graph)
         err, name = driver.cuKernelGetName(params.kern) if int(params.kern) else driver.cuFuncGetName(params.func)
         assert int(err) == 0 and want in name, name
+
+
+@pytest.mark.parametrize("block,N,K", [(64, 160, 512), (128, 96, 2176)])
+def test_any_byte_as_zero_point(block, N, K):
+    """The quantizer's zero points have four bits, but callers may bring their own: any byte, as up to eight rows."""
+    w = gaussian_weight(N, K, seed=1)
+    packed, scales, _ = O.quant_prepack(block, True, w.numpy(), True)
+    zp = (np.arange(K // block * N) * 37 % 256).astype(np.uint8)
+    ideal = O.dequant_ideal(block, True, K, N, packed, scales, zp).T
+    for M in (1, 8, 9, 16):
+        a = gaussian_act(M, K, seed=M).numpy()
+        want = a.astype(np.float64) @ ideal
+        # one fp16 rounding, and fp32 sums of K terms of up to 255 scales each (up to eight rows 1024 + 15)
+        tol = 2.0 ** -11 * np.abs(want).max() + K ** 0.5 * 1039 * float(np.abs(a).max()) * 2.0 ** -23 * float(np.abs(scales).max())
+        assert np.abs(gpu_gemm(block, True, a, N, packed, scales, zp) - want).max() <= tol, M
