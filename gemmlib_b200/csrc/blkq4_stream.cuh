@@ -1,4 +1,4 @@
-// Device helpers of the decode kernel (blkq4_gemv_stream.cu).
+// Device helpers of the decode kernel (blkq4_gemv_stream.cuh).
 #pragma once
 
 #include <cuda_fp16.h>

@@ -4,7 +4,7 @@ import pytest
 
 from oracle import blkq4_oracle as O
 from tests._util import bits, gaussian_act, gaussian_weight
-from tests.test_gemm_gpu import gpu_gemm, kat_problem
+from tests.test_gemm_gpu import gpu_gemm, kat_problem, only_kernel_node
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,26 @@ def test_known_answers(block, N, K, has_zp):
     for M in (1, 2, 5, 8):
         a, *packed = kat_problem(block, True, has_zp, M, N, K)
         assert (bits(gpu_gemm(block, True, a, N, *packed)) == bits(O.dequant_gemm(block, True, a, N, *packed))).all(), M
+
+
+@pytest.mark.parametrize("K", [4096, 1024])
+def test_few_instances_are_loaded_together(K):
+    """The first launch of a process loads every kernel of the file that has the launched one: 92 in one file took 12.4 ms, 40 take 2.5."""
+    torch, driver = pytest.importorskip("torch"), pytest.importorskip("cuda.bindings.driver")
+    from gemmlib_b200 import capi
+
+    N = 32
+    a, out = torch.zeros(1, K, dtype=torch.float16, device="cuda"), torch.empty(1, N, dtype=torch.float16, device="cuda")
+    qw, qs = torch.zeros(K * N // 2, dtype=torch.uint8, device="cuda"), torch.zeros(K * N // 64, dtype=torch.float16, device="cuda")
+    graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):
+        capi.gemm(64, True, 1, N, K, a, qw, qs, None, out, stream=stream.cuda_stream)
+    params = only_kernel_node(driver, graph)
+    func = params.func
+    if int(params.kern):
+        err, func = driver.cuKernelGetFunction(params.kern)
+        assert int(err) == 0
+    err, module = driver.cuFuncGetModule(func)
+    assert int(err) == 0
+    err, count = driver.cuModuleGetFunctionCount(module)
+    assert int(err) == 0 and count <= 48, count
