@@ -1,7 +1,7 @@
 // Skinny W4A16 kernels (M <= 16) for sm_100a: out[M,N] = A[M,K] x dequant(W4[K,N]).
 // This file holds the dispatch (launch_gemv: decode kernel -> skinny tensor-core kernel, both in files of their
-// own, -> the TMA kernel and the generic kernel below) and the two kernels that take what the first two refuse: the fused
-// exchange of shapes off the decode kernel, other blockings, meta that is not 16-byte aligned.
+// own, -> the generic kernel below) and two kernels: the generic one, which takes what the first two refuse (other blockings, meta
+// that is not 16-byte aligned), and the TMA kernel of the fused exchange off the decode kernel's shapes.
 //
 // This regime is bound by HBM bandwidth: every packed weight byte is read once
 // and used for at most 16 outputs, so the kernel is organised around the weight
@@ -269,7 +269,7 @@ gemv_kernel(const __half* __restrict__ a, const uint8_t* __restrict__ packed,
 
 
 // ------------------------------------------------------------------------------------------
-// Fast path: column-wise blocks of 64 or 128 (every 64-k step of a column has ONE scale).
+// TMA kernel of the fused exchange: column-wise blocks of 64 or 128 (every 64-k step of a column has ONE scale).
 //
 // Memory side.  Persistent CTAs (one per SM) walk a static list of 16-column tiles.  A
 // producer warp streams the packed weights through a ring of shared-memory slots with TMA
@@ -316,9 +316,7 @@ constexpr long long kGemvWaitCycles = 2000000000ll;
 
 struct PersistParams {
   const __half* a;
-  __half* out;
-  const __half* bias;  // fp16 [N] added to the fp16 result, or null
-  GatherTable gt;      // gt.world > 0: the result goes to every rank's gathered buffer instead of `out`
+  GatherTable gt;    // the result goes to every rank's gathered buffer
   int M, N, K;
   int block_shift;   // 6 or 7
   int tiles;         // N / 16
@@ -486,14 +484,10 @@ gemv_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
 
     float total[MT][4];
     int cur_lt = -1;
-    // Gather mode: the call's epoch is one past the calls completed so far (the word only changes
+    // The call's epoch is one past the calls completed so far (the word only changes
     // when every CTA of this call has finished); even / odd epochs alternate between two buffers.
-    unsigned gather_epoch = 0;
-    size_t gather_off = 0;
-    if (p.gt.world > 0) {
-      gather_epoch = *reinterpret_cast<volatile unsigned*>(p.gt.base[p.gt.rank] + kGatherEpochOff) + 1u;
-      gather_off = kGatherCtrlBytes + (size_t)(gather_epoch & 1u) * p.gt.buf_bytes;
-    }
+    const unsigned gather_epoch = *reinterpret_cast<volatile unsigned*>(p.gt.base[p.gt.rank] + kGatherEpochOff) + 1u;
+    const size_t gather_off = kGatherCtrlBytes + (size_t)(gather_epoch & 1u) * p.gt.buf_bytes;
 
     // Leaves this warp's partial sums of local tile `lt` in its own slot of the tile's buffer;
     // the warp that arrives last adds the slots up in a fixed order (the result does not depend
@@ -550,13 +544,9 @@ gemv_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
             const int m = 8 * j + 2 * t + (e & 1);
             if (m < p.M) {
               const __half h = __float2half_rn(sum[j][e]);
-              if (p.gt.world > 0) {
-                // this rank's columns of the gathered [M, n_total] result, in every rank's buffer
-                const size_t off = gather_off + ((size_t)m * p.gt.n_total + (size_t)p.gt.rank * p.N + n) * sizeof(__half);
-                for (int r = 0; r < p.gt.world; ++r) *reinterpret_cast<__half*>(p.gt.base[r] + off) = h;
-              } else {
-                p.out[(size_t)m * p.N + n] = p.bias ? __hadd(h, p.bias[n]) : h;
-              }
+              // this rank's columns of the gathered [M, n_total] result, in every rank's buffer
+              const size_t off = gather_off + ((size_t)m * p.gt.n_total + (size_t)p.gt.rank * p.N + n) * sizeof(__half);
+              for (int r = 0; r < p.gt.world; ++r) *reinterpret_cast<__half*>(p.gt.base[r] + off) = h;
             }
           }
         __syncwarp();
@@ -650,7 +640,7 @@ gemv_persistent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
       if (lane == 0) mbar_arrive(bar_empty + 8 * slot);
     }
     if (ok && cur_lt >= 0) flush(cur_lt);
-    if (p.gt.world > 0 && ok) {
+    if (ok) {
       // Publish.  A chain of release / acquire links, each at the narrowest scope that spans it:
       // storing lanes -> lane 0 of their warp (__syncwarp), warps -> the CTA's last warp (fence +
       // shared counter, CTA scope), CTAs -> the grid's last CTA (system fence + global counter),
@@ -684,16 +674,13 @@ static int env_int(const char* name) {
 }
 
 constexpr size_t kMaxDynamicSmem = 227 * 1024;
-const char* const kTooMuchSmem = "shared memory";
 
 template <int MT, bool HAS_ZP>
 std::string launch_persistent_T(int M, int N, int K, int block, cudaStream_t stream, const __half* a,
                                 const uint8_t* packed, const __half* scales, const uint8_t* zp,
-                                __half* out, const __half* bias, bool early_fetch,
-                                const GatherTable* gt = nullptr) {
+                                bool early_fetch, const GatherTable& gt) {
   PersistParams p{};
-  p.a = a; p.out = out; p.bias = bias;
-  if (gt) p.gt = *gt; p.M = M; p.N = N; p.K = K;
+  p.a = a; p.gt = gt; p.M = M; p.N = N; p.K = K;
   p.block_shift = block == 64 ? 6 : 7;
   p.tiles = N / 16;
   p.nsub = (K + kUnitKBytes - 1) / kUnitKBytes;  // the last unit may be partial
@@ -717,7 +704,7 @@ std::string launch_persistent_T(int M, int N, int K, int block, cudaStream_t str
                       (size_t)(MT == 1 ? kAccBufsMax : 2) * kCons * MT * 4 * 32 * sizeof(float) +
                       (size_t)(K / 64) * 8 * MT * (HAS_ZP ? 2 : 1) * sizeof(float) +
                       (p.a_smem ? (size_t)M * K * 2 : 0);
-  if (smem > kMaxDynamicSmem) return kTooMuchSmem;  // very long K with 9..16 rows: the generic kernel takes it
+  if (smem > kMaxDynamicSmem) return "unsupported: K too long for the fused gather at this M";
   auto kern = gemv_persistent_kernel<MT, HAS_ZP>;
   static std::atomic<int> granted[64];
   cudaError_t e = ensure_dynamic_smem(kern, smem, granted);
@@ -784,21 +771,16 @@ int read_gemv_error() {
   return v;
 }
 
-// Both are read once: a group of layers has to take the same kernel as its layers' own calls.
-static int generic_only() {
-  static const int v = env_int("BLKQ4_GEMV_GENERIC");
-  return v;
-}
+// Read once: a group of layers has to take the same kernel as its layers' own calls.
 bool gemv_stream_off() {
-  static const int v = env_int("BLKQ4_GEMV_NO_STREAM");
-  return v != 0 || generic_only() != 0;
+  static const bool off = env_int("BLKQ4_GEMV_NO_STREAM") != 0 || env_int("BLKQ4_GEMV_GENERIC") != 0;
+  return off;
 }
 
 std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
                         const __half* a, const uint8_t* packed, const __half* scales,
                         const uint8_t* zp, __half* out, const __half* bias, unsigned flags) {
   if (M < 1 || M > 16) return "skinny kernel needs 1 <= M <= 16";
-  const bool early = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) != 0;
   static const int env_warps = env_int("BLKQ4_GEMV_WARPS"), env_u = env_int("BLKQ4_GEMV_U");
   // Warps per CTA = K splits.  Each warp should see at least four 64-k steps.
   const int steps = K / 64;
@@ -816,17 +798,6 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
                               : std::string(kStreamUnsupported);
     if (r != kStreamUnsupported) return r;
     if (tc) return launch_skinny_tc(block, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
-  }
-  // Fast path: one scale per 64-k step; at least one 512-k unit (the last one may be partial), meta
-  // rows and pointers 16-byte aligned (TMA), shared memory for the per-step terms within reach.
-  if (colwise && block >= 64 && !generic_only() && K >= kUnitKBytes && K <= 32768 &&
-      reinterpret_cast<uintptr_t>(scales) % 16 == 0 && (!zp || reinterpret_cast<uintptr_t>(zp) % 16 == 0)) {
-    const std::string r =
-        (M <= 8) ? (zp ? launch_persistent_T<1, true>(M, N, K, block, stream, a, packed, scales, zp, out, bias, early)
-                       : launch_persistent_T<1, false>(M, N, K, block, stream, a, packed, scales, zp, out, bias, early))
-                 : (zp ? launch_persistent_T<2, true>(M, N, K, block, stream, a, packed, scales, zp, out, bias, early)
-                       : launch_persistent_T<2, false>(M, N, K, block, stream, a, packed, scales, zp, out, bias, early));
-    if (r != kTooMuchSmem) return r;
   }
   // Row-wise blocking carries 48 bytes of meta per chunk in registers, so it fetches
   // fewer steps at a time.
@@ -865,12 +836,11 @@ std::string launch_gemv_gather(int block, bool colwise, int M, int N, int K, cud
         reinterpret_cast<uintptr_t>(scales) % 16 == 0 && (!zp || reinterpret_cast<uintptr_t>(zp) % 16 == 0)))
     return "unsupported: the fused gather runs on the column-wise block >= 64 fast path only";
   const bool early = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) != 0;
-  const std::string r =
-      (M <= 8) ? (zp ? launch_persistent_T<1, true>(M, N, K, block, stream, a, packed, scales, zp, nullptr, nullptr, early, &gt)
-                     : launch_persistent_T<1, false>(M, N, K, block, stream, a, packed, scales, zp, nullptr, nullptr, early, &gt))
-               : (zp ? launch_persistent_T<2, true>(M, N, K, block, stream, a, packed, scales, zp, nullptr, nullptr, early, &gt)
-                     : launch_persistent_T<2, false>(M, N, K, block, stream, a, packed, scales, zp, nullptr, nullptr, early, &gt));
-  return r == kTooMuchSmem ? std::string("unsupported: K too long for the fused gather at this M") : r;
+  if (M <= 8)
+    return zp ? launch_persistent_T<1, true>(M, N, K, block, stream, a, packed, scales, zp, early, gt)
+              : launch_persistent_T<1, false>(M, N, K, block, stream, a, packed, scales, zp, early, gt);
+  return zp ? launch_persistent_T<2, true>(M, N, K, block, stream, a, packed, scales, zp, early, gt)
+            : launch_persistent_T<2, false>(M, N, K, block, stream, a, packed, scales, zp, early, gt);
 }
 
 }  // namespace blkq4

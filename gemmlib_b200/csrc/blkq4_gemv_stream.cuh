@@ -146,7 +146,7 @@ __device__ __noinline__ void redo_non_finite_rows(const __half* a, const uint8_t
 // us, block 64: M = 8: 2048 x 2048 4.1 / 3.4, 4096 x 4096 7.9 / 6.8, 4096 x 11008 13.5 / 10.8, 8192 x 28672 43.0 / 37.9; M = 4:
 // 3.2 / 2.9, 5.9 / 5.5, 10.4 / 9.2, 36.2 / 33.9.  One and two rows keep kOwnSums whatever it costs (M = 1: 512 x 11008 4.3 / 3.5, 4096 x 4096
 // 4.4 / 4.2, 4096 x 11008 8.5 / 7.9, 8192 x 28672 27.3 / 28.7): the fp32 sums round otherwise in another order, and a model's results
-// would no longer be, to the bit, those it had.  With TAIL it is kPerStep for them too, as the TMA kernel has it.
+// would no longer be, to the bit, those it had.  With TAIL it is kPerStep for them too, as the TMA kernel, which had those shapes, has it.
 // (As part of the accumulator's initial value, which is a thousand times larger than the sum, the term would be rounded there:
 // relative error against 64 bits 2.0853e-4, with either of these 2.0841e-4.)
 //

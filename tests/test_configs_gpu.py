@@ -106,7 +106,7 @@ def c4_full():
 
 @pytest.mark.parametrize("M", [1, 16, 64, 1024, 4096])
 def test_config_c4_full_width(c4_full, M):
-    """configs[3] at N = 28672: decode kernel (M=1), TMA skinny kernel (16), tensor-core kernel (64 and up)."""
+    """configs[3] at N = 28672: decode kernel (M=1), skinny tensor-core kernel (16), tensor-core kernel (64 and up)."""
     c4_full.check(M, seed=40 + M)
 
 
@@ -145,11 +145,10 @@ def test_config_c5_prefill(c5_layer):
 @pytest.mark.parametrize("shape", [(64, True, 352, 2048), (128, False, 256, 4096), (64, False, 4736, 2304),
                                    (128, True, 160, 3072)], ids=lambda s: "-".join(map(str, s)))
 def test_decode_kernel_exact_on_known_answers(shape, M):
-    """The decode kernel (M <= 8, K >= 2048 in whole groups of 256) and, for M 9..16, the generic skinny
+    """The decode kernel (M <= 8, K >= 2048 in whole groups of 256) and, for M 9..16, the skinny tensor-core
     kernel on the reference tests' known-answer family, where every product and partial sum is exact:
-    equal bits.  (The family stops being exact near K = 8192 - its sums leave the fp16 range - so the
-    kernel with two row groups, which takes M 9..16 from K = 8192 on, is covered by the Gaussian
-    full-width case of configs[3] at M = 16 instead.)"""
+    equal bits.  (The family stops being exact near K = 8192 - its sums leave the fp16 range; longer K at
+    M = 16 is covered by the Gaussian full-width case.)"""
     from gemmlib_b200 import capi
 
     block, has_zp, N, K = shape

@@ -94,14 +94,13 @@ def test_gaussian_tolerance(block, colwise, has_zp, M):
     check_gaussian(block, colwise, has_zp, M, 384, 512)
 
 
-# Shapes that walk the streaming skinny kernel's corners: more tiles than SMs, fewer tiles than
-# SMs, K not a multiple of 1024, fewer units per tile than consumer warps (K < 8192), 9..16
-# rows, very long K.
+# Shapes that walk the corners of the decode kernel and, for 9..16 rows, the skinny tensor-core kernel: more tiles than SMs, fewer
+# tiles than SMs, K not a multiple of 1024, very long K.
 STREAM_CASES = [
     (64, False, 1, 4736, 1024), (64, True, 3, 2400, 1280), (128, False, 8, 160, 3072),
     (128, True, 16, 4768, 2048), (64, True, 9, 2432, 5120), (64, False, 2, 1600, 16384),
-    (128, True, 16, 64, 32768),  # per-step terms would not fit in shared memory: generic kernel
-    (64, True, 1, 4096, 11008), (128, False, 5, 512, 1664),  # K not a multiple of 512: partial last unit
+    (128, True, 16, 64, 32768),
+    (64, True, 1, 4096, 11008), (128, False, 5, 512, 1664),  # K not a multiple of 256: a short last group of steps
 ]
 
 
