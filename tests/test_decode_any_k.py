@@ -4,9 +4,21 @@ import pytest
 
 from oracle import blkq4_oracle as O
 from tests._util import bits, gaussian_act, gaussian_weight
-from tests.test_gemm_gpu import gpu_gemm, kat_problem, only_kernel_node
+from tests.test_gemm_gpu import gpu_gemm, kat_problem, only_kernel_node, to_cuda
 
 pytestmark = pytest.mark.gpu
+
+
+def check_bias(block, a, N, packed, plain):
+    """A bias is added in fp16 to the rounded result, and changes nothing else."""
+    torch = pytest.importorskip("torch")
+    from gemmlib_b200 import capi
+
+    bias = gaussian_act(1, N, seed=3).numpy().ravel()
+    out = torch.full((a.shape[0], N), float("nan"), dtype=torch.float16, device="cuda")
+    capi.gemm(block, True, a.shape[0], N, a.shape[1], to_cuda(a), *(to_cuda(x) for x in packed), out, bias=to_cuda(bias))
+    torch.cuda.synchronize()
+    assert (bits(out.cpu().numpy()) == bits(plain + bias)).all()
 
 
 # one step; fewer groups than warps, the last one short or not; one group each and a short one; an uneven slice; N of one tile and many
@@ -31,6 +43,7 @@ def test_any_k(K, block, has_zp):
         got = gpu_gemm(block, True, a, N, *packed)
         assert np.abs(got - want).max() <= tol, M
         assert (bits(gpu_gemm(block, True, a, N, *packed, flags=capi.EARLY_WEIGHT_FETCH)) == bits(got)).all(), M
+        check_bias(block, a, N, packed, got)
 
 
 @pytest.mark.parametrize("block,N,K", [(64, 352, 576), (64, 96, 1088), (128, 160, 640)])

@@ -4,6 +4,7 @@ import pytest
 
 from oracle import blkq4_oracle as O
 from tests._util import bits, gaussian_act, gaussian_weight
+from tests.test_decode_any_k import check_bias
 from tests.test_gemm_gpu import gpu_gemm, kat_problem, only_kernel_node
 
 pytestmark = pytest.mark.gpu
@@ -22,6 +23,7 @@ def check(block, has_zp, M, N, K):
     got = gpu_gemm(block, True, a, N, *packed)
     assert np.abs(got - want).max() <= tol, (M, N, K)
     assert (bits(gpu_gemm(block, True, a, N, *packed, flags=capi.EARLY_WEIGHT_FETCH)) == bits(got)).all(), (M, N, K)
+    check_bias(block, a, N, packed, got)
 
 
 # K: half a step; one; an odd number of 64; parts of a cluster, even and not; N: part of a tile; several; more tiles than SMs (two rounds)
