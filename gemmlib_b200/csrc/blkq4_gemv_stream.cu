@@ -61,41 +61,40 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
     return kStreamUnsupported;
   // M <= 2: see the kernel; a launch of several matrices decides as their own launches do
   const Zp zp_as = !zp ? Zp::kNone : M > 2 || tail || bs < 0 ? Zp::kPerStep : Zp::kOwnSums;
-  // Two CTAs per SM (this launch's and the next one's) share 227 KB.  Where they fit, rings of two groups are enough from 4096 k on:
-  // with four, the first copies of all CTAs, 19 MB, stand before the activations, which everything waits for.  Measured on B200, four
-  // groups / two, us, block 64 with zero points: M = 1: 7168 x 4096 6.2 / 5.7, 11008 x 4096 8.5 / 8.0, 4096 x 11008 7.9 / 7.7, 8192 x 28672
-  // 27.4 / 27.2; M = 4: 4096 x 11008 9.2 / 8.9; M = 8: 4096 x 4096 6.8 / 6.4, 4096 x 11008 10.8 / 10.2; two decoder blocks of 4096 and 11008
-  // as one graph, M = 1, 79.8 / 75.8 (three groups 77.7; five and six as four).  2048 x 2048, M = 1, block 128 2.36 / 2.42: four there.
-  // A CTA alone on its SM takes four: 11008 x 4096, M = 4 11.8 / 12.5; 8192 x 28672, M = 8, symmetric 33.4 / 36.1.
+  // Two CTAs fit on an SM, this launch's and the next one's, if each takes less than half of its shared memory.  The grid has one CTA per
+  // SM, so that the second slot is the next launch's (its weights stream in while this launch computes), or two, which
+  // doubles the warps that compute: worth it only when the tiles then still divide evenly enough.  Gather mode: one, so that the
+  // whole grid is resident while it waits.
   constexpr size_t kHalfSm = (size_t)(227 * 1024) / 2 - 1024, kWholeSm = (size_t)227 * 1024;
   const size_t smem4 = stream_smem_bytes(M, K, zp_as, 4, bs), smem2 = stream_smem_bytes(M, K, zp_as, 2, bs);
   if (smem2 > kWholeSm) return kStreamUnsupported;
-  const bool two_groups = smem2 <= kHalfSm ? K >= 4096 || smem4 > kHalfSm : smem4 > kWholeSm;
+  const int sms = sm_count(), tiles = grp ? grp->tile_end[grp->count - 1] : N / 16;
+  const int rounds2 = (tiles + 2 * sms - 1) / (2 * sms);
+  const bool two_per_sm = !gt && smem2 <= kHalfSm && tiles > sms && (double)tiles / (2.0 * sms) / rounds2 >= 0.85;
+  // Groups in flight per warp.  With four, the first copies of all CTAs stand before the activations, which everything waits for: 19 MB where
+  // there are two CTAs per SM.  Two are enough there, and where they hold a warp's whole slice of a tile (up to 4096 k); a CTA
+  // alone on its SM has too little in flight with two of a longer slice.  Measured on B200, two / four groups, time ratio, M = 1 and 2 with
+  // the early weight fetch: two CTAs per SM (N = 4096 and 8192) 4096 k 0.86 to 1.00, 5120 0.94 to 0.99, 8192 0.90 to 0.99, 11008 0.96 to 1.03;
+  // one CTA per SM (N = 1024, 2048, 3584, 14336) 2048 to 4096 k 0.92 to 1.07, mean 0.99, 4352 1.06 to 1.21, 8192 1.00 to 1.25, 11008 1.12 to
+  // 1.26 (1 x 11008 x 14336 27.3 / 24.1 us); short last groups of one CTA per SM: 2112 1.0 to 1.1, 4160 and 5696 1.0 to 1.15.  In gather mode:
+  // 4096 k 0.97 to 1.00, 5120 x 1728 1.08, 8192 x 14336 1.11.
+  // Two decoder blocks of 4096 and 11008 as one graph, M = 1, four / two groups 79.8 / 75.8 us (three groups 77.7; five and six as four).
+  // Where two CTAs fit with rings of two only, those are taken; a CTA that is alone on its SM in any case takes four: 11008 x 4096, M = 4
+  // 11.8 / 12.5; 8192 x 28672, M = 8, symmetric 33.4 / 36.1.
+  const bool slice_fits = !tail && bs >= 0 && K <= 2 * kWarps * group_k;
+  const bool two_groups = smem2 <= kHalfSm ? two_per_sm || slice_fits || smem4 > kHalfSm : smem4 > kWholeSm;
   StreamLaunch l{};
   StreamParams& p = l.p;
   l.ring = two_groups ? 2 : 4;
   l.smem = two_groups ? smem2 : smem4;
   p.a = a; p.out = out; p.bias = bias; p.packed = packed; p.scales = scales; p.zp = zp;
   p.M = M; p.N = N; p.K = K;
-  p.tiles = N / 16;
+  p.tiles = tiles;
   p.steps = K / 64;
   p.a_pitch = K + a_padding(bs);
   if (gt) p.gt = *gt;
-  if (grp) {
-    p.grp = *grp;
-    p.tiles = grp->tile_end[grp->count - 1];
-  }
-  const int sms = sm_count();
-  // One CTA per SM leaves the second CTA slot of every SM to the next launch (its weights stream in
-  // while this launch computes).  Two per SM double the warps that compute; worth it only when the
-  // tiles then still divide evenly enough.
-  int grid = p.tiles < sms ? p.tiles : sms;
-  if (!gt && l.smem <= kHalfSm && p.tiles > sms) {  // gather mode: one CTA per SM, so that the whole grid is resident while it waits
-    const int per2 = (p.tiles + 2 * sms - 1) / (2 * sms);
-    const double eff2 = (double)p.tiles / (2.0 * sms) / per2;
-    if (eff2 >= 0.85) grid = p.tiles < 2 * sms ? p.tiles : 2 * sms;
-  }
-  l.grid = grid;
+  if (grp) p.grp = *grp;
+  l.grid = two_per_sm ? (tiles < 2 * sms ? tiles : 2 * sms) : tiles < sms ? tiles : sms;
   l.one_by_one = M == 1 || (M == 2 && K >= 8192);
   l.zp = zp_as;
   l.stream = stream;

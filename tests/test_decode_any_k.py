@@ -54,19 +54,24 @@ def test_known_answers(block, N, K, has_zp):
         assert (bits(gpu_gemm(block, True, a, N, *packed)) == bits(O.dequant_gemm(block, True, a, N, *packed))).all(), M
 
 
-@pytest.mark.parametrize("K", [4096, 1024])
-def test_few_instances_are_loaded_together(K):
-    """The first launch of a process loads every kernel of the file that has the launched one: 92 in one file took 12.4 ms, 40 take 2.5."""
+def launch_parameters(M, N, K):
+    """Of a plain call, block 64, symmetric."""
     torch, driver = pytest.importorskip("torch"), pytest.importorskip("cuda.bindings.driver")
     from gemmlib_b200 import capi
 
-    N = 32
-    a, out = torch.zeros(1, K, dtype=torch.float16, device="cuda"), torch.empty(1, N, dtype=torch.float16, device="cuda")
+    a, out = torch.zeros(M, K, dtype=torch.float16, device="cuda"), torch.empty(M, N, dtype=torch.float16, device="cuda")
     qw, qs = torch.zeros(K * N // 2, dtype=torch.uint8, device="cuda"), torch.zeros(K * N // 64, dtype=torch.float16, device="cuda")
     graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
     with torch.cuda.graph(graph, stream=stream):
-        capi.gemm(64, True, 1, N, K, a, qw, qs, None, out, stream=stream.cuda_stream)
-    params = only_kernel_node(driver, graph)
+        capi.gemm(64, True, M, N, K, a, qw, qs, None, out, stream=stream.cuda_stream)
+    return only_kernel_node(driver, graph)
+
+
+@pytest.mark.parametrize("K", [4096, 1024])
+def test_few_instances_are_loaded_together(K):
+    """The first launch of a process loads every kernel of the file that has the launched one: 92 in one file took 12.4 ms, 40 take 2.5."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    params = launch_parameters(1, 32, K)
     func = params.func
     if int(params.kern):
         err, func = driver.cuKernelGetFunction(params.kern)
@@ -75,3 +80,14 @@ def test_few_instances_are_loaded_together(K):
     assert int(err) == 0
     err, count = driver.cuModuleGetFunctionCount(module)
     assert int(err) == 0 and count <= 48, count
+
+
+@pytest.mark.parametrize("M,N,K,ring", [(1, 4096, 8192, 2), (1, 11008, 4096, 2), (2, 1024, 2048, 2), (1, 2048, 8192, 4), (1, 14336, 11008, 4),
+                                        (2, 3584, 5120, 4), (1, 1024, 4160, 4), (4, 3584, 8192, 2), (1, 8192, 4160, 2)])
+def test_rings(M, N, K, ring):
+    """A CTA alone on its SM has four groups of steps in flight where a slice of K is longer than two."""
+    slot = 2048 + 4 * 48  # a group's weights, scales and zero points
+    smem = launch_parameters(M, N, K).sharedMemBytes
+    steps, rows = K // 64, M + M % 2
+    rest = steps * 64 + 2 * 8 * 16 * rows * 4 + 256 + M * (K + 8) * 2
+    assert smem == 8 * ring * slot + rest, (smem - rest) / 8 / slot
