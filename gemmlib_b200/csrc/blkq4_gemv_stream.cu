@@ -95,7 +95,7 @@ std::string launch_gemv_stream(int block, bool colwise, int M, int N, int K, cud
   if (gt) p.gt = *gt;
   if (grp) p.grp = *grp;
   l.grid = two_per_sm ? (tiles < 2 * sms ? tiles : 2 * sms) : tiles < sms ? tiles : sms;
-  l.one_by_one = M == 1 || (M == 2 && K >= 8192);
+  l.one_by_one = M == 1 || (M == 2 && (tail ? K >= 8192 : K > 3 * kWarps * group_k));
   l.zp = zp_as;
   l.stream = stream;
   l.early = (flags & BLKQ4_GEMM_EARLY_WEIGHT_FETCH) != 0;

@@ -121,8 +121,10 @@ __device__ __noinline__ void redo_non_finite_rows(const __half* a, const uint8_t
 // Shared memory: rings [kWarps][D][slot_bytes] | s_corr [blocks of K, or steps][4] float4 | s_asum [the same][8] (zero points)
 //                | s_part [2][PW][16][MS] | s_stage [8][16] fp16 (gather) | s_a [M][a_pitch]
 // MZ: rows whose activations are staged at a time: one after the other (2), or all together (8), which saves a round trip to L2 per
-// row but runs a longer code.  Two rows one after the other / together, us, symmetric blocks of 64: 512 x 512 1.9 / 1.7, 1024 x 4096
-// 2.5 / 2.4, 2048 x 2048 2.7 / 2.5, 4096 x 4096 4.6 / 4.6, 8192 x 28672 26.0 / 26.8, 11008 x 4096 8.7 / 9.8: together below 8192 k.
+// row but runs a longer code.  Two rows one after the other / together, us, block 64 with the early weight fetch: symmetric 512 x 512
+// 1.9 / 1.7, 2048 x 1024 2.27 / 2.23, 3072 x 2048 3.5 / 3.3, 4096 x 4096 4.6 / 4.6, 6144 x 4096 5.9 / 5.9 (with zero points 6.4 / 6.4), but
+// 6400 x 4096 5.9 / 6.7 (6.4 / 7.4), 7168 x 4096 6.2 / 7.0 (6.6 / 7.5), 8192 x 28672 26.0 / 26.8, 11008 x 4096 8.7 / 9.8: together up to three
+// whole groups of steps a warp (6144 k).  With short last groups 6208 x 1024 4.8 / 4.7, 7232 x 2048 5.8 / 5.7: together below 8192 k.
 //
 // GATHER (N-sharded layer, one process per GPU).  The exchange is latency-bound (a few tens of KB per
 // rank), so it carries its own flags: the adding warp stores the tile's results into EVERY rank's

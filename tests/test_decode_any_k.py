@@ -1,4 +1,6 @@
 """The decode kernel where K is not whole groups of four steps for each of its eight warps."""
+import re
+
 import numpy as np
 import pytest
 
@@ -91,3 +93,13 @@ def test_rings(M, N, K, ring):
     steps, rows = K // 64, M + M % 2
     rest = steps * 64 + 2 * 8 * 16 * rows * 4 + 256 + M * (K + 8) * 2
     assert smem == 8 * ring * slot + rest, (smem - rest) / 8 / slot
+
+
+@pytest.mark.parametrize("K,together", [(2048, True), (6144, True), (6400, False), (7168, False), (7232, True), (8256, False)])
+def test_staging_of_two_rows(K, together):
+    """Two rows are staged together where that is faster: up to three whole groups of steps a warp, and below 8192 k with short groups."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    params = launch_parameters(2, 32, K)
+    err, name = driver.cuKernelGetName(params.kern) if int(params.kern) else driver.cuFuncGetName(params.func)
+    # gemv_stream_kernel<zero points, groups per ring, rows staged at a time, ...>
+    assert int(err) == 0 and re.search(rb"Li[24]ELi([28])E", name).group(1) == (b"8" if together else b"2"), name
