@@ -410,6 +410,7 @@ gemv_stream_kernel(const StreamParams p) {
                        : (uint32_t)((4 * g + (b ^ chunk_xor)) * 16 + t * 4);
 
   uint32_t src = ring_addr;
+  bool not_a_number = false;  // TAIL: among the outputs that this lane has added up
   for (int tl = 0; tl < my_tiles; ++tl) {
     uint32_t a_addr = a_base, c_addr = c_base, as_addr = asum_base;
     for (int j2 = 0; j2 < myg; ++j2) {
@@ -598,7 +599,6 @@ gemv_stream_kernel(const StreamParams p) {
         out = p.grp.out[i];
         bias = p.grp.bias[i];
       }
-      bool not_a_number = false;
       for (int idx = lane; idx < 16 * M; idx += 32) {
         const int row = idx & 15, m = idx >> 4;
         float sum = 0.0f;
@@ -611,7 +611,6 @@ gemv_stream_kernel(const StreamParams p) {
         else out[(size_t)m * n_out + n] = bias ? __hadd(h, bias[n]) : h;
         if (TAIL) not_a_number |= isnan(sum);
       }
-      if (TAIL && __any_sync(0xffffffffu, not_a_number)) redo_non_finite_rows<(BS < 0 ? 6 + BS : 6), 6 + BS>(p.a, p.packed, p.scales, p.zp, out, bias, M, n_out, K, s_corr, tile);
       if (GATHER) {
         // this rank's 16 columns of row m as eight flagged words, into every rank's buffer
         __syncwarp();
@@ -626,6 +625,9 @@ gemv_stream_kernel(const StreamParams p) {
     }
   }
   cp_async_wait<0>();
+  if (TAIL && __any_sync(0xffffffffu, not_a_number))
+    for (int tl = warp; tl < my_tiles; tl += W)  // the tiles that this warp has added up
+      redo_non_finite_rows<(BS < 0 ? 6 + BS : 6), 6 + BS>(p.a, p.packed, p.scales, p.zp, p.out, p.bias, M, N, K, s_corr, blockIdx.x + tl * gridDim.x);
   if (GATHER) {
     uint8_t* local = p.gt.base[p.gt.rank];
     // receiver: this CTA's share of the words of the complete result
