@@ -410,7 +410,14 @@ gemv_stream_kernel(const StreamParams p) {
                        : (uint32_t)((4 * g + (b ^ chunk_xor)) * 16 + t * 4);
 
   uint32_t src = ring_addr;
-  bool not_a_number = false;  // TAIL: among the outputs that this lane has added up
+  float zeros = 0.0f;  // TAIL: NaN once this lane has added up an output that is
+  // The warps look at it once, after their last tile.  (A vote per tile takes up to a tenth where a CTA has many short tiles; but the
+  // compiler's schedule of the steps of symmetric blocks of 128 is better with it: M = 1, 2 and 4 1.03, 1.00 and 0.99 of the time without
+  // either, at the end 1.05, 1.03 and 1.03.)
+  constexpr bool kVotePerTile = TAIL && BS == 1 && ZP == Zp::kNone;
+  auto redo_tile = [&](int tl) {
+    redo_non_finite_rows<(BS < 0 ? 6 + BS : 6), 6 + BS>(p.a, p.packed, p.scales, p.zp, p.out, p.bias, M, N, K, s_corr, blockIdx.x + tl * gridDim.x);
+  };
   for (int tl = 0; tl < my_tiles; ++tl) {
     uint32_t a_addr = a_base, c_addr = c_base, as_addr = asum_base;
     for (int j2 = 0; j2 < myg; ++j2) {
@@ -609,7 +616,11 @@ gemv_stream_kernel(const StreamParams p) {
         const __half h = __float2half_rn(sum);
         if (GATHER) s_stage[idx] = h;  // [m][16]
         else out[(size_t)m * n_out + n] = bias ? __hadd(h, bias[n]) : h;
-        if (TAIL) not_a_number |= isnan(sum);
+        if (TAIL) zeros = fmaf(sum, 0.0f, zeros);
+      }
+      if (kVotePerTile) {
+        if (__any_sync(0xffffffffu, isnan(zeros))) redo_tile(tl);
+        zeros = 0.0f;
       }
       if (GATHER) {
         // this rank's 16 columns of row m as eight flagged words, into every rank's buffer
@@ -625,9 +636,8 @@ gemv_stream_kernel(const StreamParams p) {
     }
   }
   cp_async_wait<0>();
-  if (TAIL && __any_sync(0xffffffffu, not_a_number))
-    for (int tl = warp; tl < my_tiles; tl += W)  // the tiles that this warp has added up
-      redo_non_finite_rows<(BS < 0 ? 6 + BS : 6), 6 + BS>(p.a, p.packed, p.scales, p.zp, p.out, p.bias, M, N, K, s_corr, blockIdx.x + tl * gridDim.x);
+  if (TAIL && !kVotePerTile && __any_sync(0xffffffffu, isnan(zeros)))
+    for (int tl = warp; tl < my_tiles; tl += W) redo_tile(tl);  // the tiles that this warp has added up
   if (GATHER) {
     uint8_t* local = p.gt.base[p.gt.rank];
     // receiver: this CTA's share of the words of the complete result
