@@ -416,14 +416,34 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
          reinterpret_cast<uintptr_t>(zp) % 16 == 0;
 }
 
-// Up to eight rows the decode kernel reads whole columns, one tile of 16 after the other; few tiles of long K leave SMs idle that
-// a split of K here uses.  Measured on B200, decode kernel / this one, us, block 64 with zero points: 8192 x 1024 M = 3 0.90 of the
-// time, M = 8 0.70; 11008 x 1024 M = 3 0.88, M = 7 0.63; 8192 x 4096 M = 3 1.08, M = 6 0.94, M = 8 0.86; 11008 x 4096 M = 6 0.89;
-// 8192 x 8192 M = 8 0.95, M = 6 1.03; 5632 x 2048 0.87 to 1.00; 4096 x 4096 M = 4 1.22, M = 8 0.99; 8192 x 28672 M = 8 1.18.
-// K that is a multiple of 256 stays there: layers of such K may share a launch of the decode kernel, with the bits of their own calls.
+// Up to eight rows the decode kernel's CTAs take 16 columns at a time, whose end costs a barrier and the addition of eight partial
+// sums, and one or two of its eight warps may have a group of steps more than the others; this kernel takes 128 columns, and time
+// that hardly depends on the rows, but a launch that cannot start early costs 2.9 us in place of 1.4.  The kernel must not depend on whether
+// it can (the results would), so that the lines lie where the two are equal in the geometric mean of both kinds of launches.
+// K in whole groups from 2048 on stays with the decode kernel: layers of such K may share a launch there, with the bits of their own
+// calls.  Measured on B200, decode kernel / this one with the early weight fetch (without), us, block 64 with zero points, K x N:
+//   K < 512: M = 3 64 x 2048 2.1 / 2.0 (2.9 / 3.5: there), 192 x 6144 3.3 / 2.3 (4.2 / 4.0); M = 5 192 x 2048 2.6 / 2.2 (3.4 / 3.9);
+//     M = 8 256 x 2048 2.9 / 2.3 (3.7 / 3.9), 448 x 2048 3.0 / 2.7 (3.9 / 4.5)
+//   512 to 703: M = 5 512 x 6144 3.8 / 2.7 (4.6 / 4.6), 512 x 11008 4.6 / 3.5 (6.1 / 5.5); M = 8 512 x 2048 3.0 / 2.6 (3.8 / 4.5: there);
+//     two rounds of tiles: M = 5 512 x 22528 0.94 of the time, M = 8 640 x 28672 0.85, 768 x 28672 0.90
+//   704 to 2047: M = 8 768 x 8192 4.3 / 3.2 (5.7 / 6.1), 1024 x 6144 4.6 / 3.8 (6.0 / 6.8), 1536 x 6144 5.1 / 5.1 (6.7 / 7.1: there);
+//     M = 5 768 x 11008 5.1 / 4.0 (6.6 / 6.2); M = 6 1536 x 14336 7.5 / 6.6 (9.3 / 8.4), 1536 x 18944 7.5 / 7.3 (9.3 / 8.7), 1792 x 11008 1.1
+//   2048 to 4095: M = 7 2112 x 3072 5.6 / 5.2 (7.3 / 6.7), M = 8 3200 x 1024 0.90, 3200 x 11008 1.05 (86 tiles: 62 SMs without work); M = 6 1.0 to 1.1
+//   from 4096 on, few columns: M = 5 5184 x 2048 6.7 / 5.9 (7.6 / 7.7), M = 8 5184 x 4096 9.3 / 7.8 (11.0 / 9.3), 6208 x 1024 8.5 / 5.4 (10.1 / 7.6);
+//     M = 3 6208 x 1024 6.3 / 5.4 (7.5 / 7.6), 8256 x 1024
+//     7.9 / 6.2, 8256 x 2048 9.0 / 7.3; M = 6 8256 x 4096 12.1 / 9.9; many: M = 8 8256 x 8192 18.4 / 15.1, 8256 x 18944 0.85; M = 6 8256 x 6144 14.3 / 14.3
 bool skinny_tc_is_faster(int M, int N, int K) {
-  if (K < 8192 || K % 256 == 0 || M < 3) return false;
-  return N <= (M < 6 ? 16 : 32) * sm_count();
+  if ((K >= 2048 && K % 256 == 0) || M < 3) return false;
+  const int sms = sm_count(), tiles = (N + TILE_N - 1) / TILE_N;
+  const bool few = N <= 32 * sms;
+  if (K < 512) return tiles <= sms ? M >= (!few ? 3 : K < 256 ? 5 : 7) : K > 256 && M >= 5;
+  if (K < 704) return !few && M >= (tiles <= sms ? 3 : 5);
+  if (tiles > sms) return false;
+  if (K < 1152) return N > 64 * sms ? M >= 5 : !few && M >= 7;
+  if (tiles * 2 > sms && tiles * 10 < sms * 7) return false;  // neither split nor enough tiles for the SMs
+  if (K < 2048) return N > 64 * sms && M >= 6;
+  if (K < 4096 || !few) return M >= 7;
+  return M >= (N > 16 * sms ? 6 : K < 6144 ? 5 : 3);
 }
 
 std::string launch_skinny_tc(int block, int M, int N, int K, cudaStream_t stream, const __half* a, const uint8_t* packed,

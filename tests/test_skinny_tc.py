@@ -42,6 +42,13 @@ def test_long_k_of_few_rows(M, N, K):
     check(64, True, M, N, K)
 
 
+@pytest.mark.parametrize("M,N,K", [(5, 96, 64), (3, 4768, 192), (8, 160, 320), (7, 18976, 448), (4, 4800, 512), (8, 4768, 1088),
+                                   (6, 14336, 1984), (7, 544, 2112), (8, 14336, 2112), (5, 544, 4160), (3, 96, 6208)])
+@pytest.mark.parametrize("has_zp", [True, False])
+def test_few_rows(M, N, K, has_zp):
+    check(64, has_zp, M, N, K)
+
+
 @pytest.mark.parametrize("block,N,K", [(64, 352, 2048), (128, 160, 3072), (64, 96, 1088), (64, 2080, 576)])
 @pytest.mark.parametrize("has_zp", [True, False])
 def test_known_answers(block, N, K, has_zp):
@@ -50,7 +57,18 @@ def test_known_answers(block, N, K, has_zp):
         assert (bits(gpu_gemm(block, True, a, N, *packed)) == bits(O.dequant_gemm(block, True, a, N, *packed))).all(), M
 
 
-@pytest.mark.parametrize("M,N,K,kernel", [(9, 4096, 4096, b"skinny_tc"), (8, 4096, 4096, b"gemv_stream"), (5, 2048, 11008, b"gemv_stream"),
+# few rows: on either side of the rules, K below 512 and not in whole groups
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 11008, 64, b"gemv_kernel"), (1, 18944, 256, b"gemv_stream"), (1, 18976, 256, b"gemv_kernel"), (2, 11008, 320, b"gemv_stream"),
+                                          (8, 4768, 64, b"gemv_kernel"), (8, 2048, 64, b"skinny_tc"), (4, 2048, 192, b"gemv_stream"),
+                                          (5, 2048, 192, b"skinny_tc"), (3, 4768, 448, b"skinny_tc"), (6, 160, 256, b"gemv_stream"),
+                                          (7, 160, 448, b"skinny_tc"), (3, 18976, 256, b"gemv_kernel"), (5, 18976, 320, b"skinny_tc"),
+                                          (4, 18976, 320, b"gemv_stream"), (3, 6144, 640, b"skinny_tc"), (8, 4096, 640, b"gemv_stream"),
+                                          (5, 11008, 1024, b"skinny_tc"), (6, 8192, 1024, b"gemv_stream"), (7, 8192, 1024, b"skinny_tc"),
+                                          (5, 11008, 1536, b"gemv_stream"), (8, 11008, 1536, b"gemv_stream"), (6, 14336, 1536, b"skinny_tc"), (8, 18976, 768, b"gemv_stream"),
+                                          (7, 3072, 2112, b"skinny_tc"), (6, 3072, 2112, b"gemv_stream"), (8, 11008, 2112, b"gemv_stream"),
+                                          (5, 2048, 5184, b"skinny_tc"), (5, 4096, 5184, b"gemv_stream"), (6, 4096, 5184, b"skinny_tc"),
+                                          (3, 2048, 6208, b"skinny_tc"), (7, 8192, 6208, b"skinny_tc"), (8, 8192, 8192, b"gemv_stream"),
+                                          (9, 4096, 4096, b"skinny_tc"), (8, 4096, 4096, b"gemv_stream"), (5, 2048, 11008, b"gemv_stream"),
                                           (5, 2048, 8256, b"skinny_tc"), (2, 2048, 8256, b"gemv_stream"), (6, 8192, 8256, b"gemv_stream")])
 def test_which_kernel(M, N, K, kernel):
     driver = pytest.importorskip("cuda.bindings.driver")
