@@ -943,7 +943,8 @@ constexpr int kCostK = 3072, kMinPlannedRows = 48;
 // costs more than it gains below 2048 k (whole / in two: K = 832 to 1088 0.68 to 0.90, 1856 0.83, 2048 0.92, 2496 1.00), one in
 // four does not (1.0 to 1.4); above, only five or more parts say that the SMs would stay idle with low tiles too.  Fewer than eight
 // column tiles leave them idle in any case: those keep their parts.
-// Apart from that the answer does not depend on the columns, so that layers cut alike alone are mostly cut alike in a group.
+// The columns count through `parts`, which is what fills the SMs with high tiles, and through that limit: layers of one K can be cut
+// otherwise than a group of them, and gemm_tc_group_keeps_bits says which may share a launch.
 inline int short_k_parts(int M, int n_tiles, int K, int parts) {
   if (n_tiles < 8) return parts;
   if (M <= 64) return parts >= 3 || K >= 2048 ? parts : 1;
@@ -952,6 +953,9 @@ inline int short_k_parts(int M, int n_tiles, int K, int parts) {
 
 // Predicted time in us, by least squares over the candidates of the problems above (rms error 10 %): start-up, then per round of
 // tiles the 64-k steps of one and its end, then the exchange between the parts of a cluster or of balanced ranges.
+// The constants are the kernels': after a change of their steps or ends they are fitted again, by timing every height of compute_plan's
+// loop, and plan_high_tiles, on random problems in its range (graphs of launches with the early weight fetch; blocks of 64 with zero
+// points column-wise, of 32 row-wise) and least squares of the relative error over the terms of one_cta and balanced_pairs.
 struct TileCost {
   double start, step, step_row, end, end_row;
 };
@@ -971,8 +975,16 @@ struct CostModel {
     return us(pair, BM, items / (double)pairs, steps64) + balanced;
   }
 };
-constexpr CostModel kColumnWise{{1.5869, 0.165, 0, 0.6429, 0}, {2.272, 0.1311, 0.0004, 0, 0.0083}, {1.4118, 0.1161, 0.0009, 0, 0.0098}, {5.4188, 0.1224, 0.0009, 0, 0.003}, 1.13, 0.0071, 0.21, 6.6},
-    kRowWise{{0.8339, 0.2595, 0, 0.5351, 0}, {1.6446, 0.219, 0.0004, 0, 0.0074}, {1.2523, 0.2433, 0.0005, 0, 0.0096}, {5.7228, 0.2428, 0.0007, 0, 0.0019}, 1.42, 0.0048, 0.29, 6.3};
+constexpr CostModel kColumnWise{{1.5869, 0.165, 0, 0.6429, 0},
+                               {2.272, 0.1311, 0.0004, 0, 0.0083},
+                               {1.4118, 0.1161, 0.0009, 0, 0.0098},
+                               {5.4188, 0.1224, 0.0009, 0, 0.003},
+                               1.13, 0.0071, 0.21, 6.6},
+    kRowWise{{0.8339, 0.2595, 0, 0.5351, 0},
+             {1.6446, 0.219, 0.0004, 0, 0.0074},
+             {1.2523, 0.2433, 0.0005, 0, 0.0096},
+             {5.7228, 0.2428, 0.0007, 0, 0.0019},
+             1.42, 0.0048, 0.29, 6.3};
 
 struct TcPlan {
   bool pair;

@@ -23,8 +23,8 @@
 //   * At the end of a tile the warps leave their partial sums in shared memory, the CTA meets at one
 //     barrier, and one warp (rotating) adds them in a fixed order, rounds to fp16 and stores.
 //
-// Instruction economy matters here: with the weight loads left out the kernel still takes 0.93 of its time (M = 1,
-// 4096 x 11008, B200), so the ~58 instructions of a 64-k step and their latencies set its pace and not HBM:
+// Instruction economy matters here: with the copies left out after the first the kernel still takes 0.89 of its time (M = 1,
+// 4096 x 11008, B200; 8192 x 28672 0.86), so the ~58 instructions of a 64-k step and their latencies set its pace and not HBM:
 // immediate-offset shared-memory loads, no predicates, no index math.
 //
 // Dequantization numerics: exact in fp32 up to the accumulation order (no fp16 rounding of scale * q);
@@ -33,7 +33,7 @@
 //
 // The instances are spread over three files - blkq4_gemv_stream.cu (one matrix, groups), blkq4_gemv_stream_gather.cu and
 // blkq4_gemv_stream_tail.cu - because CUDA loads a file's kernels together when the first of them is launched: with all 92 in one the first
-// decode call of a process took 12.4 ms, now 2.5.
+// decode call of a process took 12.4 ms, now 2.5.  Those of the exchange take 128 registers and spill 4 or 8 bytes, the others none.
 #pragma once
 
 #include <cstddef>
@@ -163,6 +163,7 @@ __device__ __noinline__ void redo_non_finite_rows(const __half* a, const uint8_t
 // BS < 0: blocks of 32 and 16, a row of scales and zero points, an activation-only term and a sum per block.  An mma adds up over the
 // four lanes of a column, so the lanes share a block's 16-byte chunks: 8 bytes each for blocks of 32, 4 for blocks of 16.  The
 // activations are staged in that order, 16 bytes a lane and 32 k, and the chunks lie in the slot so that the reads hit all banks.
+// These blocks have the TAIL form only, also where K is whole groups; a form without its tests was not measured.
 //
 // BS: steps of a quantization block, as a shift (0: blocks of 64, 1: of 128).  The two steps of a 128-k block share scale and
 // zero point: one load and conversion of them, two accumulators with independent mma chains, one scaling of their sum.
@@ -438,7 +439,9 @@ gemv_stream_kernel(const StreamParams p) {
           const float nsz = -s * z;
 #pragma unroll
           for (int v = 0; v < (1 << BS); ++v) {
-            if (M > 0) {  // always: without the branch the compiler's schedule is 1 to 2 % slower (M = 1, 4096 x 11008 8.5 / 8.6)
+            // Always.  Without the branch nvcc 12.9 schedules blocks of 128 up to 2 % slower (M = 1 4096 x 11008 7.9 / 8.0, 8192 x 28672 26.1 /
+            // 26.7 us; blocks of 64 alike): to be timed again with another compiler.
+            if (M > 0) {
               const float2 as = lds_f2<0>(as_addr + (u + v) * 32);
               ztot[0] = fmaf(nsz, as.x, ztot[0]);
               ztot[1] = fmaf(nsz, as.y, ztot[1]);
