@@ -777,19 +777,6 @@ bool gemv_stream_off() {
   return off;
 }
 
-// Up to eight rows, K below 512, blocks of 64 and 128: the decode kernel takes up to 296 tiles of 16 columns at a time, and where one has
-// only a step or a few, its end is what counts; the generic kernel has all tiles in flight.  The line lies where both kinds of launches
-// together are equal, as in skinny_tc_is_faster.  Measured on B200, generic / decode kernel with the early weight fetch (without), us,
-// block 64 with zero points, K x N: M = 1 64 x 11008 2.7 / 2.8 (2.7 / 3.7), 64 x 28672 3.2 / 3.4 (3.2 / 4.3), 256 x 28672 4.8 / 4.6 (4.7 / 5.9);
-// 256 x 12288 1.2 of the time, 320 x 28672 1.1, 64 x 4096 2.6 / 1.8 (2.6 / 2.6), 192 x 8192 3.3 / 2.6 (3.3 / 3.4): there.  From three rows on against
-// the skinny tensor-core kernel: 64 x 8192, M = 3 2.7 / 2.1 (2.7 / 3.7), 192 x 28672, M = 8 4.3 / 4.1 (4.3 / 5.8), but 128 x 11008, M = 3
-// 3.0 / 2.4 (3.1 / 3.6): there.
-static bool generic_is_faster(int M, int N, int K) {
-  const int sms = sm_count();
-  if (M <= 2) return (K < 256 && N > 64 * sms) || (K == 256 && N > 128 * sms);
-  return K <= 256 && (N > 128 * sms || (K == 64 && N > 32 * sms));
-}
-
 std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream_t stream,
                         const __half* a, const uint8_t* packed, const __half* scales,
                         const uint8_t* zp, __half* out, const __half* bias, unsigned flags) {
@@ -805,12 +792,12 @@ std::string launch_gemv(int block, bool colwise, int M, int N, int K, cudaStream
   // Decode shapes first: the cp.async stream kernel (blkq4_gemv_stream.cu); then the skinny tensor-core kernel (blkq4_skinny_tc.cu),
   // which has the rest of the column-wise blocks of 64 and 128.
   if (!gemv_stream_off()) {
-    const bool tc = skinny_tc_takes(block, colwise, M, N, K, scales, zp), generic = tc && M <= 8 && generic_is_faster(M, N, K);
-    const std::string r = M <= 8 && !generic && !(tc && skinny_tc_is_faster(M, N, K))
+    const bool tc = skinny_tc_takes(block, colwise, M, N, K, scales, zp);
+    const std::string r = M <= 8 && !(tc && skinny_tc_is_faster(M, N, K))
                               ? launch_gemv_stream(block, colwise, M, N, K, stream, a, packed, scales, zp, out, bias, flags)
                               : std::string(kStreamUnsupported);
     if (r != kStreamUnsupported) return r;
-    if (tc && !generic) return launch_skinny_tc(block, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
+    if (tc) return launch_skinny_tc(block, M, N, K, stream, a, packed, scales, zp, out, bias, flags);
   }
   // Row-wise blocking carries 48 bytes of meta per chunk in registers, so it fetches
   // fewer steps at a time.

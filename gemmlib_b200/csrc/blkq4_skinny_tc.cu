@@ -422,8 +422,10 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
 // it can (the results would), so that the lines lie where the two are equal in the geometric mean of both kinds of launches.
 // K in whole groups from 2048 on stays with the decode kernel: layers of such K may share a launch there, with the bits of their own
 // calls.  Measured on B200, decode kernel / this one with the early weight fetch (without), us, block 64 with zero points, K x N:
-//   K < 512: M = 3 64 x 2048 2.1 / 2.0 (2.9 / 3.5: there), 192 x 6144 3.3 / 2.3 (4.2 / 4.0); M = 5 192 x 2048 2.6 / 2.2 (3.4 / 3.9);
-//     M = 8 256 x 2048 2.9 / 2.3 (3.7 / 3.9), 448 x 2048 3.0 / 2.7 (3.9 / 4.5)
+//   K < 512: M = 1 128 x 11008 0.82 of the time, 64 x 28672 3.4 / 3.1 (4.3 / 4.4), 256 x 18944 1.00 (there), 64 x 4096 1.8 / 2.1 (2.6 / 3.6: there); M = 3 64 x 2048 2.1 / 2.0 (2.9 / 3.5: there), 192 x 6144 3.3 / 2.3 (4.2 / 4.0); M = 5 192 x 2048 2.6 / 2.2 (3.4 / 3.9);
+//     M = 8 256 x 2048 2.9 / 2.3 (3.7 / 3.9), 448 x 2048 3.0 / 2.7 (3.9 / 4.5); two rounds of tiles: M = 8 192 x 28672 6.3 / 4.1 (7.4 / 5.8),
+//     M = 3 320 x 22528 0.95.  (The generic kernel, which rounds the weights to fp16, takes 3.2 for 64 x 28672 and 4.3 for 192 x 28672
+//     with either launch: slower than this one with the early fetch, faster without.)
 //   512 to 703: M = 5 512 x 6144 3.8 / 2.7 (4.6 / 4.6), 512 x 11008 4.6 / 3.5 (6.1 / 5.5); M = 8 512 x 2048 3.0 / 2.6 (3.8 / 4.5: there);
 //     two rounds of tiles: M = 5 512 x 22528 0.94 of the time, M = 8 640 x 28672 0.85, 768 x 28672 0.90
 //   704 to 2047: M = 8 768 x 8192 4.3 / 3.2 (5.7 / 6.1), 1024 x 6144 4.6 / 3.8 (6.0 / 6.8), 1536 x 6144 5.1 / 5.1 (6.7 / 7.1: there);
@@ -433,10 +435,11 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
 //     M = 3 6208 x 1024 6.3 / 5.4 (7.5 / 7.6), 8256 x 1024
 //     7.9 / 6.2, 8256 x 2048 9.0 / 7.3; M = 6 8256 x 4096 12.1 / 9.9; many: M = 8 8256 x 8192 18.4 / 15.1, 8256 x 18944 0.85; M = 6 8256 x 6144 14.3 / 14.3
 bool skinny_tc_is_faster(int M, int N, int K) {
-  if ((K >= 2048 && K % 256 == 0) || M < 3) return false;
+  if (K >= 2048 && K % 256 == 0) return false;
   const int sms = sm_count(), tiles = (N + TILE_N - 1) / TILE_N;
   const bool few = N <= 32 * sms;
-  if (K < 512) return tiles <= sms ? M >= (!few ? 3 : K < 256 ? 5 : 7) : K > 256 && M >= 5;
+  if (M < 3) return K < 256 && N > 64 * sms;
+  if (K < 512) return M >= (few ? (K < 256 ? 5 : 7) : tiles <= sms || K <= 256 ? 3 : 5);
   if (K < 704) return !few && M >= (tiles <= sms ? 3 : 5);
   if (tiles > sms) return false;
   if (K < 1152) return N > 64 * sms ? M >= 5 : !few && M >= 7;

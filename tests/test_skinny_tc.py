@@ -58,10 +58,10 @@ def test_known_answers(block, N, K, has_zp):
 
 
 # few rows: on either side of the rules, K below 512 and not in whole groups
-@pytest.mark.parametrize("M,N,K,kernel", [(1, 11008, 64, b"gemv_kernel"), (1, 18944, 256, b"gemv_stream"), (1, 18976, 256, b"gemv_kernel"), (2, 11008, 320, b"gemv_stream"),
-                                          (8, 4768, 64, b"gemv_kernel"), (8, 2048, 64, b"skinny_tc"), (4, 2048, 192, b"gemv_stream"),
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 11008, 64, b"skinny_tc"), (2, 9472, 192, b"gemv_stream"), (1, 18976, 256, b"gemv_stream"), (2, 11008, 320, b"gemv_stream"),
+                                          (3, 4768, 64, b"skinny_tc"), (8, 2048, 64, b"skinny_tc"), (4, 2048, 192, b"gemv_stream"),
                                           (5, 2048, 192, b"skinny_tc"), (3, 4768, 448, b"skinny_tc"), (6, 160, 256, b"gemv_stream"),
-                                          (7, 160, 448, b"skinny_tc"), (3, 18976, 256, b"gemv_kernel"), (5, 18976, 320, b"skinny_tc"),
+                                          (7, 160, 448, b"skinny_tc"), (3, 18976, 256, b"skinny_tc"), (5, 18976, 320, b"skinny_tc"),
                                           (4, 18976, 320, b"gemv_stream"), (3, 6144, 640, b"skinny_tc"), (8, 4096, 640, b"gemv_stream"),
                                           (5, 11008, 1024, b"skinny_tc"), (6, 8192, 1024, b"gemv_stream"), (7, 8192, 1024, b"skinny_tc"),
                                           (5, 11008, 1536, b"gemv_stream"), (8, 11008, 1536, b"gemv_stream"), (6, 14336, 1536, b"skinny_tc"), (8, 18976, 768, b"gemv_stream"),
