@@ -422,7 +422,8 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
 // it can (the results would), so that the lines lie where the two are equal in the geometric mean of both kinds of launches.
 // K in whole groups from 2048 on stays with the decode kernel: layers of such K may share a launch there, with the bits of their own
 // calls.  Measured on B200, decode kernel / this one with the early weight fetch (without), us, block 64 with zero points, K x N:
-//   K < 512: M = 1 128 x 11008 0.82 of the time, 64 x 28672 3.4 / 3.1 (4.3 / 4.4), 256 x 18944 1.00 (there), 64 x 4096 1.8 / 2.1 (2.6 / 3.6: there); M = 3 64 x 2048 2.1 / 2.0 (2.9 / 3.5: there), 192 x 6144 3.3 / 2.3 (4.2 / 4.0); M = 5 192 x 2048 2.6 / 2.2 (3.4 / 3.9);
+//   K < 512: M = 1 128 x 11008 0.82 of the time, 64 x 28672 3.4 / 3.1 (4.3 / 4.4), 256 x 18944 1.00 (there), 64 x 4096 1.8 / 2.1
+//     (2.6 / 3.6: there); M = 3 64 x 2048 2.1 / 2.0 (2.9 / 3.5: there), 192 x 6144 3.3 / 2.3 (4.2 / 4.0); M = 5 192 x 2048 2.6 / 2.2 (3.4 / 3.9);
 //     M = 8 256 x 2048 2.9 / 2.3 (3.7 / 3.9), 448 x 2048 3.0 / 2.7 (3.9 / 4.5); two rounds of tiles: M = 8 192 x 28672 6.3 / 4.1 (7.4 / 5.8),
 //     M = 3 320 x 22528 0.95.  (The generic kernel, which rounds the weights to fp16, takes 3.2 for 64 x 28672 and 4.3 for 192 x 28672
 //     with either launch: slower than this one with the early fetch, faster without.)
@@ -432,8 +433,8 @@ bool skinny_tc_takes(int block, bool colwise, int M, int N, int K, const void* s
 //     M = 5 768 x 11008 5.1 / 4.0 (6.6 / 6.2); M = 6 1536 x 14336 7.5 / 6.6 (9.3 / 8.4), 1536 x 18944 7.5 / 7.3 (9.3 / 8.7), 1792 x 11008 1.1
 //   2048 to 4095: M = 7 2112 x 3072 5.6 / 5.2 (7.3 / 6.7), M = 8 3200 x 1024 0.90, 3200 x 11008 1.05 (86 tiles: 62 SMs without work); M = 6 1.0 to 1.1
 //   from 4096 on, few columns: M = 5 5184 x 2048 6.7 / 5.9 (7.6 / 7.7), M = 8 5184 x 4096 9.3 / 7.8 (11.0 / 9.3), 6208 x 1024 8.5 / 5.4 (10.1 / 7.6);
-//     M = 3 6208 x 1024 6.3 / 5.4 (7.5 / 7.6), 8256 x 1024
-//     7.9 / 6.2, 8256 x 2048 9.0 / 7.3; M = 6 8256 x 4096 12.1 / 9.9; many: M = 8 8256 x 8192 18.4 / 15.1, 8256 x 18944 0.85; M = 6 8256 x 6144 14.3 / 14.3
+//     M = 3 6208 x 1024 6.3 / 5.4 (7.5 / 7.6), 8256 x 1024 7.9 / 6.2, 8256 x 2048 9.0 / 7.3; M = 6 8256 x 4096 12.1 / 9.9; many columns:
+//     M = 8 8256 x 8192 18.4 / 15.1, 8256 x 18944 0.85 of the time; M = 6 8256 x 6144 14.3 / 14.3
 bool skinny_tc_is_faster(int M, int N, int K) {
   if (K >= 2048 && K % 256 == 0) return false;
   const int sms = sm_count(), tiles = (N + TILE_N - 1) / TILE_N;
